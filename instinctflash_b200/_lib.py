@@ -100,6 +100,18 @@ def available() -> bool:
     return any(_open(p) is not None for p in library_candidates())
 
 
+def _bind_calls(handle) -> None:
+    """Hand the entry points' addresses to the native call path (``csrc/host_calls.cpp``)."""
+    import torch  # noqa: F401  (its libraries have to be loaded first)
+
+    try:
+        from . import _calls
+    except ImportError as exc:
+        raise RuntimeError(f"the call path _calls.so is unavailable ({exc}). Build it with "
+                           "`python -m instinctflash_b200.build`.") from exc
+    _calls.bind({name: ctypes.cast(getattr(handle, name), _p).value for name in SIGNATURES})
+
+
 def lib():
     """The loaded library with argument types set.  Raises when it cannot be loaded."""
     global _LIB
@@ -111,6 +123,7 @@ def lib():
                     fn = getattr(handle, name)
                     fn.restype, fn.argtypes = restype, argtypes
                 handle.path = path
+                _bind_calls(handle)
                 _LIB = handle
                 break
         else:

@@ -5,6 +5,22 @@ import torch
 
 from .. import _lib
 
+try:
+    from .. import _calls as native
+except ImportError:
+    class _Unbuilt:
+        """Stands in for ``_calls`` where it has not been built: takes no call, so that every operator
+        goes on to ``launch`` and raises there."""
+
+        def __getattr__(self, name):
+            return lambda *args: None
+
+    native = _Unbuilt()
+
+# The operators of this package ask ``native`` first: it launches what it can (plain tensors on the
+# current device) from C++ and answers False for everything else, which then goes through the checks
+# below in Python: they raise what is wrong, or launch with the operand's device made current.
+
 E4M3 = torch.float8_e4m3fn
 
 

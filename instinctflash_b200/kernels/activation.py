@@ -15,13 +15,15 @@ from __future__ import annotations
 import torch
 
 from .. import _lib
-from ._common import E4M3, launch, ld, rows, same_device, vec
+from ._common import E4M3, launch, ld, native, rows, same_device, vec
 
 GELU_TANH = 0
 SILU = 1
 
 
 def gated_act_quant(gu, q, q_scale, *, row=None, col=None, act=GELU_TANH, num_warps=None):
+    if native.gated_act_quant(gu, q, q_scale, row, col, act):
+        return
     rows(gu, "gu", (torch.float32, torch.bfloat16, torch.float16))
     rows(q, "q", (E4M3,))
     M, F2 = gu.shape

@@ -13,7 +13,7 @@ from __future__ import annotations
 import torch
 
 from .. import _lib
-from ._common import E4M3, launch, ld, same_device
+from ._common import E4M3, launch, ld, native, same_device
 
 
 def _next_power_of_two(n: int) -> int:
@@ -38,6 +38,9 @@ def attn_combine(split: SplitWorkspace, out=None, *, heads_q: int, heads_kv: int
                  batch: int = 1, q8=None, q8_scale=None):
     """Merge the partials in ``split``; write ``out`` [B, Tq, Hq, D] (optional) and/or the quantised
     rows ``q8`` [Tq, Hq*D] e4m3 with ``q8_scale`` [Tq] (batch 1 only, as in the reference)."""
+    if native.attn_combine(split.po, split.pm, split.pl, split.splits, batch, tokens, heads_q, heads_kv, head_dim, out, q8,
+                           q8_scale):
+        return out
     if out is None and q8 is None:
         raise ValueError("nothing to write: give out, q8, or both")
     if heads_q % heads_kv:

@@ -18,7 +18,7 @@ from dataclasses import dataclass
 import torch
 
 from .. import _lib
-from ._common import E4M3, launch, ld, rows, same_device, vec
+from ._common import E4M3, launch, ld, native, rows, same_device, vec
 
 FP8_MAX = 448.0
 
@@ -68,6 +68,8 @@ def _operands(a: torch.Tensor, w: Fp8Weight):
 
 def gemm(a: torch.Tensor, w: Fp8Weight, out: torch.Tensor) -> torch.Tensor:
     """out[M, N] (bf16) = a[M, K] (e4m3) @ w.w[N, K]^T, unscaled raw accumulator."""
+    if native.gemm(a, w.w, out):
+        return out
     M, N, K = _operands(a, w)
     rows(out, "out", (torch.bfloat16,))
     if tuple(out.shape) != (M, N):
@@ -87,6 +89,9 @@ def fp8_linear(a: torch.Tensor, a_scale: torch.Tensor | None, w: Fp8Weight, out:
     ``a_scale`` is [M] (per token) or a single element (per tensor); ``w.scale`` likewise
     [N] or one element.  ``bias`` overrides ``w.bias`` (float32 or bf16).
     """
+    if native.fp8_linear(a, a_scale, w.w, w.scale, bias if bias is not None else (w.bias if use_weight_bias else None),
+                         out, exact):
+        return out
     M, N, K = _operands(a, w)
     rows(out, "out", (torch.float32, torch.bfloat16, torch.float16))
     if tuple(out.shape) != (M, N):
@@ -120,6 +125,8 @@ def fp8_linear_residual(a: torch.Tensor, a_scale: torch.Tensor, w: Fp8Weight, re
     res[m, n] += (r * a_scale[m] * w.scale[n] (+ bias[n])) (* gate[idx[m], n]), r the bf16-rounded
     accumulator; stored in ``res``'s dtype (float32, or bf16 for the Wan residual stream).
     """
+    if native.fp8_linear_residual(a, a_scale, w.w, w.scale, bias, gate, gate_index, res):
+        return res
     M, N, K = _operands(a, w)
     rows(res, "res", (torch.float32, torch.bfloat16))
     if tuple(res.shape) != (M, N):
@@ -148,6 +155,8 @@ def fp8_linear_gated(a: torch.Tensor, a_scale: torch.Tensor, w: Fp8Weight, h: to
     q, q_scale)`` finishes the operator: together they write the codes and scales of
     ``gemm`` + ``gated_act_quant`` bit for bit.  ``act``: 0 GELU-tanh, 1 SiLU.
     """
+    if native.fp8_linear_gated(a, a_scale, w.w, w.scale, h, amax, act):
+        return h
     rows(a, "a", (E4M3,))
     rows(w.w, "w.w", (E4M3,))
     rows(h, "h", (torch.float32,))
@@ -184,6 +193,8 @@ def gemm_partials(a: torch.Tensor, w: Fp8Weight, out: torch.Tensor) -> torch.Ten
     """Split-K ``gemm`` for skinny activations: ``out`` [S, M, N] float32 receives the partial sums of
     S K ranges (no scales, no rounding); ``norm.residual_norm_quant(..., delta=out)`` adds the planes
     in order, rounds the sum to bf16 (the raw accumulator's rounding point) and goes on as usual."""
+    if native.gemm_partials(a, w.w, out):
+        return out
     M, N, K = _operands(a, w)
     if out.dtype != torch.float32 or out.ndim != 3 or tuple(out.shape[1:]) != (M, N) or not out.is_contiguous():
         raise ValueError(f"out must be a contiguous float32 [S, {M}, {N}] tensor")

@@ -14,7 +14,7 @@ import ctypes
 import torch
 
 from .. import _lib
-from ._common import E4M3, launch, ld, rows, same_device, vec
+from ._common import E4M3, launch, ld, native, rows, same_device, vec
 
 FP8_MAX = 448.0
 _FLOATS = (torch.float32, torch.bfloat16, torch.float16)
@@ -22,6 +22,8 @@ _FLOATS = (torch.float32, torch.bfloat16, torch.float16)
 
 def row_quant(x, q, q_scale, *, row=None, col=None, bias=None, gelu=False, num_warps=None):
     """q[m] = e4m3((x[m] * row[m] * col + bias) [-> gelu_tanh] / s[m]), s[m] = rowmax / 448."""
+    if native.row_quant(x, q, q_scale, row, col, bias, gelu):
+        return
     rows(x, "x", _FLOATS)
     rows(q, "q", (E4M3,))
     M, D = x.shape
@@ -88,6 +90,8 @@ def quant_from_amax(h, amax, q, q_scale, zero=None):
     """``row_quant_from_amax`` as a flat kernel (rows cut into pieces for separate CTAs): the same
     codes and scales; ``amax`` is left as it is and ``zero`` (another [M] float32 buffer, or None) is
     cleared instead -- two buffers of row maxima alternate between consecutive gated GEMMs."""
+    if native.quant_from_amax(h, amax, q, q_scale, zero):
+        return
     rows(h, "h", (torch.float32,))
     M, F = h.shape
     rows(q, "q", (E4M3,))
@@ -106,6 +110,8 @@ def quant_from_amax(h, amax, q, q_scale, zero=None):
 
 def dequant_rows(x, y, *, row=None, col=None, bias=None, block=None, num_warps=4):
     """y[m] = x[m] * row[m] * col + bias (float dtypes in and out)."""
+    if native.dequant_rows(x, y, row, col, bias):
+        return
     rows(x, "x", _FLOATS)
     rows(y, "y", _FLOATS)
     M, D = x.shape
@@ -132,6 +138,9 @@ def residual_norm_quant(res, *, delta=None, delta_row=None, delta_col=None, bias
     ``res`` is float32 (bf16 for the Wan residual stream) and updated in place; ``gate``,
     ``mod_scale`` and ``mod_shift`` are [D] or, with ``mod_index`` (int32 [M]), tables [n, D].
     """
+    if router is None and native.residual_norm_quant(res, delta, delta_row, delta_col, bias, gate, write_res, layernorm,
+                                                     weight, beta, mod_scale, mod_shift, q, q_scale, y, eps, mod_index):
+        return
     return _residual_norm_quant(res, delta, delta_row, delta_col, bias, gate, write_res, layernorm, weight, beta,
                                 mod_scale, mod_shift, q, q_scale, y, eps, router, mod_index, None, None)
 

@@ -11,7 +11,7 @@ from __future__ import annotations
 import torch
 
 from .. import _lib
-from ._common import launch, rows, vec
+from ._common import launch, native, rows, vec
 
 _FLOATS = (torch.float32, torch.bfloat16, torch.float16)
 
@@ -46,6 +46,9 @@ def _index(t, name, n, device):
 def qkv_split(qkv, q_out, k_out, v_out, *, heads_q, heads_kv, head_dim, row=None, col=None, bias=None,
               inv_freq=None, pos=None, sections=None, q_norm=None, k_norm=None, norm_eps=1e-6, kv_base=0):
     """q_out [T, HQ, HD]; k_out/v_out [S, HKV, HD] written at rows ``kv_base + t``."""
+    if native.qkv_split(qkv, q_out, k_out, v_out, heads_q, heads_kv, head_dim, row, col, bias, inv_freq, pos, sections,
+                        q_norm, k_norm, norm_eps, kv_base):
+        return
     if q_out.dtype != k_out.dtype or k_out.dtype != v_out.dtype:
         raise ValueError("q/k/v outputs must share a dtype")
     if q_out.dtype not in _FLOATS:

@@ -12,7 +12,7 @@ from __future__ import annotations
 import torch
 
 from .. import _lib
-from ._common import launch, rows, vec
+from ._common import launch, native, rows, vec
 from .rope import _FLOATS, _index
 
 
@@ -30,6 +30,9 @@ def wan_qkv(raw, q_out, *, heads, head_dim, tokens, k_pool=None, v_pool=None, sl
             bias=None, q_norm=None, k_norm=None, pos=None, sections=None, inv_freq=None, eps=1e-6, num_warps=8):
     """raw [B*T, parts*H*HD] (parts: Q, then K, then V); q_out [B*T, H*HD];
     k_pool / v_pool [B, S, H*HD] written at rows ``slots[t]`` (or ``t``)."""
+    if native.wan_qkv(raw, q_out, heads, head_dim, tokens, k_pool, v_pool, slots, row, col, bias, q_norm, k_norm, pos,
+                      sections, inv_freq, eps):
+        return
     rows(raw, "raw", _FLOATS)
     rows(q_out, "q_out", _FLOATS)
     n_rows = raw.shape[0]

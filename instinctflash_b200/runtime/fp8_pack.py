@@ -12,7 +12,7 @@ from __future__ import annotations
 import torch
 
 from .. import _lib
-from ..kernels._common import launch
+from ..kernels._common import launch, native
 
 
 def _check(x):
@@ -33,6 +33,9 @@ def pack_bf16_e4m3(x: torch.Tensor, scale: torch.Tensor) -> torch.Tensor:
 
 
 def dynamic_pack_bf16_e4m3(x: torch.Tensor):
+    packed = native.dynamic_pack(x)
+    if packed:
+        return packed
     _check(x)
     if not x.numel():
         raise ValueError("Dynamic FP8 packing requires nonempty contiguous CUDA BF16 input")

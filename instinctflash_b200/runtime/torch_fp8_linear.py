@@ -13,6 +13,7 @@ import torch
 from torch import nn
 
 from ..kernels.fp8 import Fp8Weight, fp8_linear
+from ..kernels._common import native
 from .fp8_pack import dynamic_pack_bf16_e4m3
 
 
@@ -72,8 +73,15 @@ class SM100FP8Linear(nn.Module):
         self.register_buffer("weight_scale", scale)
         self.register_buffer("bias", bias)
 
-    @torch.no_grad()
     def forward(self, x):
+        # the plain case in one native call (allocations, pack, GEMM): a module called from Python for 50 tokens
+        # spent 55 us on the host for 10 us of kernels
+        packed = self._buffers
+        y = native.projection(x, packed["weight_fp8"], packed["weight_scale"], packed["bias"])
+        return self._forward(x) if y is None else y
+
+    @torch.no_grad()
+    def _forward(self, x):
         if x.ndim < 1 or x.shape[-1] != self.in_features:
             raise ValueError("FP8 projection input has incompatible feature dimension")
         if x.dtype != torch.bfloat16 or x.device != self.weight_fp8.device:
