@@ -42,12 +42,6 @@ struct CombineArgs {
   int tokens, batch, group, heads_kv, head_dim, block_d, splits;
 };
 
-__device__ __forceinline__ float ex2_approx_ftz(float a) {
-  float r;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
-  return r;
-}
-
 __global__ void __launch_bounds__(kCombineThreads) attn_combine_quant_kernel(const CombineArgs a) {
   grid_dependency_wait();  // the partials come from the kernel before this one in the stream
   grid_launch_dependents();

@@ -20,6 +20,16 @@ __device__ __forceinline__ float ex2_approx(float a) {
   asm("ex2.approx.f32 %0, %1;" : "=f"(r) : "f"(a));
   return r;
 }
+__device__ __forceinline__ float ex2_approx_ftz(float a) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+  return r;
+}
+__device__ __forceinline__ float rcp_approx_ftz(float a) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+  return r;
+}
 __device__ __forceinline__ float rsqrt_approx_ftz(float a) {
   float r;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
@@ -29,6 +39,17 @@ __device__ __forceinline__ float rsqrt_approx_ftz(float a) {
 __device__ __forceinline__ float max_f32(float a, float b) {
   float r;
   asm("max.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+// max(m, |a|, |b|) and the maximum of |a| over the warp, NaN operands dropped as by max.f32.
+__device__ __forceinline__ float max_abs_f32(float m, float a, float b) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(m), "f"(fabsf(a)), "f"(fabsf(b)));
+  return r;
+}
+__device__ __forceinline__ float warp_max_abs_f32(float a) {
+  float r;
+  asm volatile("redux.sync.max.abs.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(a));
   return r;
 }
 // Two floats -> two e4m3 codes, round-to-nearest-even, saturating to +-448.

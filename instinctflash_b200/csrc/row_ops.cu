@@ -6,6 +6,7 @@
 
 #include "../../include/iflb200.h"
 #include "launch.cuh"
+#include "row_stream.cuh"
 #include "rowmath.cuh"
 
 // The file compiles as one translation unit, or as three (IFLB200_ROW_PART = 0, 1, 2) so that
@@ -1029,6 +1030,9 @@ static int row_quant_impl(const void* x, int x_dtype, int64_t ld_x, int M, int K
                     (phase == 1 || (aligned8(q) && ld_q % 8 == 0)) && (!col || aligned16(col)) &&
                     (!bias || aligned16(bias));
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  if (fast && gelu && phase == 0 && x_dtype != IFLB200_F32 && g_row_tpr_override == 0 &&
+      launch_gelu_quant_stream({x, ld_x, M, K, row, col, bias, a.q, ld_q, qs}, x_dtype == IFLB200_F16, s))
+    return (int)cudaGetLastError();
   if (x_dtype == IFLB200_BF16) launch_row_quant<__nv_bfloat16>(a, fast, s);
   else if (x_dtype == IFLB200_F16) launch_row_quant<__half>(a, fast, s);
   else launch_row_quant<float>(a, fast, s);
@@ -1226,6 +1230,14 @@ static int resnorm_impl(void* res, int res_dtype, int64_t ld_res, int M, int D, 
     if (st != IFLB200_OK) return st;
     return (int)cudaGetLastError();
   }
+  // one affine after the norm, or none; per-row tables, a second output and a residual that is not
+  // stored stay with the one-row-per-group kernels
+  const bool modulated = mod_scale != nullptr;
+  if (fast && res_dtype == IFLB200_BF16 && layernorm && q && !y && !mod_index && (write_res || !delta) &&
+      !(modulated && (weight || beta)) && g_row_tpr_override == 0 &&
+      launch_residual_norm_stream({res, ld_res, M, D, a.delta, ld_delta, a.drow, a.dcol, a.bias, a.gate,
+                                   modulated ? mod_scale : weight, modulated ? mod_shift : beta, modulated, eps, a.q, ld_q, qs}, s))
+    return (int)cudaGetLastError();
   if (res_dtype == IFLB200_F32) launch_resnorm<float>(a, fast, s);
   else launch_resnorm<__nv_bfloat16>(a, fast, s);
   return (int)cudaGetLastError();

@@ -1,0 +1,87 @@
+"""The row kernels for many rows: same codes as the one-row-per-group kernels (GELU quantiser), the
+oracle's values (residual + layer norm + quantiser) at the edges of their range."""
+import pytest
+import torch
+
+from util import assert_quant_close_to_oracle, code_steps, i32, u8
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+E4M3 = torch.float8_e4m3fn
+
+
+@pytest.fixture(scope="module")
+def lib():
+    from instinctflash_b200 import _lib
+    return _lib.lib()
+
+
+def narrow(lib, call):
+    """``call`` on the kernels that give each row a group of 256 threads."""
+    assert lib.iflb200_row_set_group(256) == 0
+    try:
+        call()
+        torch.cuda.synchronize()
+    finally:
+        assert lib.iflb200_row_set_group(0) == 0
+
+
+# widths: smallest, not a whole number of chunks per thread, two groups of 448, the widest; rows: fewer than
+# two turns, a last turn with one row, several turns
+@pytest.mark.parametrize("M,K,dtype,bias", [(2100, 1032, torch.bfloat16, True), (297, 14336, torch.bfloat16, True),
+                                            (890, 13824, torch.float16, False), (301, 16384, torch.bfloat16, True),
+                                            (1185, 6152, torch.float16, True), (296, 8200, torch.bfloat16, False)])
+def test_gelu_quantiser_bits(lib, M, K, dtype, bias):
+    from instinctflash_b200.kernels import norm
+    from oracle import oracle as O
+    g = torch.Generator(device=DEV).manual_seed(M + K)
+    x = (torch.randn(M, K, device=DEV, generator=g) * 30).to(dtype)
+    row = torch.rand(M, device=DEV, generator=g) * 0.1
+    col = torch.rand(K, device=DEV, generator=g) * 2
+    b = torch.randn(K, device=DEV, generator=g) if bias else None
+    outs = []
+    for run in (lambda f: f(), lambda f: narrow(lib, f)):
+        q, s = torch.full((M, K + 8), 1.0, device=DEV).to(E4M3), torch.empty(M, device=DEV)
+        run(lambda: norm.row_quant(x, q[:, :K], s, row=row, col=col, bias=b, gelu=True))
+        outs.append((q, s))
+    torch.cuda.synchronize()
+    assert torch.equal(u8(outs[0][0]), u8(outs[1][0])) and torch.equal(i32(outs[0][1]), i32(outs[1][1]))
+    pick = torch.tensor([0, M // 2, M - 1], device=DEV)
+    qo, so = O.row_quant(x[pick].cpu(), row=row[pick].cpu(), col=col.cpu(), bias=None if b is None else b.cpu(), gelu=True)
+    assert_quant_close_to_oracle(outs[0][0][pick][:, :K], outs[0][1][pick], qo, so, f"{M}x{K}")
+
+
+@pytest.mark.parametrize("M,D,delta,gate,affine", [(2960, 1032, True, True, "mod"), (593, 5120, True, True, "norm"),
+                                                   (1777, 3072, True, False, "mod"), (300, 8192, True, True, "mod"),
+                                                   (600, 5128, False, False, None), (1500, 2048, False, False, "mod")])
+def test_residual_norm_rows(M, D, delta, gate, affine):
+    from instinctflash_b200.kernels import norm
+    from oracle import oracle as O
+    g = torch.Generator(device=DEV).manual_seed(M + D)
+
+    def randn(*shape, scale=1.0):
+        return torch.randn(*shape, device=DEV, generator=g) * scale
+
+    res = randn(M, D).to(torch.bfloat16)
+    kw, per_row = {}, {}
+    if delta:
+        per_row = {"delta": randn(M, D, scale=100.0).to(torch.bfloat16), "delta_row": torch.rand(M, device=DEV, generator=g) * 0.02}
+        kw = {"delta_col": randn(D), "bias": randn(D)}
+    if gate:
+        kw["gate"] = randn(D)
+    if affine:
+        names = ("mod_scale", "mod_shift") if affine == "mod" else ("weight", "beta")
+        kw.update({names[0]: randn(D, scale=0.2), names[1]: randn(D, scale=0.2)})
+    pick = torch.tensor([0, 1, M // 2, M - 2, M - 1], device=DEV)
+    want = O.residual_norm_quant(res[pick].cpu(), layernorm=True, **{k: v[pick].cpu() for k, v in per_row.items()},
+                                 **{k: v.cpu() for k, v in kw.items()})
+    q, s = torch.full((M, D + 8), 1.0, device=DEV).to(E4M3), torch.full((M,), -1.0, device=DEV)
+    norm.residual_norm_quant(res, layernorm=True, q=q[:, :D], q_scale=s, **per_row, **kw)
+    torch.cuda.synchronize()
+    assert (s > 0).all()
+    assert torch.equal(res[pick].cpu(), want["res"])   # elementwise: no sum in it
+    assert (q[:, D:].float() == 1.0).all()
+    # the order of the two sums of D terms is free: D * 2^-24 each, well under 1e-5 of the scale here
+    assert ((s[pick].cpu() - want["qs"]).abs() / want["qs"]).max().item() < 1e-5
+    steps = code_steps(q[pick][:, :D], want["q"])
+    assert steps.max().item() <= 1 and (steps != 0).float().mean().item() < 2e-3
