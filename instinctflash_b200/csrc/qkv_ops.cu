@@ -22,6 +22,7 @@
 
 #include "../../include/iflb200.h"
 #include "launch.cuh"
+#include "row_stream.cuh"
 #include "rowmath.cuh"
 
 namespace iflb200 {
@@ -614,6 +615,11 @@ extern "C" int iflb200_wan_qkv(const void* raw, int raw_dtype, int64_t ld_raw, i
                     (!k_pool || (aligned16(k_pool) && k_stride_b % oe == 0 && k_stride_s % oe == 0)) &&
                     (!v_pool || (aligned16(v_pool) && v_stride_b % oe == 0 && v_stride_s % oe == 0));
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  if (fast && raw_dtype == IFLB200_BF16 && out_dtype != IFLB200_F32 &&
+      launch_wan_qkv_stream({raw, ld_raw, rows, tokens, parts, (int)D, head_dim, row, col, bias, q_norm, k_norm, eps, inv_freq, pos,
+                             ld_pos, sections, slots, q_out, k_pool, v_pool, ld_q, k_stride_b, k_stride_s, v_stride_b, v_stride_s},
+                            out_dtype == IFLB200_F16, s))
+    return (int)cudaGetLastError();
   cudaError_t e;
   if (raw_dtype == IFLB200_BF16) e = launch_wan_qkv<__nv_bfloat16>(a, parts, out_dtype, fast, s);
   else if (raw_dtype == IFLB200_F16) e = launch_wan_qkv<__half>(a, parts, out_dtype, fast, s);

@@ -107,6 +107,7 @@ __device__ __forceinline__ void stage_vector(float*& dst, const float* src, int 
 // Meeting of one group of `threads` threads (whole warps, barrier `id`) over a value per warp; `slots` are
 // the group's, kMaxWarps of them, the neutral element (0) beyond its warps.
 constexpr int kMaxWarps = 16;
+constexpr int kMaxGroups = 12;  // one named barrier each, barrier 0 is the CTA's
 template <bool IS_MAX>
 __device__ __forceinline__ float group_meet(float v, float* slots, int warp, int id, int threads) {
   if (IS_MAX) {
@@ -148,7 +149,7 @@ StreamGeom stream_geom(int M, int K, int vectors, int row_bytes, int max_threads
   StreamGeom g;
   g.tg = ((K / 8 + kChunks - 1) / kChunks + 31) / 32 * 32;
   g.groups = max_threads / g.tg;
-  if (g.groups > 15) g.groups = 15;  // one named barrier each, barrier 0 is the CTA's
+  if (g.groups > kMaxGroups) g.groups = kMaxGroups;
   const size_t fixed = (size_t)vectors * K * 4;
   while (g.groups > 0 && fixed + (size_t)g.groups * row_bytes > kSmemLimit) --g.groups;
   if (g.groups < 2 || M < g.groups * sms) {
@@ -169,7 +170,7 @@ bool launch_stream(const StreamGeom& g, int sms, cudaStream_t s, const KArgs& a)
     if (cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimit) != cudaSuccess) return false;
     granted[dev] = true;
   }
-  launch_dep(kKernel, dim3(sms), dim3(g.tg * g.groups), g.smem, s, 1, dependent_launch_for(a.M), a, g.tg);
+  launch_dep(kKernel, dim3(sms), dim3(g.tg * g.groups), g.smem, s, 1, dependent_launch_for(a.rows_of_call()), a, g.tg);
   return true;
 }
 
@@ -188,13 +189,13 @@ bool launch_stream(const StreamGeom& g, int sms, cudaStream_t s, const KArgs& a)
 template <typename XT, bool BIAS, int THREADS>
 __global__ void __launch_bounds__(THREADS, 1) gelu_quant_stream_kernel(const GeluStreamArgs a, int tg) {
   extern __shared__ __align__(16) uint8_t smem[];
-  __shared__ __align__(16) float red[2][15][kMaxWarps];
+  __shared__ __align__(16) float red[2][kMaxGroups][kMaxWarps];
   const int g = threadIdx.x / tg, t = threadIdx.x - g * tg, groups = blockDim.x / tg;
   const uint32_t s_col = smem_u32(smem) + t * 16, s_bias = s_col + a.K * 4;
   const int half_bytes = a.K * 2;
   const uint32_t slot = smem_u32(smem) + a.K * (BIAS ? 8 : 4) + g * a.K * 2 + t * 16;
   const XT* x = reinterpret_cast<const XT*>(a.x) + t * 8;
-  for (int i = threadIdx.x; i < 2 * 15 * kMaxWarps; i += blockDim.x) (&red[0][0][0])[i] = 0.0f;
+  for (int i = threadIdx.x; i < 2 * kMaxGroups * kMaxWarps; i += blockDim.x) (&red[0][0][0])[i] = 0.0f;
 
   grid_dependency_wait();  // inputs may come from the kernel before this one in the stream
   grid_launch_dependents();
@@ -278,7 +279,7 @@ template <bool DELTA, bool GATE, bool AFFINE>
 __global__ void __launch_bounds__(kResNormThreads, 1) residual_norm_stream_kernel(const ResNormStreamArgs a, int tg) {
   constexpr int kVectors = (DELTA ? 2 : 0) + (GATE ? 1 : 0) + (AFFINE ? 2 : 0);
   extern __shared__ __align__(16) uint8_t smem[];
-  __shared__ __align__(16) float red[3][15][kMaxWarps];
+  __shared__ __align__(16) float red[3][kMaxGroups][kMaxWarps];
   const int g = threadIdx.x / tg, t = threadIdx.x - g * tg, groups = blockDim.x / tg;
   const uint32_t vec0 = smem_u32(smem) + t * 16;
   const int half_bytes = a.D * 2;
@@ -288,7 +289,7 @@ __global__ void __launch_bounds__(kResNormThreads, 1) residual_norm_stream_kerne
   const uint32_t slot_delta = slot_res + a.D * 2;
   __nv_bfloat16* res = reinterpret_cast<__nv_bfloat16*>(a.res) + t * 8;
   const float fD = (float)a.D;
-  for (int i = threadIdx.x; i < 3 * 15 * kMaxWarps; i += blockDim.x) (&red[0][0][0])[i] = 0.0f;
+  for (int i = threadIdx.x; i < 3 * kMaxGroups * kMaxWarps; i += blockDim.x) (&red[0][0][0])[i] = 0.0f;
 
   grid_dependency_wait();  // inputs may come from the kernel before this one in the stream
   grid_launch_dependents();
@@ -408,6 +409,185 @@ bool resnorm_form(const ResNormStreamArgs& a, int sms, cudaStream_t s) {
   return launch_stream<residual_norm_stream_kernel<DELTA, GATE, AFFINE>>(g, sms, s, a);
 }
 
+// --------------------------------------------------------------------------------------------
+// QKV consumer of a diffusion block (iflb200_wan_qkv): dequantise, RMS norm of Q and K over their full
+// width, rotate pairs (2j, 2j+1), store Q densely and K / V into pool rows.
+//
+// 2 bytes per element in, 2 out.  A group takes the parts (Q, K, V) of a row in turn; slots as above, the
+// vectors of all parts (eight of D floats) stay in shared memory.  The angles of a token are
+// shared by its heads and by Q and K: the group computes one sine and cosine per pair of a head, into a
+// table that the first meeting of the row makes visible.  4680 x 9216: 61.6 -> 43.7 us with one
+// CTA per (row, part) before, 16384 x 15360: 367 -> 232 (4.3 TB/s, issue slots 62 % busy).
+// --------------------------------------------------------------------------------------------
+constexpr int kWanThreads = 768;
+
+template <typename OT>
+__device__ __forceinline__ uint4 narrow(const Eight& v);
+template <>
+__device__ __forceinline__ uint4 narrow<__nv_bfloat16>(const Eight& v) {
+  uint32_t w[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    float lo, hi;
+    unpack2(v.p[i], lo, hi);
+    const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+    w[i] = *reinterpret_cast<const uint32_t*>(&h);
+  }
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+template <>
+__device__ __forceinline__ uint4 narrow<__half>(const Eight& v) {
+  uint32_t w[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    float lo, hi;
+    unpack2(v.p[i], lo, hi);
+    const __half2 h = __floats2half2_rn(lo, hi);
+    w[i] = *reinterpret_cast<const uint32_t*>(&h);
+  }
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+template <typename OT>
+__global__ void __launch_bounds__(kWanThreads, 1) wan_qkv_stream_kernel(const WanStreamArgs a, int tg) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  __shared__ __align__(16) float red[2][kMaxGroups][kMaxWarps];
+  const int D = a.D;
+  const int g = threadIdx.x / tg, t = threadIdx.x - g * tg, groups = blockDim.x / tg;
+  const int half_bytes = D * 2, step = a.bias ? 8 : 4;  // bytes of a part's vectors per column
+  const uint32_t vec0 = smem_u32(smem) + t * 16;
+  const uint32_t s_qn = vec0 + a.parts * D * step, s_kn = s_qn + (a.q_norm ? D * 4 : 0);
+  const uint32_t slot = s_kn + (a.k_norm ? D * 4 : 0) + g * D * 2;
+  // cosines, then sines, of the pairs of a head: a table per group, behind the slots
+  float* cosines = reinterpret_cast<float*>(smem + (slot - t * 16 - g * D * 2 - smem_u32(smem)) + groups * D * 2) + g * a.HD;
+  const int pair0 = (t * 8 % a.HD) >> 1;           // of the thread's first chunk
+  const bool same_pairs = tg * 8 % a.HD == 0;      // and of all its chunks
+  const __nv_bfloat16* raw = reinterpret_cast<const __nv_bfloat16*>(a.raw) + t * 8;
+  for (int i = threadIdx.x; i < 2 * kMaxGroups * kMaxWarps; i += blockDim.x) (&red[0][0][0])[i] = 0.0f;
+
+  grid_dependency_wait();  // inputs may come from the kernel before this one in the stream
+  grid_launch_dependents();
+  const int stride = gridDim.x * groups;
+  int row = blockIdx.x * groups + g;
+  auto fetch = [&](int r, int part, int it) {
+    copy16_async(slot + it * tg * 16, raw + (int64_t)r * a.ld_raw + (int64_t)part * D + it * tg * 8);
+  };
+  // the angle of pair t of a head (tg covers the pairs): its frequency stays here, the position of the next
+  // row's token is read a row ahead
+  const bool rope = a.inv_freq != nullptr, turns_pair = rope && t < a.HD / 2;
+  const float freq = turns_pair ? a.inv_freq[t] : 0.0f;
+  const float* pos = turns_pair ? a.pos + a.sections[t] : nullptr;
+  float rs = 1.0f, at = 0.0f;
+  if (row < a.rows) {
+#pragma unroll
+    for (int it = 0; it < kChunks; ++it)
+      if ((it * tg + t) * 8 < D) fetch(row, 0, it);
+    if (a.row) rs = a.row[row];
+    if (turns_pair) at = pos[(int64_t)(row % a.tokens) * a.ld_pos];
+  }
+  copy_commit();
+  float* dst = reinterpret_cast<float*>(smem);
+  for (int p = 0; p < a.parts; ++p) {
+    stage_vector(dst, a.col + (int64_t)p * D, D, 0.0f);
+    if (a.bias) stage_vector(dst, a.bias + (int64_t)p * D, D, 0.0f);
+  }
+  if (a.q_norm) stage_vector(dst, a.q_norm, D, 0.0f);
+  if (a.k_norm) stage_vector(dst, a.k_norm, D, 0.0f);
+  __syncthreads();
+
+  int turn = 0;
+  int b = 0, tok = 0;
+  for (int part = 0; row < a.rows;) {
+    if (part == 0) {
+      b = row / a.tokens;
+      tok = row - b * a.tokens;
+    }
+    const bool last = part + 1 == a.parts, more = !last || row + stride < a.rows;
+    const int next_row = last ? row + stride : row, next_part = last ? 0 : part + 1;
+    const bool norm = part == 0 ? a.q_norm != nullptr : (part == 1 && a.k_norm != nullptr);
+    if (part == 0 && turns_pair) {  // for Q and K of this row
+      const float ang = __fmul_rn(at, freq);
+      cosines[t] = cosf(ang);
+      cosines[a.HD / 2 + t] = sinf(ang);
+    }
+    float rs_next = rs;
+    if (last && more) {
+      if (a.row) rs_next = a.row[next_row];
+      if (turns_pair) at = pos[(int64_t)(next_row % a.tokens) * a.ld_pos];
+    }
+    const uint32_t s_col = vec0 + part * D * step, s_bias = s_col + D * 4;
+    copy_wait_all();
+    Eight x[kChunks];
+    uint64_t acc = 0;
+#pragma unroll
+    for (int it = 0; it < kChunks; ++it) {
+      if ((it * tg + t) * 8 < D) {
+        x[it] = widen(lds16(slot + it * tg * 16), __nv_bfloat16());
+        if (more) fetch(next_row, next_part, it);  // the slot has been read by the only thread that uses it
+        if (a.row) scale(x[it], rs);
+        if (a.bias) mul_add(x[it], lds_f32x8(s_col + it * tg * 16, half_bytes), lds_f32x8(s_bias + it * tg * 16, half_bytes));
+        else mul(x[it], lds_f32x8(s_col + it * tg * 16, half_bytes));
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc = fma2(x[it].p[i], x[it].p[i], acc);
+      }
+    }
+    copy_commit();
+    if (norm) {
+      float s0, s1;
+      unpack2(acc, s0, s1);
+      const float sum = group_meet<false>(__fadd_rn(s0, s1), red[turn][g], t >> 5, 1 + g, tg);
+      const float rstd = rsqrt_approx_ftz(__fadd_rn(div_full(sum, (float)D), a.eps));
+      const uint32_t s_w = part == 0 ? s_qn : s_kn;
+#pragma unroll
+      for (int it = 0; it < kChunks; ++it) {
+        if ((it * tg + t) * 8 < D) {
+          scale(x[it], rstd);
+          mul(x[it], lds_f32x8(s_w + it * tg * 16, half_bytes));
+        }
+      }
+      turn ^= 1;
+    } else if (rope && part == 0) {
+      named_bar_sync(1 + g, tg);
+    }
+    if (rope && part < 2) {
+      float4 co, si;
+#pragma unroll
+      for (int it = 0; it < kChunks; ++it) {
+        if ((it * tg + t) * 8 < D) {
+          if (it == 0 || !same_pairs) {  // the chunk lies inside one head
+            const int j = it == 0 ? pair0 : ((it * tg + t) * 8 % a.HD) >> 1;
+            co = *reinterpret_cast<const float4*>(cosines + j);
+            si = *reinterpret_cast<const float4*>(cosines + a.HD / 2 + j);
+          }
+          const float c[4] = {co.x, co.y, co.z, co.w}, n[4] = {si.x, si.y, si.z, si.w};
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            // (a, b) <- (a cos - b sin, b cos + a sin): sine products rounded, cosine products fused
+            float lo, hi;
+            unpack2(x[it].p[i], lo, hi);
+            x[it].p[i] = fma2(x[it].p[i], pack2(c[i], c[i]), mul2(pack2(hi, lo), pack2(-n[i], n[i])));
+          }
+        }
+      }
+    }
+    if (rope && last) named_bar_sync(1 + g, tg);  // the table has been read: the next row may replace it
+    OT* out;
+    if (part == 0) {
+      out = reinterpret_cast<OT*>(a.q) + (int64_t)row * a.ld_q;
+    } else {
+      const int64_t place = a.slots ? a.slots[tok] : tok;
+      out = part == 1 ? reinterpret_cast<OT*>(a.k) + (int64_t)b * a.sk_b + place * a.sk_s
+                      : reinterpret_cast<OT*>(a.v) + (int64_t)b * a.sv_b + place * a.sv_s;
+    }
+#pragma unroll
+    for (int it = 0; it < kChunks; ++it)
+      if ((it * tg + t) * 8 < D) *reinterpret_cast<uint4*>(out + (it * tg + t) * 8) = narrow<OT>(x[it]);
+    row = next_row;
+    part = next_part;
+    rs = rs_next;
+  }
+}
+
 }  // namespace
 
 bool launch_gelu_quant_stream(const GeluStreamArgs& a, bool half, cudaStream_t s) {
@@ -422,6 +602,15 @@ bool launch_residual_norm_stream(const ResNormStreamArgs& a, cudaStream_t s) {
   if (!a.delta) return a.scale ? resnorm_form<false, false, true>(a, sms, s) : resnorm_form<false, false, false>(a, sms, s);
   if (!a.drow || !a.dcol || !a.bias || !a.scale) return false;
   return a.gate ? resnorm_form<true, true, true>(a, sms, s) : resnorm_form<true, false, true>(a, sms, s);
+}
+
+bool launch_wan_qkv_stream(const WanStreamArgs& a, bool half, cudaStream_t s) {
+  const int sms = sm_count();
+  if (sms == 0 || !a.col || a.D <= 1024 || a.D > 16384 || a.HD % 8) return false;
+  const int vectors = a.parts * (a.bias ? 2 : 1) + (a.q_norm ? 1 : 0) + (a.k_norm ? 1 : 0);
+  StreamGeom g = stream_geom(a.rows, a.D, vectors, a.D * 2 + a.HD * 4, kWanThreads, sms);
+  if (g.groups == 0 || g.tg < a.HD / 2) return false;
+  return half ? launch_stream<wan_qkv_stream_kernel<__half>>(g, sms, s, a) : launch_stream<wan_qkv_stream_kernel<__nv_bfloat16>>(g, sms, s, a);
 }
 
 }  // namespace iflb200

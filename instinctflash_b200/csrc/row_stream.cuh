@@ -13,6 +13,7 @@ struct GeluStreamArgs {
   const void* x;
   int64_t ld_x;
   int M, K;
+  int rows_of_call() const { return M; }
   const float* row;
   const float* col;
   const float* bias;
@@ -27,6 +28,7 @@ struct ResNormStreamArgs {
   void* res;
   int64_t ld_res;
   int M, D;
+  int rows_of_call() const { return M; }
   const __nv_bfloat16* delta;  // or null
   int64_t ld_delta;
   const float *drow, *dcol, *bias, *gate;
@@ -41,5 +43,21 @@ struct ResNormStreamArgs {
 // layer norm of a bf16 residual, updated in place when there is a delta; every buffer on the 16-byte
 // rule (codes: 8), D a multiple of 8
 bool launch_residual_norm_stream(const ResNormStreamArgs& a, cudaStream_t s);
+
+struct WanStreamArgs {
+  const void* raw;  // bf16 [rows, parts * D]
+  int64_t ld_raw;
+  int rows, tokens, parts, D, HD;
+  int rows_of_call() const { return rows; }
+  const float *row, *col, *bias, *q_norm, *k_norm;
+  float eps;
+  const float *inv_freq, *pos;
+  int64_t ld_pos;
+  const int32_t *sections, *slots;
+  void *q, *k, *v;
+  int64_t ld_q, sk_b, sk_s, sv_b, sv_s;
+};
+// f16 (`half`) or bf16 outputs; every buffer and stride on the 16-byte rule, D and HD multiples of 8
+bool launch_wan_qkv_stream(const WanStreamArgs& a, bool half, cudaStream_t s);
 
 }  // namespace iflb200

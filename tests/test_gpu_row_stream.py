@@ -85,3 +85,45 @@ def test_residual_norm_rows(M, D, delta, gate, affine):
     assert ((s[pick].cpu() - want["qs"]).abs() / want["qs"]).max().item() < 1e-5
     steps = code_steps(q[pick][:, :D], want["q"])
     assert steps.max().item() <= 1 and (steps != 0).float().mean().item() < 2e-3
+
+
+# heads narrower than a thread's stride (its chunks lie at different pairs), one part only, no norm, pool slots
+@pytest.mark.parametrize("B,T,H,HD,parts,norm,dtype", [(2, 700, 24, 128, 3, True, torch.float16), (1, 1801, 9, 120, 3, False, torch.bfloat16),
+                                                       (1, 1900, 12, 128, 1, True, torch.bfloat16), (1, 593, 40, 128, 3, True, torch.float16)])
+def test_wan_qkv_rows(lib, B, T, H, HD, parts, norm, dtype):
+    from instinctflash_b200.kernels import rope, wan
+    from oracle import oracle as O
+    g = torch.Generator(device=DEV).manual_seed(T)
+    D, R = H * HD, B * T
+    raw = torch.randn(R, parts * D, device=DEV, generator=g).to(torch.bfloat16)
+    row = torch.rand(R, device=DEV, generator=g)
+    col, bias = torch.rand(parts * D, device=DEV, generator=g), torch.randn(parts * D, device=DEV, generator=g)
+    w = {n: torch.rand(D, device=DEV, generator=g) + 0.5 if norm else None for n in ("q_norm", "k_norm")}
+    pos = (torch.rand(T, 3, device=DEV, generator=g) * 60).floor()
+    sec = (torch.arange(HD // 2, device=DEV) % 3).int()
+    inv = rope.rope_inv_freq(HD, 10000.0, DEV)
+    slots = torch.randperm(T, device=DEV, generator=g).int()
+    q = torch.full((R, D + 8), 7.0, device=DEV, dtype=dtype)
+    pools = [torch.empty(B, T, D, device=DEV, dtype=dtype) if parts > 1 + i else None for i in range(2)]
+    wan.wan_qkv(raw, q[:, :D], heads=H, head_dim=HD, tokens=T, k_pool=pools[0], v_pool=pools[1], slots=slots, row=row, col=col,
+                bias=bias, pos=pos, sections=sec, inv_freq=inv, **w)
+    torch.cuda.synchronize()
+    tok = torch.tensor([0, 1, T // 2, T - 1], device=DEV)
+    for b in range(B):
+        rows = b * T + tok
+        want = O.wan_qkv(raw[rows].cpu(), heads=H, head_dim=HD, tokens=len(tok), parts=parts, row=row[rows].cpu(), col=col.cpu(),
+                         bias=bias.cpu(), pos=pos[tok].cpu(), sections=sec.cpu(), inv_freq=inv.cpu(), out_dtype=dtype,
+                         **{n: None if t is None else t.cpu() for n, t in w.items()})
+        got = [q[rows][:, :D]] + [None if p is None else p[b][slots[tok].long()] for p in pools]
+        ulp = 2.0 ** -10 if dtype == torch.float16 else 2.0 ** -7
+        for i, (a, e) in enumerate(zip(got, want)):
+            if a is None:
+                continue
+            a, e = a.cpu().float(), e.reshape(len(tok), D).float()
+            if i == 2:
+                assert torch.equal(a, e)   # V: no sum and no angle in it
+            # one rounding of the output apart (the sum of squares is free in its order, sine and cosine are the
+            # libraries'): relative to the pair's magnitude, since a rotation can cancel
+            mag = e.reshape(-1, 2).norm(dim=1).repeat_interleave(2).reshape(e.shape)
+            assert ((a - e).abs() <= ulp * mag + 1e-6).all(), (i, ((a - e).abs() / mag).max())
+    assert (q[:, D:] == 7.0).all()
