@@ -3,8 +3,8 @@
 //   out[M,N] = epilogue( sum_k A[m,k] * W[n,k] )        A [M,K], W [N,K], both K-major
 //
 // Persistent, warp-specialised, one CTA per SM:
-//   warp 0      TMA producer: cp.async.bulk.tensor loads of a 128 x 128-byte A tile and a
-//               BN x 128-byte W tile per stage, 128-byte swizzle, completion on an mbarrier;
+//   warp 0      TMA producer of W: cp.async.bulk.tensor loads of a BN x 128-byte tile per stage,
+//               128-byte swizzle, completion on an mbarrier; the last warp the same for A (128 rows);
 //   warp 1      MMA issuer: one thread issues tcgen05.mma (128 x BN x 32 per instruction,
 //               four per stage) into one of two TMEM accumulators and commits the stage's
 //               "empty" barrier / the accumulator's "full" barrier;
@@ -30,7 +30,7 @@ namespace iflb200 {
 
 constexpr int BM = 128;
 constexpr int BK = 128;  // bytes == e4m3 elements per stage along K
-constexpr int kGemmThreads = 320;  // TMA warp, MMA warp, eight epilogue warps
+constexpr int kGemmThreads = 352;  // W producer, MMA warp, eight epilogue warps, A producer
 constexpr int kPrefetchSteps = 8;  // W boxes warmed in L2 ahead of the grid dependency wait
 constexpr int kEpilogueWarps = 8;   // two per TMEM lane quadrant, each draining half of the columns
 constexpr uint64_t kWaitBudgetNs = 2000000000ull;  // 2 s per wait, then abort
@@ -161,19 +161,19 @@ __device__ __forceinline__ void tile_place(const GemmParams& p, int tile, int& m
   tile_coords(p, tile, m_blk, n_blk);
 }
 
-// Bounded wait on an mbarrier phase.  Returns false when the CTA is aborting.
+// Bounded wait of a converged warp on an mbarrier phase.  Returns false when the CTA is aborting.
 __device__ __forceinline__ bool wait_bounded(uint32_t bar, uint32_t parity, volatile uint32_t* abort,
                                              uint32_t code) {
-  if (mbar_try_wait(bar, parity)) return true;
+  if (__all_sync(0xFFFFFFFFu, mbar_try_wait(bar, parity))) return true;
   uint64_t t0 = 0;
   uint32_t spins = 0;
   while (true) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if (*abort) return false;
+    if (__all_sync(0xFFFFFFFFu, mbar_try_wait(bar, parity))) return true;
+    if (__any_sync(0xFFFFFFFFu, *abort)) return false;
     if (++spins > 2048) {
       if (t0 == 0) t0 = globaltimer_ns();
       __nanosleep(128);
-      if (globaltimer_ns() - t0 > g_gemm_wait_budget_ns) {
+      if (__any_sync(0xFFFFFFFFu, globaltimer_ns() - t0 > g_gemm_wait_budget_ns)) {
         *abort = 1;
         atomicCAS(&g_timeout_record[0], 0u, code);
         return false;
@@ -181,6 +181,40 @@ __device__ __forceinline__ bool wait_bounded(uint32_t bar, uint32_t parity, vola
     }
   }
 }
+
+// The ring of shared-memory stages as one producer warp walks it.  Each operand has a warp of its own:
+// one TMA instruction with its barrier traffic takes an issuing warp about 250 clocks however small the
+// box (330 from a branch on one lane instead of elect.sync), two warps overlap theirs.  With both
+// operands on one lane a 128-byte K step took 0.41 us whatever the tile -- 790 clocks for 520 of MMA
+// work -- although TMA brings an SM 115 bytes a clock from L2.
+template <int STAGES>
+struct Ring {
+  int stage = 0;
+  uint32_t phase = 0;
+  uint32_t armed = 0;        // stages this warp has armed at least once
+  uint32_t last_parity = 0;  // parity of its last arming per stage
+  __device__ __forceinline__ void arm() {
+    armed |= 1u << stage;
+    last_parity = (last_parity & ~(1u << stage)) | (phase << stage);
+  }
+  __device__ __forceinline__ void advance() {
+    if (++stage == STAGES) {
+      stage = 0;
+      phase ^= 1;
+    }
+  }
+  // Every load this warp issued must have landed before the CTA's shared memory can go away.  Normal exit: the
+  // consumer has already waited on all of them, these return at once.  Abort: bounded.
+  __device__ __forceinline__ void drain(uint32_t full0) const {
+    for (int s = 0; s < STAGES; ++s) {
+      if (armed & (1u << s)) {
+        const uint32_t par = (last_parity >> s) & 1u;
+        uint32_t spins = 0;
+        while (!mbar_try_wait(full0 + 8u * s, par) && ++spins < (1u << 20)) __nanosleep(64);
+      }
+    }
+  }
+};
 
 template <int BN>
 __device__ __forceinline__ void epilogue_chunk(const GemmParams& p, const uint32_t (&acc)[32], int m,
@@ -702,7 +736,7 @@ __device__ __forceinline__ void epilogue_swapped(const GemmParams& p, const CUte
 // columns of the same hidden units; p.N counts hidden units.
 // EW: epilogue warps (8, or 16 for the gated form: EW / 4 per TMEM lane quadrant).
 template <int BN, int STAGES, int SPLIT, bool SWAP = false, bool GATED = false, int EW = kEpilogueWarps, int SL = 1>
-__global__ void __launch_bounds__(64 + 32 * EW, 1)
+__global__ void __launch_bounds__(96 + 32 * EW, 1)
 gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w,
                     const __grid_constant__ CUtensorMap tm_out, const GemmParams p) {
   using L = SmemLayout<BN, STAGES, EW, SL>;
@@ -759,7 +793,7 @@ gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
     prefetch_tensormap(&tm_a);
     prefetch_tensormap(&tm_w);
     for (int s = 0; s < STAGES; ++s) {
-      mbar_init(full_bar(s), 1);
+      mbar_init(full_bar(s), 2);  // one arrival per producer
       mbar_init(empty_bar(s), 1);
     }
     for (int a = 0; a < 2; ++a) {
@@ -780,125 +814,63 @@ gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
   const uint32_t tmem_base = *tmem_slot;
   if (threadIdx.x == 0) GEMM_TRACE(2);  // barriers initialised, tensor memory allocated
 
-  // Everything above touched no global memory.  While the kernel before this one in the stream
-  // drains, pull the first W boxes of this CTA's first tile towards L2 (a prefetch cannot read
-  // stale data into the kernel: the loads proper are issued after the dependency wait and L2 is
-  // the coherence point), then wait for that kernel's results.
-  if (warp == 0 && lane == 0 && tile_first < p.num_tiles) {
-    int m_blk, n_blk, grp;
-    tile_place(p, tile_first, m_blk, n_blk, grp);
-    const int kb_end = kb1 < kb0 + kPrefetchSteps ? kb1 : kb0 + kPrefetchSteps;
-    for (int kb = kb0; kb < kb_end; kb += SL) {
-      if constexpr (GATED) {
-        tma_prefetch_l2_3d(&tm_w, kb * BK, n_blk * (BN / 2), 0);
-      } else if constexpr (SL > 1) {
-        tma_prefetch_l2_3d(&tm_w, 0, n_blk * BN, kb);
-      } else {
-        tma_prefetch_l2_2d(&tm_w, kb * BK, n_blk * BN);
-      }
+  // Everything above touched no global memory.  Everything below that reads what another kernel may have
+  // written waits for that kernel first: the producer of the activations and the epilogue warps.  The
+  // weights are not an output of the kernel before this one (contract: see iflb200_gemm_fp8_raw), so their
+  // producer starts at once, and their DRAM round trip -- the longest single latency of a 4 us
+  // skinny kernel -- runs while that kernel drains.
+  const bool w_producer = warp == 0, a_producer = warp == 2 + EW;
+  if (w_producer || a_producer) {
+    // ------------------------------------------------------------------ TMA producers
+    const bool weights = SWAP ? a_producer : w_producer;
+    if (!weights) {
+      grid_dependency_wait();
+      if (lane == 0) GEMM_TRACE(3);  // the kernel before this one has completed
     }
-  }
-
-  if (warp == 0) {
-    // ------------------------------------------------------------------ TMA producer
-    // The one thread that issues loads waits for the kernel before this one; the epilogue warps
-    // are ordered behind it through the barriers (and re-check below), the MMA warp touches no
-    // global memory.  Fewer waiting threads matter: a CTA that became resident early sits beside
-    // a kernel that is still running.
-    // The weight boxes of the first stages are issued BEFORE the dependency wait.  The weights are not
-    // an output of the kernel before this one (the activations are), so their DRAM round trip -- the
-    // longest single latency of a 4 us skinny kernel -- runs while that kernel drains; after the wait
-    // only the activation boxes (mostly L2 hits) remain.  (Contract: see iflb200_gemm_fp8_raw.)
-    int early = 0;
-    if constexpr (!SWAP) {  // (in the swapped form the operand behind tm_a is the weight matrix)
-      if (lane == 0 && tile_first < p.num_tiles) {
-        int m_blk, n_blk, grp;
-        tile_place(p, tile_first, m_blk, n_blk, grp);
-        for (int kb = kb0; kb < kb1 && early < STAGES; kb += SL, ++early) {
-          mbar_arrive_expect_tx(full_bar(early), (uint32_t)(SL * p.a_bytes) + L::kBBytes);
-          const uint32_t sw = base + early * L::kStageBytes + L::kABytes;
-          if constexpr (SL > 1) tma_load_3d(sw, &tm_w, full_bar(early), 0, n_blk * BN, kb);
-          else if constexpr (GATED) tma_load_3d(sw, &tm_w, full_bar(early), kb * BK, n_blk * (BN / 2), 0);
-          else tma_load_2d(sw, &tm_w, full_bar(early), kb * BK, n_blk * BN);
-        }
-      }
-      early = __shfl_sync(0xFFFFFFFFu, early, 0);
-    }
-    if (lane == 0) grid_dependency_wait();
-    if (lane == 0) GEMM_TRACE(3);  // the kernel before this one has completed
-    __syncwarp();
-    int stage = 0;
-    uint32_t phase = 0;
-    uint32_t armed = (1u << early) - 1u;  // stages armed at least once (the early ones: first phase, parity 0)
-    uint32_t last_parity = 0;             // parity of the last arming per stage
+    const uint32_t bytes = w_producer ? (uint32_t)L::kBBytes : (uint32_t)(SL * p.a_bytes);
+    Ring<STAGES> ring;
     bool ok = true;
     uint32_t it = 0;
-    int fill = 0;              // stage fills issued so far
     for (int tile = tile_first; ok && tile < p.num_tiles; tile += tile_stride, ++it) {
       int m_blk, n_blk, grp;
       tile_place(p, tile, m_blk, n_blk, grp);
       const int a_row = grp * p.group_rows + m_blk * BM;  // rows past a block's end belong to the next block: loaded, never stored
-      for (int kb = kb0; kb < kb1; kb += SL, ++fill) {
-        if (fill < early) {
-          // armed above with its weight box in flight (stage == fill, first phase): the activation box only
-          if (lane == 0) {
-            if constexpr (SL > 1) tma_load_3d(base + stage * L::kStageBytes, &tm_a, full_bar(stage), 0, a_row, kb);
-            else tma_load_2d(base + stage * L::kStageBytes, &tm_a, full_bar(stage), kb * BK, a_row);
-          }
-          armed |= 1u << stage;
-          last_parity = (last_parity & ~(1u << stage)) | (phase << stage);
-          __syncwarp();
-          if (++stage == STAGES) {
-            stage = 0;
-            phase ^= 1;
-          }
-          continue;
-        }
-        ok = __all_sync(0xFFFFFFFFu, wait_bounded(empty_bar(stage), phase ^ 1, abort_flag,
-                                                  (1u << 24) | (1u << 16) | (it & 0xFFFF)));
+      for (int kb = kb0; kb < kb1; kb += SL) {
+        ok = wait_bounded(empty_bar(ring.stage), ring.phase ^ 1, abort_flag, (1u << 24) | (1u << 16) | (it & 0xFFFF));
         if (!ok) break;
-        if (lane == 0) {
-          mbar_arrive_expect_tx(full_bar(stage), (uint32_t)(SL * p.a_bytes) + L::kBBytes);
-          const uint32_t sa = base + stage * L::kStageBytes;
-          if constexpr (SL > 1) {
-            // SL slabs of each operand per instruction; slabs past the end of K read as zeros
-            tma_load_3d(sa, &tm_a, full_bar(stage), 0, a_row, kb);
-            tma_load_3d(sa + L::kABytes, &tm_w, full_bar(stage), 0, n_blk * BN, kb);
+        if (elect_one()) {
+          const uint32_t bar = full_bar(ring.stage), sa = base + ring.stage * L::kStageBytes, sw = sa + L::kABytes;
+          mbar_arrive_expect_tx(bar, bytes);
+          if (w_producer) {
+            // SL slabs per instruction (slabs past the end of K read as zeros); the gated form's weight is mapped
+            // as [2][F][K]: gate rows, then the up rows of the same hidden units, in one load
+            if constexpr (SL > 1) tma_load_3d(sw, &tm_w, bar, 0, n_blk * BN, kb);
+            else if constexpr (GATED) tma_load_3d(sw, &tm_w, bar, kb * BK, n_blk * (BN / 2), 0);
+            else tma_load_2d(sw, &tm_w, bar, kb * BK, n_blk * BN);
           } else {
-          tma_load_2d(sa, &tm_a, full_bar(stage), kb * BK, a_row);
-          if constexpr (GATED) {
-            // gate rows, then the up rows of the same hidden units: one B operand of BN rows, one
-            // load (the weight is mapped as [2][F][K]; a second TMA instruction per stage cost the
-            // main loop about a tenth of its rate)
-            tma_load_3d(sa + L::kABytes, &tm_w, full_bar(stage), kb * BK, n_blk * (BN / 2), 0);
-          } else {
-            tma_load_2d(sa + L::kABytes, &tm_w, full_bar(stage), kb * BK, n_blk * BN);
-          }
+            if constexpr (SL > 1) tma_load_3d(sa, &tm_a, bar, 0, a_row, kb);
+            else tma_load_2d(sa, &tm_a, bar, kb * BK, a_row);
           }
         }
-        armed |= 1u << stage;
-        last_parity = (last_parity & ~(1u << stage)) | (phase << stage);
         __syncwarp();
-        if (++stage == STAGES) {
-          stage = 0;
-          phase ^= 1;
+        ring.arm();
+        ring.advance();
+        if (weights && it == 0 && kb == kb0 + (STAGES - 1) * SL && elect_one()) {
+          // the ring is full: until its first stage is free, pull the boxes behind it towards L2
+          for (int kp = kb + SL; kp < kb1 && kp < kb0 + kPrefetchSteps; kp += SL) {
+            if constexpr (SWAP) tma_prefetch_l2_2d(&tm_a, kp * BK, a_row);
+            else if constexpr (GATED) tma_prefetch_l2_3d(&tm_w, kp * BK, n_blk * (BN / 2), 0);
+            else if constexpr (SL > 1) tma_prefetch_l2_3d(&tm_w, 0, n_blk * BN, kp);
+            else tma_prefetch_l2_2d(&tm_w, kp * BK, n_blk * BN);
+          }
         }
       }
     }
     // This CTA's last loads are in flight: the next kernel in the stream may be scheduled now
     // (it becomes resident as CTAs of this grid leave and waits for the grid to complete).
     // Not earlier: CTAs parked at their dependency wait for the length of a long GEMM slow it.
-    grid_launch_dependents();
-    // Drain: every load this warp issued must have landed before the CTA's shared memory can
-    // go away.  Normal exit: the consumer has already waited on all of them, these return at
-    // once.  Abort: bounded.
-    for (int s = 0; s < STAGES; ++s) {
-      if (armed & (1u << s)) {
-        const uint32_t par = (last_parity >> s) & 1u;
-        uint32_t spins = 0;
-        while (!mbar_try_wait(full_bar(s), par) && ++spins < (1u << 20)) __nanosleep(64);
-      }
-    }
+    if (!weights) grid_launch_dependents();
+    ring.drain(full_bar(0));
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
     int stage = 0;
@@ -908,18 +880,16 @@ gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
     for (int tile = tile_first; ok && tile < p.num_tiles; tile += tile_stride, ++it) {
       const uint32_t acc = it & 1u;
       const uint32_t acc_phase = (it >> 1) & 1u;
-      ok = __all_sync(0xFFFFFFFFu, wait_bounded(tempty_bar(acc), acc_phase ^ 1, abort_flag,
-                                                (2u << 24) | (2u << 16) | (it & 0xFFFF)));
+      ok = wait_bounded(tempty_bar(acc), acc_phase ^ 1, abort_flag, (2u << 24) | (2u << 16) | (it & 0xFFFF));
       if (!ok) break;
       tc_fence_after();
       const uint32_t d_tmem = tmem_base + acc * kAccStride;
       for (int kb = kb0; kb < kb1; kb += SL) {
-        ok = __all_sync(0xFFFFFFFFu, wait_bounded(full_bar(stage), phase, abort_flag,
-                                                  (2u << 24) | (3u << 16) | (it & 0xFFFF)));
+        ok = wait_bounded(full_bar(stage), phase, abort_flag, (2u << 24) | (3u << 16) | (it & 0xFFFF));
         if (!ok) break;
         tc_fence_after();
         if (lane == 0 && it == 0 && kb == kb0) GEMM_TRACE(4);  // first operands have landed
-        if (lane == 0) {
+        if (elect_one()) {
           const uint32_t sa = base + stage * L::kStageBytes;
 #pragma unroll
           for (int sl = 0; sl < SL; ++sl) {
@@ -942,7 +912,7 @@ gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
         }
       }
       if (!ok) break;
-      if (lane == 0) mma_commit(tfull_bar(acc));  // accumulator complete
+      if (elect_one()) mma_commit(tfull_bar(acc));  // accumulator complete
       if (lane == 0 && it == 0) GEMM_TRACE(5);  // last MMA of the first tile issued
       __syncwarp();
     }
@@ -988,8 +958,7 @@ gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
         gated_scales<BN, EW / 4>(p, n_blk * (BN / 2), half, lane, cgl, cul);
         rs_early = (row_ok && p.row) ? __ldg(p.row + (int64_t)m * p.row_stride) : 1.0f;
       }
-      ok = __all_sync(0xFFFFFFFFu, wait_bounded(tfull_bar(acc), acc_phase, abort_flag,
-                                                (3u << 24) | (4u << 16) | (it & 0xFFFF)));
+      ok = wait_bounded(tfull_bar(acc), acc_phase, abort_flag, (3u << 24) | (4u << 16) | (it & 0xFFFF));
       if (!ok) break;
       tc_fence_after();
       if (warp == 2 && lane == 0 && it == 0) GEMM_TRACE(6);  // first accumulator complete
@@ -1063,7 +1032,7 @@ gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
     const int quad = warp & 3;
     const int half = (warp - 2) >> 2;
     const int row = quad * 32 + lane;
-    const bool reducing = warp >= 2 && !*abort_flag && tile_first < p.num_tiles;
+    const bool reducing = warp >= 2 && warp < 2 + EW && !*abort_flag && tile_first < p.num_tiles;
     cluster_arrive();
     cluster_wait();  // every CTA of the cluster has finished its main loop: the stage rings are free
     if (reducing) {
@@ -1235,7 +1204,7 @@ gemm_fp8_tc5_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
-      mbar_init(full_bar(s), 1);   // leader's producer arms it; bytes of both CTAs complete it
+      mbar_init(full_bar(s), 2);   // the leader's two producers arm it; bytes of both CTAs complete it
       mbar_init(empty_bar(s), 1);  // one multicast commit from the leader
     }
     for (int a = 0; a < 2; ++a) {
@@ -1258,38 +1227,33 @@ gemm_fp8_tc5_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
   cluster_sync_all();  // barriers of both CTAs initialised before any remote signal
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  grid_dependency_wait();
 
-  if (warp == 0) {
-    // ------------------------------------------------------------------ TMA producer (both CTAs)
-    int stage = 0;
-    uint32_t phase = 0;
+  const bool w_producer = warp == 0, a_producer = warp == 2 + kEpilogueWarps;
+  if (w_producer || a_producer) {
+    // ------------------------------------------------------------------ TMA producers (both CTAs)
+    // A warp per operand, the weights' one ahead of the dependency wait, as in the single-CTA kernel.
+    const bool weights = SWAP ? a_producer : w_producer;
+    if (!weights) grid_dependency_wait();
+    Ring<STAGES> ring;
     bool ok = true;
     uint32_t it = 0;
     for (int tile = pair_id; ok && tile < p.num_tiles; tile += pair_stride, ++it) {
       int m_blk, n_blk;
       tile_coords(p, tile, m_blk, n_blk);
-      const int m0 = m_blk * 2 * BM + (int)rank * BM;
-      const int n0 = n_blk * BN + (int)rank * (BN / 2);
+      const int row = w_producer ? n_blk * BN + (int)rank * (BN / 2) : m_blk * 2 * BM + (int)rank * BM;
       for (int kb = 0; kb < p.num_k; ++kb) {
-        ok = __all_sync(0xFFFFFFFFu, wait_bounded(empty_bar(stage), phase ^ 1, abort_flag,
-                                                  (1u << 24) | (1u << 16) | (it & 0xFFFF)));
+        ok = wait_bounded(empty_bar(ring.stage), ring.phase ^ 1, abort_flag, (1u << 24) | (1u << 16) | (it & 0xFFFF));
         if (!ok) break;
-        if (lane == 0) {
-          if (leader) mbar_arrive_expect_tx(full_bar(stage), 2 * L::kStageBytes);
-          const uint32_t sa = base + stage * L::kStageBytes;
-          const uint32_t lead_full = full_bar(stage) & kPeerBitMask;
-          tma_load_2d_pair(sa, &tm_a, lead_full, kb * BK, m0);
-          tma_load_2d_pair(sa + L::kABytes, &tm_w, lead_full, kb * BK, n0);
+        if (elect_one()) {
+          if (leader) mbar_arrive_expect_tx(full_bar(ring.stage), 2u * (w_producer ? L::kBBytes : L::kABytes));
+          const uint32_t dst = base + ring.stage * L::kStageBytes + (w_producer ? L::kABytes : 0);
+          tma_load_2d_pair(dst, w_producer ? &tm_w : &tm_a, full_bar(ring.stage) & kPeerBitMask, kb * BK, row);
         }
         __syncwarp();
-        if (++stage == STAGES) {
-          stage = 0;
-          phase ^= 1;
-        }
+        ring.advance();
       }
     }
-    grid_launch_dependents();  // last loads issued: the next kernel may be scheduled
+    if (!weights) grid_launch_dependents();  // last loads issued: the next kernel may be scheduled
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (leader only)
     if (leader) {
@@ -1300,17 +1264,15 @@ gemm_fp8_tc5_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
       for (int tile = pair_id; ok && tile < p.num_tiles; tile += pair_stride, ++it) {
         const uint32_t acc = (ACC == 2) ? (it & 1u) : 0u;
         const uint32_t acc_phase = (ACC == 2) ? ((it >> 1) & 1u) : (it & 1u);
-        ok = __all_sync(0xFFFFFFFFu, wait_bounded(tempty_bar(acc), acc_phase ^ 1, abort_flag,
-                                                  (2u << 24) | (2u << 16) | (it & 0xFFFF)));
+        ok = wait_bounded(tempty_bar(acc), acc_phase ^ 1, abort_flag, (2u << 24) | (2u << 16) | (it & 0xFFFF));
         if (!ok) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * kAccStride;
         for (int kb = 0; kb < p.num_k; ++kb) {
-          ok = __all_sync(0xFFFFFFFFu, wait_bounded(full_bar(stage), phase, abort_flag,
-                                                    (2u << 24) | (3u << 16) | (it & 0xFFFF)));
+          ok = wait_bounded(full_bar(stage), phase, abort_flag, (2u << 24) | (3u << 16) | (it & 0xFFFF));
           if (!ok) break;
           tc_fence_after();
-          if (lane == 0) {
+          if (elect_one()) {
             const uint32_t sa = base + stage * L::kStageBytes;
             const uint64_t da = make_kmajor_sw128_desc(sa);
             const uint64_t db = make_kmajor_sw128_desc(sa + L::kABytes);
@@ -1326,7 +1288,7 @@ gemm_fp8_tc5_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
           }
         }
         if (!ok) break;
-        if (lane == 0) mma_commit_pair(tfull_bar(acc), 3);  // accumulator complete in both CTAs
+        if (elect_one()) mma_commit_pair(tfull_bar(acc), 3);  // accumulator complete in both CTAs
         __syncwarp();
       }
     }
@@ -1346,6 +1308,7 @@ gemm_fp8_tc5_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
     bool ok = true;
     uint32_t it = 0;
     int swap_buf = 0;
+    grid_dependency_wait();  // scales and residual operands may come from the kernel before this one
     for (int tile = pair_id; ok && tile < p.num_tiles; tile += pair_stride, ++it) {
       int m_blk, n_blk;
       tile_coords(p, tile, m_blk, n_blk);
@@ -1361,8 +1324,7 @@ gemm_fp8_tc5_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
         cv = fetch_column_vectors(p, n_blk * BN + col_begin, col_end - col_begin, lane);
         rs_early = (row_ok && p.row) ? __ldg(p.row + (int64_t)m * p.row_stride) : 1.0f;
       }
-      ok = __all_sync(0xFFFFFFFFu, wait_bounded(tfull_bar(acc), acc_phase, abort_flag,
-                                                (3u << 24) | (4u << 16) | (it & 0xFFFF)));
+      ok = wait_bounded(tfull_bar(acc), acc_phase, abort_flag, (3u << 24) | (4u << 16) | (it & 0xFFFF));
       if (!ok) break;
       tc_fence_after();
       const uint32_t t_row = tmem_base + ((uint32_t)(quad * 32) << 16) + acc * kAccStride;
@@ -1573,7 +1535,7 @@ static int launch_gemm_form(const CUtensorMap& ta, const CUtensorMap& tw, const 
     attr_set[dev] = true;
   }
   const cudaError_t e = launch_dep(gemm_fp8_tc5_kernel<BN, STAGES, SPLIT, SWAP, GATED, EW, SL>, dim3(grid),
-                                   dim3(64 + 32 * EW), L::kDynamic, s, p.split_k,
+                                   dim3(96 + 32 * EW), L::kDynamic, s, p.split_k,
                                    dependent_launch_for(SWAP ? p.N : p.M), ta, tw, to, p);
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
