@@ -257,9 +257,10 @@ IFLB200_API int iflb200_gemm_fp8_raw(const void* a, int64_t ld_a, const void* w,
                          int M, int N, int K, void* out, int64_t ld_out, void* stream);
 
 /*
- * Split-K for skinny activations (M <= 128): K is divided into `splits` ranges, each range of each
- * 64-column tile goes to its own CTA (tiles x splits CTAs, so that a deep reduction with few
- * output columns still uses the whole GPU), and every CTA writes its fp32 partial sums:
+ * Split-K for skinny activations: K is divided into `splits` ranges, each range of each tile (64
+ * columns for M <= 128, 256 above) goes to its own CTA, so that a deep reduction with few
+ * output columns still uses the whole GPU, and leaves its fp32 partial sums (the ranges, and so the
+ * bits of the planes, do not depend on M):
  *   out[s][m][n] = sum over the s-th K range of a[m,k] * w[n,k]       (no scales, no rounding)
  * The consumer (iflb200_residual_norm_quant_partials) adds the planes in split order, so the
  * result does not depend on timing.  K a multiple of 128; splits <= ceil(K / 512); `out` is

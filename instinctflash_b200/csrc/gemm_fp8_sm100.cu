@@ -732,6 +732,8 @@ __device__ __forceinline__ void epilogue_swapped(const GemmParams& p, const CUte
 // ones.  The 64-wide kernel of the skinny-M regime exists only in form 2, so that the launches of a
 // layer, split or not, run the same code: there a second GEMM kernel per layer cost about 1 us per
 // launch in instruction fetch (0.2 ms per pass of the M = 50 stack).
+// SPLIT 3: the planes form for more than 128 rows: (tile, K range) units on a persistent grid, each leaving
+// its fp32 partial sums in a plane; K is cut as in the skinny form, so the planes' bits are the same.
 // GATED: the gated form (see epilogue_gated): a tile pairs BN/2 gate columns with the BN/2 up
 // columns of the same hidden units; p.N counts hidden units.
 // EW: epilogue warps (8, or 16 for the gated form: EW / 4 per TMEM lane quadrant).
@@ -778,16 +780,30 @@ gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
   // Split-K: the S CTAs of a cluster work on the same tile, CTA r on K steps [kb0, kb1); one
   // tile per CTA (the host launches tiles x S CTAs, at most one wave).
   // Partials: K split over independent CTAs (no cluster), each writing its fp32 partial sums.
+  constexpr bool PLANES = SPLIT == 3;
   const bool partials = SPLIT == 2 && p.partials > 1;
   const bool split = !partials && (SPLIT == 1 || (SPLIT == 2 && p.split_k > 1));
-  const int k_parts = partials ? p.partials : (split ? p.split_k : 1);
+  const int k_parts = partials || PLANES ? p.partials : (split ? p.split_k : 1);
   const int split_rank = partials ? (int)blockIdx.x % k_parts : (split ? (int)cluster_ctarank() : 0);
-  const int tile_first = k_parts > 1 ? (int)blockIdx.x / k_parts : (int)blockIdx.x;
-  const int tile_stride = k_parts > 1 ? p.num_tiles : (int)gridDim.x;
-  // K ranges in whole stages (SL slabs each)
-  const int k_stages = (p.num_k + SL - 1) / SL;
-  const int kb0 = k_parts > 1 ? (int)(((int64_t)k_stages * split_rank) / k_parts) * SL : 0;
-  const int kb1 = k_parts > 1 ? min(p.num_k, (int)(((int64_t)k_stages * (split_rank + 1)) / k_parts) * SL) : p.num_k;
+  // a unit of work is a tile, or (tile, K range) in the planes form
+  const int tile_first = !PLANES && k_parts > 1 ? (int)blockIdx.x / k_parts : (int)blockIdx.x;
+  const int tile_stride = !PLANES && k_parts > 1 ? p.num_tiles : (int)gridDim.x;
+  const int units = PLANES ? p.num_tiles * k_parts : p.num_tiles;
+  auto tile_of = [&](int unit) { return PLANES ? unit / k_parts : unit; };
+  // K ranges in whole stages of the skinny form (SL slabs each; the planes form cuts K where that form does)
+  constexpr int kUnit = PLANES ? 4 : SL;
+  const int k_stages = (p.num_k + kUnit - 1) / kUnit;
+  auto range_begin = [&](int rank) { return k_parts > 1 ? (int)(((int64_t)k_stages * rank) / k_parts) * kUnit : 0; };
+  auto range_end = [&](int rank) {
+    return k_parts > 1 ? min(p.num_k, (int)(((int64_t)k_stages * (rank + 1)) / k_parts) * kUnit) : p.num_k;
+  };
+  int kb0 = range_begin(split_rank), kb1 = range_end(split_rank);
+  auto enter_unit = [&](int unit) {
+    if constexpr (PLANES) {
+      kb0 = range_begin(unit % k_parts);
+      kb1 = range_end(unit % k_parts);
+    }
+  };
 
   if (threadIdx.x == 0) {
     prefetch_tensormap(&tm_a);
@@ -831,9 +847,10 @@ gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
     Ring<STAGES> ring;
     bool ok = true;
     uint32_t it = 0;
-    for (int tile = tile_first; ok && tile < p.num_tiles; tile += tile_stride, ++it) {
+    for (int unit = tile_first; ok && unit < units; unit += tile_stride, ++it) {
       int m_blk, n_blk, grp;
-      tile_place(p, tile, m_blk, n_blk, grp);
+      tile_place(p, tile_of(unit), m_blk, n_blk, grp);
+      enter_unit(unit);
       const int a_row = grp * p.group_rows + m_blk * BM;  // rows past a block's end belong to the next block: loaded, never stored
       for (int kb = kb0; kb < kb1; kb += SL) {
         ok = wait_bounded(empty_bar(ring.stage), ring.phase ^ 1, abort_flag, (1u << 24) | (1u << 16) | (it & 0xFFFF));
@@ -877,7 +894,8 @@ gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
     uint32_t phase = 0;
     bool ok = true;
     uint32_t it = 0;
-    for (int tile = tile_first; ok && tile < p.num_tiles; tile += tile_stride, ++it) {
+    for (int unit = tile_first; ok && unit < units; unit += tile_stride, ++it) {
+      enter_unit(unit);
       const uint32_t acc = it & 1u;
       const uint32_t acc_phase = (it >> 1) & 1u;
       ok = wait_bounded(tempty_bar(acc), acc_phase ^ 1, abort_flag, (2u << 24) | (2u << 16) | (it & 0xFFFF));
@@ -933,9 +951,10 @@ gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
     bool ok = true;
     uint32_t it = 0;
     int swap_buf = 0;
-    for (int tile = tile_first; ok && tile < p.num_tiles; tile += tile_stride, ++it) {
+    for (int unit = tile_first; ok && unit < units; unit += tile_stride, ++it) {
       int m_blk, n_blk, grp;
-      tile_place(p, tile, m_blk, n_blk, grp);
+      tile_place(p, tile_of(unit), m_blk, n_blk, grp);
+      enter_unit(unit);
       const CUtensorMap* tm_dst = p.groups > 1 ? p.out_maps + grp : &tm_out;
       const uint32_t acc = it & 1u;
       const uint32_t acc_phase = (it >> 1) & 1u;
@@ -991,7 +1010,7 @@ gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
         const int col_tma_end = col_begin + (col_end - col_begin) / per_store * per_store;
         epilogue_tma_store<BN>(p, tm_dst, t_row, staging, staging_ptr, m_blk * BM + quad * 32, n_blk * BN,
                                col_begin, col_tma_end, rs, lane,
-                               (SPLIT == 2 && p.partials >= 1) ? split_rank : -1,  // a plane map takes a 3-D store
+                               PLANES ? unit % k_parts : ((SPLIT == 2 && p.partials >= 1) ? split_rank : -1),  // a plane map takes a 3-D store
                                prefetch ? &cv : nullptr);
         if (BN % 64 != 0 && col_tma_end < col_end) {
           const int n0 = n_blk * BN + col_tma_end;
@@ -1793,13 +1812,13 @@ static int make_partials_map(CUtensorMap* tm, void* ptr, int M, int N, int64_t l
 
 // Split-K over independent CTAs for skinny activations: out[s][m][n] = sum over the s-th K range of
 // a[m,k] * w[n,k], fp32, no scales, no rounding; the consumer sums the planes in order (and rounds
-// the sum to bf16, the raw accumulator's rounding point).  K a multiple of 128, M <= 128.
+// the sum to bf16, the raw accumulator's rounding point).  K a multiple of 128.
 static int run_gemm_partials(const void* a, int64_t ld_a, const void* w, int64_t ld_w, int M, int N, int K, int splits,
                              float* out, int64_t ld_out, void* stream) {
   if (M < 0 || N < 0 || K < 0 || splits < 1) return IFLB200_ERR_ARG;
   if (M == 0 || N == 0) return IFLB200_OK;
   if (!a || !w || !out) return IFLB200_ERR_ARG;
-  if (K < BK || K % BK || N % 16 || M > BM) return IFLB200_ERR_SHAPE;
+  if (K < BK || K % BK || N % 16) return IFLB200_ERR_SHAPE;
   const int num_k = K / BK;
   if (splits > (num_k + 3) / 4) return IFLB200_ERR_SHAPE;  // every split owns at least one stage of four slabs
   if (ld_a < K || ld_w < K || ld_out < N) return IFLB200_ERR_ARG;
@@ -1817,23 +1836,35 @@ static int run_gemm_partials(const void* a, int64_t ld_a, const void* w, int64_t
   p.split_k = 1;
   p.partials = splits;
   p.tma_store = 1;
-  p.num_m = 1;
-  p.num_n = (N + 63) / 64;
+  p.num_m = (M + BM - 1) / BM;
+  // more than 128 rows: 256-wide tiles (a (tile, range) unit per SM at 400 x 1024 x 4096 with eight ranges)
+  const int bn = M <= BM || N < 256 ? 64 : 256;
+  p.num_n = (N + bn - 1) / bn;
   p.num_k = num_k;
-  p.num_tiles = p.num_n;
-  p.group_m = 1;
+  p.num_tiles = p.num_m * p.num_n;
+  p.group_m = g_cfg_group_m > 0 ? g_cfg_group_m : 8;
   const int a_rows = activation_box_rows(M);
   p.a_bytes = a_rows * BK;
   CUtensorMap ta, tw, to;
-  st = make_slab_map(&ta, a, M, K, ld_a, a_rows, 4);
-  if (st != IFLB200_OK) return st;
-  st = make_slab_map(&tw, w, N, K, ld_w, 64, 4);
-  if (st != IFLB200_OK) return st;
   st = make_partials_map(&to, out, M, N, ld_out, splits);
   if (st != IFLB200_OK) return st;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  g_last_launch[0] = 1 + 16; g_last_launch[1] = 64; g_last_launch[2] = splits; g_last_launch[3] = 104;
-  return launch_gemm_form<64, 2, 2, false, false, kEpilogueWarps, 4>(ta, tw, to, p, p.num_tiles * splits, s);
+  if (M <= BM) {
+    st = make_slab_map(&ta, a, M, K, ld_a, a_rows, 4);
+    if (st != IFLB200_OK) return st;
+    st = make_slab_map(&tw, w, N, K, ld_w, 64, 4);
+    if (st != IFLB200_OK) return st;
+    g_last_launch[0] = 1 + 16; g_last_launch[1] = 64; g_last_launch[2] = splits; g_last_launch[3] = 104;
+    return launch_gemm_form<64, 2, 2, false, false, kEpilogueWarps, 4>(ta, tw, to, p, p.num_tiles * splits, s);
+  }
+  st = make_tensor_map(&ta, a, M, K, ld_a, a_rows);
+  if (st != IFLB200_OK) return st;
+  st = make_tensor_map(&tw, w, N, K, ld_w, bn);
+  if (st != IFLB200_OK) return st;
+  const int64_t units = (int64_t)p.num_tiles * splits;
+  const int grid = units < dev->sm_count ? (int)units : dev->sm_count;
+  g_last_launch[0] = 1 + 16; g_last_launch[1] = bn; g_last_launch[2] = splits; g_last_launch[3] = 0;
+  return bn == 64 ? launch_gemm_form<64, 8, 3>(ta, tw, to, p, grid, s) : launch_gemm_form<256, 4, 3>(ta, tw, to, p, grid, s);
 }
 
 // Row blocks to several destinations: a holds `groups` blocks of `group_rows` rows; block g's

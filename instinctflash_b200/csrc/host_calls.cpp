@@ -263,7 +263,7 @@ PyObject* gemm_partials(PyObject*, Args v, Py_ssize_t nargs) {  // a, w, out [S,
   Call c;
   const Mat a = c.mat(v[0], kCodes), w = c.mat(v[1], kCodes);
   const at::Tensor* o = c.tensor(v[2]);
-  if (!o || !c.ready() || !gemm_shapes(a, w) || a.rows > 128 || a.cols % 128 || o->scalar_type() != ScalarType::Float ||
+  if (!o || !c.ready() || !gemm_shapes(a, w) || a.cols % 128 || o->scalar_type() != ScalarType::Float ||
       o->dim() != 3 || o->size(1) != a.rows || o->size(2) != w.rows || !o->is_contiguous() || o->size(0) > 1024)
     Py_RETURN_FALSE;
   float* out = static_cast<float*>(o->data_ptr());

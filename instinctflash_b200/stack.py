@@ -156,7 +156,10 @@ class LinearStack:
     """Static buffers + the per-layer call sequence.  ``ops`` supplies the operators."""
 
     def __init__(self, spec: StackSpec, weights, device, ops=None, *, fused="auto", fuse_residual: bool = False,
-                 split_partials: bool = True):
+                 split_partials: bool = True, split_rows: int | None = None):
+        # split_rows: cut K for the partial-sum projections as for that many rows (a batch of episodes keeps the
+        # bits of one episode's stack); by default for this stack's own
+        split_rows = spec.M if split_rows is None else split_rows
         self.spec, self.weights, self.dev = spec, weights, torch.device(device)
         self.ops = ops or native_ops()
         # fused forms exist only in this package's operator set; "auto" takes the gated epilogue where the
@@ -168,7 +171,7 @@ class LinearStack:
         self.fuse_residual = fuse_residual and hasattr(self.ops, "fp8_linear_residual")
         # skinny activations: deep, narrow projections (down, o) run split-K over independent CTAs, the
         # residual kernel adds the fp32 partial sums (this package's operators only)
-        self.split_partials = (split_partials and spec.kind == "gemma" and spec.M <= 128 and
+        self.split_partials = (split_partials and spec.kind == "gemma" and split_rows <= 128 and
                                hasattr(self.ops, "gemm_partials"))
         M, D, F = spec.M, spec.hidden, spec.ffn
         dev, bf16, f32 = self.dev, torch.bfloat16, torch.float32
@@ -186,7 +189,7 @@ class LinearStack:
         if self.split_partials:
             sms = torch.cuda.get_device_properties(dev).multi_processor_count
             ks = [k for name, n, k in spec.linears() if n == D and name in ("o", "down")]
-            self.splits = {k: self.ops.partial_splits(M, D, k, sms) for k in ks}
+            self.splits = {k: self.ops.partial_splits(split_rows, D, k, sms) for k in ks}
             self.part = torch.zeros(max(self.splits.values(), default=1) * M * D, dtype=f32, device=dev)
         self.attn = None
         self.launches_per_forward = 0
@@ -340,33 +343,89 @@ class HostPipeline:
         main.wait_stream(self.d2h)
 
 
-class EpisodeBatch:
-    """``episodes`` independent inferences of one stack on one GPU: one ``LinearStack`` each (own
-    activations, residual stream and scales) over shared weights, captured as parallel branches
-    of ONE CUDA graph, so that the GPU always has several short dependent chains to pick kernels
-    from.  Every GEMM keeps the row count of a single episode.  Independent robot episodes are what
-    the skinny action-expert configuration shards over GPUs; this is the per-GPU part."""
+class _Episode(LinearStack):
+    """One episode of a batch that runs stacked along the rows: the same interface as a stack of its
+    own, over its rows of the batch's buffers."""
 
-    def __init__(self, spec: StackSpec, weights, device, episodes: int, **stack_kw):
-        self.spec, self.dev = spec, torch.device(device)
-        self.stacks = [LinearStack(spec, weights, device, **stack_kw) for _ in range(episodes)]
-        self.streams = [torch.cuda.Stream(self.dev) for _ in range(episodes)]
+    def __init__(self, batch: LinearStack, index: int, spec: StackSpec):
+        self.batch, self.spec, self.weights, self.dev, self.ops = batch, spec, batch.weights, batch.dev, batch.ops
+        self.fused, self.fuse_residual, self.split_partials = batch.fused, batch.fuse_residual, batch.split_partials
+        self.rows = slice(index * spec.M, (index + 1) * spec.M)
+        self.res = batch.res[self.rows]
+        self.scale = [t[self.rows] for t in batch.scale]
+        if hasattr(batch, "h"):
+            self.h, self.amax = batch.h[self.rows], batch.amax[:, self.rows]
+        if self.split_partials:
+            self.splits, self.part = batch.splits, batch.part   # scratch: this episode's planes from its start
+        self.attn = None
         self.launches_per_forward = 0
 
+    def _q8(self, cols):
+        return self.batch._q8(cols)[self.rows]
+
+    def _raw(self, cols):
+        return self.batch._raw(cols)[self.rows]
+
+
+class EpisodeBatch:
+    """``episodes`` independent inferences of one stack on one GPU over shared weights.  Independent robot
+    episodes are what the skinny action-expert configuration shards over GPUs; this is the per-GPU part.
+
+    Skinny decoder stacks (at most 128 rows an episode) run stacked along the rows: one launch per operator
+    for all episodes.  Every operator works row by row and the K ranges stay those of one episode, so
+    each episode has the bits of a stack of its own.  As parallel branches of one graph the GPU's
+    front end could not feed the branches -- 8 episodes of 50 rows, 18 layers: 864 kernels at 1.7 us each,
+    1498 us, against 108 kernels of 400 rows.  Other stacks, whose kernels fill the GPU by themselves,
+    are captured as parallel branches: one ``LinearStack`` each."""
+
+    def __init__(self, spec: StackSpec, weights, device, episodes: int, **stack_kw):
+        self.spec, self.dev, self.episodes = spec, torch.device(device), episodes
+        self.launches_per_forward = 0   # of all episodes: a launch counts once for every episode it serves
+        self.merged = None
+        if spec.kind == "gemma" and spec.M <= 128 and episodes > 1:
+            wide = StackSpec(**{**spec.__dict__, "M": spec.M * episodes})
+            merged = LinearStack(wide, weights, device, split_rows=spec.M, **stack_kw)
+            if hasattr(merged.ops, "gemm_partials"):    # this package's operators: K ranges by rows of one episode
+                self.merged = merged
+                self.attn_rows = torch.zeros(wide.M, max(spec.o_in, 16), dtype=torch.bfloat16, device=self.dev)
+                self.stacks = [_Episode(merged, i, spec) for i in range(episodes)]
+                return
+        self.stacks = [LinearStack(spec, weights, device, **stack_kw) for _ in range(episodes)]
+        self.streams = [torch.cuda.Stream(self.dev) for _ in range(episodes)]
+
     def load(self, x, attn):
+        """``x``: one input for all episodes, or one each; ``attn``: the attention output of all of them."""
         xs = x if isinstance(x, (list, tuple)) else [x] * len(self.stacks)
-        for st, xi in zip(self.stacks, xs):
-            st.load(xi, attn)
+        if self.merged is None:
+            for st, xi in zip(self.stacks, xs):
+                st.load(xi, attn)
+            return
+        torch._foreach_copy_([st.res for st in self.stacks], list(xs))
+        for st in self.stacks:
+            st.attn = attn
+        self.attn = attn
+        o, m = self.merged.ops, self.merged
+        o.residual_norm_quant(m.res, layernorm=False, q=m._q8(self.spec.hidden), q_scale=m.scale[0])
 
     def forward(self):
-        """Fork every episode onto its own stream, join on the current one."""
-        main = torch.cuda.current_stream(self.dev)
-        for st, side in zip(self.stacks, self.streams):
-            side.wait_stream(main)
-            with torch.cuda.stream(side):
-                st.forward()
-        for side in self.streams:
-            main.wait_stream(side)
+        """Every episode's pass (branches are forked onto their own streams and joined on the current one)."""
+        if self.merged is not None:
+            if self.spec.o_in:
+                if self.attn.dtype != self.attn_rows.dtype:
+                    self.attn_rows = self.attn_rows.to(self.attn.dtype)
+                self.attn_rows.view(self.episodes, self.spec.M, -1).copy_(self.attn)
+            self.merged.attn = self.attn_rows
+            self.merged.forward()
+            for st in self.stacks:
+                st.launches_per_forward = self.merged.launches_per_forward
+        else:
+            main = torch.cuda.current_stream(self.dev)
+            for st, side in zip(self.stacks, self.streams):
+                side.wait_stream(main)
+                with torch.cuda.stream(side):
+                    st.forward()
+            for side in self.streams:
+                main.wait_stream(side)
         self.launches_per_forward = sum(st.launches_per_forward for st in self.stacks)
         return [st.res for st in self.stacks]
 
