@@ -724,6 +724,13 @@ residual_norm_quant_kernel(const ResNormArgs a) {
 constexpr int kPackThreads = 256;
 constexpr int kPackMaxCtas = 1024;
 
+__device__ __forceinline__ uint32_t max_bf16_bits(const uint4& u, uint32_t best) {
+  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+  for (int k = 0; k < 4; ++k) best = max(best, max(w[k] & 0x7FFFu, (w[k] >> 16) & 0x7FFFu));
+  return best;
+}
+
 // Maximum of |x| as an integer maximum of the bf16 magnitude bits: finite values order like
 // their bits, and every NaN pattern is larger than infinity, so NaN propagates.
 __global__ void __launch_bounds__(kPackThreads)
@@ -737,14 +744,13 @@ amax_partial_kernel(const uint16_t* __restrict__ x, int64_t n, uint32_t* __restr
   const int64_t stride = (int64_t)gridDim.x * kPackThreads;
   if (vec) {
     const uint4* xv = reinterpret_cast<const uint4*>(x);
-    for (int64_t i = (int64_t)blockIdx.x * kPackThreads + threadIdx.x; i < nvec; i += stride) {
-      const uint4 u = xv[i];
-      const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+    // four loads in flight per thread (one at a time left a 4680 x 3072 tensor at 2.3 TB/s)
+    for (int64_t i0 = (int64_t)blockIdx.x * kPackThreads + threadIdx.x; i0 < nvec; i0 += 4 * stride) {
+      uint4 u[4];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        best = max(best, w[k] & 0x7FFFu);
-        best = max(best, (w[k] >> 16) & 0x7FFFu);
-      }
+      for (int k = 0; k < 4; ++k) u[k] = i0 + k * stride < nvec ? xv[i0 + k * stride] : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) best = max_bf16_bits(u[k], best);
     }
     for (int64_t i = nvec * 8 + (int64_t)blockIdx.x * kPackThreads + threadIdx.x; i < n; i += stride)
       best = max(best, (uint32_t)x[i] & 0x7FFFu);
@@ -762,9 +768,43 @@ amax_partial_kernel(const uint16_t* __restrict__ x, int64_t n, uint32_t* __restr
   }
 }
 
+__device__ __forceinline__ float scale_of_bits(uint32_t best) {  // the maximum's magnitude bits -> max(amax, 1e-12) / 448
+  if (best > 0x7F80u) return __uint_as_float(0x7FC00000u);
+  return __fmul_rn(fmaxf(__uint_as_float(best << 16), 1e-12f), (float)(1.0 / 448.0));
+}
+
 __device__ __forceinline__ float pack_one(float x, float scale) {
   const float d = __fdiv_rn(x, scale);
   return (d != d) ? d : fminf(fmaxf(d, -448.0f), 448.0f);
+}
+
+// Eight codes of x / scale.  The quotient is the correctly rounded one by Markstein's correction (P. Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor", 1990): with r = 1 / scale
+// correctly rounded and q = x r, the remainder x - q scale is exact in one fma and q + r (x - q scale)
+// rounds to the quotient, in three packed instructions per pair instead of a division each.  Where the
+// remainder underflows, the code is zero either way; a scale that is not finite takes the division
+// (`r` is then NaN).  The conversion saturates, which is the clamp to +-448.  Compared on the GPU for every
+// bf16 maximum and every bf16 x: no code differs.
+__device__ __forceinline__ uint2 pack_eight(const uint4& u, float scale, float r) {
+  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+  float f[8];
+  const bool fast = r == r;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const float lo = __uint_as_float(w[k] << 16), hi = __uint_as_float(w[k] & 0xFFFF0000u);
+    if (fast) {  // of -x: a zero keeps its sign that way, the codes' signs are turned back below
+      const uint64_t x2 = pack2(lo, hi), n2 = pack2(-r, -r), q = mul2(x2, n2);
+      unpack2(fma2(fma2(q, pack2(scale, scale), x2), n2, q), f[2 * k], f[2 * k + 1]);
+    } else {
+      f[2 * k] = pack_one(lo, scale);
+      f[2 * k + 1] = pack_one(hi, scale);
+    }
+  }
+  const uint32_t turn = fast ? 0x80808080u : 0u;
+  return make_uint2(cvt_e4m3x4(f[0], f[1], f[2], f[3]) ^ turn, cvt_e4m3x4(f[4], f[5], f[6], f[7]) ^ turn);
+}
+__device__ __forceinline__ float reciprocal_for_pack(float scale) {
+  return scale > 1e-20f && scale < 1e37f ? __frcp_rn(scale) : __uint_as_float(0x7FC00000u);
 }
 
 // n_partial > 0: dynamic scale from the partial maxima (every CTA recomputes it; CTA 0 writes
@@ -786,13 +826,7 @@ pack_kernel(const uint16_t* __restrict__ x, int64_t n, const uint32_t* __restric
     __syncthreads();
     if (threadIdx.x == 0) {
       for (int i = 1; i < kPackThreads / 32; ++i) best = max(best, red[i]);
-      float sc;
-      if (best > 0x7F80u) {
-        sc = __uint_as_float(0x7FC00000u);
-      } else {
-        const float amax = __uint_as_float(best << 16);
-        sc = __fmul_rn(fmaxf(amax, 1e-12f), (float)(1.0 / 448.0));
-      }
+      const float sc = scale_of_bits(best);
       s_scale = sc;
       if (blockIdx.x == 0) *scale_out = sc;
     }
@@ -806,20 +840,67 @@ pack_kernel(const uint16_t* __restrict__ x, int64_t n, const uint32_t* __restric
   const int64_t stride = (int64_t)gridDim.x * kPackThreads;
   const int64_t nvec = vec ? n / 8 : 0;
   const uint4* xv = reinterpret_cast<const uint4*>(x);
-  for (int64_t i = (int64_t)blockIdx.x * kPackThreads + threadIdx.x; i < nvec; i += stride) {
-    const uint4 u = xv[i];
-    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-    float f[8];
+  // with a caller's own scale the row may hold NaN or a quotient out of range: by division
+  const float r = n_partial > 0 ? reciprocal_for_pack(scale) : __uint_as_float(0x7FC00000u);
+  for (int64_t i0 = (int64_t)blockIdx.x * kPackThreads + threadIdx.x; i0 < nvec; i0 += 4 * stride) {
+    uint4 u[4];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      f[2 * k] = pack_one(__uint_as_float(w[k] << 16), scale);
-      f[2 * k + 1] = pack_one(__uint_as_float(w[k] & 0xFFFF0000u), scale);
-    }
-    reinterpret_cast<uint2*>(q)[i] =
-        make_uint2(cvt_e4m3x4(f[0], f[1], f[2], f[3]), cvt_e4m3x4(f[4], f[5], f[6], f[7]));
+    for (int k = 0; k < 4; ++k) u[k] = i0 + k * stride < nvec ? xv[i0 + k * stride] : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (i0 + k * stride < nvec) reinterpret_cast<uint2*>(q)[i0 + k * stride] = pack_eight(u[k], scale, r);
   }
   for (int64_t i = nvec * 8 + (int64_t)blockIdx.x * kPackThreads + threadIdx.x; i < n; i += stride)
     q[i] = (uint8_t)(cvt_e4m3x2(pack_one(__uint_as_float((uint32_t)x[i] << 16), scale), 0.0f) & 0xFF);
+}
+
+// Small tensors: the whole dynamic pack in one launch.  A cluster of eight CTAs keeps the tensor in
+// registers between the maximum and the cast; the maxima of the CTAs meet in distributed shared memory.
+// The two kernels above are two launches and two passes for a few microseconds of work: 50 x 1024
+// inputs took 5 us of a 10 us projection.  Up to 2^17 elements; above, eight SMs are
+// slower than two passes of the whole GPU.
+constexpr int kPackCluster = 8, kPackClusterThreads = 1024;
+constexpr int64_t kPackClusterMax = (int64_t)kPackCluster * kPackClusterThreads * 8 * 2;
+
+template <int V>
+__global__ void __cluster_dims__(kPackCluster, 1, 1) __launch_bounds__(kPackClusterThreads)
+pack_cluster_kernel(const uint4* __restrict__ x, int nvec, float* __restrict__ scale_out, uint2* __restrict__ q) {
+  __shared__ uint32_t red[kPackClusterThreads / 32];
+  __shared__ uint32_t maxima[kPackCluster];
+  const int rank = (int)cluster_ctarank();
+  grid_dependency_wait();  // x may come from the kernel before this one in the stream
+  grid_launch_dependents();
+  uint4 u[V];
+  uint32_t best = 0;
+#pragma unroll
+  for (int v = 0; v < V; ++v) {
+    const int i = (v * kPackCluster + rank) * kPackClusterThreads + threadIdx.x;
+    u[v] = i < nvec ? x[i] : make_uint4(0u, 0u, 0u, 0u);
+  }
+#pragma unroll
+  for (int v = 0; v < V; ++v) best = max_bf16_bits(u[v], best);
+  best = __reduce_max_sync(0xFFFFFFFFu, best);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = best;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    best = __reduce_max_sync(0xFFFFFFFFu, red[threadIdx.x]);
+    if (threadIdx.x < kPackCluster) {
+      uint32_t peer;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(smem_u32(&maxima[rank])), "r"(threadIdx.x));
+      asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(peer), "r"(best) : "memory");
+    }
+  }
+  cluster_sync_all();
+  best = maxima[0];
+#pragma unroll
+  for (int k = 1; k < kPackCluster; ++k) best = max(best, maxima[k]);
+  const float scale = scale_of_bits(best), r = reciprocal_for_pack(scale);
+  if (rank == 0 && threadIdx.x == 0) *scale_out = scale;
+#pragma unroll
+  for (int v = 0; v < V; ++v) {
+    const int i = (v * kPackCluster + rank) * kPackClusterThreads + threadIdx.x;
+    if (i < nvec) q[i] = pack_eight(u[v], scale, r);
+  }
 }
 
 #endif  // pack kernels
@@ -1295,6 +1376,18 @@ static int pack_grid(int64_t n) {
   return (int)ctas;
 }
 
+// The one-launch form where it applies.
+static bool launch_pack_cluster(const void* x, int64_t n, void* q, float* scale, cudaStream_t s) {
+  if (n > kPackClusterMax || n % 8 || !aligned16(x) || !aligned8(q)) return false;
+  const int nvec = (int)(n / 8);
+  const dim3 grid(kPackCluster), block(kPackClusterThreads);
+  auto xv = reinterpret_cast<const uint4*>(x);
+  auto qv = reinterpret_cast<uint2*>(q);
+  if (nvec <= kPackCluster * kPackClusterThreads) launch_dep(pack_cluster_kernel<1>, grid, block, 0, s, 1, dependent_launch_for(1), xv, nvec, scale, qv);
+  else launch_dep(pack_cluster_kernel<2>, grid, block, 0, s, 1, dependent_launch_for(1), xv, nvec, scale, qv);
+  return true;
+}
+
 extern "C" size_t iflb200_pack_workspace_bytes(int64_t n) {
   return (size_t)pack_grid(n < 0 ? 0 : n) * sizeof(uint32_t);
 }
@@ -1308,6 +1401,7 @@ extern "C" int iflb200_dynamic_pack_bf16_e4m3(const void* x, int64_t n, void* q,
     return IFLB200_ERR_ALIGN;
   const int grid = pack_grid(n);
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  if (launch_pack_cluster(x, n, q, scale, s)) return (int)cudaGetLastError();
   uint32_t* partial = reinterpret_cast<uint32_t*>(workspace);
   launch_dep(amax_partial_kernel, dim3(grid), dim3(kPackThreads), 0, s, 1, dependent_launch_for(n >> 12), reinterpret_cast<const uint16_t*>(x), n, partial);
   launch_dep(pack_kernel, dim3(grid), dim3(kPackThreads), 0, s, 1, dependent_launch_for(n >> 12), reinterpret_cast<const uint16_t*>(x), n, partial, grid,
