@@ -549,10 +549,8 @@ __device__ __forceinline__ float round_through<__nv_bfloat16>(float x) {
   return __bfloat162float(__float2bfloat16_rn(x));
 }
 
-// PART: the delta arrives as fp32 partial sums of a K-split GEMM (a.dpart) instead of a raw bf16
-// accumulator; a separate instantiation so that the ordinary one keeps its registers.
-template <typename RT, int TPR, int IT, bool FAST, bool PART = false>
-__global__ void __launch_bounds__(kRowThreads, PART ? 2 : resnorm_min_blocks<IT>())
+template <typename RT, int TPR, int IT, bool FAST>
+__global__ void __launch_bounds__(kRowThreads, resnorm_min_blocks<IT>())
 residual_norm_quant_kernel(const ResNormArgs a) {
   row_dependency_wait();  // inputs may come from the kernel before this one in the stream
   row_trigger();
@@ -562,8 +560,6 @@ residual_norm_quant_kernel(const ResNormArgs a) {
   const bool live = m < a.M;
   RT* rr = reinterpret_cast<RT*>(a.res) + (live ? (int64_t)m * a.ld_res : 0);
   const __nv_bfloat16* dr = a.delta ? a.delta + (live ? (int64_t)m * a.ld_delta : 0) : nullptr;
-  const float* dp = PART ? a.dpart + (live ? (int64_t)m * a.ld_delta : 0) : nullptr;
-  const int64_t dp_plane = (int64_t)a.M * a.ld_delta;
   const int64_t mofs = (live && a.mod_index) ? (int64_t)a.mod_index[m] * a.D : 0;
   const float drs = (live && a.drow) ? a.drow[m] : 1.0f;
   const float fD = (float)a.D;
@@ -575,7 +571,7 @@ residual_norm_quant_kernel(const ResNormArgs a) {
     const int c0 = (it * TPR + t) * 8;
     const bool on = it < a.iters && live && c0 < a.D;
     rres[it] = fetch<FAST, RT>(rr, c0, a.D, on);
-    rdel[it] = fetch<FAST, __nv_bfloat16>(dr, c0, a.D, on && dr != nullptr && !PART);
+    rdel[it] = fetch<FAST, __nv_bfloat16>(dr, c0, a.D, on && dr != nullptr);
   }
   float x[IT][8];
   float sum = 0.0f, sumsq = 0.0f;
@@ -584,33 +580,9 @@ residual_norm_quant_kernel(const ResNormArgs a) {
     const int c0 = (it * TPR + t) * 8;
     unpack(rres[it], x[it]);
     if (it < a.iters && live && c0 < a.D) {
-      if (dr || PART) {
+      if (dr) {
         float d[8], cs[8], bs[8], gs[8];
-        if constexpr (PART) {
-          // kGroup planes in flight together (all eight for rows of one chunk per thread: the skinny
-          // expert shapes, where a second dependent round trip is a tenth of the kernel), added in split order
-          constexpr int kGroup = IT == 1 ? 8 : 4;
-#pragma unroll
-          for (int i = 0; i < 8; ++i) d[i] = 0.0f;
-#pragma unroll 1
-          for (int s0 = 0; s0 < a.dsplits; s0 += kGroup) {
-            float e[kGroup][8];
-#pragma unroll
-            for (int sp = 0; sp < kGroup; ++sp)
-              if (s0 + sp < a.dsplits) load_f32<FAST>(dp + (s0 + sp) * dp_plane, c0, a.D, e[sp]);
-#pragma unroll
-            for (int sp = 0; sp < kGroup; ++sp) {
-              if (s0 + sp < a.dsplits) {
-#pragma unroll
-                for (int i = 0; i < 8; ++i) d[i] = (s0 + sp == 0) ? e[sp][i] : __fadd_rn(d[i], e[sp][i]);
-              }
-            }
-          }
-#pragma unroll
-          for (int i = 0; i < 8; ++i) d[i] = __bfloat162float(__float2bfloat16_rn(d[i]));
-        } else {
-          unpack(rdel[it], d);
-        }
+        unpack(rdel[it], d);
         if (a.dcol) load_f32<FAST>(a.dcol, c0, a.D, cs);
         if (a.bias) load_f32<FAST>(a.bias, c0, a.D, bs);
         if (a.gate) load_f32<FAST>(a.gate + mofs, c0, a.D, gs);
@@ -701,21 +673,263 @@ residual_norm_quant_kernel(const ResNormArgs a) {
     const int c0 = (it * TPR + t) * 8;
     if (it < a.iters && c0 < a.D) store_codes<FAST>(qr, c0, a.D, x[it], inv);
   }
-  if constexpr (PART) {
+}
+
+#if IFLB200_ROW_PART == 2 || IFLB200_ROW_PART == -1
+// --------------------------------------------------------------------------------------------
+// residual_norm_quant for a delta that arrives as fp32 planes of a K-split GEMM (p of them: 4 p bytes per
+// element where the bf16 accumulator has 2), one CTA per row.
+//
+// Bound by latency and by how many rows are in flight at once: a thread owns IT quads of columns 1024
+// apart, so that every access of a warp is 512 contiguous bytes, all loads of the row -- residual,
+// PL planes, column scales -- are issued before the first use, and the registers are held down
+// so that a few hundred rows are resident together.  Eight columns a thread, chunk after chunk and plane
+// group after plane group before: 50 x 1024 with eight planes 2.9 -> 2.3 us, 816 x 2048 with two 7.6 -> 5.6.
+// PL: planes loaded together (further ones follow in groups of PL).
+// --------------------------------------------------------------------------------------------
+template <typename T>
+struct Quad;
+template <>
+struct Quad<float> {
+  float4 u;
+  __device__ __forceinline__ void load(const float* p) { u = *reinterpret_cast<const float4*>(p); }
+  __device__ __forceinline__ void widen(float (&o)[4]) const { o[0] = u.x; o[1] = u.y; o[2] = u.z; o[3] = u.w; }
+};
+template <>
+struct Quad<__nv_bfloat16> {
+  uint2 u;
+  __device__ __forceinline__ void load(const __nv_bfloat16* p) { u = *reinterpret_cast<const uint2*>(p); }
+  __device__ __forceinline__ void widen(float (&o)[4]) const {
+    o[0] = __uint_as_float(u.x << 16); o[1] = __uint_as_float(u.x & 0xFFFF0000u);
+    o[2] = __uint_as_float(u.y << 16); o[3] = __uint_as_float(u.y & 0xFFFF0000u);
+  }
+};
+__device__ __forceinline__ void load_quad(const float* p, float (&o)[4]) {
+  Quad<float> q;
+  q.load(p);
+  q.widen(o);
+}
+__device__ __forceinline__ void store_quad(void* base, int dtype, int64_t off, const float (&v)[4]) {
+  if (dtype == IFLB200_F32) {
+    *reinterpret_cast<float4*>(reinterpret_cast<float*>(base) + off) = make_float4(v[0], v[1], v[2], v[3]);
+    return;
+  }
+  uint32_t w[2];
 #pragma unroll
-    for (int k = 0; k < kMaxMirrors; ++k) {
-      if (k < a.mirrors) {
-        if (t == 0) a.qs_mirror[k][m] = scale;
-        uint8_t* qm = a.q_mirror[k] + (int64_t)m * a.ld_q;
+  for (int i = 0; i < 2; ++i)
+    w[i] = dtype == IFLB200_BF16 ? (f32_to_bf16_bits(v[2 * i]) | (f32_to_bf16_bits(v[2 * i + 1]) << 16))
+                                 : (f32_to_f16_bits(v[2 * i]) | (f32_to_f16_bits(v[2 * i + 1]) << 16));
+  *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(base) + off) = make_uint2(w[0], w[1]);
+}
+
+// Sum or maximum of magnitudes over the CTA; `slots` is used once per row.
+template <bool IS_MAX>
+__device__ __forceinline__ float row_cta_reduce(float v, float* slots) {
+  if (IS_MAX) {
+    v = warp_max_abs_f32(v);
+  } else {
 #pragma unroll
-        for (int it = 0; it < IT; ++it) {
-          const int c0 = (it * TPR + t) * 8;
-          if (it < a.iters && c0 < a.D) store_codes<FAST>(qm, c0, a.D, x[it], inv);
+    for (int o = 16; o > 0; o >>= 1) v = __fadd_rn(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
+  }
+  if ((threadIdx.x & 31) == 0) slots[threadIdx.x >> 5] = v;
+  __syncthreads();
+  const float4 a = reinterpret_cast<const float4*>(slots)[0], b = reinterpret_cast<const float4*>(slots)[1];
+  if (IS_MAX) return max_f32(max_f32(max_f32(a.x, a.y), max_f32(a.z, a.w)), max_f32(max_f32(b.x, b.y), max_f32(b.z, b.w)));
+  return __fadd_rn(__fadd_rn(__fadd_rn(a.x, a.y), __fadd_rn(a.z, a.w)), __fadd_rn(__fadd_rn(b.x, b.y), __fadd_rn(b.z, b.w)));
+}
+
+// Resident CTAs per SM that the registers have to leave room for: about 4 * IT * (PL + 4) live values and the
+// addresses.
+template <int IT, int PL>
+__host__ __device__ constexpr int row_cta_min_blocks() {
+  return IT * (PL + 4) <= 12 ? 4 : (IT * (PL + 4) <= 18 ? 3 : 2);
+}
+
+template <typename RT, int IT, int PL>
+__global__ void __launch_bounds__(kRowThreads, row_cta_min_blocks<IT, PL>())
+residual_norm_planes_kernel(const ResNormArgs a) {
+  static_assert(kRowThreads == 256, "eight warps per row");
+  __shared__ __align__(16) float red[3][kRowThreads / 32];
+  constexpr int kStep = kRowThreads * 4;
+  const int m = blockIdx.x, c = threadIdx.x * 4;
+  row_dependency_wait();  // inputs may come from the kernel before this one in the stream
+  row_trigger();
+  RT* rr = reinterpret_cast<RT*>(a.res) + (int64_t)m * a.ld_res + c;
+  const int64_t mofs = a.mod_index ? (int64_t)a.mod_index[m] * a.D + c : c;
+  const float drs = a.drow ? a.drow[m] : 1.0f;
+
+  Quad<RT> rres[IT];
+  Quad<float> plane[PL][IT], dcol[IT];
+  const float* dp = a.dpart + (int64_t)m * a.ld_delta + c;
+  const int64_t dp_plane = (int64_t)a.M * a.ld_delta;
+#pragma unroll
+  for (int it = 0; it < IT; ++it) {
+    if (it * kStep + c < a.D) {
+      rres[it].load(rr + it * kStep);
+      if (a.dcol) dcol[it].load(a.dcol + c + it * kStep);
+    }
+#pragma unroll
+    for (int s = 0; s < PL; ++s)
+      if (s < a.dsplits && it * kStep + c < a.D) plane[s][it].load(dp + s * dp_plane + it * kStep);
+  }
+  float x[IT][4];
+  float sum = 0.0f;
+#pragma unroll
+  for (int it = 0; it < IT; ++it) {
+    const int o = it * kStep;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) x[it][i] = 0.0f;
+    if (o + c < a.D) {
+      rres[it].widen(x[it]);
+      float d[4], op[4];
+      plane[0][it].widen(d);  // the planes in split order, then the raw accumulator's rounding point
+#pragma unroll
+      for (int s = 1; s < PL; ++s) {
+        if (s < a.dsplits) {
+          float e[4];
+          plane[s][it].widen(e);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) d[i] = __fadd_rn(d[i], e[i]);
+        }
+      }
+      if (PL < 8) {
+#pragma unroll 1
+        for (int s0 = PL; s0 < a.dsplits; s0 += PL) {
+          float e[PL][4];
+#pragma unroll
+          for (int s = 0; s < PL; ++s)
+            if (s0 + s < a.dsplits) load_quad(dp + (s0 + s) * dp_plane + o, e[s]);
+#pragma unroll
+          for (int s = 0; s < PL; ++s) {
+            if (s0 + s < a.dsplits) {
+#pragma unroll
+              for (int i = 0; i < 4; ++i) d[i] = __fadd_rn(d[i], e[s][i]);
+            }
+          }
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) d[i] = __bfloat162float(__float2bfloat16_rn(d[i]));
+      ChainV<4> ch(d);
+      if (a.drow) ch.mul(drs);
+      if (a.dcol) {
+        dcol[it].widen(op);
+        ch.mul(op);
+      }
+      if (a.bias) {
+        load_quad(a.bias + c + o, op);
+        ch.add(op);
+      }
+      if (a.gate) {
+        load_quad(a.gate + mofs + o, op);
+        ch.mul(op);
+      }
+      ch.add(x[it]);  // x + d, contracted with d's last multiply when there is one
+      ch.done(x[it]);
+      if (a.write_res) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x[it][i] = round_through<RT>(x[it][i]);
+        store_quad(a.res, dtype_of<RT>(), (int64_t)m * a.ld_res + c + o, x[it]);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) sum = a.layernorm ? __fadd_rn(sum, x[it][i]) : __fmaf_rn(x[it][i], x[it][i], sum);
+    }
+  }
+  if (a.q == nullptr && a.y == nullptr) return;  // residual update only (uniform across the CTA)
+
+  const float fD = (float)a.D;
+  sum = row_cta_reduce<false>(sum, red[0]);
+  if (a.layernorm) {
+    const float mean = div_full(sum, fD);
+    sum = 0.0f;
+#pragma unroll
+    for (int it = 0; it < IT; ++it) {
+      if (it * kStep + c < a.D) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          x[it][i] = __fadd_rn(x[it][i], -mean);
+          sum = __fmaf_rn(x[it][i], x[it][i], sum);
         }
       }
     }
+    sum = row_cta_reduce<false>(sum, red[1]);
+  }
+  const float rstd = rsqrt_approx_ftz(__fadd_rn(div_full(sum, fD), a.eps));
+  float amax = 0.0f;
+#pragma unroll
+  for (int it = 0; it < IT; ++it) {
+    const int o = it * kStep;
+    if (o + c < a.D) {
+      float op[4];
+      ChainV<4> ch(x[it]);
+      ch.mul(rstd);
+      if (a.weight) {
+        load_quad(a.weight + c + o, op);
+        ch.mul(op);
+      }
+      if (a.beta) {
+        load_quad(a.beta + c + o, op);
+        ch.add(op);
+      }
+      if (a.mod_scale) {
+        load_quad(a.mod_scale + mofs + o, op);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) op[i] = __fadd_rn(op[i], 1.0f);
+        ch.mul(op);
+        load_quad(a.mod_shift + mofs + o, op);
+        ch.add(op);
+      }
+      ch.done(x[it]);
+      amax = max_abs_f32(max_abs_f32(amax, x[it][0], x[it][1]), x[it][2], x[it][3]);
+      if (a.y) store_quad(a.y, a.y_dtype, (int64_t)m * a.ld_y + c + o, x[it]);
+    }
+  }
+  if (a.q == nullptr) return;
+  amax = row_cta_reduce<true>(amax, red[2]);
+  float scale, inv;
+  quant_scales(amax, scale, inv);
+  if (threadIdx.x == 0) a.qs[m] = scale;
+  uint8_t* q = a.q + (int64_t)m * a.ld_q + c;
+#pragma unroll
+  for (int it = 0; it < IT; ++it) {
+    if (it * kStep + c < a.D) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) x[it][i] = __fmul_rn(x[it][i], inv);
+      const uint32_t code = cvt_e4m3x4(x[it][0], x[it][1], x[it][2], x[it][3]);
+      *reinterpret_cast<uint32_t*>(q + it * kStep) = code;
+#pragma unroll
+      for (int k = 0; k < kMaxMirrors; ++k)
+        if (k < a.mirrors) *reinterpret_cast<uint32_t*>(a.q_mirror[k] + (int64_t)m * a.ld_q + c + it * kStep) = code;
+    }
+  }
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int k = 0; k < kMaxMirrors; ++k)
+      if (k < a.mirrors) a.qs_mirror[k][m] = scale;
   }
 }
+
+// Rows of at most 8192 columns on the aligned path; planes in groups that fit the registers.
+template <typename RT, int IT, int PL>
+static void launch_resnorm_planes_form(const ResNormArgs& a, cudaStream_t s) {
+  launch_dep(residual_norm_planes_kernel<RT, IT, PL>, dim3(a.M), dim3(kRowThreads), 0, s, 1, dependent_launch_for(a.M), a);
+}
+template <typename RT>
+static void launch_resnorm_planes(const ResNormArgs& a, cudaStream_t s) {
+  const int quads = (a.D + 1023) / 1024;
+  switch (quads) {
+    case 1: return a.dsplits <= 4 ? launch_resnorm_planes_form<RT, 1, 4>(a, s) : launch_resnorm_planes_form<RT, 1, 8>(a, s);
+    case 2:
+      return a.dsplits <= 2   ? launch_resnorm_planes_form<RT, 2, 2>(a, s)
+             : a.dsplits <= 4 ? launch_resnorm_planes_form<RT, 2, 4>(a, s)
+                              : launch_resnorm_planes_form<RT, 2, 8>(a, s);
+    case 3: return launch_resnorm_planes_form<RT, 3, 2>(a, s);
+    case 4: return launch_resnorm_planes_form<RT, 4, 4>(a, s);
+    case 5: return launch_resnorm_planes_form<RT, 5, 2>(a, s);
+    default: return launch_resnorm_planes_form<RT, 8, 1>(a, s);
+  }
+}
+#endif
 
 #if IFLB200_ROW_PART == 1 || IFLB200_ROW_PART == -1
 // --------------------------------------------------------------------------------------------
@@ -1011,38 +1225,6 @@ static void launch_gated(GatedArgs a, bool fast, cudaStream_t s) {
     launch_dep(gated_act_quant_kernel<XT, TPR, IT, true>, dim3(grid), dim3(kRowThreads), 0, s, 1, dependent_launch_for(a.M), a);
   });
 }
-// The partial-sum form: rows of at most 8192 columns on the aligned path.
-template <typename RT>
-static int launch_resnorm_partials(ResNormArgs a, bool fast, cudaStream_t s) {
-  if (!fast || a.D > 8192) return IFLB200_ERR_SHAPE;
-  if (a.D <= 1024) {
-    a.iters = 1;
-    launch_dep(residual_norm_quant_kernel<RT, 128, 1, true, true>, dim3((a.M + 1) / 2), dim3(kRowThreads), 0, s, 1,
-               dependent_launch_for(a.M), a);
-  } else if (a.D <= 2048) {
-    a.iters = 1;
-    launch_dep(residual_norm_quant_kernel<RT, kRowThreads, 1, true, true>, dim3(a.M), dim3(kRowThreads), 0, s, 1,
-               dependent_launch_for(a.M), a);
-  } else if (a.D <= 3072) {  // 128 threads x 3 chunks use every chunk slot; two rows per CTA
-    a.iters = 3;
-    launch_dep(residual_norm_quant_kernel<RT, 128, 3, true, true>, dim3((a.M + 1) / 2), dim3(kRowThreads), 0, s, 1,
-               dependent_launch_for(a.M), a);
-  } else if (a.D <= 4096) {
-    a.iters = 2;
-    launch_dep(residual_norm_quant_kernel<RT, kRowThreads, 2, true, true>, dim3(a.M), dim3(kRowThreads), 0, s, 1,
-               dependent_launch_for(a.M), a);
-  } else if (a.D <= 6144) {
-    a.iters = 3;
-    launch_dep(residual_norm_quant_kernel<RT, kRowThreads, 3, true, true>, dim3(a.M), dim3(kRowThreads), 0, s, 1,
-               dependent_launch_for(a.M), a);
-  } else {
-    a.iters = 4;
-    launch_dep(residual_norm_quant_kernel<RT, kRowThreads, 4, true, true>, dim3(a.M), dim3(kRowThreads), 0, s, 1,
-               dependent_launch_for(a.M), a);
-  }
-  return IFLB200_OK;
-}
-
 template <typename RT>
 static void launch_resnorm(ResNormArgs a, bool fast, cudaStream_t s) {
   if (!fast) {
@@ -1145,15 +1327,44 @@ extern "C" int iflb200_row_max_sharded(const void* x, int x_dtype, int64_t ld_x,
 
 #if IFLB200_ROW_PART == 0 || IFLB200_ROW_PART == -1
 // Quantiser pass over fp32 rows whose maxima are already known (the second half of the gated GEMM):
-// no reduction, so a row is cut into pieces of 2048 columns for separate CTAs and the pass runs as a
-// flat elementwise kernel (816 x 16384: 6528 CTAs instead of 816 CTAs that each hold a whole row).
+// no reduction, so a row is cut into pieces for separate CTAs and the pass runs as a flat elementwise
+// kernel (816 x 16384: 3264 CTAs instead of 816 CTAs that each hold a whole row).
 // The maxima are read, never written; `amax_zero` (another buffer, or NULL) is cleared for the
 // producer after next -- clearing the buffer that is being read would race with the row's other CTAs.
-template <bool FAST>
+// Five bytes per element, mostly from L2: a thread takes Q quads 1024 columns apart, every access of a
+// warp contiguous and all of them in flight (one pair of loads per thread before: 816 x 16384 10.2 us).
+template <int Q>
 __global__ void __launch_bounds__(kRowThreads)
 quant_from_amax_kernel(const float* __restrict__ h, int64_t ld_h, int M, int F, const float* __restrict__ amax,
                        float* __restrict__ amax_zero, uint8_t* __restrict__ q, int64_t ld_q, float* __restrict__ qs) {
   row_dependency_wait();  // h and amax come from the kernel before this one in the stream
+  row_trigger();
+  const int m = blockIdx.y;
+  const int c0 = blockIdx.x * (kRowThreads * 4 * Q) + threadIdx.x * 4;
+  const float* src = h + (int64_t)m * ld_h + c0;
+  uint8_t* dst = q + (int64_t)m * ld_q + c0;
+  float4 v[Q];
+#pragma unroll
+  for (int i = 0; i < Q; ++i)
+    if (c0 + i * kRowThreads * 4 < F) v[i] = *reinterpret_cast<const float4*>(src + i * kRowThreads * 4);
+  float scale, inv;
+  quant_scales(amax[m], scale, inv);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    qs[m] = scale;
+    if (amax_zero) amax_zero[m] = 0.0f;
+  }
+#pragma unroll
+  for (int i = 0; i < Q; ++i)
+    if (c0 + i * kRowThreads * 4 < F)
+      *reinterpret_cast<uint32_t*>(dst + i * kRowThreads * 4) =
+          cvt_e4m3x4(__fmul_rn(v[i].x, inv), __fmul_rn(v[i].y, inv), __fmul_rn(v[i].z, inv), __fmul_rn(v[i].w, inv));
+}
+
+// The same for any alignment and width.
+__global__ void __launch_bounds__(kRowThreads)
+quant_from_amax_any_kernel(const float* __restrict__ h, int64_t ld_h, int M, int F, const float* __restrict__ amax,
+                           float* __restrict__ amax_zero, uint8_t* __restrict__ q, int64_t ld_q, float* __restrict__ qs) {
+  row_dependency_wait();
   row_trigger();
   const int m = blockIdx.y;
   const int c0 = (blockIdx.x * kRowThreads + threadIdx.x) * 8;
@@ -1165,8 +1376,8 @@ quant_from_amax_kernel(const float* __restrict__ h, int64_t ld_h, int M, int F, 
   }
   if (c0 >= F) return;
   float v[8];
-  load_f32<FAST>(h + (int64_t)m * ld_h, c0, F, v);
-  store_codes<FAST>(q + (int64_t)m * ld_q, c0, F, v, inv);
+  load_f32<false>(h + (int64_t)m * ld_h, c0, F, v);
+  store_codes<false>(q + (int64_t)m * ld_q, c0, F, v, inv);
 }
 
 extern "C" int iflb200_quant_from_amax(const float* h, int64_t ld_h, int M, int F, const float* amax, float* amax_zero,
@@ -1177,14 +1388,16 @@ extern "C" int iflb200_quant_from_amax(const float* h, int64_t ld_h, int M, int 
   if (ld_h < F || ld_q < F) return IFLB200_ERR_ARG;
   if (M > 65535) return IFLB200_ERR_SHAPE;
   const bool fast = F % 8 == 0 && aligned16(h) && (ld_h * 4) % 16 == 0 && aligned8(q) && ld_q % 8 == 0;
-  const dim3 grid((unsigned)((F + kRowThreads * 8 - 1) / (kRowThreads * 8)), (unsigned)M);
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  if (fast)
-    launch_dep(quant_from_amax_kernel<true>, grid, dim3(kRowThreads), 0, s, 1, dependent_launch_for(M), h, ld_h, M, F, amax,
-               amax_zero, reinterpret_cast<uint8_t*>(q), ld_q, qs);
-  else
-    launch_dep(quant_from_amax_kernel<false>, grid, dim3(kRowThreads), 0, s, 1, dependent_launch_for(M), h, ld_h, M, F, amax,
-               amax_zero, reinterpret_cast<uint8_t*>(q), ld_q, qs);
+  uint8_t* codes = reinterpret_cast<uint8_t*>(q);
+  auto launch = [&](auto kernel, int columns) {
+    launch_dep(kernel, dim3((unsigned)((F + columns - 1) / columns), (unsigned)M), dim3(kRowThreads), 0, s, 1,
+               dependent_launch_for(M), h, ld_h, M, F, amax, amax_zero, codes, ld_q, qs);
+  };
+  // few rows: shorter pieces, so that every SM has one
+  if (!fast) launch(quant_from_amax_any_kernel, kRowThreads * 8);
+  else if ((int64_t)M * F >= (int64_t)1 << 21) launch(quant_from_amax_kernel<4>, kRowThreads * 16);
+  else launch(quant_from_amax_kernel<1>, kRowThreads * 4);
   return (int)cudaGetLastError();
 }
 #endif
@@ -1306,9 +1519,9 @@ static int resnorm_impl(void* res, int res_dtype, int64_t ld_res, int M, int D, 
                     (!y || (aligned16(y) && (ld_y * esize(y_dtype)) % 16 == 0)) && tables_ok;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (delta_splits) {
-    const int st = res_dtype == IFLB200_F32 ? launch_resnorm_partials<float>(a, fast, s)
-                                            : launch_resnorm_partials<__nv_bfloat16>(a, fast, s);
-    if (st != IFLB200_OK) return st;
+    if (!fast || D > 8192) return IFLB200_ERR_SHAPE;
+    if (res_dtype == IFLB200_F32) launch_resnorm_planes<float>(a, s);
+    else launch_resnorm_planes<__nv_bfloat16>(a, s);
     return (int)cudaGetLastError();
   }
   // one affine after the norm, or none; per-row tables, a second output and a residual that is not

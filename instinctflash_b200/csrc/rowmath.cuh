@@ -64,53 +64,55 @@ struct Chain {
   }
 };
 
-// The same for the eight elements of a chunk at once.  Which operations exist is decided by
+// The same for the elements of a chunk (an even number of them) at once.  Which operations exist is decided by
 // kernel arguments, the same for every element, so `pending` is uniform: the compiler emits
 // one uniform branch per stage and chunk instead of selects per element.
-struct Chain8 {
-  float v[8];
-  float p[8];
+template <int N>
+struct ChainV {
+  float v[N];
+  float p[N];
   bool pending;
-  __device__ __forceinline__ explicit Chain8(const float (&x)[8]) : pending(false) {
+  __device__ __forceinline__ explicit ChainV(const float (&x)[N]) : pending(false) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = x[i];
+    for (int i = 0; i < N; ++i) v[i] = x[i];
   }
   __device__ __forceinline__ void flush() {
     if (pending) {
 #pragma unroll
-      for (int i = 0; i < 8; i += 2) unpack2(mul2(pack2(v[i], v[i + 1]), pack2(p[i], p[i + 1])), v[i], v[i + 1]);
+      for (int i = 0; i < N; i += 2) unpack2(mul2(pack2(v[i], v[i + 1]), pack2(p[i], p[i + 1])), v[i], v[i + 1]);
     }
   }
-  __device__ __forceinline__ void mul(const float (&f)[8]) {
+  __device__ __forceinline__ void mul(const float (&f)[N]) {
     flush();
 #pragma unroll
-    for (int i = 0; i < 8; ++i) p[i] = f[i];
+    for (int i = 0; i < N; ++i) p[i] = f[i];
     pending = true;
   }
   __device__ __forceinline__ void mul(float f) {
     flush();
 #pragma unroll
-    for (int i = 0; i < 8; ++i) p[i] = f;
+    for (int i = 0; i < N; ++i) p[i] = f;
     pending = true;
   }
-  __device__ __forceinline__ void add(const float (&c)[8]) {
+  __device__ __forceinline__ void add(const float (&c)[N]) {
     if (pending) {
 #pragma unroll
-      for (int i = 0; i < 8; i += 2)
+      for (int i = 0; i < N; i += 2)
         unpack2(fma2(pack2(v[i], v[i + 1]), pack2(p[i], p[i + 1]), pack2(c[i], c[i + 1])), v[i], v[i + 1]);
       pending = false;
     } else {
 #pragma unroll
-      for (int i = 0; i < 8; i += 2) unpack2(add2(pack2(v[i], v[i + 1]), pack2(c[i], c[i + 1])), v[i], v[i + 1]);
+      for (int i = 0; i < N; i += 2) unpack2(add2(pack2(v[i], v[i + 1]), pack2(c[i], c[i + 1])), v[i], v[i + 1]);
     }
   }
-  __device__ __forceinline__ void done(float (&out)[8]) {
+  __device__ __forceinline__ void done(float (&out)[N]) {
     flush();
     pending = false;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) out[i] = v[i];
+    for (int i = 0; i < N; ++i) out[i] = v[i];
   }
 };
+using Chain8 = ChainV<8>;
 
 // gelu_pytorch_tanh as written in the reference: 0.5*v*(1 + (2/(1+exp(-2*inner)) - 1)),
 // inner = 0.79788456*(v + 0.044715*v^3), with exp lowered to ex2.approx and the division to
