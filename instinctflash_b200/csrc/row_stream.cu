@@ -145,9 +145,9 @@ struct StreamGeom {
   int tg = 0, groups = 0;
   size_t smem = 0;
 };
-StreamGeom stream_geom(int M, int K, int vectors, int row_bytes, int max_threads, int sms) {
+StreamGeom stream_geom(int M, int K, int vectors, int row_bytes, int max_threads, int sms, int chunks = kChunks) {
   StreamGeom g;
-  g.tg = ((K / 8 + kChunks - 1) / kChunks + 31) / 32 * 32;
+  g.tg = ((K / 8 + chunks - 1) / chunks + 31) / 32 * 32;
   g.groups = max_threads / g.tg;
   if (g.groups > kMaxGroups) g.groups = kMaxGroups;
   const size_t fixed = (size_t)vectors * K * 4;
@@ -186,7 +186,7 @@ bool launch_stream(const StreamGeom& g, int sms, cudaStream_t s, const KArgs& a)
 // row they were 8 bytes beside 3 of HBM traffic.  4680 x 14336: 106 -> 62 us, 16384 x 13824: 343 -> 183,
 // the special-function unit busy for half of it.
 // --------------------------------------------------------------------------------------------
-template <typename XT, bool BIAS, int THREADS>
+template <typename XT, bool BIAS, int THREADS, int CHUNKS>
 __global__ void __launch_bounds__(THREADS, 1) gelu_quant_stream_kernel(const GeluStreamArgs a, int tg) {
   extern __shared__ __align__(16) uint8_t smem[];
   __shared__ __align__(16) float red[2][kMaxGroups][kMaxWarps];
@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(THREADS, 1) gelu_quant_stream_kernel(const Gel
   auto fetch = [&](int row, int it) { copy16_async(slot + it * tg * 16, x + (int64_t)row * a.ld_x + it * tg * 8); };
   if (m < a.M) {
 #pragma unroll
-    for (int it = 0; it < kChunks; ++it)
+    for (int it = 0; it < CHUNKS; ++it)
       if ((it * tg + t) * 8 < a.K) fetch(m, it);
     rs = a.row[m];
   }
@@ -220,10 +220,10 @@ __global__ void __launch_bounds__(THREADS, 1) gelu_quant_stream_kernel(const Gel
     const bool more = next < a.M;
     const float rs_next = more ? a.row[next] : 1.0f;
     copy_wait_all();
-    Eight v[kChunks];
+    Eight v[CHUNKS];
     float amax = 0.0f;
 #pragma unroll
-    for (int it = 0; it < kChunks; ++it) {
+    for (int it = 0; it < CHUNKS; ++it) {
       if ((it * tg + t) * 8 < a.K) {
         v[it] = widen(lds16(slot + it * tg * 16), XT());
         if (more) fetch(next, it);  // the slot has been read by the only thread that uses it
@@ -243,23 +243,24 @@ __global__ void __launch_bounds__(THREADS, 1) gelu_quant_stream_kernel(const Gel
     if (t == 0) a.qs[m] = scale_out;
     uint8_t* q = a.q + (int64_t)m * a.ld_q + t * 8;
 #pragma unroll
-    for (int it = 0; it < kChunks; ++it)
+    for (int it = 0; it < CHUNKS; ++it)
       if ((it * tg + t) * 8 < a.K) store_codes(q + it * tg * 8, v[it], inv);
     rs = rs_next;
   }
 }
 
-template <typename XT, int THREADS>
+template <typename XT, int THREADS, int CHUNKS>
 bool gelu_form(const GeluStreamArgs& a, int sms, cudaStream_t s) {
-  const StreamGeom g = stream_geom(a.M, a.K, a.bias ? 2 : 1, a.K * 2, THREADS, sms);
+  const StreamGeom g = stream_geom(a.M, a.K, a.bias ? 2 : 1, a.K * 2, THREADS, sms, CHUNKS);
   if (g.groups == 0) return false;
-  return a.bias ? launch_stream<gelu_quant_stream_kernel<XT, true, THREADS>>(g, sms, s, a)
-                : launch_stream<gelu_quant_stream_kernel<XT, false, THREADS>>(g, sms, s, a);
+  return a.bias ? launch_stream<gelu_quant_stream_kernel<XT, true, THREADS, CHUNKS>>(g, sms, s, a)
+                : launch_stream<gelu_quant_stream_kernel<XT, false, THREADS, CHUNKS>>(g, sms, s, a);
 }
 template <typename XT>
 bool gelu_width(const GeluStreamArgs& a, int sms, cudaStream_t s) {
-  // two groups of 448 threads hold rows of up to 14336 columns with eight more registers a thread
-  return a.K <= 14336 ? gelu_form<XT, 896>(a, sms, s) : gelu_form<XT, 1024>(a, sms, s);
+  // two groups of 448 threads hold rows of up to 14336 columns with eight more registers a thread; wider rows are
+  // faster with eight chunks on half the threads (16384 x 16384 221 -> 207 us; 16384 x 13824 is not, 183 -> 199)
+  return a.K <= 14336 ? gelu_form<XT, 896, 4>(a, sms, s) : gelu_form<XT, 512, 8>(a, sms, s);
 }
 
 // --------------------------------------------------------------------------------------------
