@@ -1192,7 +1192,8 @@ struct PairSmemLayout {
   static constexpr int kDynamic = kTotal + 1024;
 };
 
-template <int BN, int STAGES, int ACC, bool SWAP = false>
+// PLANES: (tile, K range) units as in the single-CTA kernel's planes form.
+template <int BN, int STAGES, int ACC, bool SWAP = false, bool PLANES = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
 gemm_fp8_tc5_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w,
                          const __grid_constant__ CUtensorMap tm_out, const GemmParams p) {
@@ -1220,6 +1221,16 @@ gemm_fp8_tc5_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
   const bool leader = rank == 0;
   const int pair_id = blockIdx.x >> 1;
   const int pair_stride = gridDim.x >> 1;
+  const int parts = PLANES ? p.partials : 1;
+  const int units = p.num_tiles * parts;
+  auto range_begin = [&](int part) { return PLANES ? (int)(((int64_t)((p.num_k + 3) / 4) * part) / parts) * 4 : 0; };
+  int kb0 = 0, kb1 = p.num_k;
+  auto enter_unit = [&](int unit) {
+    if constexpr (PLANES) {
+      kb0 = range_begin(unit % parts);
+      kb1 = min(p.num_k, range_begin(unit % parts + 1));
+    }
+  };
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -1256,11 +1267,12 @@ gemm_fp8_tc5_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
     Ring<STAGES> ring;
     bool ok = true;
     uint32_t it = 0;
-    for (int tile = pair_id; ok && tile < p.num_tiles; tile += pair_stride, ++it) {
+    for (int unit = pair_id; ok && unit < units; unit += pair_stride, ++it) {
       int m_blk, n_blk;
-      tile_coords(p, tile, m_blk, n_blk);
+      tile_coords(p, unit / parts, m_blk, n_blk);
+      enter_unit(unit);
       const int row = w_producer ? n_blk * BN + (int)rank * (BN / 2) : m_blk * 2 * BM + (int)rank * BM;
-      for (int kb = 0; kb < p.num_k; ++kb) {
+      for (int kb = kb0; kb < kb1; ++kb) {
         ok = wait_bounded(empty_bar(ring.stage), ring.phase ^ 1, abort_flag, (1u << 24) | (1u << 16) | (it & 0xFFFF));
         if (!ok) break;
         if (elect_one()) {
@@ -1280,14 +1292,15 @@ gemm_fp8_tc5_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
       uint32_t phase = 0;
       bool ok = true;
       uint32_t it = 0;
-      for (int tile = pair_id; ok && tile < p.num_tiles; tile += pair_stride, ++it) {
+      for (int unit = pair_id; ok && unit < units; unit += pair_stride, ++it) {
+        enter_unit(unit);
         const uint32_t acc = (ACC == 2) ? (it & 1u) : 0u;
         const uint32_t acc_phase = (ACC == 2) ? ((it >> 1) & 1u) : (it & 1u);
         ok = wait_bounded(tempty_bar(acc), acc_phase ^ 1, abort_flag, (2u << 24) | (2u << 16) | (it & 0xFFFF));
         if (!ok) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * kAccStride;
-        for (int kb = 0; kb < p.num_k; ++kb) {
+        for (int kb = kb0; kb < kb1; ++kb) {
           ok = wait_bounded(full_bar(stage), phase, abort_flag, (2u << 24) | (3u << 16) | (it & 0xFFFF));
           if (!ok) break;
           tc_fence_after();
@@ -1297,7 +1310,7 @@ gemm_fp8_tc5_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
             const uint64_t db = make_kmajor_sw128_desc(sa + L::kABytes);
 #pragma unroll
             for (int j = 0; j < BK / 32; ++j)
-              mma_f8f6f4_pair(d_tmem, da + 2 * j, db + 2 * j, kIdesc, (kb | j) != 0 ? 1u : 0u);
+              mma_f8f6f4_pair(d_tmem, da + 2 * j, db + 2 * j, kIdesc, kb > kb0 || j > 0 ? 1u : 0u);
             mma_commit_pair(empty_bar(stage), 3);  // stage free in both CTAs
           }
           __syncwarp();
@@ -1328,9 +1341,10 @@ gemm_fp8_tc5_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
     uint32_t it = 0;
     int swap_buf = 0;
     grid_dependency_wait();  // scales and residual operands may come from the kernel before this one
-    for (int tile = pair_id; ok && tile < p.num_tiles; tile += pair_stride, ++it) {
+    for (int unit = pair_id; ok && unit < units; unit += pair_stride, ++it) {
       int m_blk, n_blk;
-      tile_coords(p, tile, m_blk, n_blk);
+      tile_coords(p, unit / parts, m_blk, n_blk);
+      enter_unit(unit);
       const uint32_t acc = (ACC == 2) ? (it & 1u) : 0u;
       const uint32_t acc_phase = (ACC == 2) ? ((it >> 1) & 1u) : (it & 1u);
       const int m = m_blk * 2 * BM + (int)rank * BM + quad * 32 + lane;
@@ -1360,7 +1374,7 @@ gemm_fp8_tc5_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
       if (p.tma_store) {
         epilogue_tma_store<BN>(p, &tm_out, t_row, staging, staging_ptr,
                                m_blk * 2 * BM + (int)rank * BM + quad * 32, n_blk * BN, col_begin, col_end, rs, lane,
-                               -1, prefetch ? &cv : nullptr);
+                               PLANES ? unit % parts : -1, prefetch ? &cv : nullptr);
       } else {
 #pragma unroll 1
         for (int c = col_begin / 32; c < col_end / 32; ++c) {
@@ -1572,7 +1586,7 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tw, const CUten
   }
 }
 
-template <int BN, int STAGES, int ACC, bool SWAP = false>
+template <int BN, int STAGES, int ACC, bool SWAP = false, bool PLANES = false>
 static int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tw, const CUtensorMap& to,
                             const GemmParams& p, int grid, cudaStream_t s) {
   using L = PairSmemLayout<BN, STAGES>;
@@ -1580,12 +1594,12 @@ static int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tw, const 
   int dev = 0;
   cudaGetDevice(&dev);
   if (!attr_set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_fp8_tc5_pair_kernel<BN, STAGES, ACC, SWAP>,
+    cudaError_t e = cudaFuncSetAttribute(gemm_fp8_tc5_pair_kernel<BN, STAGES, ACC, SWAP, PLANES>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, L::kDynamic);
     if (e != cudaSuccess) return (int)e;
     attr_set[dev] = true;
   }
-  const cudaError_t e = launch_dep(gemm_fp8_tc5_pair_kernel<BN, STAGES, ACC, SWAP>, dim3(grid), dim3(kGemmThreads),
+  const cudaError_t e = launch_dep(gemm_fp8_tc5_pair_kernel<BN, STAGES, ACC, SWAP, PLANES>, dim3(grid), dim3(kGemmThreads),
                                    L::kDynamic, s, 1, dependent_launch_for(SWAP ? p.N : p.M), ta, tw, to, p);
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
@@ -1621,13 +1635,15 @@ static int run_gemm(const void* a, int64_t ld_a, const void* w, int64_t ld_w, Ge
   // single CTAs in 9; 14336 x 3072 149.5 against 161.2; but 3072 x 14336 186 against 150 where the
   // pairs need 4 waves for 3).  So the pair kernel is taken when its wave count, weighted by that
   // factor, is below the single-CTA one.
+  // Below 2048 rows only where there are at least two waves to save in (816 x 8192 x 2048 15.4 against
+  // 16.0 us, 1300 x 12288 x 3072 39.7 against 42.4; the one wave of 1500 x 2048 x 4096 is 15.4 against 14.9).
   bool pair_by_heuristic = false;
-  if (g_cfg_mode == 0 && g_cfg_tile_n == 0 && g_cfg_split_k == 0 && p.M >= 2048 && p.N >= 256) {
+  if (g_cfg_mode == 0 && g_cfg_tile_n == 0 && g_cfg_split_k == 0 && p.M >= 512 && p.N >= 256) {
     const int64_t single_tiles = (int64_t)((p.M + BM - 1) / BM) * ((p.N + 255) / 256);
     const int64_t pair_tiles = (int64_t)((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + 255) / 256);
     const int64_t single_waves = (single_tiles + dev->sm_count - 1) / dev->sm_count;
     const int64_t pair_waves = (pair_tiles + dev->sm_count / 2 - 1) / (dev->sm_count / 2);
-    pair_by_heuristic = pair_waves * 87 < single_waves * 100;
+    pair_by_heuristic = pair_waves * 87 < single_waves * 100 && (p.M >= 2048 || single_waves >= 2);
   }
   if ((g_cfg_mode >= 2 || pair_by_heuristic) && p.N >= 256) {
     // CTA pairs: 256 x 256 tiles, each CTA loads 128 rows of A and 128 rows of W per K step.
@@ -1656,11 +1672,11 @@ static int run_gemm(const void* a, int64_t ld_a, const void* w, int64_t ld_w, Ge
                            : launch_gemm_pair<PBN, 6, 2>(ta, tw, to, p, grid, s);  // two accumulators
   }
 
-  // Tile width by a measured cost model: one 128-byte K step of a CTA costs about 590 / 690 /
-  // 830 cycles for a 64 / 128 / 256 wide tile (24 / 32 / 48 KB through the SM's L2 port per
-  // step; 192 and 224 interpolate), the kernel takes waves x steps x that, plus a fixed cost per
-  // wave for prologue and the exposed epilogue.  The widths that are not powers of two are for
-  // wave quantisation (7 row blocks x 32768 columns: 896 tiles of 256 = 6.05 waves of 148 SMs, i.e.
+  // Tile width by a measured cost model: one 128-byte K step of a CTA costs about 385 / 510 / 720 cycles for a
+  // 64 / 128 / 256 wide tile: 24 / 32 / 48 KB are written to shared memory and read back by the tensor core
+  // through one port of 128 bytes a clock (192 and 224 interpolate).  The kernel takes waves x steps x that,
+  // plus a fixed cost per wave for prologue and the exposed epilogue.  The widths that are not powers of two
+  // are for wave quantisation (7 row blocks x 32768 columns: 896 tiles of 256 = 6.05 waves of 148 SMs, i.e.
   // 7, but 1029 tiles of 224 = 6.95 waves of narrower tiles).  Timed alone the 224-wide kernel is
   // 2 % faster on that shape, inside the layer stack it was 4 us per launch slower (its 448-byte
   // tile rows start off the 128-byte line grid), so the model does not choose them by itself.
@@ -1669,7 +1685,7 @@ static int run_gemm(const void* a, int64_t ld_a, const void* w, int64_t ld_w, Ge
   int split = 1;
   {
     const int widths[5] = {256, 224, 192, 128, 64};
-    const int64_t step_cycles[5] = {830, 790, 750, 690, 590};
+    const int64_t step_cycles[5] = {720, 680, 640, 510, 385};
     const int64_t steps = (p.K + BK - 1) / BK;
     int64_t best = 0;
     int best_bn = 0;
@@ -1686,7 +1702,8 @@ static int run_gemm(const void* a, int64_t ld_a, const void* w, int64_t ld_w, Ge
         if (sk > 1 && (tiles * sk > dev->sm_count || steps / sk < 8 || widths[i] / sk < 32)) continue;
         if (sk > 1 && (widths[i] & (widths[i] - 1))) continue;  // the reduction splits power-of-two widths
         const int64_t waves = sk > 1 ? 1 : (tiles + dev->sm_count - 1) / dev->sm_count;
-        const int64_t cost = waves * ((steps / sk) * step_cycles[i] + 2500 + (sk > 1 ? 18000 : 0));
+        const int64_t exchange = sk > 1 ? 5000 + 65 * widths[i] * (sk - 1) / sk : 0;  // barriers, columns handed over
+        const int64_t cost = waves * ((steps / sk) * step_cycles[i] + 2500 + exchange);
         if (best_bn == 0 || cost < best) {
           best = cost;
           best_bn = widths[i];
@@ -1857,12 +1874,27 @@ static int run_gemm_partials(const void* a, int64_t ld_a, const void* w, int64_t
     g_last_launch[0] = 1 + 16; g_last_launch[1] = 64; g_last_launch[2] = splits; g_last_launch[3] = 104;
     return launch_gemm_form<64, 2, 2, false, false, kEpilogueWarps, 4>(ta, tw, to, p, p.num_tiles * splits, s);
   }
+  // CTA pairs where blocks of 256 rows pad little and their units need no more waves: two thirds of the traffic per K step, which is what these launches wait for.
+  // 816 x 2048 x 16384 in two ranges 28.6 against 29.7 us, 640 rows in three 22.8 against 23.3.
+  const int pair_m = (M + 2 * BM - 1) / (2 * BM), sm_pairs = dev->sm_count / 2;
+  const int64_t pair_units = (int64_t)pair_m * p.num_n * splits, single_units = (int64_t)p.num_tiles * splits;
+  const int64_t pair_waves = (pair_units + sm_pairs - 1) / sm_pairs;
+  const int64_t single_waves = (single_units + dev->sm_count - 1) / dev->sm_count;
+  if (bn == 256 && g_cfg_mode != 1 && pair_m * 2 * BM * 4 <= M * 5 + 16 && pair_waves <= single_waves) {
+    st = make_tensor_map(&ta, a, M, K, ld_a, BM);
+    if (st != IFLB200_OK) return st;
+    st = make_tensor_map(&tw, w, N, K, ld_w, BM);
+    if (st != IFLB200_OK) return st;
+    p.num_m = pair_m;
+    p.num_tiles = p.num_m * p.num_n;
+    g_last_launch[0] = 3 + 16; g_last_launch[1] = bn; g_last_launch[2] = splits; g_last_launch[3] = 6;
+    return launch_gemm_pair<256, 6, 2, false, true>(ta, tw, to, p, 2 * (int)(pair_units < sm_pairs ? pair_units : sm_pairs), s);
+  }
   st = make_tensor_map(&ta, a, M, K, ld_a, a_rows);
   if (st != IFLB200_OK) return st;
   st = make_tensor_map(&tw, w, N, K, ld_w, bn);
   if (st != IFLB200_OK) return st;
-  const int64_t units = (int64_t)p.num_tiles * splits;
-  const int grid = units < dev->sm_count ? (int)units : dev->sm_count;
+  const int grid = single_units < dev->sm_count ? (int)single_units : dev->sm_count;
   g_last_launch[0] = 1 + 16; g_last_launch[1] = bn; g_last_launch[2] = splits; g_last_launch[3] = 0;
   return bn == 64 ? launch_gemm_form<64, 8, 3>(ta, tw, to, p, grid, s) : launch_gemm_form<256, 4, 3>(ta, tw, to, p, grid, s);
 }
@@ -1945,7 +1977,7 @@ static int run_gemm_gated(const void* a, int64_t ld_a, const void* w, int64_t ld
   p.num_k = (K + BK - 1) / BK;
   // tile width (gate + up columns) by the cost model of the ordinary form
   const int widths[3] = {256, 128, 64};
-  const int64_t step_cycles[3] = {830, 690, 590};
+  const int64_t step_cycles[3] = {720, 510, 385};
   int bn = g_cfg_tile_n == 256 || g_cfg_tile_n == 128 || g_cfg_tile_n == 64 ? g_cfg_tile_n : 0;
   if (bn == 0) {
     int64_t best = 0;

@@ -182,11 +182,19 @@ def fp8_linear_gated(a: torch.Tensor, a_scale: torch.Tensor, w: Fp8Weight, h: to
 
 def partial_splits(M: int, N: int, K: int, sm_count: int = 148) -> int:
     """How many K ranges ``gemm_partials`` should use for a skinny projection: enough (tile, range)
-    pairs to occupy the GPU, every range at least four 128-byte K slabs, at most eight planes."""
-    if M > 128 or K % 128:
+    pairs to occupy the GPU, every range at least four 128-byte K slabs, at most eight planes.
+
+    Above 128 rows the planes pay where one wave of tiles leaves much of the GPU idle and the
+    reduction is deep (a range of at least sixteen slabs outlasts its fp32 tile): the consumer adds the
+    planes on its way, while the cluster form of the GEMM exchanges them through distributed shared memory
+    first."""
+    if K % 128:
         return 1
-    tiles = (N + 63) // 64
-    return max(1, min(8, sm_count // max(1, tiles), (K // 128) // 4))
+    if M <= 128:
+        tiles, slabs = (N + 63) // 64, 4
+    else:
+        tiles, slabs = ((M + 127) // 128) * ((N + 255) // 256), 16
+    return max(1, min(8, sm_count // max(1, tiles), (K // 128) // slabs))
 
 
 def gemm_partials(a: torch.Tensor, w: Fp8Weight, out: torch.Tensor) -> torch.Tensor:

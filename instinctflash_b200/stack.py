@@ -169,9 +169,9 @@ class LinearStack:
             fused = spec.M > 128
         self.fused = bool(fused) and hasattr(self.ops, "fp8_linear_gated")
         self.fuse_residual = fuse_residual and hasattr(self.ops, "fp8_linear_residual")
-        # skinny activations: deep, narrow projections (down, o) run split-K over independent CTAs, the
+        # deep, narrow projections (down, o) whose tiles do not fill the GPU run split-K over independent CTAs, the
         # residual kernel adds the fp32 partial sums (this package's operators only)
-        self.split_partials = (split_partials and spec.kind == "gemma" and split_rows <= 128 and
+        self.split_partials = (split_partials and spec.kind == "gemma" and
                                hasattr(self.ops, "gemm_partials"))
         M, D, F = spec.M, spec.hidden, spec.ffn
         dev, bf16, f32 = self.dev, torch.bfloat16, torch.float32
@@ -382,7 +382,7 @@ class EpisodeBatch:
         self.spec, self.dev, self.episodes = spec, torch.device(device), episodes
         self.launches_per_forward = 0   # of all episodes: a launch counts once for every episode it serves
         self.merged = None
-        if spec.kind == "gemma" and spec.M <= 128 and episodes > 1:
+        if spec.kind == "gemma" and spec.M <= 128 and episodes > 1 and spec.M * episodes <= 65535:
             wide = StackSpec(**{**spec.__dict__, "M": spec.M * episodes})
             merged = LinearStack(wide, weights, device, split_rows=spec.M, **stack_kw)
             if hasattr(merged.ops, "gemm_partials"):    # this package's operators: K ranges by rows of one episode
@@ -403,7 +403,6 @@ class EpisodeBatch:
         torch._foreach_copy_([st.res for st in self.stacks], list(xs))
         for st in self.stacks:
             st.attn = attn
-        self.attn = attn
         o, m = self.merged.ops, self.merged
         o.residual_norm_quant(m.res, layernorm=False, q=m._q8(self.spec.hidden), q_scale=m.scale[0])
 
@@ -411,9 +410,14 @@ class EpisodeBatch:
         """Every episode's pass (branches are forked onto their own streams and joined on the current one)."""
         if self.merged is not None:
             if self.spec.o_in:
-                if self.attn.dtype != self.attn_rows.dtype:
-                    self.attn_rows = self.attn_rows.to(self.attn.dtype)
-                self.attn_rows.view(self.episodes, self.spec.M, -1).copy_(self.attn)
+                attn = [st.attn for st in self.stacks]
+                if attn[0].dtype != self.attn_rows.dtype:
+                    self.attn_rows = self.attn_rows.to(attn[0].dtype)
+                rows = self.attn_rows.view(self.episodes, self.spec.M, -1)
+                if all(t is attn[0] for t in attn):   # one output for all of them, as load() leaves it
+                    rows.copy_(attn[0])
+                else:
+                    torch._foreach_copy_(list(rows), attn)
             self.merged.attn = self.attn_rows
             self.merged.forward()
             for st in self.stacks:
