@@ -58,6 +58,7 @@ struct GemmParams {
   int out_dtype;
   int64_t ld_out;
   int split_k;     // > 1: the CTAs of a cluster share one tile, each a K range; partials are summed over DSMEM
+  int m64;         // lean form: MMAs of M = 64 (at most 64 rows; the output map's box has 16 rows then)
   int a_bytes;     // bytes one activation box delivers per K step: 128 x (rows of the box)
   int partials;    // > 1: K is split over that many independent CTAs per tile; each writes its fp32 partial
                    // accumulator to out[split][M][ld_out] (summed in split order by the consumer)
@@ -734,6 +735,10 @@ __device__ __forceinline__ void epilogue_swapped(const GemmParams& p, const CUte
 // launch in instruction fetch (0.2 ms per pass of the M = 50 stack).
 // SPLIT 3: the planes form for more than 128 rows: (tile, K range) units on a persistent grid, each leaving
 // its fp32 partial sums in a plane; K is cut as in the skinny form, so the planes' bits are the same.
+// SPLIT 4: the lean form of the skinny regime: planes or one range, TMA stores, no cluster and no direct stores.
+// Every launch of a 4 us kernel fetches its instructions cold, so the code that a skinny layer stack never
+// reaches is left out; and up to 64 rows its MMAs read 64 activation rows instead of 128 (38 clocks each
+// for 48: a third of the main loop of a K = 1024 tile).
 // GATED: the gated form (see epilogue_gated): a tile pairs BN/2 gate columns with the BN/2 up
 // columns of the same hidden units; p.N counts hidden units.
 // EW: epilogue warps (8, or 16 for the gated form: EW / 4 per TMEM lane quadrant).
@@ -780,9 +785,13 @@ gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
   // Split-K: the S CTAs of a cluster work on the same tile, CTA r on K steps [kb0, kb1); one
   // tile per CTA (the host launches tiles x S CTAs, at most one wave).
   // Partials: K split over independent CTAs (no cluster), each writing its fp32 partial sums.
-  constexpr bool PLANES = SPLIT == 3;
-  const bool partials = SPLIT == 2 && p.partials > 1;
+  constexpr bool PLANES = SPLIT == 3, LEAN = SPLIT == 4;
+  const bool partials = (SPLIT == 2 || LEAN) && p.partials > 1;
   const bool split = !partials && (SPLIT == 1 || (SPLIT == 2 && p.split_k > 1));
+  // At most 64 rows: MMAs of M = 64, whose row i lies in lane i % 16 of quadrant i / 16
+  const bool m64 = LEAN && p.m64;
+  const int quad_rows = m64 ? 16 : 32;
+  const uint32_t idesc = m64 ? make_idesc_e4m3_f32(64, BN) : kIdesc;
   const int k_parts = partials || PLANES ? p.partials : (split ? p.split_k : 1);
   const int split_rank = partials ? (int)blockIdx.x % k_parts : (split ? (int)cluster_ctarank() : 0);
   // a unit of work is a tile, or (tile, K range) in the planes form
@@ -918,7 +927,7 @@ gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
 #pragma unroll
             for (int j = 0; j < BK / 32; ++j) {
               // 32 bytes further along K inside the swizzled 128-byte row: +2 in 16-byte units.
-              mma_f8f6f4(d_tmem, da + 2 * j, db + 2 * j, kIdesc, (kb + sl > kb0 || j > 0) ? 1u : 0u);
+              mma_f8f6f4(d_tmem, da + 2 * j, db + 2 * j, idesc, (kb + sl > kb0 || j > 0) ? 1u : 0u);
             }
           }
           mma_commit(empty_bar(stage));  // stage reusable once these MMAs have read it
@@ -963,9 +972,9 @@ gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
       // same thing before its first load), then this tile's per-column operands and row scale, so
       // that their latency runs under the main loop instead of after it.
       if (it == 0) grid_dependency_wait();
-      const int m = m_blk * BM + quad * 32 + lane;
-      const bool row_ok = m < p.M;
-      const bool prefetch = !SWAP && !GATED && !split && p.tma_store && p.epilogue != EPI_RAW && col_end - col_begin <= 128;
+      const int m = m_blk * BM + quad * quad_rows + lane;
+      const bool row_ok = m < p.M && (!LEAN || lane < quad_rows);
+      const bool prefetch = !SWAP && !GATED && !split && (LEAN || p.tma_store) && p.epilogue != EPI_RAW && col_end - col_begin <= 128;
       ColumnVectors cv;
       float rs_early = 1.0f;
       if (prefetch) {
@@ -1003,14 +1012,14 @@ gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
       if (split) {
         // one tile per CTA: the partial accumulator stays in tensor memory; the exchange with
         // the other CTAs of the cluster follows the role loops
-      } else if (p.tma_store) {
+      } else if (LEAN || p.tma_store) {
         // whole 128-byte pieces through shared memory and TMA; a 32-column remainder of a
         // 224-wide tile (two-byte outputs) straight from registers
         const int per_store = (p.out_dtype == IFLB200_F32 || p.half_rows) ? 32 : 64;
         const int col_tma_end = col_begin + (col_end - col_begin) / per_store * per_store;
-        epilogue_tma_store<BN>(p, tm_dst, t_row, staging, staging_ptr, m_blk * BM + quad * 32, n_blk * BN,
+        epilogue_tma_store<BN>(p, tm_dst, t_row, staging, staging_ptr, m_blk * BM + quad * quad_rows, n_blk * BN,
                                col_begin, col_tma_end, rs, lane,
-                               PLANES ? unit % k_parts : ((SPLIT == 2 && p.partials >= 1) ? split_rank : -1),  // a plane map takes a 3-D store
+                               PLANES ? unit % k_parts : (((SPLIT == 2 || LEAN) && p.partials >= 1) ? split_rank : -1),  // a plane map takes a 3-D store
                                prefetch ? &cv : nullptr);
         if (BN % 64 != 0 && col_tma_end < col_end) {
           const int n0 = n_blk * BN + col_tma_end;
@@ -1042,7 +1051,7 @@ gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
     __syncwarp();
   }
 
-  if (split) {
+  if (!LEAN && split) {
     // CTA r of the cluster reduces columns [r*BN/S, (r+1)*BN/S) of the tile: its own partial
     // comes from tensor memory, the peers write theirs into its shared memory, and the sum runs
     // in rank order (fixed, so the result does not depend on timing); then the consumer
@@ -1476,13 +1485,13 @@ static int make_gated_weight_map(CUtensorMap* tm, const void* ptr, int F, int K,
   return r == CUDA_SUCCESS ? IFLB200_OK : IFLB200_ERR_DRIVER;
 }
 
-// [M, N] output matrix of 2- or 4-byte elements; box = 128 bytes x 32 rows, 128-byte swizzle.
-static int make_out_map(CUtensorMap* tm, void* ptr, int M, int N, int64_t ld, int esize, int row_bytes = 128) {
+// [M, N] output matrix of 2- or 4-byte elements; box = row_bytes x box_rows, swizzled over that many bytes.
+static int make_out_map(CUtensorMap* tm, void* ptr, int M, int N, int64_t ld, int esize, int row_bytes = 128, int box_rows = 32) {
   EncodeTiledFn enc = get_encode_fn();
   if (!enc) return IFLB200_ERR_DRIVER;
   const cuuint64_t dims[2] = {(cuuint64_t)N, (cuuint64_t)M};
   const cuuint64_t strides[1] = {(cuuint64_t)ld * esize};
-  const cuuint32_t box[2] = {(cuuint32_t)(row_bytes / esize), 32u};
+  const cuuint32_t box[2] = {(cuuint32_t)(row_bytes / esize), (cuuint32_t)box_rows};
   const cuuint32_t estr[2] = {1, 1};
   const CUresult r = enc(tm, esize == 2 ? CU_TENSOR_MAP_DATA_TYPE_UINT16 : CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, ptr,
                          dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -1800,7 +1809,13 @@ static int run_gemm(const void* a, int64_t ld_a, const void* w, int64_t ld_w, Ge
     if (make_slab_map(&sa_map, a, p.M, p.K, ld_a, a_rows, 4) == IFLB200_OK &&
         make_slab_map(&sw_map, w, p.N, p.K, ld_w, bn, 4) == IFLB200_OK) {
       g_last_launch[3] = 104;
-      return launch_gemm_form<64, 2, 2, false, false, kEpilogueWarps, 4>(sa_map, sw_map, to, p, grid, s);
+      if (split > 1 || !p.tma_store) return launch_gemm_form<64, 2, 2, false, false, kEpilogueWarps, 4>(sa_map, sw_map, to, p, grid, s);
+      p.m64 = p.M <= 64;
+      if (p.m64) {
+        st = make_out_map(&to, p.out, p.M, p.N, p.ld_out, oes, p.half_rows ? 64 : 128, 16);
+        if (st != IFLB200_OK) return st;
+      }
+      return launch_gemm_form<64, 2, 4, false, false, kEpilogueWarps, 4>(sa_map, sw_map, to, p, grid, s);
     }
   }
   switch (bn) {
@@ -1813,13 +1828,13 @@ static int run_gemm(const void* a, int64_t ld_a, const void* w, int64_t ld_w, Ge
   }
 }
 
-// [splits][M][N] fp32 partial sums; box = 32 columns (128 bytes) x 32 rows x 1 plane.
-static int make_partials_map(CUtensorMap* tm, void* ptr, int M, int N, int64_t ld, int splits) {
+// [splits][M][N] fp32 partial sums; box = 32 columns (128 bytes) x box_rows x 1 plane.
+static int make_partials_map(CUtensorMap* tm, void* ptr, int M, int N, int64_t ld, int splits, int box_rows) {
   EncodeTiledFn enc = get_encode_fn();
   if (!enc) return IFLB200_ERR_DRIVER;
   const cuuint64_t dims[3] = {(cuuint64_t)N, (cuuint64_t)M, (cuuint64_t)splits};
   const cuuint64_t strides[2] = {(cuuint64_t)ld * 4, (cuuint64_t)ld * 4 * (cuuint64_t)M};
-  const cuuint32_t box[3] = {32u, 32u, 1u};
+  const cuuint32_t box[3] = {32u, (cuuint32_t)box_rows, 1u};
   const cuuint32_t estr[3] = {1, 1, 1};
   const CUresult r = enc(tm, CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, ptr, dims, strides, box, estr,
                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
@@ -1863,7 +1878,7 @@ static int run_gemm_partials(const void* a, int64_t ld_a, const void* w, int64_t
   const int a_rows = activation_box_rows(M);
   p.a_bytes = a_rows * BK;
   CUtensorMap ta, tw, to;
-  st = make_partials_map(&to, out, M, N, ld_out, splits);
+  st = make_partials_map(&to, out, M, N, ld_out, splits, M <= 64 ? 16 : 32);
   if (st != IFLB200_OK) return st;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (M <= BM) {
@@ -1872,7 +1887,8 @@ static int run_gemm_partials(const void* a, int64_t ld_a, const void* w, int64_t
     st = make_slab_map(&tw, w, N, K, ld_w, 64, 4);
     if (st != IFLB200_OK) return st;
     g_last_launch[0] = 1 + 16; g_last_launch[1] = 64; g_last_launch[2] = splits; g_last_launch[3] = 104;
-    return launch_gemm_form<64, 2, 2, false, false, kEpilogueWarps, 4>(ta, tw, to, p, p.num_tiles * splits, s);
+    p.m64 = M <= 64;
+    return launch_gemm_form<64, 2, 4, false, false, kEpilogueWarps, 4>(ta, tw, to, p, p.num_tiles * splits, s);
   }
   // CTA pairs where blocks of 256 rows pad little and their units need no more waves: two thirds of the traffic per K step, which is what these launches wait for.
   // 816 x 2048 x 16384 in two ranges 28.6 against 29.7 us, 640 rows in three 22.8 against 23.3.
