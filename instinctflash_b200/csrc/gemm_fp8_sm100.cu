@@ -58,7 +58,6 @@ struct GemmParams {
   int out_dtype;
   int64_t ld_out;
   int split_k;     // > 1: the CTAs of a cluster share one tile, each a K range; partials are summed over DSMEM
-  int m64;         // lean form: MMAs of M = 64 (at most 64 rows; the output map's box has 16 rows then)
   int a_bytes;     // bytes one activation box delivers per K step: 128 x (rows of the box)
   int partials;    // > 1: K is split over that many independent CTAs per tile; each writes its fp32 partial
                    // accumulator to out[split][M][ld_out] (summed in split order by the consumer)
@@ -123,14 +122,15 @@ __device__ __forceinline__ float ld_dsmem_f32(uint32_t addr) {
 // SL: 128-byte K slabs per stage.  With SL > 1 one TMA instruction per operand brings SL slabs (the
 // operands are mapped as [K / 128][rows][128 bytes]): a skinny GEMM's main loop is bound by the
 // rate at which one SM can issue TMA instructions (about 0.2 us each, measured), not by bytes.
-template <int BN, int STAGES, int EW = kEpilogueWarps, int SL = 1>
+// AR: activation rows of a stage (64: the lean form for at most 64 rows).
+template <int BN, int STAGES, int EW = kEpilogueWarps, int SL = 1, int AR = BM>
 struct SmemLayout {
-  static constexpr int kABytes = BM * BK * SL;
+  static constexpr int kABytes = AR * BK * SL;
   static constexpr int kBBytes = BN * BK * SL;
   static constexpr int kStageBytes = kABytes + kBBytes;
   // epilogue staging: one 32-row buffer per epilogue warp (TMA-store source), 128 bytes per row
-  // with eight epilogue warps, 64 with sixteen
-  static constexpr int kWarpStaging = EW > 8 ? 2048 : 4096;
+  // with eight epilogue warps, 64 with sixteen; a warp of the 64-row form has 16 rows
+  static constexpr int kWarpStaging = EW > 8 || AR == 64 ? 2048 : 4096;
   static constexpr int kStagingOffset = STAGES * kStageBytes;
   static constexpr int kBarOffset = kStagingOffset + EW * kWarpStaging;
   // full[STAGES], empty[STAGES], tmem_full[2], tmem_empty[2], then the TMEM base word and the
@@ -420,9 +420,10 @@ __device__ __forceinline__ void epilogue_values(const GemmParams& p, const uint3
 // Consumer arithmetic and output cast of 32 consecutive columns of this lane's row, written into
 // the lane's 128-byte staging row (128-byte swizzle: 16-byte chunk index ^ (lane & 7)).  `sub` is
 // the column offset inside the staged piece: 0 or 32 for two-byte outputs, 0 for four-byte ones.
+// `live`: the lane holds a row (a warp of the 64-row form has sixteen, and staging for no more).
 __device__ __forceinline__ void stage_columns(const GemmParams& p, const uint32_t (&r)[32], int n_abs, float rs,
                                               uint8_t* mine, int sub, int lane, bool pre = false, float csl = 0.0f,
-                                              float bsl = 0.0f) {
+                                              float bsl = 0.0f, bool live = true) {
   const int es = (p.out_dtype == IFLB200_F32) ? 4 : 2;
   if (es == 2) {
     // 32 values = 64 bytes = four 16-byte chunks; chunk index within the 128-byte row
@@ -437,7 +438,7 @@ __device__ __forceinline__ void stage_columns(const GemmParams& p, const uint32_
         u.y = pack_bf16x2(__uint_as_float(r[8 * j + 2]), __uint_as_float(r[8 * j + 3]));
         u.z = pack_bf16x2(__uint_as_float(r[8 * j + 4]), __uint_as_float(r[8 * j + 5]));
         u.w = pack_bf16x2(__uint_as_float(r[8 * j + 6]), __uint_as_float(r[8 * j + 7]));
-        *reinterpret_cast<uint4*>(mine + (((first + j) ^ sw) * 16)) = u;
+        if (live) *reinterpret_cast<uint4*>(mine + (((first + j) ^ sw) * 16)) = u;
       }
     } else {
       float y[32];
@@ -456,7 +457,7 @@ __device__ __forceinline__ void stage_columns(const GemmParams& p, const uint32_
           u.z = pack_f16x2(y[8 * j + 4], y[8 * j + 5]);
           u.w = pack_f16x2(y[8 * j + 6], y[8 * j + 7]);
         }
-        *reinterpret_cast<uint4*>(mine + (((first + j) ^ sw) * 16)) = u;
+        if (live) *reinterpret_cast<uint4*>(mine + (((first + j) ^ sw) * 16)) = u;
       }
     }
   } else {
@@ -464,8 +465,9 @@ __device__ __forceinline__ void stage_columns(const GemmParams& p, const uint32_
     epilogue_values(p, r, n_abs, rs, y, pre, csl, bsl);
 #pragma unroll
     for (int j = 0; j < 8; ++j)
-      *reinterpret_cast<float4*>(mine + ((j ^ (lane & 7)) * 16)) =
-          make_float4(y[4 * j + 0], y[4 * j + 1], y[4 * j + 2], y[4 * j + 3]);
+      if (live)
+        *reinterpret_cast<float4*>(mine + ((j ^ (lane & 7)) * 16)) =
+            make_float4(y[4 * j + 0], y[4 * j + 1], y[4 * j + 2], y[4 * j + 3]);
   }
 }
 
@@ -473,7 +475,7 @@ __device__ __forceinline__ void stage_columns(const GemmParams& p, const uint32_
 // memory.  128 bytes of each output row (64 two-byte or 32 four-byte columns) are staged with
 // the 128-byte swizzle and written by one TMA store, so global memory sees whole 128-byte lines
 // instead of 16-byte pieces of 32 different rows.
-template <int BN>
+template <int BN, int ROWS = 32>
 __device__ __forceinline__ void epilogue_tma_store(const GemmParams& p, const CUtensorMap* tm_out, uint32_t t_row,
                                                    uint32_t staging, uint8_t* staging_ptr, int row0, int n_base,
                                                    int col_begin, int col_end, float rs, int lane, int z = -1,
@@ -498,9 +500,9 @@ __device__ __forceinline__ void epilogue_tma_store(const GemmParams& p, const CU
         const int k = (c + sub - col_begin) >> 5;  // which of the warp's 32-column chunks (uniform)
         const float csl = k == 0 ? cv->cs[0] : (k == 1 ? cv->cs[1] : (k == 2 ? cv->cs[2] : cv->cs[3]));
         const float bsl = k == 0 ? cv->bs[0] : (k == 1 ? cv->bs[1] : (k == 2 ? cv->bs[2] : cv->bs[3]));
-        stage_columns(p, r, n0 + sub, rs, mine, sub, lane, true, csl, bsl);
+        stage_columns(p, r, n0 + sub, rs, mine, sub, lane, true, csl, bsl, lane < ROWS);
       } else {
-        stage_columns(p, r, n0 + sub, rs, mine, sub, lane);
+        stage_columns(p, r, n0 + sub, rs, mine, sub, lane, false, 0.0f, 0.0f, lane < ROWS);
       }
       GEMM_TRACE_IN_HELPER(11, threadIdx.x == 64 && c == col_begin && sub == 0);  // first chunk staged
     }
@@ -742,17 +744,18 @@ __device__ __forceinline__ void epilogue_swapped(const GemmParams& p, const CUte
 // GATED: the gated form (see epilogue_gated): a tile pairs BN/2 gate columns with the BN/2 up
 // columns of the same hidden units; p.N counts hidden units.
 // EW: epilogue warps (8, or 16 for the gated form: EW / 4 per TMEM lane quadrant).
-template <int BN, int STAGES, int SPLIT, bool SWAP = false, bool GATED = false, int EW = kEpilogueWarps, int SL = 1>
+template <int BN, int STAGES, int SPLIT, bool SWAP = false, bool GATED = false, int EW = kEpilogueWarps, int SL = 1, int AR = BM>
 __global__ void __launch_bounds__(96 + 32 * EW, 1)
 gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w,
                     const __grid_constant__ CUtensorMap tm_out, const GemmParams p) {
-  using L = SmemLayout<BN, STAGES, EW, SL>;
+  using L = SmemLayout<BN, STAGES, EW, SL, AR>;
+  static_assert(AR == BM || SPLIT == 4, "64-row stages: lean form only");
   static_assert(EW == kEpilogueWarps || GATED, "only the gated epilogue is written for more than eight warps");
   static_assert(SL == 1 || (!GATED && !SWAP), "several slabs per load: ordinary form only");
   // two accumulators, each at a power-of-two column offset; BN in {64, 128, 192, 224, 256}
   constexpr uint32_t kAccStride = BN <= 64 ? 64 : (BN <= 128 ? 128 : 256);
   constexpr uint32_t kTmemCols = 2 * kAccStride;
-  constexpr uint32_t kIdesc = make_idesc_e4m3_f32(BM, BN);
+  constexpr uint32_t kIdesc = make_idesc_e4m3_f32(AR, BN);
 
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
@@ -789,9 +792,7 @@ gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
   const bool partials = (SPLIT == 2 || LEAN) && p.partials > 1;
   const bool split = !partials && (SPLIT == 1 || (SPLIT == 2 && p.split_k > 1));
   // At most 64 rows: MMAs of M = 64, whose row i lies in lane i % 16 of quadrant i / 16
-  const bool m64 = LEAN && p.m64;
-  const int quad_rows = m64 ? 16 : 32;
-  const uint32_t idesc = m64 ? make_idesc_e4m3_f32(64, BN) : kIdesc;
+  constexpr int quad_rows = AR / 4;
   const int k_parts = partials || PLANES ? p.partials : (split ? p.split_k : 1);
   const int split_rank = partials ? (int)blockIdx.x % k_parts : (split ? (int)cluster_ctarank() : 0);
   // a unit of work is a tile, or (tile, K range) in the planes form
@@ -927,7 +928,7 @@ gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
 #pragma unroll
             for (int j = 0; j < BK / 32; ++j) {
               // 32 bytes further along K inside the swizzled 128-byte row: +2 in 16-byte units.
-              mma_f8f6f4(d_tmem, da + 2 * j, db + 2 * j, idesc, (kb + sl > kb0 || j > 0) ? 1u : 0u);
+              mma_f8f6f4(d_tmem, da + 2 * j, db + 2 * j, kIdesc, (kb + sl > kb0 || j > 0) ? 1u : 0u);
             }
           }
           mma_commit(empty_bar(stage));  // stage reusable once these MMAs have read it
@@ -1017,7 +1018,7 @@ gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
         // 224-wide tile (two-byte outputs) straight from registers
         const int per_store = (p.out_dtype == IFLB200_F32 || p.half_rows) ? 32 : 64;
         const int col_tma_end = col_begin + (col_end - col_begin) / per_store * per_store;
-        epilogue_tma_store<BN>(p, tm_dst, t_row, staging, staging_ptr, m_blk * BM + quad * quad_rows, n_blk * BN,
+        epilogue_tma_store<BN, quad_rows>(p, tm_dst, t_row, staging, staging_ptr, m_blk * BM + quad * quad_rows, n_blk * BN,
                                col_begin, col_tma_end, rs, lane,
                                PLANES ? unit % k_parts : (((SPLIT == 2 || LEAN) && p.partials >= 1) ? split_rank : -1),  // a plane map takes a 3-D store
                                prefetch ? &cv : nullptr);
@@ -1561,22 +1562,22 @@ static int g_cfg_slabs = 0;  // 1: one K slab per TMA instruction everywhere (ex
 static int g_cfg_gated_warps = 0;  // gated form, 256-wide tiles: 0 heuristic, 8 or 16 epilogue warps
 static int g_cfg_mode = 0;  // 0 auto, 1 single-CTA tiles only, 2 CTA pairs with one accumulator, 3 CTA pairs with two
 
-template <int BN, int STAGES, int SPLIT, bool SWAP = false, bool GATED = false, int EW = kEpilogueWarps, int SL = 1>
+template <int BN, int STAGES, int SPLIT, bool SWAP = false, bool GATED = false, int EW = kEpilogueWarps, int SL = 1, int AR = BM>
 static int launch_gemm_form(const CUtensorMap& ta, const CUtensorMap& tw, const CUtensorMap& to, const GemmParams& p,
                             int grid, cudaStream_t s) {
-  using L = SmemLayout<BN, STAGES, EW, SL>;
+  using L = SmemLayout<BN, STAGES, EW, SL, AR>;
   static_assert(L::kDynamic <= 227 * 1024, "stage ring + staging exceed the shared memory of an SM");
   static bool attr_set[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return IFLB200_ERR_DEVICE;
   if (!attr_set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_fp8_tc5_kernel<BN, STAGES, SPLIT, SWAP, GATED, EW, SL>,
+    cudaError_t e = cudaFuncSetAttribute(gemm_fp8_tc5_kernel<BN, STAGES, SPLIT, SWAP, GATED, EW, SL, AR>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, L::kDynamic);
     if (e != cudaSuccess) return (int)e;
     attr_set[dev] = true;
   }
-  const cudaError_t e = launch_dep(gemm_fp8_tc5_kernel<BN, STAGES, SPLIT, SWAP, GATED, EW, SL>, dim3(grid),
+  const cudaError_t e = launch_dep(gemm_fp8_tc5_kernel<BN, STAGES, SPLIT, SWAP, GATED, EW, SL, AR>, dim3(grid),
                                    dim3(96 + 32 * EW), L::kDynamic, s, p.split_k,
                                    dependent_launch_for(SWAP ? p.N : p.M), ta, tw, to, p);
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
@@ -1593,6 +1594,12 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tw, const CUten
     }
     return launch_gemm_form<BN, STAGES, 0>(ta, tw, to, p, grid, s);
   }
+}
+
+static int launch_lean(const CUtensorMap& ta, const CUtensorMap& tw, const CUtensorMap& to, const GemmParams& p, int grid,
+                       cudaStream_t s) {
+  return p.M <= 64 ? launch_gemm_form<64, 3, 4, false, false, kEpilogueWarps, 4, 64>(ta, tw, to, p, grid, s)
+                   : launch_gemm_form<64, 2, 4, false, false, kEpilogueWarps, 4>(ta, tw, to, p, grid, s);
 }
 
 template <int BN, int STAGES, int ACC, bool SWAP = false, bool PLANES = false>
@@ -1810,12 +1817,11 @@ static int run_gemm(const void* a, int64_t ld_a, const void* w, int64_t ld_w, Ge
         make_slab_map(&sw_map, w, p.N, p.K, ld_w, bn, 4) == IFLB200_OK) {
       g_last_launch[3] = 104;
       if (split > 1 || !p.tma_store) return launch_gemm_form<64, 2, 2, false, false, kEpilogueWarps, 4>(sa_map, sw_map, to, p, grid, s);
-      p.m64 = p.M <= 64;
-      if (p.m64) {
+      if (p.M <= 64) {  // the lean form stores sixteen rows at a time then
         st = make_out_map(&to, p.out, p.M, p.N, p.ld_out, oes, p.half_rows ? 64 : 128, 16);
         if (st != IFLB200_OK) return st;
       }
-      return launch_gemm_form<64, 2, 4, false, false, kEpilogueWarps, 4>(sa_map, sw_map, to, p, grid, s);
+      return launch_lean(sa_map, sw_map, to, p, grid, s);
     }
   }
   switch (bn) {
@@ -1869,8 +1875,17 @@ static int run_gemm_partials(const void* a, int64_t ld_a, const void* w, int64_t
   p.partials = splits;
   p.tma_store = 1;
   p.num_m = (M + BM - 1) / BM;
-  // more than 128 rows: 256-wide tiles (a (tile, range) unit per SM at 400 x 1024 x 4096 with eight ranges)
-  const int bn = M <= BM || N < 256 ? 64 : 256;
+  // more than 128 rows: the width with the least waves x steps x clocks (as in run_gemm; an fp32 tile's epilogue
+  // and the prologue are 4000 a wave)
+  int bn = 64;
+  if (M > BM && N >= 256) {
+    auto cost = [&](int width, int clocks) {
+      const int64_t units = (int64_t)p.num_m * ((N + width - 1) / width) * splits;
+      const int steps = ((num_k + 3) / 4 + splits - 1) / splits * 4;
+      return (units + dev->sm_count - 1) / dev->sm_count * ((int64_t)steps * clocks + 4000);
+    };
+    if (cost(256, 720) <= cost(64, 385)) bn = 256;
+  }
   p.num_n = (N + bn - 1) / bn;
   p.num_k = num_k;
   p.num_tiles = p.num_m * p.num_n;
@@ -1887,8 +1902,7 @@ static int run_gemm_partials(const void* a, int64_t ld_a, const void* w, int64_t
     st = make_slab_map(&tw, w, N, K, ld_w, 64, 4);
     if (st != IFLB200_OK) return st;
     g_last_launch[0] = 1 + 16; g_last_launch[1] = 64; g_last_launch[2] = splits; g_last_launch[3] = 104;
-    p.m64 = M <= 64;
-    return launch_gemm_form<64, 2, 4, false, false, kEpilogueWarps, 4>(ta, tw, to, p, p.num_tiles * splits, s);
+    return launch_lean(ta, tw, to, p, p.num_tiles * splits, s);
   }
   // CTA pairs where blocks of 256 rows pad little and their units need no more waves: two thirds of the traffic per K step, which is what these launches wait for.
   // 816 x 2048 x 16384 in two ranges 28.6 against 29.7 us, 640 rows in three 22.8 against 23.3.

@@ -25,8 +25,14 @@ __device__ __forceinline__ void row_dependency_wait() {
   __syncthreads();
 }
 
-// Row kernels let the next kernel in the stream be scheduled as soon as their last CTAs start.
+// Row kernels let the next kernel in the stream be scheduled as soon as their last CTAs start -- before
+// their own dependency wait where the caller says so (early_trigger_for).
 __device__ __forceinline__ void row_trigger() { grid_launch_dependents(); }
+__device__ __forceinline__ void row_begin(int early) {
+  if (early) row_trigger();
+  row_dependency_wait();
+  if (!early) row_trigger();
+}
 
 // CTAs have 256 threads.  A row is owned by a group of TPR threads, each holding IT chunks of 8
 // elements: narrow rows share a CTA (TPR = 32 / 64 / 128, one chunk per thread), wide rows take
@@ -242,6 +248,7 @@ __host__ __device__ constexpr int resnorm_min_blocks() {
 constexpr int kMaxMirrors = 7;  // copies of a result in the buffers of the other GPUs of a group of up to eight
 
 struct RowQuantArgs {
+  int early;  // see row_begin
   const void* x;
   int64_t ld_x;
   int M, K, iters;
@@ -277,8 +284,7 @@ __device__ __forceinline__ void write_row_max(const RowQuantArgs& a, int m, floa
 template <typename XT, int TPR, int IT, bool PLAIN, bool FAST>
 __global__ void __launch_bounds__(kRowThreads, PLAIN ? (IT <= 2 ? 4 : 3) : row_min_blocks<IT>())
 row_quant_kernel(const RowQuantArgs a) {
-  row_dependency_wait();  // inputs may come from the kernel before this one in the stream
-  row_trigger();
+  row_begin(a.early);  // inputs may come from the kernel before this one in the stream
   __shared__ float red[kRowThreads / 32];
   const int t = threadIdx.x % TPR;
   const int m = blockIdx.x * (kRowThreads / TPR) + threadIdx.x / TPR;
@@ -377,6 +383,7 @@ row_quant_kernel(const RowQuantArgs a) {
 // issue, not by HBM: ~40 instructions per element (the reference's ex2.approx / div.full chains).
 // --------------------------------------------------------------------------------------------
 struct GatedArgs {
+  int early;  // see row_begin
   const void* gu;
   int64_t ld_gu;
   int M, F, iters;
@@ -391,8 +398,7 @@ struct GatedArgs {
 template <typename XT, int TPR, int IT, bool FAST>
 __global__ void __launch_bounds__(kRowThreads, row_min_blocks<IT>())
 gated_act_quant_kernel(const GatedArgs a) {
-  row_dependency_wait();  // inputs may come from the kernel before this one in the stream
-  row_trigger();
+  row_begin(a.early);  // inputs may come from the kernel before this one in the stream
   __shared__ float red[kRowThreads / 32];
   const int t = threadIdx.x % TPR;
   const int m = blockIdx.x * (kRowThreads / TPR) + threadIdx.x / TPR;
@@ -506,6 +512,7 @@ __global__ void __launch_bounds__(256) dequant_rows_kernel(const DequantArgs a) 
 // residual_norm_quant: (f32 residual) 2D delta + 4D res in, 4D res + D codes out, + 4 bytes.
 // --------------------------------------------------------------------------------------------
 struct ResNormArgs {
+  int early;  // see row_begin
   void* res;
   int64_t ld_res;
   int M, D, iters;
@@ -552,8 +559,7 @@ __device__ __forceinline__ float round_through<__nv_bfloat16>(float x) {
 template <typename RT, int TPR, int IT, bool FAST>
 __global__ void __launch_bounds__(kRowThreads, resnorm_min_blocks<IT>())
 residual_norm_quant_kernel(const ResNormArgs a) {
-  row_dependency_wait();  // inputs may come from the kernel before this one in the stream
-  row_trigger();
+  row_begin(a.early);  // inputs may come from the kernel before this one in the stream
   __shared__ float red[3][kRowThreads / 32];
   const int t = threadIdx.x % TPR;
   const int m = blockIdx.x * (kRowThreads / TPR) + threadIdx.x / TPR;
@@ -752,8 +758,7 @@ residual_norm_planes_kernel(const ResNormArgs a) {
   __shared__ __align__(16) float red[3][kRowThreads / 32];
   constexpr int kStep = kRowThreads * 4;
   const int m = blockIdx.x, c = threadIdx.x * 4;
-  row_dependency_wait();  // inputs may come from the kernel before this one in the stream
-  row_trigger();
+  row_begin(a.early);  // inputs may come from the kernel before this one in the stream
   RT* rr = reinterpret_cast<RT*>(a.res) + (int64_t)m * a.ld_res + c;
   const int64_t mofs = a.mod_index ? (int64_t)a.mod_index[m] * a.D + c : c;
   const float drs = a.drow ? a.drow[m] : 1.0f;
@@ -1284,6 +1289,7 @@ static int row_quant_impl(const void* x, int x_dtype, int64_t ld_x, int M, int K
   a.row = row; a.col = col; a.bias = bias; a.gelu = gelu;
   a.q = reinterpret_cast<uint8_t*>(q); a.ld_q = ld_q; a.qs = qs;
   a.phase = phase; a.amax = amax;
+  a.early = early_trigger_for(reinterpret_cast<cudaStream_t>(stream));
   a.mirrors = mirrors;
   for (int k = 0; k < kMaxMirrors; ++k) {
     a.amax_mirror[k] = k < mirrors ? amax_mirrors[k] : nullptr;
@@ -1294,7 +1300,7 @@ static int row_quant_impl(const void* x, int x_dtype, int64_t ld_x, int M, int K
                     (!bias || aligned16(bias));
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (fast && gelu && phase == 0 && x_dtype != IFLB200_F32 && g_row_tpr_override == 0 &&
-      launch_gelu_quant_stream({x, ld_x, M, K, row, col, bias, a.q, ld_q, qs}, x_dtype == IFLB200_F16, s))
+      launch_gelu_quant_stream({x, ld_x, M, K, row, col, bias, a.q, ld_q, qs, a.early}, x_dtype == IFLB200_F16, s))
     return (int)cudaGetLastError();
   if (x_dtype == IFLB200_BF16) launch_row_quant<__nv_bfloat16>(a, fast, s);
   else if (x_dtype == IFLB200_F16) launch_row_quant<__half>(a, fast, s);
@@ -1336,9 +1342,8 @@ extern "C" int iflb200_row_max_sharded(const void* x, int x_dtype, int64_t ld_x,
 template <int Q>
 __global__ void __launch_bounds__(kRowThreads)
 quant_from_amax_kernel(const float* __restrict__ h, int64_t ld_h, int M, int F, const float* __restrict__ amax,
-                       float* __restrict__ amax_zero, uint8_t* __restrict__ q, int64_t ld_q, float* __restrict__ qs) {
-  row_dependency_wait();  // h and amax come from the kernel before this one in the stream
-  row_trigger();
+                       float* __restrict__ amax_zero, uint8_t* __restrict__ q, int64_t ld_q, float* __restrict__ qs, int early) {
+  row_begin(early);  // h and amax come from the kernel before this one in the stream
   const int m = blockIdx.y;
   const int c0 = blockIdx.x * (kRowThreads * 4 * Q) + threadIdx.x * 4;
   const float* src = h + (int64_t)m * ld_h + c0;
@@ -1363,9 +1368,8 @@ quant_from_amax_kernel(const float* __restrict__ h, int64_t ld_h, int M, int F, 
 // The same for any alignment and width.
 __global__ void __launch_bounds__(kRowThreads)
 quant_from_amax_any_kernel(const float* __restrict__ h, int64_t ld_h, int M, int F, const float* __restrict__ amax,
-                           float* __restrict__ amax_zero, uint8_t* __restrict__ q, int64_t ld_q, float* __restrict__ qs) {
-  row_dependency_wait();
-  row_trigger();
+                           float* __restrict__ amax_zero, uint8_t* __restrict__ q, int64_t ld_q, float* __restrict__ qs, int early) {
+  row_begin(early);
   const int m = blockIdx.y;
   const int c0 = (blockIdx.x * kRowThreads + threadIdx.x) * 8;
   float scale, inv;
@@ -1392,7 +1396,7 @@ extern "C" int iflb200_quant_from_amax(const float* h, int64_t ld_h, int M, int 
   uint8_t* codes = reinterpret_cast<uint8_t*>(q);
   auto launch = [&](auto kernel, int columns) {
     launch_dep(kernel, dim3((unsigned)((F + columns - 1) / columns), (unsigned)M), dim3(kRowThreads), 0, s, 1,
-               dependent_launch_for(M), h, ld_h, M, F, amax, amax_zero, codes, ld_q, qs);
+               dependent_launch_for(M), h, ld_h, M, F, amax, amax_zero, codes, ld_q, qs, early_trigger_for(s));
   };
   // few rows: shorter pieces, so that every SM has one
   if (!fast) launch(quant_from_amax_any_kernel, kRowThreads * 8);
@@ -1416,6 +1420,7 @@ extern "C" int iflb200_gated_act_quant(const void* gu, int gu_dtype, int64_t ld_
   GatedArgs a;
   a.gu = gu; a.ld_gu = ld_gu; a.M = M; a.F = F; a.row = row; a.col = col; a.act = act;
   a.q = reinterpret_cast<uint8_t*>(q); a.ld_q = ld_q; a.qs = qs;
+  a.early = early_trigger_for(reinterpret_cast<cudaStream_t>(stream));
   const int es = esize(gu_dtype);
   const bool fast = F % 8 == 0 && aligned16(gu) && (ld_gu * es) % 16 == 0 && aligned8(q) && ld_q % 8 == 0 &&
                     (!col || aligned16(col));
@@ -1501,6 +1506,7 @@ static int resnorm_impl(void* res, int res_dtype, int64_t ld_res, int M, int D, 
   a.q = reinterpret_cast<uint8_t*>(q); a.ld_q = ld_q; a.qs = qs;
   a.y = y; a.y_dtype = y_dtype; a.ld_y = ld_y;
   a.mirrors = mirrors;
+  a.early = early_trigger_for(reinterpret_cast<cudaStream_t>(stream));
   bool mirrors_ok = true;
   for (int k = 0; k < kMaxMirrors; ++k) {
     a.q_mirror[k] = k < mirrors ? reinterpret_cast<uint8_t*>(q_mirrors[k]) : nullptr;
@@ -1530,7 +1536,7 @@ static int resnorm_impl(void* res, int res_dtype, int64_t ld_res, int M, int D, 
   if (fast && res_dtype == IFLB200_BF16 && layernorm && q && !y && !mod_index && (write_res || !delta) &&
       !(modulated && (weight || beta)) && g_row_tpr_override == 0 &&
       launch_residual_norm_stream({res, ld_res, M, D, a.delta, ld_delta, a.drow, a.dcol, a.bias, a.gate,
-                                   modulated ? mod_scale : weight, modulated ? mod_shift : beta, modulated, eps, a.q, ld_q, qs}, s))
+                                   modulated ? mod_scale : weight, modulated ? mod_shift : beta, modulated, eps, a.q, ld_q, qs, a.early}, s))
     return (int)cudaGetLastError();
   if (res_dtype == IFLB200_F32) launch_resnorm<float>(a, fast, s);
   else launch_resnorm<__nv_bfloat16>(a, fast, s);

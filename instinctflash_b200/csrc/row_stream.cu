@@ -197,8 +197,9 @@ __global__ void __launch_bounds__(THREADS, 1) gelu_quant_stream_kernel(const Gel
   const XT* x = reinterpret_cast<const XT*>(a.x) + t * 8;
   for (int i = threadIdx.x; i < 2 * kMaxGroups * kMaxWarps; i += blockDim.x) (&red[0][0][0])[i] = 0.0f;
 
+  if (a.early) grid_launch_dependents();
   grid_dependency_wait();  // inputs may come from the kernel before this one in the stream
-  grid_launch_dependents();
+  if (!a.early) grid_launch_dependents();
   const int stride = gridDim.x * groups;
   int m = blockIdx.x * groups + g;
   float rs = 1.0f;
@@ -292,8 +293,9 @@ __global__ void __launch_bounds__(kResNormThreads, 1) residual_norm_stream_kerne
   const float fD = (float)a.D;
   for (int i = threadIdx.x; i < 3 * kMaxGroups * kMaxWarps; i += blockDim.x) (&red[0][0][0])[i] = 0.0f;
 
+  if (a.early) grid_launch_dependents();
   grid_dependency_wait();  // inputs may come from the kernel before this one in the stream
-  grid_launch_dependents();
+  if (!a.early) grid_launch_dependents();
   const int stride = gridDim.x * groups;
   int m = blockIdx.x * groups + g;
   float rs = 1.0f;

@@ -20,6 +20,7 @@ struct GeluStreamArgs {
   uint8_t* q;
   int64_t ld_q;
   float* qs;
+  int early;  // let the next kernel be scheduled before the dependency wait
 };
 // x: bf16 or f16, every buffer on the 16-byte rule (codes: 8), K a multiple of 8
 bool launch_gelu_quant_stream(const GeluStreamArgs& a, bool half, cudaStream_t s);
@@ -39,6 +40,7 @@ struct ResNormStreamArgs {
   uint8_t* q;
   int64_t ld_q;
   float* qs;
+  int early;  // let the next kernel be scheduled before the dependency wait
 };
 // layer norm of a bf16 residual, updated in place when there is a delta; every buffer on the 16-byte
 // rule (codes: 8), D a multiple of 8

@@ -14,6 +14,7 @@ through memory.
 from __future__ import annotations
 
 from dataclasses import dataclass
+from functools import lru_cache
 
 import torch
 
@@ -180,21 +181,41 @@ def fp8_linear_gated(a: torch.Tensor, a_scale: torch.Tensor, w: Fp8Weight, h: to
     return h
 
 
+@lru_cache(maxsize=None)
 def partial_splits(M: int, N: int, K: int, sm_count: int = 148) -> int:
-    """How many K ranges ``gemm_partials`` should use for a skinny projection: enough (tile, range)
-    pairs to occupy the GPU, every range at least four 128-byte K slabs, at most eight planes.
+    """How many K ranges ``gemm_partials`` should use for a narrow projection whose consumer adds the
+    planes: up to 128 rows enough (tile, range) pairs to occupy the GPU, every range at least four
+    128-byte K slabs, at most eight planes.
 
-    Above 128 rows the planes pay where one wave of tiles leaves much of the GPU idle and the
-    reduction is deep (a range of at least sixteen slabs outlasts its fp32 tile): the consumer adds the
-    planes on its way, while the cluster form of the GEMM exchanges them through distributed shared memory
-    first."""
+    Above 128 rows the number with the least estimated time, 1 where the unsplit GEMM is as good.  In SM clocks: a
+    slab of a 128 x 64 / 256 tile 385 / 720 (bytes through the shared-memory port), 4000 a wave for
+    prologue and fp32 epilogue (2500 for bf16), every plane written and read back at 2500 bytes a clock.
+    Four decoder layers of 2048 x 16384: 315 -> 300 us at 301 rows (six planes against the GEMM that splits
+    K over a cluster), 438 -> 402 at 640 (three)."""
     if K % 128:
         return 1
+    slabs = K // 128
     if M <= 128:
-        tiles, slabs = (N + 63) // 64, 4
-    else:
-        tiles, slabs = ((M + 127) // 128) * ((N + 255) // 256), 16
-    return max(1, min(8, sm_count // max(1, tiles), (K // 128) // slabs))
+        return max(1, min(8, sm_count // max(1, (N + 63) // 64), slabs // 4))
+    blocks, plane = (M + 127) // 128, 8 * M * N // 2500
+
+    def cost(splits, width, clocks, wave):
+        units = blocks * ((N + width - 1) // width) * splits
+        steps = min(slabs, 4 * -(-(-(-slabs // 4)) // splits))
+        return -(-units // sm_count) * (steps * clocks + wave)
+
+    plain = [(width, clocks) for width, clocks in ((64, 385), (128, 510), (256, 720)) if width == 64 or N >= width]
+    unsplit = min(cost(1, w, c, 2500) for w, c in plain)
+    for ranges in (2, 4):   # over a cluster: one wave, partial sums handed over through distributed shared memory
+        for width, clocks in plain:
+            if blocks * ((N + width - 1) // width) * ranges <= sm_count and slabs // ranges >= 8 and width // ranges >= 32:
+                unsplit = min(unsplit, slabs // ranges * clocks + 7500 + 65 * width * (ranges - 1) // ranges)
+    best, least = 1, unsplit + plane // 2
+    for splits in range(2, min(8, (slabs + 3) // 4) + 1):
+        time = min(cost(splits, w, c, 4000) for w, c in plain if w != 128) + splits * plane
+        if time < least:
+            best, least = splits, time
+    return best
 
 
 def gemm_partials(a: torch.Tensor, w: Fp8Weight, out: torch.Tensor) -> torch.Tensor:

@@ -10,7 +10,7 @@ The same driver runs any set of operators with the reference's signatures (``ops
 so the reference's own kernels can be timed through it.
 
 With this package's operators the driver uses the fused forms by default (``fused="auto"``: for
-more than 128 rows): the gated activation is evaluated in the gate_up GEMM's epilogue (``fp8_linear_gated`` +
+more than 64 rows): the gated activation is evaluated in the gate_up GEMM's epilogue (``fp8_linear_gated`` +
 ``row_quant_from_amax`` instead of ``gemm`` + ``gated_act_quant``), bit-identical to the unfused
 sequence; ``fused=False`` keeps the reference's three-launch structure per linear.
 """
@@ -162,11 +162,12 @@ class LinearStack:
         split_rows = spec.M if split_rows is None else split_rows
         self.spec, self.weights, self.dev = spec, weights, torch.device(device)
         self.ops = ops or native_ops()
-        # fused forms exist only in this package's operator set; "auto" takes the gated epilogue where the
-        # GEMM is long enough to hide it (measured: with M = 50 the two-kernel gated form is slower
-        # than gemm + gated_act_quant, whose single row kernel costs one short launch)
+        # fused forms exist only in this package's operator set; "auto" takes the gated epilogue where its
+        # extra short launch costs no more than the row kernel it replaces (a layer of 1024 x 4096: 26.6
+        # against 27.1 us at 50 rows, equal at 64, 30.9 against 30.4 at 96; 2048 x 16384 at 80 rows 58.1
+        # against 54.0)
         if fused == "auto":
-            fused = spec.M > 128
+            fused = spec.M > 64
         self.fused = bool(fused) and hasattr(self.ops, "fp8_linear_gated")
         self.fuse_residual = fuse_residual and hasattr(self.ops, "fp8_linear_residual")
         # deep, narrow projections (down, o) whose tiles do not fill the GPU run split-K over independent CTAs, the
