@@ -372,20 +372,20 @@ class EpisodeBatch:
     """``episodes`` independent inferences of one stack on one GPU over shared weights.  Independent robot
     episodes are what the skinny action-expert configuration shards over GPUs; this is the per-GPU part.
 
-    Skinny decoder stacks (at most 128 rows an episode) run stacked along the rows: one launch per operator
-    for all episodes.  Every operator works row by row and the K ranges stay those of one episode, so
-    each episode has the bits of a stack of its own.  As parallel branches of one graph the GPU's
-    front end could not feed the branches -- 8 episodes of 50 rows, 18 layers: 864 kernels at 1.7 us each,
-    1498 us, against 108 kernels of 400 rows.  Other stacks, whose kernels fill the GPU by themselves,
-    are captured as parallel branches: one ``LinearStack`` each."""
+    Decoder stacks run stacked along the rows: one launch per operator for all episodes.  Every operator
+    works row by row; up to 128 rows an episode the K ranges stay those of one episode, so each has the
+    bits of a stack of its own, above that only the order of a K-split sum may differ.  As parallel
+    branches of one graph the GPU's front end could not feed the branches -- 8 episodes of 50 rows, 18
+    layers: 864 kernels at 1.7 us each, 1498 us, against 90 kernels of 400 rows.  Other stacks are captured
+    as parallel branches: one ``LinearStack`` each."""
 
     def __init__(self, spec: StackSpec, weights, device, episodes: int, **stack_kw):
         self.spec, self.dev, self.episodes = spec, torch.device(device), episodes
         self.launches_per_forward = 0   # of all episodes: a launch counts once for every episode it serves
         self.merged = None
-        if spec.kind == "gemma" and spec.M <= 128 and episodes > 1 and spec.M * episodes <= 65535:
+        if spec.kind == "gemma" and episodes > 1 and spec.M * episodes <= 65535:
             wide = StackSpec(**{**spec.__dict__, "M": spec.M * episodes})
-            merged = LinearStack(wide, weights, device, split_rows=spec.M, **stack_kw)
+            merged = LinearStack(wide, weights, device, split_rows=spec.M if spec.M <= 128 else None, **stack_kw)
             if hasattr(merged.ops, "gemm_partials"):    # this package's operators: K ranges by rows of one episode
                 self.merged = merged
                 self.attn_rows = torch.zeros(wide.M, max(spec.o_in, 16), dtype=torch.bfloat16, device=self.dev)
