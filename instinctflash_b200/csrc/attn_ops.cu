@@ -27,6 +27,7 @@
 namespace iflb200 {
 
 constexpr int kCombineThreads = 512;
+constexpr int kCombineMaxCluster = 8;
 constexpr int kCombineIters = 4;  // 512 threads x 4 chunks x 4 values = 8192 values per token row
 
 struct CombineArgs {
@@ -39,31 +40,37 @@ struct CombineArgs {
   uint8_t* q;
   int64_t ld_q;
   float* qs;
-  int tokens, batch, group, heads_kv, head_dim, block_d, splits;
+  int tokens, batch, group, heads_kv, head_dim, block_d, splits, cluster;
 };
 
 // The partials of a chunk come in groups of kGroup splits, every load of a group issued before the first is
-// used: with at most kGroup splits (the engines' geometry) a token is one memory round trip.  Split by split it
-// was a chain of dependent ones (50 tokens x 8 heads x 256, 8 splits: 4.5 us between launches).
-constexpr int kGroup = 8;
-
-template <int IT>
-__global__ void __launch_bounds__(kCombineThreads) attn_combine_quant_kernel(const CombineArgs a) {
+// used: with at most kGroup = 8 splits (the engines' geometry) a token is one memory round trip.  Split by split
+// it was a chain of dependent ones (50 tokens x 8 heads x 256, 8 splits: 4.5 -> 3.1 us between launches).
+// Groups of four where there are tokens for two CTAs per SM, whose phases then cover each other.
+// CL: a cluster of a.cluster CTAs shares a token's chunks -- for few tokens, whose CTAs would each pull hundreds of
+// KB through one SM (28 tokens x 16 heads x 256, 12 splits: 7.9 us with one CTA per token) -- and the
+// row maximum meets in distributed shared memory.
+template <int IT, bool CL, int kGroup>
+__global__ void __launch_bounds__(kCombineThreads, kGroup == 4 ? 2 : 1) attn_combine_quant_kernel(const CombineArgs a) {
   const int threads = blockDim.x;
   grid_dependency_wait();  // the partials come from the kernel before this one in the stream
   grid_launch_dependents();
   __shared__ float red[kCombineThreads / 32];
-  const int t = blockIdx.x, b = blockIdx.y;
+  __shared__ float maxima[kCombineMaxCluster];
+  const int t = CL ? blockIdx.x / a.cluster : blockIdx.x, b = blockIdx.y;
   const int chunks_per_head = a.head_dim / 4;
   const int heads = a.group * a.heads_kv;
-  const int total = heads * chunks_per_head;
+  const int all = heads * chunks_per_head;
+  const int share = CL ? (all + a.cluster - 1) / a.cluster : all;
+  const int first = CL ? (int)cluster_ctarank() * share : 0;
+  const int total = min(all, first + share);  // this CTA's chunks: [first, total)
   const int n_rows = a.tokens * a.group;
   const int64_t plane = (int64_t)a.batch * a.heads_kv * n_rows;  // rows of one split
   float out[IT][4];
   float amax = 0.0f;
 #pragma unroll
   for (int it = 0; it < IT; ++it) {
-    const int c = it * threads + threadIdx.x;
+    const int c = first + it * threads + threadIdx.x;
 #pragma unroll
     for (int i = 0; i < 4; ++i) out[it][i] = 0.0f;
     if (c < total) {
@@ -137,13 +144,23 @@ __global__ void __launch_bounds__(kCombineThreads) attn_combine_quant_kernel(con
 #pragma unroll
   for (int i = 1; i < kCombineThreads / 32; ++i)
     if (i < threads / 32) amax = max_f32(amax, red[i]);
+  if (CL) {
+    if ((int)threadIdx.x < a.cluster) {
+      uint32_t peer;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(smem_u32(&maxima[cluster_ctarank()])), "r"(threadIdx.x));
+      asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(peer), "f"(amax) : "memory");
+    }
+    cluster_sync_all();
+    amax = maxima[0];
+    for (int i = 1; i < a.cluster; ++i) amax = max_f32(amax, maxima[i]);
+  }
   float scale, inv;
   quant_scales(amax, scale, inv);
-  if (threadIdx.x == 0) a.qs[t] = scale;
+  if (threadIdx.x == 0 && first == 0) a.qs[t] = scale;
   uint8_t* qr = a.q + (int64_t)t * a.ld_q;
 #pragma unroll
   for (int it = 0; it < IT; ++it) {
-    const int c = it * threads + threadIdx.x;
+    const int c = first + it * threads + threadIdx.x;
     if (c < total) {
       const int head = c / chunks_per_head, d = (c - head * chunks_per_head) * 4;
       *reinterpret_cast<uint32_t*>(qr + (int64_t)head * a.head_dim + d) =
@@ -184,10 +201,17 @@ extern "C" int iflb200_attn_combine_quant(const float* po, const float* pm, cons
   a.head_dim = head_dim; a.block_d = block_d; a.splits = splits;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   const int chunks = heads_q * (head_dim / 4);
-  const dim3 grid(tokens, batch), block(chunks <= 128 ? 128 : (chunks <= 256 ? 256 : kCombineThreads));
+  // a cluster per token while half of the GPU would stay idle and every CTA keeps a chunk per thread of four warps
+  a.cluster = 1;
+  while (a.cluster < kCombineMaxCluster && (int64_t)tokens * batch * a.cluster * 2 <= 148 && chunks >= 256 * a.cluster) a.cluster *= 2;
+  const int share = (chunks + a.cluster - 1) / a.cluster;
+  const dim3 grid(tokens * a.cluster, batch), block(share <= 128 ? 128 : (share <= 256 ? 256 : kCombineThreads));
   const bool dep = dependent_launch_for(tokens);
-  const cudaError_t e = chunks <= kCombineThreads       ? launch_dep(attn_combine_quant_kernel<1>, grid, block, 0, s, 1, dep, a)
-                        : chunks <= 2 * kCombineThreads ? launch_dep(attn_combine_quant_kernel<2>, grid, block, 0, s, 1, dep, a)
-                                                        : launch_dep(attn_combine_quant_kernel<kCombineIters>, grid, block, 0, s, 1, dep, a);
+  cudaError_t e;
+  auto go = [&](auto kernel) { return launch_dep(kernel, grid, block, 0, s, a.cluster, dep, a); };
+  if (a.cluster > 1) e = share <= kCombineThreads ? go(attn_combine_quant_kernel<1, true, 8>) : go(attn_combine_quant_kernel<kCombineIters, true, 8>);
+  else if (chunks <= kCombineThreads) e = tokens <= 296 ? go(attn_combine_quant_kernel<1, false, 8>) : go(attn_combine_quant_kernel<1, false, 4>);
+  else if (chunks <= 2 * kCombineThreads) e = tokens <= 148 ? go(attn_combine_quant_kernel<2, false, 8>) : go(attn_combine_quant_kernel<2, false, 4>);
+  else e = go(attn_combine_quant_kernel<kCombineIters, false, 4>);
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }

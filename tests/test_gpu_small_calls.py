@@ -35,7 +35,7 @@ def test_one_launch_pack(n, kind):
         assert torch.equal(u8(q), u8(want))
 
 
-@pytest.mark.parametrize("tokens,hq,hkv,hd,splits", [(3, 8, 1, 256, 9), (2, 16, 2, 64, 17), (1, 32, 8, 256, 8), (5, 4, 4, 20, 1)])
+@pytest.mark.parametrize("tokens,hq,hkv,hd,splits", [(3, 8, 1, 256, 9), (2, 16, 2, 64, 17), (1, 32, 8, 256, 8), (5, 4, 4, 20, 1), (70, 16, 4, 100, 3)])
 def test_merge_of_more_splits_than_a_group(tokens, hq, hkv, hd, splits):
     from instinctflash_b200.kernels import attention
     from oracle import oracle as O
