@@ -127,3 +127,33 @@ def test_wan_qkv_rows(lib, B, T, H, HD, parts, norm, dtype):
             mag = e.reshape(-1, 2).norm(dim=1).repeat_interleave(2).reshape(e.shape)
             assert ((a - e).abs() <= ulp * mag + 1e-6).all(), (i, ((a - e).abs() / mag).max())
     assert (q[:, D:] == 7.0).all()
+
+
+# one token; a CTA's tokens not whole, a unit round not whole; many tokens; wide heads; no norm (every bit then)
+@pytest.mark.parametrize("T,HQ,HKV,HD,norm", [(1, 8, 1, 64, True), (3001, 5, 1, 64, True), (611, 12, 4, 128, False), (301, 10, 2, 256, True), (1501, 3, 2, 256, True),
+                                              (2400, 16, 4, 64, False)])
+def test_qkv_split_tokens_per_cta(lib, T, HQ, HKV, HD, norm):
+    from instinctflash_b200.kernels import rope
+    from oracle import oracle as O
+    g = torch.Generator(device=DEV).manual_seed(T)
+    W = (HQ + 2 * HKV) * HD
+    raw = torch.randn(T, W, device=DEV, generator=g).to(torch.bfloat16)
+    kw = dict(heads_q=HQ, heads_kv=HKV, head_dim=HD)
+    per_row = dict(row=torch.rand(T, device=DEV, generator=g), pos=(torch.rand(T, 2, device=DEV, generator=g) * 900).floor())
+    vec = dict(col=torch.rand(W, device=DEV, generator=g), bias=torch.randn(W, device=DEV, generator=g),
+               inv_freq=rope.rope_inv_freq(HD, 10000.0, DEV), sections=(torch.arange(HD // 2, device=DEV) % 2).int())
+    if norm:
+        vec.update(q_norm=torch.rand(HD, device=DEV, generator=g) + 0.5, k_norm=torch.rand(HD, device=DEV, generator=g) + 0.5)
+    q = torch.full((T, HQ, HD), 7.0, device=DEV, dtype=torch.float16)
+    k, v = (torch.full((T + 9, HKV, HD), 7.0, device=DEV, dtype=torch.float16) for _ in range(2))
+    rope.qkv_split(raw, q, k, v, kv_base=5, **kw, **per_row, **vec)
+    torch.cuda.synchronize()
+    pick = torch.tensor(sorted({0, T // 3, T - 1}), device=DEV)
+    qo, ko, vo = O.qkv_split(raw[pick].cpu(), kv_rows=len(pick), **kw, **{n: t[pick].cpu() for n, t in per_row.items()},
+                             **{n: t.cpu() for n, t in vec.items()})
+    assert torch.equal(v[5 + pick].cpu(), vo)   # V: no sum and no angle in it
+    for a, e in ((q[pick].cpu().float(), qo.float()), (k[5 + pick].cpu().float(), ko.float())):
+        # a rounding of the output and one of sine or cosine, relative to the pair it rotates
+        mag = torch.stack((e[..., :HD // 2], e[..., HD // 2:])).norm(dim=0).repeat(1, 1, 2)
+        assert ((a - e).abs() <= 2.0 ** -10 * mag + 1e-6).all()
+    assert (k[:5] == 7.0).all() and (v[5 + T:] == 7.0).all()
