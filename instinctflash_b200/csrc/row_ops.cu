@@ -1073,15 +1073,15 @@ pack_kernel(const uint16_t* __restrict__ x, int64_t n, const uint32_t* __restric
     q[i] = (uint8_t)(cvt_e4m3x2(pack_one(__uint_as_float((uint32_t)x[i] << 16), scale), 0.0f) & 0xFF);
 }
 
-// Small tensors: the whole dynamic pack in one launch.  A cluster of eight CTAs keeps the tensor in
-// registers between the maximum and the cast; the maxima of the CTAs meet in distributed shared memory.
-// The two kernels above are two launches and two passes for a few microseconds of work: 50 x 1024
-// inputs took 5 us of a 10 us projection.  Up to 2^17 elements; above, eight SMs are
-// slower than two passes of the whole GPU.
-constexpr int kPackCluster = 8, kPackClusterThreads = 1024;
-constexpr int64_t kPackClusterMax = (int64_t)kPackCluster * kPackClusterThreads * 8 * 2;
+// Small tensors: the whole dynamic pack in one launch.  A cluster of eight CTAs (sixteen above 2^18
+// elements) keeps the tensor in registers between the maximum and the cast; the maxima of the CTAs meet in
+// distributed shared memory.  The two kernels above are two launches and two passes: 4.1 us whatever the size,
+// against 2.0 here at 2^16 elements, 3.2 at 2^18, 3.4 at 2^19; a cluster takes 4.3 for 680 thousand, so above
+// 2^19 they stay.
+constexpr int kPackClusterThreads = 1024;
+constexpr int64_t kPackClusterMax = (int64_t)16 * kPackClusterThreads * 8 * 4;
 
-template <int V>
+template <int kPackCluster, int V>
 __global__ void __cluster_dims__(kPackCluster, 1, 1) __launch_bounds__(kPackClusterThreads)
 pack_cluster_kernel(const uint4* __restrict__ x, int nvec, float* __restrict__ scale_out, uint2* __restrict__ q) {
   __shared__ uint32_t red[kPackClusterThreads / 32];
@@ -1599,11 +1599,26 @@ static int pack_grid(int64_t n) {
 static bool launch_pack_cluster(const void* x, int64_t n, void* q, float* scale, cudaStream_t s) {
   if (n > kPackClusterMax || n % 8 || !aligned16(x) || !aligned8(q)) return false;
   const int nvec = (int)(n / 8);
-  const dim3 grid(kPackCluster), block(kPackClusterThreads);
   auto xv = reinterpret_cast<const uint4*>(x);
   auto qv = reinterpret_cast<uint2*>(q);
-  if (nvec <= kPackCluster * kPackClusterThreads) launch_dep(pack_cluster_kernel<1>, grid, block, 0, s, 1, dependent_launch_for(1), xv, nvec, scale, qv);
-  else launch_dep(pack_cluster_kernel<2>, grid, block, 0, s, 1, dependent_launch_for(1), xv, nvec, scale, qv);
+  auto go = [&](auto kernel, int ctas) {
+    launch_dep(kernel, dim3(ctas), dim3(kPackClusterThreads), 0, s, 1, dependent_launch_for(1), xv, nvec, scale, qv);
+  };
+  const int per_thread = (nvec + 8 * kPackClusterThreads - 1) / (8 * kPackClusterThreads);  // on eight CTAs
+  if (per_thread <= 1) go(pack_cluster_kernel<8, 1>, 8);
+  else if (per_thread <= 2) go(pack_cluster_kernel<8, 2>, 8);
+  else if (per_thread <= 4) go(pack_cluster_kernel<8, 4>, 8);
+  else {
+    static bool granted[64] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+    if (!granted[dev]) {
+      if (cudaFuncSetAttribute(pack_cluster_kernel<16, 4>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+        return false;
+      granted[dev] = true;
+    }
+    go(pack_cluster_kernel<16, 4>, 16);
+  }
   return true;
 }
 

@@ -10,8 +10,8 @@ DEV = "cuda"
 E4M3 = torch.float8_e4m3fn
 
 
-# one chunk; a CTA of the cluster empty; one register chunk per thread full, and one over; the largest, and one over
-@pytest.mark.parametrize("n", [8, 8 * 1023, 65536, 65544, 131072, 131080])
+# one chunk; a CTA of the cluster empty; every count of register chunks and cluster size full, and one over
+@pytest.mark.parametrize("n", [8, 8 * 1023, 65536, 65544, 131072, 131080, 262144, 262152, 524288, 524296])
 @pytest.mark.parametrize("kind", ["normal", "zeros", "nan", "inf", "tiny"])
 def test_one_launch_pack(n, kind):
     from instinctflash_b200 import _lib
