@@ -22,6 +22,8 @@
 #include <cuda_runtime.h>
 #include <string.h>
 
+#include <type_traits>
+
 #include "../../include/iflb200.h"
 #include "launch.cuh"
 #include "rowmath.cuh"
@@ -74,6 +76,14 @@ struct GemmParams {
   int groups;
   int group_rows;
   const CUtensorMap* out_maps;
+};
+
+// The lean form's arguments: K need not be a multiple of 128.  Stages of whole slabs come through the slab maps
+// (K / 128 slabs); the stage that holds the ragged slab comes slab by slab through these, which read
+// zeros past the end of a row.
+struct LeanParams : GemmParams {
+  CUtensorMap a_tail, w_tail;
+  int full_slabs;  // K / 128
 };
 
 // role << 24 | barrier kind << 16 | low 16 bits of the tile counter; 0 = no timeout.
@@ -747,7 +757,8 @@ __device__ __forceinline__ void epilogue_swapped(const GemmParams& p, const CUte
 template <int BN, int STAGES, int SPLIT, bool SWAP = false, bool GATED = false, int EW = kEpilogueWarps, int SL = 1, int AR = BM>
 __global__ void __launch_bounds__(96 + 32 * EW, 1)
 gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w,
-                    const __grid_constant__ CUtensorMap tm_out, const GemmParams p) {
+                    const __grid_constant__ CUtensorMap tm_out,
+                    const __grid_constant__ std::conditional_t<SPLIT == 4, LeanParams, GemmParams> p) {
   using L = SmemLayout<BN, STAGES, EW, SL, AR>;
   static_assert(AR == BM || SPLIT == 4, "64-row stages: lean form only");
   static_assert(EW == kEpilogueWarps || GATED, "only the gated epilogue is written for more than eight warps");
@@ -865,6 +876,23 @@ gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
       for (int kb = kb0; kb < kb1; kb += SL) {
         ok = wait_bounded(empty_bar(ring.stage), ring.phase ^ 1, abort_flag, (1u << 24) | (1u << 16) | (it & 0xFFFF));
         if (!ok) break;
+        if constexpr (LEAN) {
+          const int have = min(SL, kb1 - kb);
+          if (kb + have > p.full_slabs) {  // the stage of the ragged slab
+            if (elect_one()) {
+              const uint32_t bar = full_bar(ring.stage), sa = base + ring.stage * L::kStageBytes, sw = sa + L::kABytes;
+              mbar_arrive_expect_tx(bar, (uint32_t)have * (bytes / SL));
+              for (int sl = 0; sl < have; ++sl) {
+                if (w_producer) tma_load_2d(sw + sl * BN * BK, &p.w_tail, bar, (kb + sl) * BK, n_blk * BN);
+                else tma_load_2d(sa + sl * p.a_bytes, &p.a_tail, bar, (kb + sl) * BK, a_row);
+              }
+            }
+            __syncwarp();
+            ring.arm();
+            ring.advance();
+            continue;
+          }
+        }
         if (elect_one()) {
           const uint32_t bar = full_bar(ring.stage), sa = base + ring.stage * L::kStageBytes, sw = sa + L::kABytes;
           mbar_arrive_expect_tx(bar, bytes);
@@ -885,6 +913,9 @@ gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
         if (weights && it == 0 && kb == kb0 + (STAGES - 1) * SL && elect_one()) {
           // the ring is full: until its first stage is free, pull the boxes behind it towards L2
           for (int kp = kb + SL; kp < kb1 && kp < kb0 + kPrefetchSteps; kp += SL) {
+            if constexpr (LEAN) {
+              if (kp >= p.full_slabs) break;
+            }
             if constexpr (SWAP) tma_prefetch_l2_2d(&tm_a, kp * BK, a_row);
             else if constexpr (GATED) tma_prefetch_l2_3d(&tm_w, kp * BK, n_blk * (BN / 2), 0);
             else if constexpr (SL > 1) tma_prefetch_l2_3d(&tm_w, 0, n_blk * BN, kp);
@@ -1455,7 +1486,7 @@ static int make_tensor_map(CUtensorMap* tm, const void* ptr, int rows, int K, in
   return r == CUDA_SUCCESS ? IFLB200_OK : IFLB200_ERR_DRIVER;
 }
 
-// [rows, K] e4m3 matrix, K a multiple of 128, seen as [K / 128][rows][128 bytes]: box = 128 bytes x
+// [rows, K] e4m3 matrix, its whole 128-byte slabs seen as [K / 128][rows][128 bytes]: box = 128 bytes x
 // box_rows x `slabs`, so that one load brings `slabs` consecutive 128-byte K slabs of the tile, each
 // laid out in shared memory like the box of make_tensor_map.
 static int make_slab_map(CUtensorMap* tm, const void* ptr, int rows, int K, int64_t ld, int box_rows, int slabs) {
@@ -1563,8 +1594,8 @@ static int g_cfg_gated_warps = 0;  // gated form, 256-wide tiles: 0 heuristic, 8
 static int g_cfg_mode = 0;  // 0 auto, 1 single-CTA tiles only, 2 CTA pairs with one accumulator, 3 CTA pairs with two
 
 template <int BN, int STAGES, int SPLIT, bool SWAP = false, bool GATED = false, int EW = kEpilogueWarps, int SL = 1, int AR = BM>
-static int launch_gemm_form(const CUtensorMap& ta, const CUtensorMap& tw, const CUtensorMap& to, const GemmParams& p,
-                            int grid, cudaStream_t s) {
+static int launch_gemm_form(const CUtensorMap& ta, const CUtensorMap& tw, const CUtensorMap& to,
+                            const std::conditional_t<SPLIT == 4, LeanParams, GemmParams>& p, int grid, cudaStream_t s) {
   using L = SmemLayout<BN, STAGES, EW, SL, AR>;
   static_assert(L::kDynamic <= 227 * 1024, "stage ring + staging exceed the shared memory of an SM");
   static bool attr_set[64] = {};
@@ -1596,9 +1627,27 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tw, const CUten
   }
 }
 
-static int launch_lean(const CUtensorMap& ta, const CUtensorMap& tw, const CUtensorMap& to, const GemmParams& p, int grid,
-                       cudaStream_t s) {
-  return p.M <= 64 ? launch_gemm_form<64, 3, 4, false, false, kEpilogueWarps, 4, 64>(ta, tw, to, p, grid, s)
+static int make_tensor_map(CUtensorMap* tm, const void* ptr, int rows, int K, int64_t ld, int box_rows);
+static int make_slab_map(CUtensorMap* tm, const void* ptr, int rows, int K, int64_t ld, int box_rows, int slabs);
+
+static int launch_lean(const void* a, int64_t ld_a, const void* w, int64_t ld_w, const CUtensorMap& to, const GemmParams& g,
+                       int grid, cudaStream_t s) {
+  LeanParams p;
+  static_cast<GemmParams&>(p) = g;
+  p.full_slabs = g.K / BK;
+  const int a_rows = g.a_bytes / BK;
+  CUtensorMap ta, tw;
+  int st = make_slab_map(&ta, a, g.M, g.K, ld_a, a_rows, 4);
+  if (st == IFLB200_OK) st = make_slab_map(&tw, w, g.N, g.K, ld_w, 64, 4);
+  if (g.K % BK) {
+    if (st == IFLB200_OK) st = make_tensor_map(&p.a_tail, a, g.M, g.K, ld_a, a_rows);
+    if (st == IFLB200_OK) st = make_tensor_map(&p.w_tail, w, g.N, g.K, ld_w, 64);
+  } else {
+    memset(&p.a_tail, 0, sizeof(p.a_tail));
+    memset(&p.w_tail, 0, sizeof(p.w_tail));
+  }
+  if (st != IFLB200_OK) return st;
+  return g.M <= 64 ? launch_gemm_form<64, 3, 4, false, false, kEpilogueWarps, 4, 64>(ta, tw, to, p, grid, s)
                    : launch_gemm_form<64, 2, 4, false, false, kEpilogueWarps, 4>(ta, tw, to, p, grid, s);
 }
 
@@ -1809,19 +1858,22 @@ static int run_gemm(const void* a, int64_t ld_a, const void* w, int64_t ld_w, Ge
   if (st != IFLB200_OK) return st;
   const int stages = g_cfg_stages;
   g_last_launch[0] = 1; g_last_launch[1] = bn; g_last_launch[2] = split; g_last_launch[3] = stages;
-  // Skinny regime (64-wide tiles): four K slabs per TMA instruction where the layout allows it
-  // (K a multiple of 128, at least one full stage per CTA); the K order is unchanged, so are the bits.
-  if (bn == 64 && g_cfg_slabs != 1 && p.K % BK == 0 && p.num_k / split >= 4 && stages == 0) {
-    CUtensorMap sa_map, sw_map;
-    if (make_slab_map(&sa_map, a, p.M, p.K, ld_a, a_rows, 4) == IFLB200_OK &&
-        make_slab_map(&sw_map, w, p.N, p.K, ld_w, bn, 4) == IFLB200_OK) {
-      g_last_launch[3] = 104;
-      if (split > 1 || !p.tma_store) return launch_gemm_form<64, 2, 2, false, false, kEpilogueWarps, 4>(sa_map, sw_map, to, p, grid, s);
+  // Skinny regime (64-wide tiles): four K slabs per TMA instruction where a CTA has at least one full stage of
+  // them; the K order is unchanged, so are the bits.
+  if (bn == 64 && g_cfg_slabs != 1 && p.num_k / split >= 4 && stages == 0) {
+    if (split == 1 && p.tma_store) {
       if (p.M <= 64) {  // the lean form stores sixteen rows at a time then
         st = make_out_map(&to, p.out, p.M, p.N, p.ld_out, oes, p.half_rows ? 64 : 128, 16);
         if (st != IFLB200_OK) return st;
       }
-      return launch_lean(sa_map, sw_map, to, p, grid, s);
+      g_last_launch[3] = 104;
+      return launch_lean(a, ld_a, w, ld_w, to, p, grid, s);
+    }
+    CUtensorMap sa_map, sw_map;
+    if (p.K % BK == 0 && make_slab_map(&sa_map, a, p.M, p.K, ld_a, a_rows, 4) == IFLB200_OK &&
+        make_slab_map(&sw_map, w, p.N, p.K, ld_w, bn, 4) == IFLB200_OK) {
+      g_last_launch[3] = 104;
+      return launch_gemm_form<64, 2, 2, false, false, kEpilogueWarps, 4>(sa_map, sw_map, to, p, grid, s);
     }
   }
   switch (bn) {
@@ -1897,12 +1949,8 @@ static int run_gemm_partials(const void* a, int64_t ld_a, const void* w, int64_t
   if (st != IFLB200_OK) return st;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (M <= BM) {
-    st = make_slab_map(&ta, a, M, K, ld_a, a_rows, 4);
-    if (st != IFLB200_OK) return st;
-    st = make_slab_map(&tw, w, N, K, ld_w, 64, 4);
-    if (st != IFLB200_OK) return st;
     g_last_launch[0] = 1 + 16; g_last_launch[1] = 64; g_last_launch[2] = splits; g_last_launch[3] = 104;
-    return launch_lean(ta, tw, to, p, p.num_tiles * splits, s);
+    return launch_lean(a, ld_a, w, ld_w, to, p, p.num_tiles * splits, s);
   }
   // CTA pairs where blocks of 256 rows pad little and their units need no more waves: two thirds of the traffic per K step, which is what these launches wait for.
   // 816 x 2048 x 16384 in two ranges 28.6 against 29.7 us, 640 rows in three 22.8 against 23.3.

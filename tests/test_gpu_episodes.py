@@ -52,3 +52,38 @@ def test_episode_batch_bits(M, hidden, ffn, o_in, episodes):
     for st, x, w in zip(batch.stacks, xs, want):   # an episode by itself, on its rows of the batch's buffers
         st.load(x, attn)
         assert torch.equal(st.forward(), w)
+
+
+# the 64-row form and its neighbours, and K whose last slab is ragged: with whole stages in front, alone in its
+# stage, in the first stage; the K order does not depend on the form, so the bits are those of 128-wide tiles
+@pytest.mark.parametrize("M", [1, 16, 17, 50, 63, 64, 65, 128, 300])
+@pytest.mark.parametrize("K", [400, 512, 528, 1040, 1152, 2032])
+def test_skinny_forms_bits(M, K):
+    from instinctflash_b200 import _lib
+    from instinctflash_b200.kernels import fp8
+    g = torch.Generator(device=DEV).manual_seed(K)
+    N = 336
+    a = torch.full((M + 1, K), 448.0, device=DEV).to(E4M3)   # a row behind the operand must not be read into it
+    a[:M] = torch.randn(M, K, device=DEV, generator=g).to(E4M3)
+    wt = torch.full((N + 1, K), 448.0, device=DEV).to(E4M3)
+    wt[:N] = torch.randn(N, K, device=DEV, generator=g).to(E4M3)
+    w = fp8.Fp8Weight(wt[:N], torch.rand(N, device=DEV, generator=g), torch.randn(N, device=DEV, generator=g))
+    s = torch.rand(M, device=DEV, generator=g)
+    outs = []
+    for tile in (64, 128):
+        assert _lib.lib().iflb200_gemm_set_config(tile, 0, 0) == 0 and _lib.lib().iflb200_gemm_set_split_k(1) == 0
+        try:
+            raw = torch.full((M, N), float("nan"), device=DEV, dtype=torch.bfloat16)
+            fp8.gemm(a[:M], w, raw)
+            y = [torch.full((M, N), float("nan"), device=DEV, dtype=t) for t in (torch.float32, torch.float16)]
+            for o in y:
+                fp8.fp8_linear(a[:M], s, w, o)
+            torch.cuda.synchronize()
+            outs.append([raw, *y])
+        finally:
+            _lib.lib().iflb200_gemm_set_config(0, 0, 0)
+            _lib.lib().iflb200_gemm_set_split_k(0)
+    for p, q in zip(*outs):
+        assert not torch.isnan(p).any() and torch.equal(p, q)
+    exact = (a[:M].double() @ wt[:N].double().T)   # exact products: the bf16 rounding of an fp32 sum
+    assert ((outs[0][0].double() - exact).abs() <= 2.0 ** -8 * exact.abs() + 1e-4 * K ** 0.5).all()
