@@ -1694,23 +1694,64 @@ static int run_gemm(const void* a, int64_t ld_a, const void* w, int64_t ld_w, Ge
   } else {
     memset(&to, 0, sizeof(to));
   }
-  // CTA pairs by choice of the heuristic.  A pair moves 32 KB per SM and K step instead of 48 KB
-  // and its 256 x 256 tile takes about 0.87 of the time two SMs need for two 128 x 256 tiles
-  // (measured per shape at M = 4680: 9216 x 3072 98.7 us on pairs in 10 waves against 103.7 us on
-  // single CTAs in 9; 14336 x 3072 149.5 against 161.2; but 3072 x 14336 186 against 150 where the
-  // pairs need 4 waves for 3).  So the pair kernel is taken when its wave count, weighted by that
-  // factor, is below the single-CTA one.
-  // Below 2048 rows only where there are at least two waves to save in (816 x 8192 x 2048 15.4 against
-  // 16.0 us, 1300 x 12288 x 3072 39.7 against 42.4; the one wave of 1500 x 2048 x 4096 is 15.4 against 14.9).
-  bool pair_by_heuristic = false;
-  if (g_cfg_mode == 0 && g_cfg_tile_n == 0 && g_cfg_split_k == 0 && p.M >= 512 && p.N >= 256) {
-    const int64_t single_tiles = (int64_t)((p.M + BM - 1) / BM) * ((p.N + 255) / 256);
-    const int64_t pair_tiles = (int64_t)((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + 255) / 256);
-    const int64_t single_waves = (single_tiles + dev->sm_count - 1) / dev->sm_count;
-    const int64_t pair_waves = (pair_tiles + dev->sm_count / 2 - 1) / (dev->sm_count / 2);
-    pair_by_heuristic = pair_waves * 87 < single_waves * 100 && (p.M >= 2048 || single_waves >= 2);
+  // Tile shape by a measured cost model: waves x (K steps x clocks of a step + 400) and the prologue and epilogue
+  // that nothing covers.  A 128-byte K step of a 64 / 128 / 256 wide tile takes about 385 / 510 / 710 clocks: 24 /
+  // 32 / 48 KB are written to shared memory and read back by the tensor core through one port of 128
+  // bytes a clock (192 and 224 interpolate).  A CTA pair's 256 x 256 tile is 32 KB per SM and 610, or 710 in a
+  // single wave, where latency shows.  Rows that do not start on 64-byte boundaries (K and strides in odd
+  // multiples of 16 or 32) make every 128-byte piece two L2 requests: 570 / 715 / 1090, pairs 830 / 870.
+  // Measured at 1792 x 1792 x 4096 and x 4112: 256-wide 14.4 and 23.1 us, pairs 15.3 and 17.9; 1300 x 12288 x
+  // 3072 42.4 and, on pairs, 39.7; 2229 x 512 x 1568 on pairs 10.0, 64-wide 7.0.
+  // The widths that are not powers of two are for wave quantisation (7 row blocks x 32768 columns: 896 tiles of
+  // 256 = 6.05 waves of 148 SMs, i.e. 7, but 1029 tiles of 224 = 6.95 waves of narrower tiles).  Timed alone the
+  // 224-wide kernel is 2 % faster on that shape, inside the layer stack it was 4 us per launch slower (its
+  // 448-byte tile rows start off the 128-byte line grid), so the model does not choose them by itself.
+  const bool aligned = (ld_a | ld_w) % 64 == 0;
+  p.num_m = (p.M + BM - 1) / BM;
+  int bn = g_cfg_tile_n;
+  int split = 1;
+  bool pair = false;
+  {
+    const int widths[5] = {256, 224, 192, 128, 64};
+    const int64_t step_cycles[2][5] = {{1090, 1000, 900, 715, 570}, {710, 680, 640, 510, 385}};
+    const int64_t steps = (p.K + BK - 1) / BK;
+    int64_t best = 0;
+    int best_bn = 0;
+    for (int i = 0; i < 5; ++i) {
+      if (g_cfg_tile_n && widths[i] != g_cfg_tile_n) continue;
+      if (!g_cfg_tile_n && (widths[i] & (widths[i] - 1))) continue;  // 192 / 224: only when asked for (see above)
+      if (!g_cfg_tile_n && widths[i] > 64 && p.N < widths[i]) continue;
+      const int64_t tiles = (int64_t)p.num_m * ((p.N + widths[i] - 1) / widths[i]);
+      // split-K over a cluster: one wave of tiles x S CTAs, S in {2, 4}, leaving each CTA >= 8 K
+      // steps and >= 32 columns to reduce; the exchange of partials over distributed shared
+      // memory, two cluster barriers and the reduction are a fixed cost per launch.
+      for (int sk = 1; sk <= 4; sk *= 2) {
+        if (g_cfg_split_k && sk != g_cfg_split_k) continue;
+        if (sk > 1 && (tiles * sk > dev->sm_count || steps / sk < 8 || widths[i] / sk < 32)) continue;
+        if (sk > 1 && (widths[i] & (widths[i] - 1))) continue;  // the reduction splits power-of-two widths
+        const int64_t waves = sk > 1 ? 1 : (tiles + dev->sm_count - 1) / dev->sm_count;
+        const int64_t exchange = sk > 1 ? 5000 + 65 * widths[i] * (sk - 1) / sk : 0;  // barriers, columns handed over
+        // up to 64 rows the lean 64-wide form moves half as much per step (24 x 4624 x 5984 9.1 us, where the
+        // cluster form of 128-wide tiles takes 19.5)
+        const int64_t clocks = widths[i] == 64 && p.M <= 64 && sk == 1 && steps >= 4 ? 280 : step_cycles[aligned][i];
+        const int64_t cost = waves * ((steps / sk) * clocks + 400) + 2100 + exchange;
+        if (best_bn == 0 || cost < best) {
+          best = cost;
+          best_bn = widths[i];
+          split = sk;
+        }
+      }
+    }
+    if (best_bn == 0 && g_cfg_mode < 2) return IFLB200_ERR_ARG;  // the forced configuration does not fit this problem
+    bn = best_bn;
+    if (g_cfg_mode == 0 && g_cfg_tile_n == 0 && g_cfg_split_k == 0 && g_cfg_swap != 2 && p.M > BM && p.N >= 256) {
+      const int64_t tiles = (int64_t)((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + 255) / 256);
+      const int64_t waves = (tiles + dev->sm_count / 2 - 1) / (dev->sm_count / 2);
+      const int64_t step = aligned ? (waves == 1 ? 710 : 610) : (waves == 1 ? 870 : 830);
+      pair = waves * (steps * step + 400) + 3100 < best;
+    }
   }
-  if ((g_cfg_mode >= 2 || pair_by_heuristic) && p.N >= 256) {
+  if ((g_cfg_mode >= 2 || pair) && p.N >= 256) {
     // CTA pairs: 256 x 256 tiles, each CTA loads 128 rows of A and 128 rows of W per K step.
     constexpr int PBN = 256;
     p.num_m = (p.M + 2 * BM - 1) / (2 * BM);
@@ -1737,48 +1778,6 @@ static int run_gemm(const void* a, int64_t ld_a, const void* w, int64_t ld_w, Ge
                            : launch_gemm_pair<PBN, 6, 2>(ta, tw, to, p, grid, s);  // two accumulators
   }
 
-  // Tile width by a measured cost model: one 128-byte K step of a CTA costs about 385 / 510 / 720 cycles for a
-  // 64 / 128 / 256 wide tile: 24 / 32 / 48 KB are written to shared memory and read back by the tensor core
-  // through one port of 128 bytes a clock (192 and 224 interpolate).  The kernel takes waves x steps x that,
-  // plus a fixed cost per wave for prologue and the exposed epilogue.  The widths that are not powers of two
-  // are for wave quantisation (7 row blocks x 32768 columns: 896 tiles of 256 = 6.05 waves of 148 SMs, i.e.
-  // 7, but 1029 tiles of 224 = 6.95 waves of narrower tiles).  Timed alone the 224-wide kernel is
-  // 2 % faster on that shape, inside the layer stack it was 4 us per launch slower (its 448-byte
-  // tile rows start off the 128-byte line grid), so the model does not choose them by itself.
-  p.num_m = (p.M + BM - 1) / BM;
-  int bn = g_cfg_tile_n;
-  int split = 1;
-  {
-    const int widths[5] = {256, 224, 192, 128, 64};
-    const int64_t step_cycles[5] = {720, 680, 640, 510, 385};
-    const int64_t steps = (p.K + BK - 1) / BK;
-    int64_t best = 0;
-    int best_bn = 0;
-    for (int i = 0; i < 5; ++i) {
-      if (g_cfg_tile_n && widths[i] != g_cfg_tile_n) continue;
-      if (!g_cfg_tile_n && (widths[i] & (widths[i] - 1))) continue;  // 192 / 224: only when asked for (see above)
-      if (!g_cfg_tile_n && widths[i] > 64 && p.N < widths[i]) continue;
-      const int64_t tiles = (int64_t)p.num_m * ((p.N + widths[i] - 1) / widths[i]);
-      // split-K over a cluster: one wave of tiles x S CTAs, S in {2, 4}, leaving each CTA >= 8 K
-      // steps and >= 32 columns to reduce; the exchange of partials over distributed shared
-      // memory, two cluster barriers and the reduction are a fixed cost per launch.
-      for (int sk = 1; sk <= 4; sk *= 2) {
-        if (g_cfg_split_k && sk != g_cfg_split_k) continue;
-        if (sk > 1 && (tiles * sk > dev->sm_count || steps / sk < 8 || widths[i] / sk < 32)) continue;
-        if (sk > 1 && (widths[i] & (widths[i] - 1))) continue;  // the reduction splits power-of-two widths
-        const int64_t waves = sk > 1 ? 1 : (tiles + dev->sm_count - 1) / dev->sm_count;
-        const int64_t exchange = sk > 1 ? 5000 + 65 * widths[i] * (sk - 1) / sk : 0;  // barriers, columns handed over
-        const int64_t cost = waves * ((steps / sk) * step_cycles[i] + 2500 + exchange);
-        if (best_bn == 0 || cost < best) {
-          best = cost;
-          best_bn = widths[i];
-          split = sk;
-        }
-      }
-    }
-    if (best_bn == 0) return IFLB200_ERR_ARG;  // the forced configuration does not fit this problem
-    bn = best_bn;
-  }
   // Swapped form for a few hundred tokens: the tokens go on the MMA's N side in tiles of the width
   // that fits them (816 tokens = 4 x 208 with 2 % padding, where 7 row blocks of 128 carry 9 %), the
   // weight rows on its M side in blocks of 128 (256 on a CTA pair), and the epilogue stores the
