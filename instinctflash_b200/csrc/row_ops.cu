@@ -1638,8 +1638,10 @@ extern "C" int iflb200_dynamic_pack_bf16_e4m3(const void* x, int64_t n, void* q,
   if (launch_pack_cluster(x, n, q, scale, s)) return (int)cudaGetLastError();
   uint32_t* partial = reinterpret_cast<uint32_t*>(workspace);
   launch_dep(amax_partial_kernel, dim3(grid), dim3(kPackThreads), 0, s, 1, dependent_launch_for(n >> 12), reinterpret_cast<const uint16_t*>(x), n, partial);
-  launch_dep(pack_kernel, dim3(grid), dim3(kPackThreads), 0, s, 1, dependent_launch_for(n >> 12), reinterpret_cast<const uint16_t*>(x), n, partial, grid,
-                                            nullptr, scale, reinterpret_cast<uint8_t*>(q));
+  // The pass over the maxima is the kernel before at any size, and it is short beside a GEMM: its
+  // successor starts early however large the tensor is (4680 x 3072 15.2 -> 14.9 us).
+  launch_dep(pack_kernel, dim3(grid), dim3(kPackThreads), 0, s, 1, dependent_launch_for(0), reinterpret_cast<const uint16_t*>(x), n, partial, grid, nullptr,
+                                            scale, reinterpret_cast<uint8_t*>(q));
   return (int)cudaGetLastError();
 }
 
@@ -1702,7 +1704,7 @@ extern "C" int iflb200_dynamic_pack_bf16_e4m3_noalloc(const void* x, int64_t n, 
   const int grid = pack_grid(n);  // <= kPackMaxCtas words of scratch, all written before they are read
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   launch_dep(amax_partial_kernel, dim3(grid), dim3(kPackThreads), 0, s, 1, dependent_launch_for(n >> 12), reinterpret_cast<const uint16_t*>(x), n, partial);
-  launch_dep(pack_kernel, dim3(grid), dim3(kPackThreads), 0, s, 1, dependent_launch_for(n >> 12), reinterpret_cast<const uint16_t*>(x), n, partial, grid, nullptr,
+  launch_dep(pack_kernel, dim3(grid), dim3(kPackThreads), 0, s, 1, dependent_launch_for(0), reinterpret_cast<const uint16_t*>(x), n, partial, grid, nullptr,
                                             scale, reinterpret_cast<uint8_t*>(q));
   return (int)cudaGetLastError();
 }
