@@ -1234,11 +1234,15 @@ struct PairSmemLayout {
 };
 
 // PLANES: (tile, K range) units as in the single-CTA kernel's planes form.
-template <int BN, int STAGES, int ACC, bool SWAP = false, bool PLANES = false>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
+// GATED: the gated form (see epilogue_gated).  The leader loads the gate rows of the tile's BN/2 hidden units,
+// its peer the up rows, so both accumulators hold BN/2 gate columns followed by their up columns; p.N counts
+// hidden units and EW is 16, as in the single-CTA kernel.
+template <int BN, int STAGES, int ACC, bool SWAP = false, bool PLANES = false, bool GATED = false, int EW = kEpilogueWarps>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(96 + 32 * EW, 1)
 gemm_fp8_tc5_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w,
                          const __grid_constant__ CUtensorMap tm_out, const GemmParams p) {
   using L = PairSmemLayout<BN, STAGES>;
+  constexpr int kWarpStaging = kStagingBytes / EW;
   constexpr uint32_t kAccStride = BN <= 128 ? 128 : 256;  // accumulators at power-of-two column offsets
   constexpr uint32_t kTmemCols = ACC * kAccStride;         // 256 or 512
   constexpr uint32_t kIdesc = make_idesc_e4m3_f32(2 * BM, BN);
@@ -1280,7 +1284,7 @@ gemm_fp8_tc5_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(tfull_bar(a), 1);
-      mbar_init(tempty_bar(a), 2 * kEpilogueWarps);  // the epilogue warps of both CTAs
+      mbar_init(tempty_bar(a), 2 * EW);  // the epilogue warps of both CTAs
     }
     tmem_slot[1] = 0;
     fence_barrier_init();
@@ -1299,7 +1303,7 @@ gemm_fp8_tc5_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  const bool w_producer = warp == 0, a_producer = warp == 2 + kEpilogueWarps;
+  const bool w_producer = warp == 0, a_producer = warp == 2 + EW;
   if (w_producer || a_producer) {
     // ------------------------------------------------------------------ TMA producers (both CTAs)
     // A warp per operand, the weights' one ahead of the dependency wait, as in the single-CTA kernel.
@@ -1312,7 +1316,8 @@ gemm_fp8_tc5_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
       int m_blk, n_blk;
       tile_coords(p, unit / parts, m_blk, n_blk);
       enter_unit(unit);
-      const int row = w_producer ? n_blk * BN + (int)rank * (BN / 2) : m_blk * 2 * BM + (int)rank * BM;
+      const int w_row = GATED ? n_blk * (BN / 2) + (int)rank * p.N : n_blk * BN + (int)rank * (BN / 2);
+      const int row = w_producer ? w_row : m_blk * 2 * BM + (int)rank * BM;
       for (int kb = kb0; kb < kb1; ++kb) {
         ok = wait_bounded(empty_bar(ring.stage), ring.phase ^ 1, abort_flag, (1u << 24) | (1u << 16) | (it & 0xFFFF));
         if (!ok) break;
@@ -1376,8 +1381,8 @@ gemm_fp8_tc5_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
       col_begin = 0;
       col_end = half == 0 ? BN : 0;
     }
-    const uint32_t staging = base + L::kStagingOffset + (uint32_t)(warp - 2) * 4096u;
-    uint8_t* staging_ptr = smem + L::kStagingOffset + (warp - 2) * 4096;
+    const uint32_t staging = base + L::kStagingOffset + (uint32_t)(warp - 2) * (uint32_t)kWarpStaging;
+    uint8_t* staging_ptr = smem + L::kStagingOffset + (warp - 2) * kWarpStaging;
     bool ok = true;
     uint32_t it = 0;
     int swap_buf = 0;
@@ -1391,11 +1396,16 @@ gemm_fp8_tc5_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
       const int m = m_blk * 2 * BM + (int)rank * BM + quad * 32 + lane;
       const bool row_ok = m < p.M;
       // this tile's per-column operands and row scale, fetched under the main loop (see ColumnVectors)
-      const bool prefetch = !SWAP && p.tma_store && p.epilogue != EPI_RAW && col_end - col_begin <= 128;
+      const bool prefetch = !SWAP && !GATED && p.tma_store && p.epilogue != EPI_RAW && col_end - col_begin <= 128;
       ColumnVectors cv;
       float rs_early = 1.0f;
       if (prefetch) {
         cv = fetch_column_vectors(p, n_blk * BN + col_begin, col_end - col_begin, lane);
+        rs_early = (row_ok && p.row) ? __ldg(p.row + (int64_t)m * p.row_stride) : 1.0f;
+      }
+      float cgl[4], cul[4];
+      if constexpr (GATED) {
+        gated_scales<BN, EW / 4>(p, n_blk * (BN / 2), half, lane, cgl, cul);
         rs_early = (row_ok && p.row) ? __ldg(p.row + (int64_t)m * p.row_stride) : 1.0f;
       }
       ok = wait_bounded(tfull_bar(acc), acc_phase, abort_flag, (3u << 24) | (4u << 16) | (it & 0xFFFF));
@@ -1405,6 +1415,14 @@ gemm_fp8_tc5_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
       if constexpr (SWAP) {
         epilogue_swapped<BN>(p, &tm_out, t_row, staging, staging_ptr, m_blk * 2 * BM + (int)rank * BM + quad * 32,
                              n_blk * BN, half, lane, swap_buf);
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(tempty_bar(acc), 0);
+        continue;
+      }
+      if constexpr (GATED) {
+        epilogue_gated<BN, EW / 4>(p, &tm_out, t_row, staging, staging_ptr, m_blk * 2 * BM + (int)rank * BM + quad * 32,
+                                   n_blk * (BN / 2), half, m, row_ok, rs_early, lane, cgl, cul);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(tempty_bar(acc), 0);
@@ -1651,7 +1669,7 @@ static int launch_lean(const void* a, int64_t ld_a, const void* w, int64_t ld_w,
                    : launch_gemm_form<64, 2, 4, false, false, kEpilogueWarps, 4>(ta, tw, to, p, grid, s);
 }
 
-template <int BN, int STAGES, int ACC, bool SWAP = false, bool PLANES = false>
+template <int BN, int STAGES, int ACC, bool SWAP = false, bool PLANES = false, bool GATED = false, int EW = kEpilogueWarps>
 static int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tw, const CUtensorMap& to,
                             const GemmParams& p, int grid, cudaStream_t s) {
   using L = PairSmemLayout<BN, STAGES>;
@@ -1659,12 +1677,12 @@ static int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tw, const 
   int dev = 0;
   cudaGetDevice(&dev);
   if (!attr_set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_fp8_tc5_pair_kernel<BN, STAGES, ACC, SWAP, PLANES>,
+    cudaError_t e = cudaFuncSetAttribute(gemm_fp8_tc5_pair_kernel<BN, STAGES, ACC, SWAP, PLANES, GATED, EW>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, L::kDynamic);
     if (e != cudaSuccess) return (int)e;
     attr_set[dev] = true;
   }
-  const cudaError_t e = launch_dep(gemm_fp8_tc5_pair_kernel<BN, STAGES, ACC, SWAP, PLANES>, dim3(grid), dim3(kGemmThreads),
+  const cudaError_t e = launch_dep(gemm_fp8_tc5_pair_kernel<BN, STAGES, ACC, SWAP, PLANES, GATED, EW>, dim3(grid), dim3(96 + 32 * EW),
                                    L::kDynamic, s, 1, dependent_launch_for(SWAP ? p.N : p.M), ta, tw, to, p);
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
@@ -2052,21 +2070,56 @@ static int run_gemm_gated(const void* a, int64_t ld_a, const void* w, int64_t ld
   p.tma_store = 1;
   p.num_m = (M + BM - 1) / BM;
   p.num_k = (K + BK - 1) / BK;
-  // tile width (gate + up columns) by the cost model of the ordinary form
+  // Tile width (gate + up columns) and CTA pairs by measured cost: steps of 720 / 510 / 385 clocks for 256 / 128 /
+  // 64-wide tiles and 600 for pairs (660 in a single wave; rows off 64-byte boundaries as in the ordinary form),
+  // 2000 per tile for the epilogue, 2500 on pairs.  A last wave that is partly filled costs half of a wave and
+  // half of its share: its CTAs find the L2 and the store path free.  The constants are the ones whose choice is
+  // closest to the fastest form over 81 sizes (65 to 1300 tokens, 1024 to 16384 hidden units, K 1024 to 5120):
+  // within 3 % at 80 of them.  With 2 x 16384 columns at K = 2048 pairs against single CTAs take 18.6 / 20.1 us for
+  // 256 tokens, 45.4 / 48.0 for 768, 55.1 / 59.1 for 1024, 81.5 / 92.0 for 1536, but 30.4 / 27.2 for 384, which
+  // pairs pad to 512; 512 tokens, 2 x 6912 columns at K = 5120 31.8 / 36.6.
+  const bool aligned = (ld_a | ld_w) % 64 == 0;
   const int widths[3] = {256, 128, 64};
-  const int64_t step_cycles[3] = {720, 510, 385};
+  const int64_t step_cycles[2][3] = {{1090, 715, 570}, {720, 510, 385}};
+  const auto cost = [&](int64_t tiles, int64_t slots, int64_t step, int64_t epilogue) {
+    const int64_t waves = (tiles + slots - 1) / slots;
+    const int64_t percent = waves == 1 ? 100 : (50 * tiles + slots - 1) / slots + 50 * waves;
+    return percent * (p.num_k * step + epilogue) / 100;
+  };
   int bn = g_cfg_tile_n == 256 || g_cfg_tile_n == 128 || g_cfg_tile_n == 64 ? g_cfg_tile_n : 0;
+  bool pair = g_cfg_mode == 3 && F >= 128;
   if (bn == 0) {
     int64_t best = 0;
     for (int i = 0; i < 3; ++i) {
-      const int64_t tiles = (int64_t)p.num_m * ((F + widths[i] / 2 - 1) / (widths[i] / 2));
-      const int64_t waves = (tiles + dev->sm_count - 1) / dev->sm_count;
-      const int64_t cost = waves * (p.num_k * step_cycles[i] + 2500);
-      if (bn == 0 || cost < best) {
-        best = cost;
+      const int64_t c = cost((int64_t)p.num_m * ((F + widths[i] / 2 - 1) / (widths[i] / 2)), dev->sm_count, step_cycles[aligned][i], 2000);
+      if (bn == 0 || c < best) {
+        best = c;
         bn = widths[i];
       }
     }
+    if (g_cfg_mode == 0 && M > BM && F >= 128) {
+      const int64_t tiles = (int64_t)((M + 2 * BM - 1) / (2 * BM)) * ((F + 127) / 128), pairs = dev->sm_count / 2;
+      const bool one_wave = tiles <= pairs;
+      pair = cost(tiles, pairs, aligned ? (one_wave ? 660 : 600) : (one_wave ? 870 : 830), 2500) + 1000 < best;
+    }
+  }
+  if (pair) {
+    // as in the ordinary form: 256 tokens x 128 hidden units, each CTA 128 rows of A and of the gate or up weights
+    p.num_m = (M + 2 * BM - 1) / (2 * BM);
+    p.num_n = (F + 127) / 128;
+    p.num_tiles = p.num_m * p.num_n;
+    p.group_m = g_cfg_group_m > 0 ? g_cfg_group_m : (p.num_m <= 24 ? p.num_m : 16);
+    const int pairs = dev->sm_count / 2;
+    CUtensorMap ta, tw, to;
+    st = make_tensor_map(&ta, a, M, K, ld_a, BM);
+    if (st != IFLB200_OK) return st;
+    st = make_tensor_map(&tw, w, 2 * F, K, ld_w, 128);
+    if (st != IFLB200_OK) return st;
+    st = make_out_map(&to, h, M, F, ld_h, 4, 64);
+    if (st != IFLB200_OK) return st;
+    g_last_launch[0] = 3 + 8; g_last_launch[1] = 256; g_last_launch[2] = 1; g_last_launch[3] = 6;
+    return launch_gemm_pair<256, 6, 2, false, false, true, 16>(ta, tw, to, p, 2 * (p.num_tiles < pairs ? p.num_tiles : pairs),
+                                                              reinterpret_cast<cudaStream_t>(stream));
   }
   p.num_n = (F + bn / 2 - 1) / (bn / 2);
   p.num_tiles = p.num_m * p.num_n;
