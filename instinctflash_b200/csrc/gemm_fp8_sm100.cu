@@ -1712,14 +1712,16 @@ static int run_gemm(const void* a, int64_t ld_a, const void* w, int64_t ld_w, Ge
   } else {
     memset(&to, 0, sizeof(to));
   }
-  // Tile shape by a measured cost model: waves x (K steps x clocks of a step + 400) and the prologue and epilogue
-  // that nothing covers.  A 128-byte K step of a 64 / 128 / 256 wide tile takes about 385 / 510 / 710 clocks: 24 /
-  // 32 / 48 KB are written to shared memory and read back by the tensor core through one port of 128
-  // bytes a clock (192 and 224 interpolate).  A CTA pair's 256 x 256 tile is 32 KB per SM and 610, or 710 in a
-  // single wave, where latency shows.  Rows that do not start on 64-byte boundaries (K and strides in odd
-  // multiples of 16 or 32) make every 128-byte piece two L2 requests: 570 / 715 / 1090, pairs 830 / 870.
-  // Measured at 1792 x 1792 x 4096 and x 4112: 256-wide 14.4 and 23.1 us, pairs 15.3 and 17.9; 1300 x 12288 x
-  // 3072 42.4 and, on pairs, 39.7; 2229 x 512 x 1568 on pairs 10.0, 64-wide 7.0.
+  // Tile shape by a measured cost model: waves x (K steps x clocks of a step + what a tile's epilogue holds up), and what
+  // the first loads and the last stores take.  A partly filled last wave, which has the L2 and the store path to itself,
+  // counts 0.7 and 0.3 of its share.  A 128-byte K step of a 64 / 128 / 256 wide tile is about 490 / 555 / 800 clocks:
+  // 24 / 32 / 48 KB are written to shared memory and read back by the tensor core through one port of 128 bytes a clock
+  // (192 and 224 interpolate; the lean form's 64 rows 315).  A CTA pair's 256 x 256 tile is 32 KB per SM and 690, or 750
+  // in a single wave, where latency shows.  Rows that do not start on 64-byte boundaries (K and strides in odd multiples
+  // of 16 or 32) make every 128-byte piece two L2 requests: 570 / 630 / 815, lean 395, pairs 650 and 585.  The constants
+  // are the ones whose choice is closest to the fastest form over 680 sizes (16 to 6000 rows, 256 to 14384 columns, K 256
+  // to 16384): 0.4 % slower on average, more than 10 % at three.  3072 columns at K = 14336: 1024 rows 44.4 us on 256-wide tiles,
+  // 40.3 on pairs; 1536 at K = 8960: 512 rows 18.4 us on 64-wide tiles, 15.5 on 128-wide ones with K split in two.
   // The widths that are not powers of two are for wave quantisation (7 row blocks x 32768 columns: 896 tiles of
   // 256 = 6.05 waves of 148 SMs, i.e. 7, but 1029 tiles of 224 = 6.95 waves of narrower tiles).  Timed alone the
   // 224-wide kernel is 2 % faster on that shape, inside the layer stack it was 4 us per launch slower (its
@@ -1731,8 +1733,13 @@ static int run_gemm(const void* a, int64_t ld_a, const void* w, int64_t ld_w, Ge
   bool pair = false;
   {
     const int widths[5] = {256, 224, 192, 128, 64};
-    const int64_t step_cycles[2][5] = {{1090, 1000, 900, 715, 570}, {710, 680, 640, 510, 385}};
+    const int64_t step_cycles[2][5] = {{815, 750, 690, 630, 570}, {800, 740, 680, 555, 490}};
+    const int64_t tile_cycles[5] = {3560, 3130, 2700, 1850, 2640}, ends[5] = {2690, 2690, 2690, 2405, 1870};
     const int64_t steps = (p.K + BK - 1) / BK;
+    const auto waves_cost = [](int64_t tiles, int64_t slots, int64_t wave) {
+      const int64_t waves = (tiles + slots - 1) / slots;
+      return waves == 1 ? wave : (7 * waves * wave + 3 * tiles * wave / slots) / 10;
+    };
     int64_t best = 0;
     int best_bn = 0;
     for (int i = 0; i < 5; ++i) {
@@ -1745,14 +1752,17 @@ static int run_gemm(const void* a, int64_t ld_a, const void* w, int64_t ld_w, Ge
       // memory, two cluster barriers and the reduction are a fixed cost per launch.
       for (int sk = 1; sk <= 4; sk *= 2) {
         if (g_cfg_split_k && sk != g_cfg_split_k) continue;
-        if (sk > 1 && (tiles * sk > dev->sm_count || steps / sk < 8 || widths[i] / sk < 32)) continue;
+        // clusters of four do not fill every group of SMs the chip allots them from: 35 of them took two waves
+        if (sk > 1 && (tiles * sk > dev->sm_count - (sk == 4 && !g_cfg_split_k ? 16 : 0) || steps / sk < 8 || widths[i] / sk < 32)) continue;
         if (sk > 1 && (widths[i] & (widths[i] - 1))) continue;  // the reduction splits power-of-two widths
-        const int64_t waves = sk > 1 ? 1 : (tiles + dev->sm_count - 1) / dev->sm_count;
-        const int64_t exchange = sk > 1 ? 5000 + 65 * widths[i] * (sk - 1) / sk : 0;  // barriers, columns handed over
+        if (sk > 1 && widths[i] == 64 && !g_cfg_split_k) continue;  // never the fastest form
+        const int64_t exchange = sk > 1 ? 6780 + 65 * widths[i] * (sk - 1) / sk : 0;  // barriers, columns handed over
         // up to 64 rows the lean 64-wide form moves half as much per step (24 x 4624 x 5984 9.1 us, where the
         // cluster form of 128-wide tiles takes 19.5)
-        const int64_t clocks = widths[i] == 64 && p.M <= 64 && sk == 1 && steps >= 4 ? 280 : step_cycles[aligned][i];
-        const int64_t cost = waves * ((steps / sk) * clocks + 400) + 2100 + exchange;
+        const bool lean = widths[i] == 64 && p.M <= 64 && sk == 1 && steps >= 4;
+        const int64_t clocks = lean ? (aligned ? 315 : 395) : step_cycles[aligned][i];
+        const int64_t wave = (steps + sk - 1) / sk * clocks + (lean ? 3285 : tile_cycles[i]);
+        const int64_t cost = waves_cost(tiles * sk, dev->sm_count, wave) + ends[i] + exchange;
         if (best_bn == 0 || cost < best) {
           best = cost;
           best_bn = widths[i];
@@ -1764,9 +1774,9 @@ static int run_gemm(const void* a, int64_t ld_a, const void* w, int64_t ld_w, Ge
     bn = best_bn;
     if (g_cfg_mode == 0 && g_cfg_tile_n == 0 && g_cfg_split_k == 0 && g_cfg_swap != 2 && p.M > BM && p.N >= 256) {
       const int64_t tiles = (int64_t)((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + 255) / 256);
-      const int64_t waves = (tiles + dev->sm_count / 2 - 1) / (dev->sm_count / 2);
-      const int64_t step = aligned ? (waves == 1 ? 710 : 610) : (waves == 1 ? 870 : 830);
-      pair = waves * (steps * step + 400) + 3100 < best;
+      const int64_t pairs = dev->sm_count / 2;
+      const int64_t step = aligned ? (tiles <= pairs ? 750 : 690) : (tiles <= pairs ? 585 : 650);
+      pair = waves_cost(tiles, pairs, steps * step + 4285) + 3595 < best;
     }
   }
   if ((g_cfg_mode >= 2 || pair) && p.N >= 256) {
