@@ -8,7 +8,7 @@
 //   warp 1      MMA issuer: one thread issues tcgen05.mma (128 x BN x 32 per instruction,
 //               four per stage) into one of two TMEM accumulators and commits the stage's
 //               "empty" barrier / the accumulator's "full" barrier;
-//   warps 2..5  epilogue: tcgen05.ld the finished accumulator (one row per thread), apply the
+//   warps 2..   epilogue (eight or sixteen): tcgen05.ld the finished accumulator (one row per thread), apply the
 //               consumer arithmetic of the reference in its exact order and store.
 // The two TMEM accumulators let the epilogue of tile i overlap the main loop of tile i+1.
 // The K loop order is a function of K alone (128-byte steps, no split), so an output element
@@ -742,9 +742,8 @@ __device__ __forceinline__ void epilogue_swapped(const GemmParams& p, const CUte
 // SPLIT: 0 = never a cluster split-K, 1 = always (p.split_k > 1), 2 = decided by p.split_k.  The
 // wide-tile kernels of the large-M regime exist in forms 0 and 1: measured inside the M = 816 layer
 // stack, a kernel that carries both code paths ran the stack 5 % slower than the two specialised
-// ones.  The 64-wide kernel of the skinny-M regime exists only in form 2, so that the launches of a
-// layer, split or not, run the same code: there a second GEMM kernel per layer cost about 1 us per
-// launch in instruction fetch (0.2 ms per pass of the M = 50 stack).
+// ones.  The 64-wide kernel exists in form 2, for what the lean form (4) below leaves out: residual and direct-store
+// epilogues, fewer than four K steps, a K split over a cluster that was asked for.
 // SPLIT 3: the planes form for more than 128 rows: (tile, K range) units on a persistent grid, each leaving
 // its fp32 partial sums in a plane; K is cut as in the skinny form, so the planes' bits are the same.
 // SPLIT 4: the lean form of the skinny regime: planes or one range, TMA stores, no cluster and no direct stores.
