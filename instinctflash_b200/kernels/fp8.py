@@ -188,31 +188,37 @@ def partial_splits(M: int, N: int, K: int, sm_count: int = 148) -> int:
     128-byte K slabs, at most eight planes.
 
     Above 128 rows the number with the least estimated time, 1 where the unsplit GEMM is as good.  In SM clocks: a
-    slab of a 128 x 64 / 256 tile 385 / 720 (bytes through the shared-memory port), 4000 a wave for
-    prologue and fp32 epilogue (2500 for bf16), every plane written and read back at 2500 bytes a clock.
+    slab of a 128 x 64 / 256 tile 380 / 700 and a wave 7500 for prologue and fp32 epilogue, every plane written
+    and read back at 3200 bytes a clock; unsplit 440 / 480 / 850 for 64 / 128 / 256 columns and 1600 a wave,
+    over a cluster 11700 and 80 a column handed over.  The constants are the ones whose choice is closest to
+    the fastest number for the GEMM and the residual kernel after it over 63 sizes (130 to 1024 rows, seven
+    shapes): more than 3 % above it at two.
     Four decoder layers of 2048 x 16384: 315 -> 300 us at 301 rows (six planes against the GEMM that splits
-    K over a cluster), 438 -> 402 at 640 (three)."""
+    K over a cluster), 438 -> 402 at 640 (three); GEMM and residual of 816 x 2048 x 8192 25.6 -> 23.4 us
+    unsplit, of 384 x 3072 x 8192 23.3 -> 21.2 in four."""
     if K % 128:
         return 1
     slabs = K // 128
     if M <= 128:
         return max(1, min(8, sm_count // max(1, (N + 63) // 64), slabs // 4))
-    blocks, plane = (M + 127) // 128, 8 * M * N // 2500
+    blocks, plane = (M + 127) // 128, 8 * M * N // 3200
 
     def cost(splits, width, clocks, wave):
         units = blocks * ((N + width - 1) // width) * splits
         steps = min(slabs, 4 * -(-(-(-slabs // 4)) // splits))
         return -(-units // sm_count) * (steps * clocks + wave)
 
-    plain = [(width, clocks) for width, clocks in ((64, 385), (128, 510), (256, 720)) if width == 64 or N >= width]
-    unsplit = min(cost(1, w, c, 2500) for w, c in plain)
-    for ranges in (2, 4):   # over a cluster: one wave, partial sums handed over through distributed shared memory
-        for width, clocks in plain:
-            if blocks * ((N + width - 1) // width) * ranges <= sm_count and slabs // ranges >= 8 and width // ranges >= 32:
-                unsplit = min(unsplit, slabs // ranges * clocks + 7500 + 65 * width * (ranges - 1) // ranges)
+    plain = [(width, clocks) for width, clocks in ((64, 440), (128, 480), (256, 850)) if width == 64 or N >= width]
+    unsplit = min(cost(1, w, c, 1600) for w, c in plain)
+    # over a cluster: one wave, partial sums handed over through distributed shared memory (35 clusters of four
+    # do not fit the chip at once)
+    for ranges, room in ((2, sm_count), (4, sm_count - 16)):
+        for width, clocks in plain[1:]:
+            if blocks * ((N + width - 1) // width) * ranges <= room and slabs // ranges >= 8:
+                unsplit = min(unsplit, slabs // ranges * clocks + 11700 + 80 * width * (ranges - 1) // ranges)
     best, least = 1, unsplit + plane // 2
     for splits in range(2, min(8, (slabs + 3) // 4) + 1):
-        time = min(cost(splits, w, c, 4000) for w, c in plain if w != 128) + splits * plane
+        time = min(cost(splits, w, c, 7500) for w, c in ((64, 380), (256, 700)) if w == 64 or N >= w) + splits * plane
         if time < least:
             best, least = splits, time
     return best
