@@ -1087,6 +1087,7 @@ pack_cluster_kernel(const uint4* __restrict__ x, int nvec, float* __restrict__ s
   __shared__ uint32_t red[kPackClusterThreads / 32];
   __shared__ uint32_t maxima[kPackCluster];
   const int rank = (int)cluster_ctarank();
+  cluster_arrive();        // this CTA runs: its shared memory may be written from now on
   grid_dependency_wait();  // x may come from the kernel before this one in the stream
   grid_launch_dependents();
   uint4 u[V];
@@ -1101,6 +1102,7 @@ pack_cluster_kernel(const uint4* __restrict__ x, int nvec, float* __restrict__ s
   best = __reduce_max_sync(0xFFFFFFFFu, best);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = best;
   __syncthreads();
+  cluster_wait();  // every CTA of the cluster has started: a store into one that has not would be lost
   if (threadIdx.x < 32) {
     best = __reduce_max_sync(0xFFFFFFFFu, red[threadIdx.x]);
     if (threadIdx.x < kPackCluster) {
@@ -1108,6 +1110,7 @@ pack_cluster_kernel(const uint4* __restrict__ x, int nvec, float* __restrict__ s
       asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(smem_u32(&maxima[rank])), "r"(threadIdx.x));
       asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(peer), "r"(best) : "memory");
     }
+    __syncwarp();  // the cluster barrier wants whole warps
   }
   cluster_sync_all();
   best = maxima[0];
