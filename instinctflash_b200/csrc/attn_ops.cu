@@ -53,6 +53,7 @@ struct CombineArgs {
 template <int IT, bool CL, int kGroup>
 __global__ void __launch_bounds__(kCombineThreads, kGroup == 4 ? 2 : 1) attn_combine_quant_kernel(const CombineArgs a) {
   const int threads = blockDim.x;
+  if (CL) cluster_arrive();  // this CTA runs: its shared memory may be written from now on
   grid_dependency_wait();  // the partials come from the kernel before this one in the stream
   grid_launch_dependents();
   __shared__ float red[kCombineThreads / 32];
@@ -135,6 +136,10 @@ __global__ void __launch_bounds__(kCombineThreads, kGroup == 4 ? 2 : 1) attn_com
       }
     }
   }
+  if (CL) {
+    __syncwarp();    // the cluster barrier wants whole warps
+    cluster_wait();  // every CTA of the cluster has started: a store into one that has not would be lost
+  }
   if (!a.q) return;  // merge only (uniform)
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) amax = max_f32(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
@@ -150,6 +155,7 @@ __global__ void __launch_bounds__(kCombineThreads, kGroup == 4 ? 2 : 1) attn_com
       asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(smem_u32(&maxima[cluster_ctarank()])), "r"(threadIdx.x));
       asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(peer), "f"(amax) : "memory");
     }
+    __syncwarp();
     cluster_sync_all();
     amax = maxima[0];
     for (int i = 1; i < a.cluster; ++i) amax = max_f32(amax, maxima[i]);

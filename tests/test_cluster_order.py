@@ -32,7 +32,7 @@ def remote_before_started(body):
     return remote is not None and (started is None or started.start() > remote.start())
 
 
-@pytest.mark.parametrize("source", ["gemm_fp8_sm100.cu", "row_ops.cu"])
+@pytest.mark.parametrize("source", ["gemm_fp8_sm100.cu", "row_ops.cu", "attn_ops.cu"])
 def test_remote_shared_memory_after_the_cluster_has_started(source):
     bodies = list(kernel_bodies((CSRC / source).read_text()))
     assert any(REMOTE.search(body) for _, body in bodies)
