@@ -251,8 +251,6 @@ IFLB200_API int iflb200_residual_norm_quant_peers(void* res, int res_dtype, int6
  * kernel; `a`, the scales and everything else are read
  * after the wait.  So `w` must not be an OUTPUT of the kernel enqueued immediately before on the
  * same stream (weights are packed at load time; activations may of course come from that kernel).
- * Inside a stream capture the row operators let the kernel behind them start early as well, so there `w`
- * must not be an output of either of the TWO kernels enqueued before.
  * Replaces: instinctflash/kernels/fp8.py:50-53 (gemm -> torch._scaled_mm).
  */
 IFLB200_API int iflb200_gemm_fp8_raw(const void* a, int64_t ld_a, const void* w, int64_t ld_w,

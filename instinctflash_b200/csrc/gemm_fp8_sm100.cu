@@ -1628,6 +1628,7 @@ static int launch_gemm_form(const CUtensorMap& ta, const CUtensorMap& tw, const 
   const cudaError_t e = launch_dep(gemm_fp8_tc5_kernel<BN, STAGES, SPLIT, SWAP, GATED, EW, SL, AR>, dim3(grid),
                                    dim3(96 + 32 * EW), L::kDynamic, s, p.split_k,
                                    dependent_launch_for(SWAP ? p.N : p.M), ta, tw, to, p);
+  note_captured_gemm(s);
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
 
@@ -1683,6 +1684,7 @@ static int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tw, const 
   }
   const cudaError_t e = launch_dep(gemm_fp8_tc5_pair_kernel<BN, STAGES, ACC, SWAP, PLANES, GATED, EW>, dim3(grid), dim3(96 + 32 * EW),
                                    L::kDynamic, s, 1, dependent_launch_for(SWAP ? p.N : p.M), ta, tw, to, p);
+  note_captured_gemm(s);
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
 

@@ -19,14 +19,41 @@ inline bool dependent_launch_for(long long rows) {
   return g_dependent_launch == 2 || (g_dependent_launch == 1 && rows <= kDependentLaunchMaxRows);
 }
 
+// The node that a stream capture of `s` stands at: the last kernel captured into it.  False outside a
+// capture, and where several branches meet.
+struct CapturePoint {
+  unsigned long long capture = 0;  // unique for the life of the process
+  cudaGraphNode_t node = nullptr;
+};
+inline bool capture_point(cudaStream_t s, CapturePoint& at) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (s == nullptr || cudaStreamIsCapturing(s, &status) != cudaSuccess || status != cudaStreamCaptureStatusActive) return false;
+  const cudaGraphNode_t* nodes = nullptr;
+  const cudaGraphEdgeData* edges = nullptr;
+  size_t n = 0;
+  if (cudaStreamGetCaptureInfo_v3(s, &status, &at.capture, nullptr, &nodes, &edges, &n) != cudaSuccess || n != 1) return false;
+  at.node = nodes[0];
+  return true;
+}
+
+// The last GEMM of this library that this thread has captured.
+inline thread_local CapturePoint t_captured_gemm;
+inline void note_captured_gemm(cudaStream_t s) {
+  CapturePoint at;
+  if (g_dependent_launch != 0 && capture_point(s, at)) t_captured_gemm = at;
+}
+
 // Whether a row kernel should let its successor be scheduled before its own dependency wait, so that the
 // GEMM behind it sets up and fetches weights while the kernel two ahead of it drains (50 rows: 27.7 -> 25.6 us
-// per expert layer).  Only inside a captured graph: there the two kernels before a GEMM are known not to
-// write its weights (contract: iflb200_gemm_fp8_raw), in an eager stream anything may precede.
+// per expert layer).  Only where the kernel before the row kernel is known to be one of this library's
+// GEMMs, which a captured graph can tell and an eager stream cannot: a GEMM lets the row kernel start only once everything
+// before the GEMM has completed, and writes accumulators, never the codes of a weight.  So the kernels still
+// running when the next GEMM reads its weights are that GEMM and the row kernel, whose output they must not
+// be anyway (contract: iflb200_gemm_fp8_raw).  Row kernels that followed one another and all signalled
+// early would let a GEMM read a weight that a kernel any number of launches ahead is still writing.
 inline int early_trigger_for(cudaStream_t s) {
-  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-  return g_dependent_launch != 0 && s != nullptr && cudaStreamIsCapturing(s, &status) == cudaSuccess &&
-         status == cudaStreamCaptureStatusActive;
+  CapturePoint at;
+  return g_dependent_launch != 0 && capture_point(s, at) && at.capture == t_captured_gemm.capture && at.node == t_captured_gemm.node;
 }
 
 template <typename... KArgs, typename... Args>
