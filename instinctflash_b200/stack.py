@@ -346,7 +346,10 @@ class HostPipeline:
 
 class _Episode(LinearStack):
     """One episode of a batch that runs stacked along the rows: the same interface as a stack of its
-    own, over its rows of the batch's buffers."""
+    own.  Its state -- residual stream, input codes and scales, row maxima -- is its rows of the batch's
+    buffers, so that the batch and the episode can take turns; what a pass only passes from one operator
+    to the next is its own from its first pass by itself, so that episodes do not write into one
+    another's, one after the other or on streams of their own."""
 
     def __init__(self, batch: LinearStack, index: int, spec: StackSpec):
         self.batch, self.spec, self.weights, self.dev, self.ops = batch, spec, batch.weights, batch.dev, batch.ops
@@ -357,15 +360,22 @@ class _Episode(LinearStack):
         if hasattr(batch, "h"):
             self.h, self.amax = batch.h[self.rows], batch.amax[:, self.rows]
         if self.split_partials:
-            self.splits, self.part = batch.splits, batch.part   # scratch: this episode's planes from its start
+            self.splits = batch.splits
         self.attn = None
         self.launches_per_forward = 0
 
-    def _q8(self, cols):
-        return self.batch._q8(cols)[self.rows]
+    def __getattr__(self, name):
+        # scratch of a pass: the widest operand codes and raw accumulators, the planes of a K split
+        if name not in ("q8", "raw", "part"):
+            raise AttributeError(f"{type(self).__name__!r} object has no attribute {name!r}")
+        whole = getattr(self.batch, name)
+        t = torch.empty(whole.numel() * self.spec.M // self.batch.spec.M, dtype=whole.dtype, device=self.dev)
+        setattr(self, name, t)
+        return t
 
-    def _raw(self, cols):
-        return self.batch._raw(cols)[self.rows]
+    def _q8(self, cols):
+        # codes of the residual stream's width outlive a pass (load() leaves them, forward() ends with them)
+        return self.batch._q8(cols)[self.rows] if cols == self.spec.hidden else super()._q8(cols)
 
 
 class EpisodeBatch:

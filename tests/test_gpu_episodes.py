@@ -54,6 +54,33 @@ def test_episode_batch_bits(M, hidden, ffn, o_in, episodes):
         assert torch.equal(st.forward(), w)
 
 
+@pytest.mark.parametrize("M,o_in", [(50, 0), (150, 2048)])
+def test_episodes_on_streams_of_their_own(M, o_in):
+    """All loaded first, then each by itself beside the others: planes, codes and accumulators of one are not
+    another's to write."""
+    from instinctflash_b200.stack import EpisodeBatch, LinearStack, StackSpec, make_inputs, make_weights
+    spec = StackSpec("expert", "gemma", 3, M, 1024, 4096, 1536, o_in=o_in, seed=6)
+    weights = make_weights(spec, DEV)
+    xs = [make_inputs(StackSpec(**{**spec.__dict__, "seed": 70 + e}), DEV)[0] for e in range(3)]
+    attn = make_inputs(spec, DEV)[1]
+    batch = EpisodeBatch(spec, weights, DEV, 3)
+    want = []
+    for x in xs:   # K cut as the batch cuts it
+        st = LinearStack(spec, weights, DEV, split_rows=M if M <= 128 else 3 * M)
+        st.load(x, attn)
+        want.append(st.forward().clone())
+    for _ in range(3):
+        batch.load(xs, attn)
+        streams = [torch.cuda.Stream() for _ in xs]
+        torch.cuda.synchronize()
+        for st, s in zip(batch.stacks, streams):
+            with torch.cuda.stream(s):
+                st.forward()
+        torch.cuda.synchronize()
+        for st, w in zip(batch.stacks, want):
+            assert torch.equal(st.res, w)
+
+
 # the 64-row form and its neighbours, and K whose last slab is ragged: with whole stages in front, alone in its
 # stage, in the first stage; the K order does not depend on the form, so the bits are those of 128-wide tiles
 @pytest.mark.parametrize("M", [1, 16, 17, 50, 63, 64, 65, 128, 300])
