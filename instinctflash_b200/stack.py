@@ -398,7 +398,9 @@ class EpisodeBatch:
             merged = LinearStack(wide, weights, device, split_rows=spec.M if spec.M <= 128 else None, **stack_kw)
             if hasattr(merged.ops, "gemm_partials"):    # this package's operators: K ranges by rows of one episode
                 self.merged = merged
-                self.attn_rows = torch.zeros(wide.M, max(spec.o_in, 16), dtype=torch.bfloat16, device=self.dev)
+                # the episodes' attention outputs side by side, a buffer per element type: a captured graph keeps
+                # the address of the one it was captured with
+                self.attn_rows = {}
                 self.stacks = [_Episode(merged, i, spec) for i in range(episodes)]
                 return
         self.stacks = [LinearStack(spec, weights, device, **stack_kw) for _ in range(episodes)]
@@ -411,25 +413,36 @@ class EpisodeBatch:
             for st, xi in zip(self.stacks, xs):
                 st.load(xi, attn)
             return
-        torch._foreach_copy_([st.res for st in self.stacks], list(xs))
-        for st in self.stacks:
+        pairs = list(zip(self.stacks, xs))
+        if pairs:
+            torch._foreach_copy_([st.res for st, _ in pairs], [xi for _, xi in pairs])
+        for st, _ in pairs:
             st.attn = attn
         o, m = self.merged.ops, self.merged
         o.residual_norm_quant(m.res, layernorm=False, q=m._q8(self.spec.hidden), q_scale=m.scale[0])
 
+    def _merged_attn(self):
+        """The episodes' attention outputs stacked along the rows."""
+        attn, shape = [st.attn for st in self.stacks], (self.spec.M, self.spec.o_in)
+        for t in attn:
+            if t is None or tuple(t.shape) != shape or t.dtype not in (torch.float32, torch.bfloat16, torch.float16):
+                raise ValueError(f"attn must be a float32, bfloat16 or float16 [{shape[0]}, {shape[1]}] tensor for every episode")
+            if t.device != self.merged.res.device or t.stride(1) != 1:
+                raise ValueError(f"attn must live on {self.merged.res.device} and be contiguous in its last dimension")
+        dtype = attn[0].dtype if len({t.dtype for t in attn}) == 1 else torch.float32   # holds either 16-bit type exactly
+        if dtype not in self.attn_rows:
+            self.attn_rows[dtype] = torch.empty(self.merged.spec.M, shape[1], dtype=dtype, device=self.dev)
+        rows = self.attn_rows[dtype].view(self.episodes, *shape)
+        if all(t is attn[0] for t in attn):   # one output for all of them, as load() leaves it
+            rows.copy_(attn[0])
+        else:
+            torch._foreach_copy_(list(rows), attn)
+        return self.attn_rows[dtype]
+
     def forward(self):
         """Every episode's pass (branches are forked onto their own streams and joined on the current one)."""
         if self.merged is not None:
-            if self.spec.o_in:
-                attn = [st.attn for st in self.stacks]
-                if attn[0].dtype != self.attn_rows.dtype:
-                    self.attn_rows = self.attn_rows.to(attn[0].dtype)
-                rows = self.attn_rows.view(self.episodes, self.spec.M, -1)
-                if all(t is attn[0] for t in attn):   # one output for all of them, as load() leaves it
-                    rows.copy_(attn[0])
-                else:
-                    torch._foreach_copy_(list(rows), attn)
-            self.merged.attn = self.attn_rows
+            self.merged.attn = self._merged_attn() if self.spec.o_in else None
             self.merged.forward()
             for st in self.stacks:
                 st.launches_per_forward = self.merged.launches_per_forward

@@ -81,3 +81,47 @@ def test_scratch_of_an_episode_is_its_own(setup):
         used = [getattr(st, name) for st in batch.stacks] + [getattr(batch.merged, name)]
         spans = sorted((t.data_ptr(), t.data_ptr() + t.numel() * t.element_size()) for t in used)
         assert all(a[1] <= b[0] for a, b in zip(spans, spans[1:])), name
+
+
+def test_fewer_inputs_than_episodes(setup):
+    """As with separate stacks, the episodes behind the last input keep what they have."""
+    batch, lone, xs, attn = setup(64)
+    batch.load(xs, attn)
+    batch.load(xs[1:2], attn)
+    lone[0].load(xs[1], attn)
+    batch.load([], attn)
+    batch.forward()
+    for st, alone in zip(batch.stacks, lone):
+        assert torch.equal(st.res, alone.forward())
+
+
+def test_attention_outputs_of_several_types(setup):
+    batch, lone, xs, attn = setup(64)
+    batch.load(xs, attn)
+    for e, dtype in enumerate((torch.float16, torch.bfloat16, torch.float32)):
+        mine = (attn.float() * (1.0 + e / 7)).to(dtype)
+        batch.stacks[e].load(xs[e], mine)
+        lone[e].load(xs[e], mine)
+    batch.forward()
+    for st, alone in zip(batch.stacks, lone):
+        assert torch.equal(st.res, alone.forward())
+
+
+def test_attention_buffer_of_a_captured_pass_stays(setup):
+    """A captured graph writes to the addresses of its capture: changing the element type in between must not
+    free them."""
+    batch, _, xs, attn = setup(64)
+    used = []
+    for dtype in (torch.bfloat16, torch.float16, torch.bfloat16):
+        batch.load(xs, attn.to(dtype))
+        batch.forward()
+        used.append(batch.merged.attn.data_ptr())
+    assert used[0] == used[2] != used[1]
+
+
+@pytest.mark.parametrize("bad", [lambda t: t[:1], lambda t: t.double(), lambda t: t.to("meta"), lambda t: t.T.contiguous().T])
+def test_attention_outputs_that_one_stack_refuses(setup, bad):
+    batch, _, xs, attn = setup(64)
+    batch.load(xs, bad(attn))
+    with pytest.raises(ValueError):
+        batch.forward()
