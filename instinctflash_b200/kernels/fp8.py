@@ -181,11 +181,15 @@ def fp8_linear_gated(a: torch.Tensor, a_scale: torch.Tensor, w: Fp8Weight, h: to
     return h
 
 
-@lru_cache(maxsize=None)
+PLANES_MAX_WIDTH = 8192   # columns that the residual kernel over planes takes
+
+
+@lru_cache(maxsize=1024)
 def partial_splits(M: int, N: int, K: int, sm_count: int = 148) -> int:
     """How many K ranges ``gemm_partials`` should use for a narrow projection whose consumer adds the
     planes: up to 128 rows enough (tile, range) pairs to occupy the GPU, every range at least four
-    128-byte K slabs, at most eight planes.
+    128-byte K slabs, at most eight planes.  1, the unsplit GEMM, for outputs wider than the residual kernel
+    over planes takes.
 
     Above 128 rows the number with the least estimated time, 1 where the unsplit GEMM is as good.  In SM clocks: a
     slab of a 128 x 64 / 256 tile 380 / 700 and a wave 7500 for prologue and fp32 epilogue, every plane written
@@ -196,7 +200,7 @@ def partial_splits(M: int, N: int, K: int, sm_count: int = 148) -> int:
     Four decoder layers of 2048 x 16384: 315 -> 300 us at 301 rows (six planes against the GEMM that splits
     K over a cluster), 438 -> 402 at 640 (three); GEMM and residual of 816 x 2048 x 8192 25.6 -> 23.4 us
     unsplit, of 384 x 3072 x 8192 23.3 -> 21.2 in four."""
-    if K % 128:
+    if K % 128 or N > PLANES_MAX_WIDTH:
         return 1
     slabs = K // 128
     if M <= 128:

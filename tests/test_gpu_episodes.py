@@ -81,6 +81,23 @@ def test_episodes_on_streams_of_their_own(M, o_in):
             assert torch.equal(st.res, w)
 
 
+# one column block wider than the residual kernel over planes takes, and the widest that it takes
+@pytest.mark.parametrize("hidden", [9216, 8192])
+def test_wide_decoder_stack_above_128_rows(hidden):
+    from instinctflash_b200.stack import LinearStack, StackSpec, make_inputs, make_weights
+    spec = StackSpec("wide", "gemma", 1, 129, hidden, 16384, 512, seed=8)
+    weights = make_weights(spec, DEV)
+    x, attn = make_inputs(spec, DEV)
+    got = []
+    for planes in (True, False):
+        st = LinearStack(spec, weights, DEV, split_partials=planes)
+        st.load(x, attn)
+        got.append(st.forward().double())
+    # the order of the K sum may differ, which can move a sum across a bf16 rounding: 2^-8 of the update's size
+    update = got[1] - x.double()
+    assert ((got[0] - got[1]).norm() / update.norm()).item() < 2.0 ** -8
+
+
 # the 64-row form and its neighbours, and K whose last slab is ragged: with whole stages in front, alone in its
 # stage, in the first stage; the K order does not depend on the form, so the bits are those of 128-wide tiles
 @pytest.mark.parametrize("M", [1, 16, 17, 50, 63, 64, 65, 128, 300])

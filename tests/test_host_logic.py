@@ -154,3 +154,12 @@ def test_qkv_consumers_reject_bad_arguments_before_launch():
     with pytest.raises(ValueError, match="CUDA"):
         wan.wan_qkv(x, torch.zeros(4, 64, dtype=torch.float16), heads=1, head_dim=64, tokens=4)
     assert rope.rope_inv_freq(8, 10000.0, "cpu").tolist() == pytest.approx([1.0, 0.1, 0.01, 0.001])
+
+
+@pytest.mark.parametrize("M,N,K", [(129, 9216, 16384), (129, 10240, 16384), (257, 16384, 16384), (50, 8208, 4096), (2000, 8208, 32768)])
+def test_no_planes_for_rows_wider_than_their_consumer_takes(M, N, K):
+    assert fp8.partial_splits(M, N, K) == 1
+
+
+def test_planes_up_to_the_widest_row_of_their_consumer():
+    assert fp8.PLANES_MAX_WIDTH == 8192 and fp8.partial_splits(129, 8192, 16384) > 1
