@@ -191,7 +191,8 @@ class LinearStack:
             sms = torch.cuda.get_device_properties(dev).multi_processor_count
             ks = [k for name, n, k in spec.linears() if n == D and name in ("o", "down")]
             self.splits = {k: self.ops.partial_splits(split_rows, D, k, sms) for k in ks}
-            self.part = torch.zeros(max(self.splits.values(), default=1) * M * D, dtype=f32, device=dev)
+            planes = max(self.splits.values(), default=1)
+            self.part = torch.zeros(planes * M * D if planes > 1 else 0, dtype=f32, device=dev)
         self.attn = None
         self.launches_per_forward = 0
 

@@ -11,7 +11,7 @@ from instinctflash_b200.stack import EpisodeBatch, LinearStack, StackSpec, make_
 EPISODES = 3
 
 
-def split_ops():
+def split_ops(planes=2):
     """The oracle's operators with K-split GEMMs, as this package's operator set has them."""
     ops = oracle_ops.ops()
 
@@ -21,7 +21,7 @@ def split_ops():
             part = oracle_ops.CpuFp8Weight(w.w[:, lo:hi].contiguous(), None)
             oracle_ops.gemm_acc(a[:, lo:hi].contiguous(), part, plane)
 
-    ops.gemm_partials, ops.partial_splits = gemm_partials, lambda M, N, K, sms: 2
+    ops.gemm_partials, ops.partial_splits = gemm_partials, lambda M, N, K, sms: planes
     return ops
 
 
@@ -125,3 +125,11 @@ def test_attention_outputs_that_one_stack_refuses(setup, bad):
     batch.load(xs, bad(attn))
     with pytest.raises(ValueError):
         batch.forward()
+
+
+def test_no_planes_are_held_where_nothing_is_split(monkeypatch):
+    monkeypatch.setattr(torch.cuda, "get_device_properties", lambda dev: SimpleNamespace(multi_processor_count=148))
+    spec = StackSpec("tiny", "gemma", layers=1, M=8, hidden=64, ffn=128, qkv=96, seed=5)
+    weights = make_weights(spec, "cpu", cpu_seeded=True)
+    held = [LinearStack(spec, weights, "cpu", ops=split_ops(planes)).part.numel() for planes in (1, 2)]
+    assert held == [0, 2 * spec.M * spec.hidden]
