@@ -22,6 +22,7 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/version.h>
 
 #include <algorithm>
 #include <cmath>
@@ -673,4 +674,9 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_calls", "Calls from tensors to li
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__calls() { return PyModule_Create(&module); }
+// `torch_version`: whose tensors this file was compiled for; the loader binds it under that torch only
+PyMODINIT_FUNC PyInit__calls() {
+  PyObject* m = PyModule_Create(&module);
+  if (m && PyModule_AddStringConstant(m, "torch_version", TORCH_VERSION) < 0) Py_CLEAR(m);
+  return m;
+}

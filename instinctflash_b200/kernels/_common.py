@@ -9,8 +9,8 @@ try:
     from .. import _calls as native
 except ImportError:
     class _Unbuilt:
-        """Stands in for ``_calls`` where it has not been built: takes no call, so that every operator
-        goes on to ``launch`` and raises there."""
+        """Stands in for a ``_calls`` that is missing or does not import: takes no call, so that every
+        operator goes on to its checks in Python and ``launch``."""
 
         def __getattr__(self, name):
             return lambda *args: None
