@@ -76,8 +76,11 @@ class SM100FP8Linear(nn.Module):
     def forward(self, x):
         # the plain case in one native call (allocations, pack, GEMM): a module called from Python for 50 tokens
         # spent 55 us on the host for 10 us of kernels
-        packed = self._buffers
-        y = native.projection(x, packed["weight_fp8"], packed["weight_scale"], packed["bias"])
+        packed = self._buffers   # (attribute look-up through nn.Module takes longer than the checks behind it)
+        try:
+            y = native.projection(x, packed["weight_fp8"], packed["weight_scale"], packed["bias"])
+        except KeyError:         # a packed tensor has become a parameter or a plain attribute
+            y = None
         return self._forward(x) if y is None else y
 
     @torch.no_grad()
