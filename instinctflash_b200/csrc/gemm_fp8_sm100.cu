@@ -1771,7 +1771,6 @@ static int run_gemm(const void* a, int64_t ld_a, const void* w, int64_t ld_w, Ge
         }
       }
     }
-    if (best_bn == 0 && g_cfg_mode < 2) return IFLB200_ERR_ARG;  // the forced configuration does not fit this problem
     bn = best_bn;
     if (g_cfg_mode == 0 && g_cfg_tile_n == 0 && g_cfg_split_k == 0 && g_cfg_swap != 2 && p.M > BM && p.N >= 256) {
       const int64_t tiles = (int64_t)((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + 255) / 256);
@@ -1806,6 +1805,7 @@ static int run_gemm(const void* a, int64_t ld_a, const void* w, int64_t ld_w, Ge
     return g_cfg_mode == 2 ? launch_gemm_pair<PBN, 6, 1>(ta, tw, to, p, grid, s)
                            : launch_gemm_pair<PBN, 6, 2>(ta, tw, to, p, grid, s);  // two accumulators
   }
+  if (bn == 0) return IFLB200_ERR_ARG;  // the forced configuration does not fit this problem
 
   // Swapped form for a few hundred tokens: the tokens go on the MMA's N side in tiles of the width
   // that fits them (816 tokens = 4 x 208 with 2 % padding, where 7 row blocks of 128 carry 9 %), the
