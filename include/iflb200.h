@@ -257,14 +257,14 @@ IFLB200_API int iflb200_gemm_fp8_raw(const void* a, int64_t ld_a, const void* w,
                          int M, int N, int K, void* out, int64_t ld_out, void* stream);
 
 /*
- * Split-K for skinny activations: K is divided into `splits` ranges, each range of each tile (64
- * columns for M <= 128, 256 above) goes to its own CTA, so that a deep reduction with few
- * output columns still uses the whole GPU, and leaves its fp32 partial sums (the ranges, and so the
- * bits of the planes, do not depend on M):
+ * Split-K for outputs whose tiles do not fill the GPU: K is divided into `splits` ranges, each range of
+ * each tile (64 columns up to 128 rows; 64 or 256 above, by estimated time, on CTA pairs where blocks of
+ * 256 rows pad little) is a unit of work of its own and leaves its fp32 partial sums (the ranges, and
+ * so the bits of the planes, do not depend on M):
  *   out[s][m][n] = sum over the s-th K range of a[m,k] * w[n,k]       (no scales, no rounding)
  * The consumer (iflb200_residual_norm_quant_partials) adds the planes in split order, so the
- * result does not depend on timing.  K a multiple of 128; splits <= ceil(K / 512); `out` is
- * scratch owned by the caller, splits * M * ld_out floats.
+ * result does not depend on timing; it takes up to eight planes of up to 8192 columns.  K a multiple
+ * of 128; splits <= ceil(K / 512); `out` is scratch owned by the caller, splits * M * ld_out floats.
  * Replaces: instinctflash/kernels/fp8.py:50-53 for the deep, narrow projections of the action
  * expert (instinctflash/engines/pi05/engine.py:244-250); the split has no reference counterpart.
  */

@@ -799,8 +799,8 @@ gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
   // tile per CTA (the host launches tiles x S CTAs, at most one wave).
   // Partials: K split over independent CTAs (no cluster), each writing its fp32 partial sums.
   constexpr bool PLANES = SPLIT == 3, LEAN = SPLIT == 4;
-  const bool partials = (SPLIT == 2 || LEAN) && p.partials > 1;
-  const bool split = !partials && (SPLIT == 1 || (SPLIT == 2 && p.split_k > 1));
+  const bool partials = LEAN && p.partials > 1;
+  const bool split = SPLIT == 1 || (SPLIT == 2 && p.split_k > 1);
   // At most 64 rows: MMAs of M = 64, whose row i lies in lane i % 16 of quadrant i / 16
   constexpr int quad_rows = AR / 4;
   const int k_parts = partials || PLANES ? p.partials : (split ? p.split_k : 1);
@@ -1050,7 +1050,7 @@ gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
         const int col_tma_end = col_begin + (col_end - col_begin) / per_store * per_store;
         epilogue_tma_store<BN, quad_rows>(p, tm_dst, t_row, staging, staging_ptr, m_blk * BM + quad * quad_rows, n_blk * BN,
                                col_begin, col_tma_end, rs, lane,
-                               PLANES ? unit % k_parts : (((SPLIT == 2 || LEAN) && p.partials >= 1) ? split_rank : -1),  // a plane map takes a 3-D store
+                               PLANES ? unit % k_parts : (LEAN && p.partials >= 1 ? split_rank : -1),  // a plane map takes a 3-D store
                                prefetch ? &cv : nullptr);
         if (BN % 64 != 0 && col_tma_end < col_end) {
           const int n0 = n_blk * BN + col_tma_end;
@@ -1082,7 +1082,7 @@ gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
     __syncwarp();
   }
 
-  if (!LEAN && split) {
+  if (split) {
     // CTA r of the cluster reduces columns [r*BN/S, (r+1)*BN/S) of the tile: its own partial
     // comes from tensor memory, the peers write theirs into its shared memory, and the sum runs
     // in rank order (fixed, so the result does not depend on timing); then the consumer
