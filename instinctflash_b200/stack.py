@@ -392,7 +392,7 @@ class EpisodeBatch:
 
     def __init__(self, spec: StackSpec, weights, device, episodes: int, **stack_kw):
         self.spec, self.dev, self.episodes = spec, torch.device(device), episodes
-        self.launches_per_forward = 0   # of all episodes: a launch counts once for every episode it serves
+        self.launches_per_forward = 0   # of all episodes together; one that serves them all counts once
         self.merged = None
         if spec.kind == "gemma" and episodes > 1 and spec.M * episodes <= 65535:
             wide = StackSpec(**{**spec.__dict__, "M": spec.M * episodes})
@@ -445,8 +445,7 @@ class EpisodeBatch:
         if self.merged is not None:
             self.merged.attn = self._merged_attn() if self.spec.o_in else None
             self.merged.forward()
-            for st in self.stacks:
-                st.launches_per_forward = self.merged.launches_per_forward
+            self.launches_per_forward = self.merged.launches_per_forward
         else:
             main = torch.cuda.current_stream(self.dev)
             for st, side in zip(self.stacks, self.streams):
@@ -455,7 +454,7 @@ class EpisodeBatch:
                     st.forward()
             for side in self.streams:
                 main.wait_stream(side)
-        self.launches_per_forward = sum(st.launches_per_forward for st in self.stacks)
+            self.launches_per_forward = sum(st.launches_per_forward for st in self.stacks)
         return [st.res for st in self.stacks]
 
     def capture(self):

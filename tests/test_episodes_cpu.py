@@ -133,3 +133,11 @@ def test_no_planes_are_held_where_nothing_is_split(monkeypatch):
     weights = make_weights(spec, "cpu", cpu_seeded=True)
     held = [LinearStack(spec, weights, "cpu", ops=split_ops(planes)).part.numel() for planes in (1, 2)]
     assert held == [0, 2 * spec.M * spec.hidden]
+
+
+def test_launches_of_a_stacked_pass_count_once(setup):
+    batch, lone, xs, attn = setup(64)
+    batch.load(xs, attn)
+    batch.forward()
+    lone[0].forward()
+    assert batch.launches_per_forward == lone[0].launches_per_forward

@@ -262,9 +262,9 @@ def test_a_wait_that_nothing_satisfies_runs_out_and_leaves_the_context_usable():
     assert torch.equal(ps.res, want)
 
 
-def test_episode_batch_branches_equal_separate_runs():
-    """Independent episodes in flight as parallel branches of one CUDA graph: every episode's
-    residual stream equals the one a lone stack computes from the same input."""
+def test_episode_batch_equals_separate_runs():
+    """Independent episodes stacked along the rows of one CUDA graph: every episode's residual stream
+    equals the one a lone stack computes from the same input."""
     from instinctflash_b200.stack import EpisodeBatch
     spec = StackSpec("expert", "gemma", 3, 50, 1024, 4096, 1536, steps=2, seed=4)
     weights = make_weights(spec, DEV)
@@ -285,7 +285,37 @@ def test_episode_batch_branches_equal_separate_runs():
     torch.cuda.synchronize()
     for st, w in zip(batch.stacks, want):
         assert torch.equal(st.res, w)
-    assert batch.launches_per_forward == 4 * batch.stacks[0].launches_per_forward
+    # one launch per operator for all four: gate_up, quantiser, down, residual and the QKV GEMM of every layer and step
+    assert batch.launches_per_forward == spec.layers * spec.steps * 5
+
+
+# rotary DiT blocks are not stacked: they run as branches of one graph
+def test_episode_batch_branches_equal_separate_runs():
+    """Independent episodes in flight as parallel branches of one CUDA graph: every episode's
+    residual stream equals the one a lone stack computes from the same input."""
+    from instinctflash_b200.stack import EpisodeBatch
+    spec = StackSpec("wan", "wan", 2, 96, 1536, 4096, 4608, o_in=1536, cross=True, seed=4)
+    weights = make_weights(spec, DEV)
+    xs = []
+    for e in range(3):
+        x, attn = make_inputs(StackSpec(**{**spec.__dict__, "seed": 40 + e}), DEV)
+        xs.append(x)
+    want = []
+    for x in xs:
+        st = LinearStack(spec, weights, DEV)
+        st.load(x, attn)
+        want.append(st.forward().clone())
+    batch = EpisodeBatch(spec, weights, DEV, 3)
+    assert batch.merged is None
+    batch.load(xs, attn)
+    g = batch.capture()
+    for _ in range(2):
+        batch.load(xs, attn)
+        g.replay()
+        torch.cuda.synchronize()
+        for st, w in zip(batch.stacks, want):
+            assert torch.equal(st.res, w)
+    assert batch.launches_per_forward == 3 * batch.stacks[0].launches_per_forward == 3 * spec.layers * 12
 
 
 def test_results_do_not_depend_on_what_ran_before():
