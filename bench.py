@@ -48,7 +48,7 @@ UNIT = "TFLOP/s"
 NOMINAL_FP8_TFLOPS = 4500.0
 NOMINAL_HBM_GBS = 8000.0
 EPISODES = 64           # independent action-expert episodes of the sharded c3 configuration
-EPISODE_BRANCHES = 8    # episodes in flight on one GPU (parallel branches of one CUDA graph)
+EPISODE_BRANCHES = 8    # episodes in flight on one GPU (stacked along the rows of one CUDA graph)
 
 
 def measured_peaks():
@@ -531,10 +531,9 @@ def max_over_ranks(ms, dist, dev):
 
 def sharded_c3_episodes(dev, dist, rank, world, steps, warmup, max_branches=EPISODE_BRANCHES):
     """64 independent action-expert episodes (M = 50 each, 18 layers x 10 flow steps), 64 / p per
-    GPU, no collective.  On each GPU up to 8 episodes are in flight as parallel branches of one CUDA
-    graph (every GEMM still has M = 50 rows; branches that reach the same layer together find its
-    weights in L2)."""
-    from instinctflash_b200.stack import SPECS, EpisodeBatch, make_inputs, make_weights
+    GPU, no collective.  On each GPU up to 8 episodes are in flight, stacked along the rows: one launch
+    per operator serves them all, and a weight is read once for all of them."""
+    from instinctflash_b200.stack import SPECS, EpisodeBatch, StackSpec, make_inputs, make_weights
     spec = SPECS["c3"]
     mine = EPISODES // world + (1 if rank < EPISODES % world else 0)
     branches = min(max_branches, max(1, mine))
@@ -551,14 +550,15 @@ def sharded_c3_episodes(dev, dist, rank, world, steps, warmup, max_branches=EPIS
         dist.barrier()
     ms = replay_ms(g, rounds * steps, stream, dev) / steps      # all of this rank's episodes, once
     ms = max_over_ranks(ms, dist, dev)
-    per_episode_bytes = stack_bytes(spec)
+    # a weight once per flow step for the episodes in flight together, everything else per episode
+    nbytes = rounds * stack_bytes(StackSpec(**{**spec.__dict__, "M": spec.M * branches}))
     peaks = measured_peaks()
     out = {"episodes": EPISODES, "episodes_per_rank": mine, "branches_per_gpu": branches, "ms_all_episodes": ms,
            "episodes_per_s": EPISODES / (ms * 1e-3), "ms_per_episode_per_gpu": ms / max(1, mine),
-           "algorithmic_gbs_per_gpu": per_episode_bytes * mine / (ms * 1e-3) / 1e9,
-           "frac_of_hbm_peak": per_episode_bytes * mine / (ms * 1e-3) / 1e9 / peaks["hbm_gbs"],
-           "note": "algorithmic bytes count every weight once per episode and flow step; branches that share a layer's "
-                   "weights through L2 read less from DRAM than that", "collective": "none"}
+           "algorithmic_gbs_per_gpu": nbytes / (ms * 1e-3) / 1e9,
+           "frac_of_hbm_peak": nbytes / (ms * 1e-3) / 1e9 / peaks["hbm_gbs"],
+           "note": "algorithmic bytes count a weight once per flow step for the episodes in flight together",
+           "collective": "none"}
     del batch, g, weights
     torch.cuda.empty_cache()
     return out
