@@ -794,7 +794,7 @@ def main():
     local_rank = int(os.environ.get("LOCAL_RANK", "0"))
     world = int(os.environ.get("WORLD_SIZE", "1"))
 
-    from instinctflash_b200.stack import SPECS, LinearStack, StackSpec, make_inputs, make_weights
+    from instinctflash_b200.specs import SPECS, StackSpec
     spec = SPECS[args.workload]
     if args.episodes > 1:
         spec = StackSpec(**{**spec.__dict__, "M": spec.M * args.episodes})
@@ -805,8 +805,9 @@ def main():
         spec = StackSpec(**{**spec.__dict__, "M": -(-spec.M // world)})
 
     if args.impl == "reference":
-        run_reference(args, spec, rank, world)
+        run_reference(args, spec, rank, world)   # none of this package's kernels or call paths is loaded
         return
+    from instinctflash_b200.stack import LinearStack, make_inputs, make_weights
 
     if not torch.cuda.is_available():
         raise SystemExit("bench.py needs a CUDA device: the FP8 linear path has no CPU fallback")
