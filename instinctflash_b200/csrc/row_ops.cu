@@ -987,45 +987,6 @@ amax_partial_kernel(const uint16_t* __restrict__ x, int64_t n, uint32_t* __restr
   }
 }
 
-__device__ __forceinline__ float scale_of_bits(uint32_t best) {  // the maximum's magnitude bits -> max(amax, 1e-12) / 448
-  if (best > 0x7F80u) return __uint_as_float(0x7FC00000u);
-  return __fmul_rn(fmaxf(__uint_as_float(best << 16), 1e-12f), (float)(1.0 / 448.0));
-}
-
-__device__ __forceinline__ float pack_one(float x, float scale) {
-  const float d = __fdiv_rn(x, scale);
-  return (d != d) ? d : fminf(fmaxf(d, -448.0f), 448.0f);
-}
-
-// Eight codes of x / scale.  The quotient is the correctly rounded one by Markstein's correction (P. Markstein,
-// "Computation of elementary functions on the IBM RISC System/6000 processor", 1990): with r = 1 / scale
-// correctly rounded and q = x r, the remainder x - q scale is exact in one fma and q + r (x - q scale)
-// rounds to the quotient, in three packed instructions per pair instead of a division each.  Where the
-// remainder underflows, the code is zero either way; a scale that is not finite takes the division
-// (`r` is then NaN).  The conversion saturates, which is the clamp to +-448.  Compared on the GPU for every
-// bf16 maximum and every bf16 x: no code differs.
-__device__ __forceinline__ uint2 pack_eight(const uint4& u, float scale, float r) {
-  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-  float f[8];
-  const bool fast = r == r;
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const float lo = __uint_as_float(w[k] << 16), hi = __uint_as_float(w[k] & 0xFFFF0000u);
-    if (fast) {  // of -x: a zero keeps its sign that way, the codes' signs are turned back below
-      const uint64_t x2 = pack2(lo, hi), n2 = pack2(-r, -r), q = mul2(x2, n2);
-      unpack2(fma2(fma2(q, pack2(scale, scale), x2), n2, q), f[2 * k], f[2 * k + 1]);
-    } else {
-      f[2 * k] = pack_one(lo, scale);
-      f[2 * k + 1] = pack_one(hi, scale);
-    }
-  }
-  const uint32_t turn = fast ? 0x80808080u : 0u;
-  return make_uint2(cvt_e4m3x4(f[0], f[1], f[2], f[3]) ^ turn, cvt_e4m3x4(f[4], f[5], f[6], f[7]) ^ turn);
-}
-__device__ __forceinline__ float reciprocal_for_pack(float scale) {
-  return scale > 1e-20f && scale < 1e37f ? __frcp_rn(scale) : __uint_as_float(0x7FC00000u);
-}
-
 // n_partial > 0: dynamic scale from the partial maxima (every CTA recomputes it; CTA 0 writes
 // it out).  n_partial == 0: fixed scale read from scale_in.
 __global__ void __launch_bounds__(kPackThreads)

@@ -1,6 +1,6 @@
 // Element-wise arithmetic shared by the row kernels and the GEMM epilogues.  Every operation
-// is an explicitly rounded fp32 instruction in the order the reference's Triton kernels
-// compile to for sm_100 (instinctflash/kernels/norm.py:44-80,135-147,168-175 and
+// is an explicitly rounded fp32 instruction in the order of the reference's source
+// (instinctflash/kernels/norm.py:44-80,135-147,168-175 and
 // instinctflash/kernels/activation.py:26-43): a multiply that feeds an add is contracted
 // into one fma.rn, every other multiply and add rounds on its own.
 #pragma once
@@ -136,8 +136,8 @@ __device__ __forceinline__ float gelu_tanh_ref(float v) {
 // The same for two elements, with fewer instructions and the same results: packed arithmetic; the
 // multiplications by -2 and log2(e) as one (a power of two is exact); ex2 and the reciprocal with
 // subnormals flushed, whose difference disappears in 1 + e and in d - 1; 2/den as 2 * rcp(den), exact
-// in the product and fused with the -1.  Compared with the function above on the GPU for all 2^32
-// inputs: no bit differs.  The GELU quantiser of 4680 x 14336 rows spent 128 us on the long form.
+// in the product and fused with the -1.  No bit differs from the function above for any of the 2^32
+// inputs (tests/exhaustive.cu compares them all).  The GELU quantiser of 4680 x 14336 rows spent 128 us on the long form.
 __device__ __forceinline__ uint64_t gelu_tanh_ref2(uint64_t v) {
   const float k1 = __uint_as_float(0x3D372713u), k2 = __uint_as_float(0x3F4C422Au), kz = -2.0f * __uint_as_float(0x3FB8AA3Bu);
   const uint64_t a1 = mul2(v, pack2(k1, k1));
@@ -181,6 +181,46 @@ __device__ __forceinline__ uint32_t f32_to_bf16_bits(float f) {
 }
 __device__ __forceinline__ uint32_t f32_to_f16_bits(float f) {
   return (uint32_t)__half_as_ushort(__float2half_rn(f));
+}
+
+// Per-tensor pack.
+__device__ __forceinline__ float scale_of_bits(uint32_t best) {  // the maximum's magnitude bits -> max(amax, 1e-12) / 448
+  if (best > 0x7F80u) return __uint_as_float(0x7FC00000u);
+  return __fmul_rn(fmaxf(__uint_as_float(best << 16), 1e-12f), (float)(1.0 / 448.0));
+}
+
+__device__ __forceinline__ float pack_one(float x, float scale) {
+  const float d = __fdiv_rn(x, scale);
+  return (d != d) ? d : fminf(fmaxf(d, -448.0f), 448.0f);
+}
+
+// Eight codes of x / scale.  The quotient is the correctly rounded one by Markstein's correction (P. Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor", 1990): with r = 1 / scale
+// correctly rounded and q = x r, the remainder x - q scale is exact in one fma and q + r (x - q scale)
+// rounds to the quotient, in three packed instructions per pair instead of a division each.  Where the
+// remainder underflows, the code is zero either way; a scale that is not finite takes the division
+// (`r` is then NaN).  The conversion saturates, which is the clamp to +-448.  No code differs for any bf16
+// maximum and any bf16 x up to it (tests/exhaustive.cu compares them all).
+__device__ __forceinline__ uint2 pack_eight(const uint4& u, float scale, float r) {
+  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+  float f[8];
+  const bool fast = r == r;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const float lo = __uint_as_float(w[k] << 16), hi = __uint_as_float(w[k] & 0xFFFF0000u);
+    if (fast) {  // of -x: a zero keeps its sign that way, the codes' signs are turned back below
+      const uint64_t x2 = pack2(lo, hi), n2 = pack2(-r, -r), q = mul2(x2, n2);
+      unpack2(fma2(fma2(q, pack2(scale, scale), x2), n2, q), f[2 * k], f[2 * k + 1]);
+    } else {
+      f[2 * k] = pack_one(lo, scale);
+      f[2 * k + 1] = pack_one(hi, scale);
+    }
+  }
+  const uint32_t turn = fast ? 0x80808080u : 0u;
+  return make_uint2(cvt_e4m3x4(f[0], f[1], f[2], f[3]) ^ turn, cvt_e4m3x4(f[4], f[5], f[6], f[7]) ^ turn);
+}
+__device__ __forceinline__ float reciprocal_for_pack(float scale) {
+  return scale > 1e-20f && scale < 1e37f ? __frcp_rn(scale) : __uint_as_float(0x7FC00000u);
 }
 
 }  // namespace iflb200

@@ -4,8 +4,8 @@ Drop-in for the three operators of ``instinctflash/kernels/norm.py``:
 ``row_quant`` (lines 128-158), ``dequant_rows`` (lines 162-185) and ``residual_norm_quant``
 (lines 26-124, without its MoE ``router`` tail).  Same argument names and meaning; the Triton
 tuning hints (``num_warps``, ``block``) are accepted and ignored.  The arithmetic follows the
-instruction order the reference compiles to on sm_100, so the e4m3 codes and scales of the
-quantiser are bit-identical to the reference's on the same inputs.
+order of the reference's source; recorded outputs of the reference on a B200 confirm that the e4m3
+codes and scales of the quantiser are bit-identical on the same inputs.
 """
 from __future__ import annotations
 
