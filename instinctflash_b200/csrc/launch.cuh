@@ -19,6 +19,15 @@ inline bool dependent_launch_for(long long rows) {
   return g_dependent_launch == 2 || (g_dependent_launch == 1 && rows <= kDependentLaunchMaxRows);
 }
 
+// Multiprocessors of the current device; 0 when it cannot be told.
+inline int device_sm_count() {
+  static int count[64] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  if (count[dev] == 0) cudaDeviceGetAttribute(&count[dev], cudaDevAttrMultiProcessorCount, dev);
+  return count[dev];
+}
+
 // The node that a stream capture of `s` stands at: the last kernel captured into it.  False outside a
 // capture, and where several branches meet.
 struct CapturePoint {

@@ -556,8 +556,10 @@ __device__ __forceinline__ float round_through<__nv_bfloat16>(float x) {
   return __bfloat162float(__float2bfloat16_rn(x));
 }
 
-template <typename RT, int TPR, int IT, bool FAST>
-__global__ void __launch_bounds__(kRowThreads, resnorm_min_blocks<IT>())
+// PART: the delta arrives as fp32 planes of a K-split GEMM (a.dpart) instead of a raw bf16 accumulator; an
+// instantiation of its own, so that the ordinary one keeps its registers.
+template <typename RT, int TPR, int IT, bool FAST, bool PART = false>
+__global__ void __launch_bounds__(kRowThreads, PART ? 2 : resnorm_min_blocks<IT>())
 residual_norm_quant_kernel(const ResNormArgs a) {
   row_begin(a.early);  // inputs may come from the kernel before this one in the stream
   __shared__ float red[3][kRowThreads / 32];
@@ -566,6 +568,8 @@ residual_norm_quant_kernel(const ResNormArgs a) {
   const bool live = m < a.M;
   RT* rr = reinterpret_cast<RT*>(a.res) + (live ? (int64_t)m * a.ld_res : 0);
   const __nv_bfloat16* dr = a.delta ? a.delta + (live ? (int64_t)m * a.ld_delta : 0) : nullptr;
+  const float* dp = PART ? a.dpart + (live ? (int64_t)m * a.ld_delta : 0) : nullptr;
+  const int64_t dp_plane = (int64_t)a.M * a.ld_delta;
   const int64_t mofs = (live && a.mod_index) ? (int64_t)a.mod_index[m] * a.D : 0;
   const float drs = (live && a.drow) ? a.drow[m] : 1.0f;
   const float fD = (float)a.D;
@@ -577,7 +581,7 @@ residual_norm_quant_kernel(const ResNormArgs a) {
     const int c0 = (it * TPR + t) * 8;
     const bool on = it < a.iters && live && c0 < a.D;
     rres[it] = fetch<FAST, RT>(rr, c0, a.D, on);
-    rdel[it] = fetch<FAST, __nv_bfloat16>(dr, c0, a.D, on && dr != nullptr);
+    rdel[it] = fetch<FAST, __nv_bfloat16>(dr, c0, a.D, on && dr != nullptr && !PART);
   }
   float x[IT][8];
   float sum = 0.0f, sumsq = 0.0f;
@@ -586,9 +590,32 @@ residual_norm_quant_kernel(const ResNormArgs a) {
     const int c0 = (it * TPR + t) * 8;
     unpack(rres[it], x[it]);
     if (it < a.iters && live && c0 < a.D) {
-      if (dr) {
+      if (dr || PART) {
         float d[8], cs[8], bs[8], gs[8];
-        unpack(rdel[it], d);
+        if constexpr (PART) {
+          // four planes in flight together, added in split order
+          constexpr int kGroup = 4;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) d[i] = 0.0f;
+#pragma unroll 1
+          for (int s0 = 0; s0 < a.dsplits; s0 += kGroup) {
+            float e[kGroup][8];
+#pragma unroll
+            for (int sp = 0; sp < kGroup; ++sp)
+              if (s0 + sp < a.dsplits) load_f32<FAST>(dp + (s0 + sp) * dp_plane, c0, a.D, e[sp]);
+#pragma unroll
+            for (int sp = 0; sp < kGroup; ++sp) {
+              if (s0 + sp < a.dsplits) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) d[i] = (s0 + sp == 0) ? e[sp][i] : __fadd_rn(d[i], e[sp][i]);
+              }
+            }
+          }
+#pragma unroll
+          for (int i = 0; i < 8; ++i) d[i] = __bfloat162float(__float2bfloat16_rn(d[i]));
+        } else {
+          unpack(rdel[it], d);
+        }
         if (a.dcol) load_f32<FAST>(a.dcol, c0, a.D, cs);
         if (a.bias) load_f32<FAST>(a.bias, c0, a.D, bs);
         if (a.gate) load_f32<FAST>(a.gate + mofs, c0, a.D, gs);
@@ -678,6 +705,20 @@ residual_norm_quant_kernel(const ResNormArgs a) {
   for (int it = 0; it < IT; ++it) {
     const int c0 = (it * TPR + t) * 8;
     if (it < a.iters && c0 < a.D) store_codes<FAST>(qr, c0, a.D, x[it], inv);
+  }
+  if constexpr (PART) {
+#pragma unroll
+    for (int k = 0; k < kMaxMirrors; ++k) {
+      if (k < a.mirrors) {
+        if (t == 0) a.qs_mirror[k][m] = scale;
+        uint8_t* qm = a.q_mirror[k] + (int64_t)m * a.ld_q;
+#pragma unroll
+        for (int it = 0; it < IT; ++it) {
+          const int c0 = (it * TPR + t) * 8;
+          if (it < a.iters && c0 < a.D) store_codes<FAST>(qm, c0, a.D, x[it], inv);
+        }
+      }
+    }
   }
 }
 
@@ -914,25 +955,43 @@ residual_norm_planes_kernel(const ResNormArgs a) {
   }
 }
 
-// Rows of at most 8192 columns on the aligned path; planes in groups that fit the registers.
+// Rows of at most 8192 columns on the aligned path.  The quads form takes its further plane groups quad by quad, each
+// a round trip, and that many registers let few rows be resident: it serves the widths and numbers of planes
+// whose loads it has all in flight.  us, quads against rows of eight columns a thread:
+//   up to 2048 columns ahead everywhere (1024, 50 rows, 8 planes 2.66 / 3.10; 2048, 816 rows, 2 planes 5.71 / 7.60);
+//   to 3072 where its three rows an SM need no more waves than the other's two pairs (300 rows, 2 planes 4.58 / 5.72,
+//   816 rows 7.82 / 10.49, but 500 rows 6.45 / 5.96; a wave over one or two planes is 0.6 of the other's: 1100 rows 9.97 /
+//   10.78), and with seven or eight planes in one wave (816 rows 18.2 / 17.1);
+//   from 4097 to 5120 with one or two planes (300 rows 8.47 / 9.02, four planes 10.8 / 10.2);
+//   not elsewhere (4096, 816 rows, 8 planes 28.9 / 26.3; 8192, 500 rows, 2 / 8 planes 16.6 / 13.5 and 70.8 / 30.8).
 template <typename RT, int IT, int PL>
 static void launch_resnorm_planes_form(const ResNormArgs& a, cudaStream_t s) {
   launch_dep(residual_norm_planes_kernel<RT, IT, PL>, dim3(a.M), dim3(kRowThreads), 0, s, 1, dependent_launch_for(a.M), a);
 }
+template <typename RT, int TPR, int IT>
+static void launch_resnorm_part_form(ResNormArgs a, cudaStream_t s) {
+  constexpr int rows = kRowThreads / TPR;
+  a.iters = IT;
+  launch_dep(residual_norm_quant_kernel<RT, TPR, IT, true, true>, dim3((a.M + rows - 1) / rows), dim3(kRowThreads), 0, s, 1,
+             dependent_launch_for(a.M), a);
+}
 template <typename RT>
 static void launch_resnorm_planes(const ResNormArgs& a, cudaStream_t s) {
-  const int quads = (a.D + 1023) / 1024;
-  switch (quads) {
-    case 1: return a.dsplits <= 4 ? launch_resnorm_planes_form<RT, 1, 4>(a, s) : launch_resnorm_planes_form<RT, 1, 8>(a, s);
-    case 2:
-      return a.dsplits <= 2   ? launch_resnorm_planes_form<RT, 2, 2>(a, s)
-             : a.dsplits <= 4 ? launch_resnorm_planes_form<RT, 2, 4>(a, s)
-                              : launch_resnorm_planes_form<RT, 2, 8>(a, s);
-    case 3: return launch_resnorm_planes_form<RT, 3, 2>(a, s);
-    case 4: return launch_resnorm_planes_form<RT, 4, 4>(a, s);
-    case 5: return launch_resnorm_planes_form<RT, 5, 2>(a, s);
-    default: return launch_resnorm_planes_form<RT, 8, 1>(a, s);
+  const int quads = (a.D + 1023) / 1024, sms = device_sm_count() > 0 ? device_sm_count() : 148;
+  if (quads == 1) return a.dsplits <= 4 ? launch_resnorm_planes_form<RT, 1, 4>(a, s) : launch_resnorm_planes_form<RT, 1, 8>(a, s);
+  if (quads == 2)
+    return a.dsplits <= 2   ? launch_resnorm_planes_form<RT, 2, 2>(a, s)
+           : a.dsplits <= 4 ? launch_resnorm_planes_form<RT, 2, 4>(a, s)
+                            : launch_resnorm_planes_form<RT, 2, 8>(a, s);
+  if (quads == 3) {
+    const int waves = (a.M + 3 * sms - 1) / (3 * sms), waves_of_pairs = (a.M + 4 * sms - 1) / (4 * sms);
+    const bool ahead = a.dsplits > 6 ? waves == 1 : (a.dsplits > 2 ? waves <= waves_of_pairs : waves * 3 <= waves_of_pairs * 5);
+    return ahead ? launch_resnorm_planes_form<RT, 3, 2>(a, s) : launch_resnorm_part_form<RT, 128, 3>(a, s);
   }
+  if (quads == 4) return launch_resnorm_part_form<RT, kRowThreads, 2>(a, s);
+  if (quads == 5 && a.dsplits <= 2) return launch_resnorm_planes_form<RT, 5, 2>(a, s);
+  if (quads <= 6) return launch_resnorm_part_form<RT, kRowThreads, 3>(a, s);
+  return launch_resnorm_part_form<RT, kRowThreads, 4>(a, s);
 }
 #endif
 

@@ -14,14 +14,6 @@
 namespace iflb200 {
 namespace {
 
-int sm_count() {
-  static int count[64] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-  if (count[dev] == 0) cudaDeviceGetAttribute(&count[dev], cudaDevAttrMultiProcessorCount, dev);
-  return count[dev];
-}
-
 // Eight elements as four packed pairs (the arithmetic below is two lanes per instruction throughout;
 // keeping the pairs packed between the steps saves the register moves around them).
 struct Eight {
@@ -594,13 +586,13 @@ __global__ void __launch_bounds__(kWanThreads, 1) wan_qkv_stream_kernel(const Wa
 }  // namespace
 
 bool launch_gelu_quant_stream(const GeluStreamArgs& a, bool half, cudaStream_t s) {
-  const int sms = sm_count();
+  const int sms = device_sm_count();
   if (sms == 0 || !a.row || !a.col || a.K <= 1024 || a.K > 16384) return false;
   return half ? gelu_width<__half>(a, sms, s) : gelu_width<__nv_bfloat16>(a, sms, s);
 }
 
 bool launch_residual_norm_stream(const ResNormStreamArgs& a, cudaStream_t s) {
-  const int sms = sm_count();
+  const int sms = device_sm_count();
   if (sms == 0 || a.D <= 1024 || a.D > 8192 || (a.scale != nullptr) != (a.shift != nullptr)) return false;
   if (!a.delta) return a.scale ? resnorm_form<false, false, true>(a, sms, s) : resnorm_form<false, false, false>(a, sms, s);
   if (!a.drow || !a.dcol || !a.bias || !a.scale) return false;
@@ -608,7 +600,7 @@ bool launch_residual_norm_stream(const ResNormStreamArgs& a, cudaStream_t s) {
 }
 
 bool launch_wan_qkv_stream(const WanStreamArgs& a, bool half, cudaStream_t s) {
-  const int sms = sm_count();
+  const int sms = device_sm_count();
   if (sms == 0 || !a.col || a.D <= 1024 || a.D > 16384 || a.HD % 8) return false;
   const int vectors = a.parts * (a.bias ? 2 : 1) + (a.q_norm ? 1 : 0) + (a.k_norm ? 1 : 0);
   StreamGeom g = stream_geom(a.rows, a.D, vectors, a.D * 2 + a.HD * 4, kWanThreads, sms);
