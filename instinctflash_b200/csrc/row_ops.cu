@@ -1421,9 +1421,14 @@ extern "C" int iflb200_quant_from_amax(const float* h, int64_t ld_h, int M, int 
     launch_dep(kernel, dim3((unsigned)((F + columns - 1) / columns), (unsigned)M), dim3(kRowThreads), 0, s, 1,
                dependent_launch_for(M), h, ld_h, M, F, amax, amax_zero, codes, ld_q, qs, early_trigger_for(s));
   };
-  // few rows: shorter pieces, so that every SM has one
+  // Pieces of 4096 columns where there is work for every SM, of 1024 while six of them a SM hold all, of 2048 between
+  // (a piece of 1024 columns is one load a thread): us for pieces of 1024 / 2048 / 4096 columns -- 50 x 4096 1.30 / 1.30 /
+  // 1.47, 150 x 4096 1.44 / 1.49 / 1.80, 500 x 4096 2.82 / 1.90 / 2.21, 150 x 13824 3.00 / 1.90 / 2.41, 2000 x 1040 4.85 /
+  // 2.85 / 2.86, 816 x 16384 14.2 / 7.62 / 5.12.
+  const int pieces = (F + kRowThreads * 4 - 1) / (kRowThreads * 4), sms = device_sm_count() > 0 ? device_sm_count() : 148;
   if (!fast) launch(quant_from_amax_any_kernel, kRowThreads * 8);
   else if ((int64_t)M * F >= (int64_t)1 << 21) launch(quant_from_amax_kernel<4>, kRowThreads * 16);
+  else if (pieces > 1 && (int64_t)M * pieces > 6 * sms) launch(quant_from_amax_kernel<2>, kRowThreads * 8);
   else launch(quant_from_amax_kernel<1>, kRowThreads * 4);
   return (int)cudaGetLastError();
 }
