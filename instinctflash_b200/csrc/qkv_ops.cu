@@ -428,9 +428,15 @@ cudaError_t launch_qkv_split_vec(const QkvSplitArgs& a, cudaStream_t s) {
   const int heads = a.HQ + 2 * a.HKV;
   const int64_t units = (int64_t)a.T * heads;
   const bool dep = dependent_launch_for(a.T);
-  // the table pays where many heads share a token's angles or there is more than the GPU holds at once (816 x 10 x
-  // 256 5.0 us against 6.0 with it, 332 x 16 x 256 4.1 against 3.4, 1968 x 10 x 128 7.0 against 6.1)
-  if (a.T >= 296 && (heads >= 14 || a.T >= 1500) && qkv_split_aligned(a, 4)) {
+  // The table pays where many heads share a token's angles or there is more than the GPU holds at once; the wider a head,
+  // the less of a unit are its angles.  Time with the table over time without, over 7 to 32 heads and 296 to 8192 tokens:
+  // 64 wide 0.75 to 0.93 from 14 heads on, with fewer 0.65 to 0.84 at 1500 tokens; 128 wide 0.75 to 1.06 from 14 heads on,
+  // fewer 0.90 to 1.02 at 1700; 256 wide 0.83 to 0.98 from 14 heads on at 1200 (1.05 to 1.3 at 816), fewer 0.92 to 1.08 at
+  // 1700.  16 or 32 heads of 256 make whole rounds of a one-token CTA: 0.84 to 1.0 while the CTAs are resident together.
+  const bool many = heads >= 14;
+  const bool table = a.HD == 256 ? a.T >= (many ? 1200 : 1700) || (heads % 16 == 0 && a.T <= 370)
+                                 : many || a.T >= (a.HD == 128 ? 1700 : 1500);
+  if (a.T >= 296 && table && qkv_split_aligned(a, 4)) {
     // tokens per CTA: as many as the angle table holds, fewer where that would leave SMs without two CTAs
     int tb = a.T / 296;
     tb = tb > 512 / a.HD ? 512 / a.HD : tb;
