@@ -212,14 +212,17 @@ extern "C" int iflb200_attn_combine_quant(const float* po, const float* pm, cons
   // 8 splits 3.0 us against 3.4 in a cluster of two; with 16 splits 4.7 against 4.4, with 16 heads 5.7 against 4.0)
   a.cluster = 1;
   const bool one_round = chunks <= kCombineThreads && splits <= 8;
-  while (!one_round && a.cluster < kCombineMaxCluster && (int64_t)tokens * batch * a.cluster * 2 <= 148 && chunks >= 256 * a.cluster) a.cluster *= 2;
+  while (!one_round && chunks > 256 && a.cluster < kCombineMaxCluster && (int64_t)tokens * batch * a.cluster * 2 <= 148 && chunks >= 256 * a.cluster) a.cluster *= 2;
   const int share = (chunks + a.cluster - 1) / a.cluster;
   const dim3 grid(tokens * a.cluster, batch), block(share <= 128 ? 128 : (share <= 256 ? 256 : kCombineThreads));
   const bool dep = dependent_launch_for(tokens);
   cudaError_t e;
   auto go = [&](auto kernel) { return launch_dep(kernel, grid, block, 0, s, a.cluster, dep, a); };
   if (a.cluster > 1) e = share <= kCombineThreads ? go(attn_combine_quant_kernel<1, true, 8>) : go(attn_combine_quant_kernel<kCombineIters, true, 8>);
-  else if (chunks <= kCombineThreads) e = tokens <= 296 ? go(attn_combine_quant_kernel<1, false, 8>) : go(attn_combine_quant_kernel<1, false, 4>);
+  // groups of eight while every token has its SM (CTAs of 512 threads: one an SM with that many registers; 296 tokens x 8 x
+  // 256, 4 / 16 splits 4.73 / 8.12 us in groups of eight, 3.47 / 6.90 in groups of four) or CTAs are small (296 tokens x 8 x
+  // 64, 8 splits 2.69 / 3.16)
+  else if (chunks <= kCombineThreads) e = tokens <= (block.x > 256 ? 148 : 296) ? go(attn_combine_quant_kernel<1, false, 8>) : go(attn_combine_quant_kernel<1, false, 4>);
   else if (chunks <= 2 * kCombineThreads) e = tokens <= 148 ? go(attn_combine_quant_kernel<2, false, 8>) : go(attn_combine_quant_kernel<2, false, 4>);
   else e = go(attn_combine_quant_kernel<kCombineIters, false, 4>);
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
