@@ -1723,6 +1723,12 @@ static int run_gemm(const void* a, int64_t ld_a, const void* w, int64_t ld_w, Ge
   // are the ones whose choice is closest to the fastest form over 680 sizes (16 to 6000 rows, 256 to 14384 columns, K 256
   // to 16384): 0.4 % slower on average, more than 10 % at three.  3072 columns at K = 14336: 1024 rows 44.4 us on 256-wide tiles,
   // 40.3 on pairs; 1536 at K = 8960: 512 rows 18.4 us on 64-wide tiles, 15.5 on 128-wide ones with K split in two.
+  // Scales and bias in the epilogue take longer than raw stores once the last tile's main loop is over, the more so the
+  // wider the tile, and most after an exchange over a cluster, where every column's operands come after the sums: so many
+  // clocks are added below (64-wide tiles 0).  In one wave the lean form's step takes less with fewer rows.  Fitted over 611
+  // sizes (1 to 8192 rows): the fused linear's choice 0.3 % slower than the fastest form, with the raw form's constants
+  // 5.4 %.  175 x 608 x 4016 15.2 us on 128-wide tiles with K split in four, 12.6 on 64-wide ones; 193 x 304 x 304 5.6 on
+  // 128-wide tiles, 4.6; 4 x 3408 x 7760 17.2 split in four, 9.8 lean.
   // The widths that are not powers of two are for wave quantisation (7 row blocks x 32768 columns: 896 tiles of
   // 256 = 6.05 waves of 148 SMs, i.e. 7, but 1029 tiles of 224 = 6.95 waves of narrower tiles).  Timed alone the
   // 224-wide kernel is 2 % faster on that shape, inside the layer stack it was 4 us per launch slower (its
@@ -1736,6 +1742,9 @@ static int run_gemm(const void* a, int64_t ld_a, const void* w, int64_t ld_w, Ge
     const int widths[5] = {256, 224, 192, 128, 64};
     const int64_t step_cycles[2][5] = {{815, 750, 690, 630, 570}, {800, 740, 680, 555, 490}};
     const int64_t tile_cycles[5] = {3560, 3130, 2700, 1850, 2640}, ends[5] = {2690, 2690, 2690, 2405, 1870};
+    const bool arithmetic = p.epilogue == EPI_DEQUANT;
+    const int64_t lean_cycles[2][3] = {{210, 280, 395}, {200, 200, 315}};
+    const int64_t arithmetic_cycles[5] = {5800, 4650, 3500, 1200, 0};
     const int64_t steps = (p.K + BK - 1) / BK;
     const auto waves_cost = [](int64_t tiles, int64_t slots, int64_t wave) {
       const int64_t waves = (tiles + slots - 1) / slots;
@@ -1761,9 +1770,11 @@ static int run_gemm(const void* a, int64_t ld_a, const void* w, int64_t ld_w, Ge
         // up to 64 rows the lean 64-wide form moves half as much per step (24 x 4624 x 5984 9.1 us, where the
         // cluster form of 128-wide tiles takes 19.5)
         const bool lean = widths[i] == 64 && p.M <= 64 && sk == 1 && steps >= 4;
-        const int64_t clocks = lean ? (aligned ? 315 : 395) : step_cycles[aligned][i];
+        const int few = !arithmetic || tiles > dev->sm_count || p.M > 32 ? 2 : (p.M > 16 ? 1 : 0);
+        const int64_t clocks = lean ? lean_cycles[aligned][few] : step_cycles[aligned][i];
         const int64_t wave = (steps + sk - 1) / sk * clocks + (lean ? 3285 : tile_cycles[i]);
-        const int64_t cost = waves_cost(tiles * sk, dev->sm_count, wave) + ends[i] + exchange;
+        const int64_t last = !arithmetic ? 0 : (sk == 1 ? arithmetic_cycles[i] : 12000);
+        const int64_t cost = waves_cost(tiles * sk, dev->sm_count, wave) + ends[i] + exchange + last;
         if (best_bn == 0 || cost < best) {
           best = cost;
           best_bn = widths[i];
@@ -1776,7 +1787,7 @@ static int run_gemm(const void* a, int64_t ld_a, const void* w, int64_t ld_w, Ge
       const int64_t tiles = (int64_t)((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + 255) / 256);
       const int64_t pairs = dev->sm_count / 2;
       const int64_t step = aligned ? (tiles <= pairs ? 750 : 690) : (tiles <= pairs ? 585 : 650);
-      pair = waves_cost(tiles, pairs, steps * step + 4285) + 3595 < best;
+      pair = waves_cost(tiles, pairs, steps * step + 4285) + 3595 + (arithmetic ? 5200 : 0) < best;
     }
   }
   if ((g_cfg_mode >= 2 || pair) && p.N >= 256) {

@@ -24,3 +24,28 @@ def test_a_split_that_does_not_fit_is_refused(mode, M, N, K, split):
         lib.iflb200_gemm_set_split_k(0)
     torch.cuda.synchronize()
     assert st == _lib.ERR_ARG and (out == 7.0).all()
+
+
+# small calls of the fused linear: no K split over a cluster, whose epilogue costs more than the K steps it saves
+@pytest.mark.parametrize("M,N,K", [(4, 3408, 7760), (175, 608, 4016), (309, 1840, 5344), (193, 304, 304), (66, 13184, 1248)])
+def test_fused_linear_keeps_the_unsplit_bits(M, N, K):
+    from instinctflash_b200 import _lib
+    from instinctflash_b200.kernels import fp8
+    lib = _lib.lib()
+    g = torch.Generator(device=DEV).manual_seed(K)
+    a = torch.randn(M, K, device=DEV, generator=g).to(E4M3)
+    w = fp8.Fp8Weight(torch.randn(N, K, device=DEV, generator=g).to(E4M3), torch.rand(N, device=DEV, generator=g),
+                      torch.randn(N, device=DEV, generator=g))
+    s = torch.rand(M, device=DEV, generator=g)
+    outs = []
+    for tile in (0, 64):
+        assert lib.iflb200_gemm_set_config(tile, 0, 0) == 0 and lib.iflb200_gemm_set_split_k(1 if tile else 0) == 0
+        try:
+            y = torch.full((M, N), float("nan"), device=DEV)
+            fp8.fp8_linear(a, s, w, y)
+            torch.cuda.synchronize()
+            outs.append(y)
+        finally:
+            lib.iflb200_gemm_set_config(0, 0, 0)
+            lib.iflb200_gemm_set_split_k(0)
+    assert torch.equal(*outs)
