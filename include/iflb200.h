@@ -68,8 +68,8 @@ IFLB200_API const char* iflb200_status_string(int status);
  * Per-token (per-row) dynamic e4m3 quantiser with the optional consumer prologue.
  *   v[m,k]  = x[m,k] (*row[m]) (*col[k]) (+bias[k])  [-> gelu_tanh]
  *   amax    = max(max_k |v|, 1e-8);  qs[m] = amax / 448;  q[m,k] = e4m3(v * (448 / amax))
- * Both divisions are PTX div.full.f32, the cast is cvt.rn.satfinite, as the reference's
- * Triton kernel compiles to on sm_100.
+ * Both divisions are PTX div.full.f32, the cast is cvt.rn.satfinite, which the
+ * reference's recorded outputs match bit for bit.
  * Replaces: instinctflash/kernels/norm.py:128-158 (_row_quant_kernel, row_quant).
  */
 IFLB200_API int iflb200_row_quant(const void* x, int x_dtype, int64_t ld_x, int M, int K,

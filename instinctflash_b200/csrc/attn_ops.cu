@@ -5,7 +5,7 @@
 // The attention kernel leaves, per split sp, batch b, KV head and query row r = token * GROUP + h,
 // an unnormalised output vector PO (BLOCK_D floats, BLOCK_D = head_dim rounded up to a power of
 // two), the running maximum PM and the running sum PL.  For one token this kernel computes, for
-// every query head and every d < head_dim, in the instruction order the reference compiles to:
+// every query head and every d < head_dim, in the order of the reference's source:
 //     m   = max over sp of PM                       (max.f32, starting from -inf)
 //     w   = ex2.approx.ftz(PM[sp] - m)
 //     l   = fma(w, PL[sp], l)                       (from 0, splits in order)

@@ -1,5 +1,5 @@
-// Inline-PTX wrappers for sm_100a: the approximate float instructions the reference's Triton
-// kernels compile to, mbarrier, TMA (cp.async.bulk.tensor) and tcgen05 (MMA, TMEM).
+// Inline-PTX wrappers for sm_100a: the approximate float instructions whose results the reference's
+// recorded outputs match, mbarrier, TMA (cp.async.bulk.tensor) and tcgen05 (MMA, TMEM).
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>

@@ -7,7 +7,7 @@
 //   wan_qkv    (instinctflash/kernels/wan.py:20-104): RMS norm over the full width of Q or K,
 //              rotary pairs (2j, 2j+1); one CTA owns one (row, part) with the part in registers.
 //
-// Element arithmetic is the order the reference's kernels compile to for sm_100: a multiply
+// Element arithmetic is the order of the reference's source, with the roundings its recorded outputs show: a multiply
 // that feeds an add is one fma.rn, every other multiply rounds on its own; of the two products
 // of a rotation the one with the sine is rounded and the one with the cosine is fused; the
 // mean of squares is div.full(sum, n), the scale rsqrt.approx.ftz; sine and cosine are the

@@ -3,7 +3,7 @@
  * for tests/, the smoke check and the CPU-baseline leg of bench.py; the product never calls it.
  *
  * Each function restates one operator of the InstinctFlash reference, element by element, in
- * the fp32 instruction order its Triton kernel compiles to for sm_100 (a multiply feeding an
+ * the order of its source, with the roundings that its recorded outputs show (a multiply feeding an
  * add is one fmaf; every other multiply/add rounds on its own):
  *   oracle_row_quant            instinctflash/kernels/norm.py:128-147
  *   oracle_dequant_rows         instinctflash/kernels/norm.py:162-175
