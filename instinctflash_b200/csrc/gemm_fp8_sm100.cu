@@ -1823,8 +1823,9 @@ static int run_gemm(const void* a, int64_t ld_a, const void* w, int64_t ld_w, Ge
   // weight rows on its M side in blocks of 128 (256 on a CTA pair), and the epilogue stores the
   // tile transposed.  Same K loop, same accumulator bits.  Two-byte raw or dequantised outputs.
   // Measured on 816 x 32768 x 2048: 54.1 us on CTA pairs, 55.7 on single CTAs, against 53.9 for the
-  // ordinary form (the main loops alone 44.8 / 46.2 / 45.5 us: a 208-wide MMA step is no shorter
-  // than a 256-wide one), so the heuristic does not take it; iflb200_gemm_set_mode(256) does.
+  // ordinary form (the main loops alone 44.8 / 46.2 / 45.5 us).  That was with one producer warp for both
+  // operands, when a K step took 0.41 us whatever the tile; it has not been measured again since each operand has
+  // its own.  The heuristic does not take it; iflb200_gemm_set_mode(256) does.
   if (g_cfg_swap != 1 && g_cfg_mode == 0 && g_cfg_tile_n == 0 && g_cfg_split_k == 0 && g_cfg_stages == 0 &&
       p.M > 256 && p.M <= 1024 && oes == 2 && p.tma_store && (p.epilogue == EPI_RAW || p.epilogue == EPI_DEQUANT)) {
     const int t_tiles = (p.M + 255) / 256;
