@@ -499,10 +499,10 @@ IFLB200_API int iflb200_set_wait_budget_us(int64_t microseconds);
 
 /*
  * Which kernel the last GEMM call of this process launched (host-side record, no device access):
- * family 1 = single-CTA tiles, 2 / 3 = CTA pairs with one / two accumulators, +4 = the swapped
- * form, +8 = the gated form (paired gate / up columns), +16 = split-K partial planes, +32 = row blocks
+ * family 1 = single-CTA tiles, 2 / 3 = CTA pairs with one / two accumulators, +4 = the tokens
+ * form (tokens on the MMA's N side), +8 = the gated form (paired gate / up columns), +16 = split-K partial planes, +32 = row blocks
  * to several destinations; the tile width in columns (tokens for the
- * swapped form); the cluster split-K factor.  Any pointer may be NULL.  For tests that must know
+ * tokens form); the cluster split-K factor.  Any pointer may be NULL.  For tests that must know
  * that a given kernel really ran.  No reference counterpart.
  */
 IFLB200_API int iflb200_gemm_last_launch(int* family, int* tile_n, int* split_k);
@@ -527,9 +527,9 @@ IFLB200_API int iflb200_set_dependent_launch(int enable);
 /* Kernel family: 0 = heuristic, 1 = single-CTA tiles only, 2 / 3 = 256x256 tiles on CTA pairs
  * (cta_group::2) with one / two tensor-memory accumulators; add 16 to store the epilogue
  * straight from registers instead of through shared memory and TMA; add 256 to take the
- * swapped form (tokens on the MMA's N side, 257..1024 tokens, two-byte raw or dequantised output;
- * not chosen by the heuristic) wherever it exists, 128 to forbid it, 512 to keep the swapped form
- * off CTA pairs; add 1024 / 2048 to run the gated form's 256-wide tiles with sixteen / eight
+ * tokens form (tokens on the MMA's N side; raw, dequantised, partial-sum and gated outputs) wherever it
+ * exists, in tiles of tile_n tokens if that is set, 128 to forbid it (512, once its single-CTA variant,
+ * changes nothing); add 1024 / 2048 to run the gated form's 256-wide tiles with sixteen / eight
  * epilogue warps; add 4096 to keep the skinny-regime kernel on one K slab per TMA instruction.
  * Any other bit is refused.  Every mode writes the same output bits.  For
  * experiments and tests.  No reference counterpart. */

@@ -673,72 +673,6 @@ __device__ __forceinline__ void epilogue_gated(const GemmParams& p, const CUtens
   if (any && row_ok) atomicMax(p.amax + m, __float_as_uint(row_max));
 }
 
-// Epilogue of the swapped form (tokens on the MMA's N side): the accumulator holds the tile
-// transposed, lane = output column n, TMEM column = token.  A warp turns 32 tokens x its 32 output
-// columns into a [token][n] block of 32 x 64 bytes in shared memory (one 2-byte store per value:
-// the 32 lanes of a store instruction fill 64 contiguous bytes of one token row, no bank
-// conflict) and writes it with one TMA store; two blocks per warp alternate.  The last chunk of a
-// token tile whose width is not a multiple of 32 starts at width - 32 and rewrites a few tokens of
-// the chunk before it with the same values.  Two-byte outputs, raw or dequantised.
-template <int BT>
-__device__ __forceinline__ void epilogue_swapped(const GemmParams& p, const CUtensorMap* tm_out, uint32_t t_row,
-                                                 uint32_t staging, uint8_t* staging_ptr, int n_row0, int tok0,
-                                                 int half, int lane, int& buf) {
-  constexpr int kChunks = (BT + 31) / 32;
-  constexpr int kFirstHalf = (kChunks + 1) / 2;
-  const int c_begin = half == 0 ? 0 : kFirstHalf, c_end = half == 0 ? kFirstHalf : kChunks;
-  const int n = n_row0 + lane;  // this lane's output column
-  const bool n_ok = n < p.M;    // p.M: rows of the MMA's M side = output columns
-  float cs = 1.0f, bs = 0.0f;
-  if (p.epilogue == EPI_DEQUANT && n_ok) {
-    if (p.col) cs = __ldg(p.col + (int64_t)n * p.col_stride);
-    if (p.bias)
-      bs = (p.bias_dtype == IFLB200_F32) ? __ldg(reinterpret_cast<const float*>(p.bias) + n)
-                                         : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.bias)[n]);
-  }
-  // `buf` lives across tiles: the two blocks alternate over the whole life of the warp, so the
-  // block about to be written is always the one whose store was issued two stores ago
-#pragma unroll 1
-  for (int c = c_begin; c < c_end; ++c) {
-    const int t0 = (c * 32 + 32 <= BT) ? c * 32 : BT - 32;  // chunk start inside the tile
-    const int tok = tok0 + t0;
-    if (tok >= p.N) continue;  // p.N: tokens
-    if (n_row0 >= p.M) continue;
-    uint32_t r[32];
-    tmem_ld_32x32b_x32(t_row + t0, r);
-    tmem_ld_wait();
-    if (lane == 0) bulk_wait_group_read<1>();  // the store issued two chunks ago has read this block
-    __syncwarp();
-    uint8_t* blk = staging_ptr + buf * 2048 + lane * 2;
-#pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      float v = __uint_as_float(r[j]);
-      if (p.epilogue == EPI_DEQUANT) {
-        if (!p.exact) v = __bfloat162float(__float2bfloat16_rn(v));
-        if (p.exact == 2) {
-          v = __fmul_rn(v, __fmul_rn(__ldg(p.row), cs));
-          if (p.bias) v = __fadd_rn(v, bs);
-        } else {
-          Chain ch(v);
-          if (p.row) ch.mul(__ldg(p.row + (int64_t)min(tok + j, p.N - 1) * p.row_stride));
-          if (p.col) ch.mul(cs);
-          if (p.bias) ch.add(bs);
-          v = ch.done();
-        }
-      }
-      const uint16_t h = p.out_dtype == IFLB200_F16 ? (uint16_t)f32_to_f16_bits(v) : (uint16_t)f32_to_bf16_bits(v);
-      *reinterpret_cast<uint16_t*>(blk + j * 64) = h;
-    }
-    fence_proxy_async_smem();
-    __syncwarp();
-    if (lane == 0) {
-      tma_store_2d(tm_out, staging + buf * 2048, n_row0, tok);
-      bulk_commit_group();
-    }
-    buf ^= 1;
-  }
-}
-
 // SPLIT: 0 = never a cluster split-K, 1 = always (p.split_k > 1), 2 = decided by p.split_k.  The
 // wide-tile kernels of the large-M regime exist in forms 0 and 1: measured inside the M = 816 layer
 // stack, a kernel that carries both code paths ran the stack 5 % slower than the two specialised
@@ -753,7 +687,7 @@ __device__ __forceinline__ void epilogue_swapped(const GemmParams& p, const CUte
 // GATED: the gated form (see epilogue_gated): a tile pairs BN/2 gate columns with the BN/2 up
 // columns of the same hidden units; p.N counts hidden units.
 // EW: epilogue warps (8, or 16 for the gated form: EW / 4 per TMEM lane quadrant).
-template <int BN, int STAGES, int SPLIT, bool SWAP = false, bool GATED = false, int EW = kEpilogueWarps, int SL = 1, int AR = BM>
+template <int BN, int STAGES, int SPLIT, bool GATED = false, int EW = kEpilogueWarps, int SL = 1, int AR = BM>
 __global__ void __launch_bounds__(96 + 32 * EW, 1)
 gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w,
                     const __grid_constant__ CUtensorMap tm_out,
@@ -761,7 +695,7 @@ gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
   using L = SmemLayout<BN, STAGES, EW, SL, AR>;
   static_assert(AR == BM || SPLIT == 4, "64-row stages: lean form only");
   static_assert(EW == kEpilogueWarps || GATED, "only the gated epilogue is written for more than eight warps");
-  static_assert(SL == 1 || (!GATED && !SWAP), "several slabs per load: ordinary form only");
+  static_assert(SL == 1 || !GATED, "several slabs per load: ordinary form only");
   // two accumulators, each at a power-of-two column offset; BN in {64, 128, 192, 224, 256}
   constexpr uint32_t kAccStride = BN <= 64 ? 64 : (BN <= 128 ? 128 : 256);
   constexpr uint32_t kTmemCols = 2 * kAccStride;
@@ -858,7 +792,7 @@ gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
   const bool w_producer = warp == 0, a_producer = warp == 2 + EW;
   if (w_producer || a_producer) {
     // ------------------------------------------------------------------ TMA producers
-    const bool weights = SWAP ? a_producer : w_producer;
+    const bool weights = w_producer;
     if (!weights) {
       grid_dependency_wait();
       if (lane == 0) GEMM_TRACE(3);  // the kernel before this one has completed
@@ -915,8 +849,7 @@ gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
             if constexpr (LEAN) {
               if (kp >= p.full_slabs) break;
             }
-            if constexpr (SWAP) tma_prefetch_l2_2d(&tm_a, kp * BK, a_row);
-            else if constexpr (GATED) tma_prefetch_l2_3d(&tm_w, kp * BK, n_blk * (BN / 2), 0);
+            if constexpr (GATED) tma_prefetch_l2_3d(&tm_w, kp * BK, n_blk * (BN / 2), 0);
             else if constexpr (SL > 1) tma_prefetch_l2_3d(&tm_w, 0, n_blk * BN, kp);
             else tma_prefetch_l2_2d(&tm_w, kp * BK, n_blk * BN);
           }
@@ -990,7 +923,6 @@ gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
     uint8_t* staging_ptr = smem + L::kStagingOffset + (warp - 2) * L::kWarpStaging;
     bool ok = true;
     uint32_t it = 0;
-    int swap_buf = 0;
     for (int unit = tile_first; ok && unit < units; unit += tile_stride, ++it) {
       int m_blk, n_blk, grp;
       tile_place(p, tile_of(unit), m_blk, n_blk, grp);
@@ -1005,7 +937,7 @@ gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
       if (it == 0) grid_dependency_wait();
       const int m = m_blk * BM + quad * quad_rows + lane;
       const bool row_ok = m < p.M && (!LEAN || lane < quad_rows);
-      const bool prefetch = !SWAP && !GATED && !split && (LEAN || p.tma_store) && p.epilogue != EPI_RAW && col_end - col_begin <= 128;
+      const bool prefetch = !GATED && !split && (LEAN || p.tma_store) && p.epilogue != EPI_RAW && col_end - col_begin <= 128;
       ColumnVectors cv;
       float rs_early = 1.0f;
       if (prefetch) {
@@ -1022,14 +954,6 @@ gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
       tc_fence_after();
       if (warp == 2 && lane == 0 && it == 0) GEMM_TRACE(6);  // first accumulator complete
       const uint32_t t_row = tmem_base + ((uint32_t)(quad * 32) << 16) + acc * kAccStride;
-      if constexpr (SWAP) {
-        epilogue_swapped<BN>(p, &tm_out, t_row, staging, staging_ptr, m_blk * BM + quad * 32, n_blk * BN, half, lane,
-                             swap_buf);
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(tempty_bar(acc));
-        continue;
-      }
       const float rs = (prefetch || GATED) ? rs_early : ((row_ok && p.row) ? __ldg(p.row + (int64_t)m * p.row_stride) : 1.0f);
       if constexpr (GATED) {
         epilogue_gated<BN, EW / 4>(p, &tm_out, t_row, staging, staging_ptr, m_blk * BM + quad * 32, n_blk * (BN / 2),
@@ -1236,7 +1160,7 @@ struct PairSmemLayout {
 // GATED: the gated form (see epilogue_gated).  The leader loads the gate rows of the tile's BN/2 hidden units,
 // its peer the up rows, so both accumulators hold BN/2 gate columns followed by their up columns; p.N counts
 // hidden units and EW is 16, as in the single-CTA kernel.
-template <int BN, int STAGES, int ACC, bool SWAP = false, bool PLANES = false, bool GATED = false, int EW = kEpilogueWarps>
+template <int BN, int STAGES, int ACC, bool PLANES = false, bool GATED = false, int EW = kEpilogueWarps>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(96 + 32 * EW, 1)
 gemm_fp8_tc5_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w,
                          const __grid_constant__ CUtensorMap tm_out, const GemmParams p) {
@@ -1306,7 +1230,7 @@ gemm_fp8_tc5_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
   if (w_producer || a_producer) {
     // ------------------------------------------------------------------ TMA producers (both CTAs)
     // A warp per operand, the weights' one ahead of the dependency wait, as in the single-CTA kernel.
-    const bool weights = SWAP ? a_producer : w_producer;
+    const bool weights = w_producer;
     if (!weights) grid_dependency_wait();
     Ring<STAGES> ring;
     bool ok = true;
@@ -1384,7 +1308,6 @@ gemm_fp8_tc5_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
     uint8_t* staging_ptr = smem + L::kStagingOffset + (warp - 2) * kWarpStaging;
     bool ok = true;
     uint32_t it = 0;
-    int swap_buf = 0;
     grid_dependency_wait();  // scales and residual operands may come from the kernel before this one
     for (int unit = pair_id; ok && unit < units; unit += pair_stride, ++it) {
       int m_blk, n_blk;
@@ -1395,7 +1318,7 @@ gemm_fp8_tc5_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
       const int m = m_blk * 2 * BM + (int)rank * BM + quad * 32 + lane;
       const bool row_ok = m < p.M;
       // this tile's per-column operands and row scale, fetched under the main loop (see ColumnVectors)
-      const bool prefetch = !SWAP && !GATED && p.tma_store && p.epilogue != EPI_RAW && col_end - col_begin <= 128;
+      const bool prefetch = !GATED && p.tma_store && p.epilogue != EPI_RAW && col_end - col_begin <= 128;
       ColumnVectors cv;
       float rs_early = 1.0f;
       if (prefetch) {
@@ -1411,14 +1334,6 @@ gemm_fp8_tc5_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
       if (!ok) break;
       tc_fence_after();
       const uint32_t t_row = tmem_base + ((uint32_t)(quad * 32) << 16) + acc * kAccStride;
-      if constexpr (SWAP) {
-        epilogue_swapped<BN>(p, &tm_out, t_row, staging, staging_ptr, m_blk * 2 * BM + (int)rank * BM + quad * 32,
-                             n_blk * BN, half, lane, swap_buf);
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive_cluster(tempty_bar(acc), 0);
-        continue;
-      }
       if constexpr (GATED) {
         epilogue_gated<BN, EW / 4>(p, &tm_out, t_row, staging, staging_ptr, m_blk * 2 * BM + (int)rank * BM + quad * 32,
                                    n_blk * (BN / 2), half, m, row_ok, rs_early, lane, cgl, cul);
@@ -1465,6 +1380,12 @@ gemm_fp8_tc5_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
     tmem_dealloc_pair(tmem_base, kTmemCols);
   }
 }
+
+}  // namespace iflb200
+
+#include "gemm_tokens.cuh"
+
+namespace iflb200 {
 
 // --------------------------------------------------------------------------------------------
 // Host side
@@ -1549,21 +1470,6 @@ static int make_out_map(CUtensorMap* tm, void* ptr, int M, int N, int64_t ld, in
   return r == CUDA_SUCCESS ? IFLB200_OK : IFLB200_ERR_DRIVER;
 }
 
-// [tokens, N] output of two-byte elements for the swapped form: box = 32 columns (64 bytes) x 32
-// token rows, no swizzle.
-static int make_out_map_swapped(CUtensorMap* tm, void* ptr, int tokens, int N, int64_t ld) {
-  EncodeTiledFn enc = get_encode_fn();
-  if (!enc) return IFLB200_ERR_DRIVER;
-  const cuuint64_t dims[2] = {(cuuint64_t)N, (cuuint64_t)tokens};
-  const cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
-  const cuuint32_t box[2] = {32u, 32u};
-  const cuuint32_t estr[2] = {1, 1};
-  const CUresult r = enc(tm, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, ptr, dims, strides, box, estr,
-                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? IFLB200_OK : IFLB200_ERR_DRIVER;
-}
-
 // Rows of the activation box.  The MMA always reads 128 rows of the stage, but with at most 120
 // activation rows the box only brings the rows that exist (rounded up to the 8-row swizzle atom):
 // the TMA unit issues one request per 128-byte box row whether the row exists or not, and for a
@@ -1599,18 +1505,17 @@ static int device_info(DeviceInfo** out) {
 
 int g_dependent_launch = 1;
 // what the last call of run_gemm launched: {family, tile width, split_k, stages}; family 1 = single-CTA
-// tiles, 2 / 3 = CTA pairs with one / two accumulators, +4 = swapped form, +8 = gated (paired columns)
+// tiles, 2 / 3 = CTA pairs with one / two accumulators, +4 = tokens form, +8 = gated (paired columns)
 static int g_last_launch[4] = {0, 0, 0, 0};
 static int g_cfg_tile_n = 0, g_cfg_stages = 0, g_cfg_group_m = 0;
 static int g_cfg_split_k = 0;  // 0: cost model, 1: never split K, 2/4/8: forced
 static int g_cfg_direct_store = 0;  // 1: epilogue stores straight from registers (experiments)
-static int g_cfg_pair_swap = 1;  // the swapped form on CTA pairs where the shape allows
-static int g_cfg_swap = 0;  // 0: cost model, 1: never, 2: always where the form exists
+static int g_cfg_tokens = 0;  // tokens form: 0 cost model, 1 never, 2 always where the form exists
 static int g_cfg_slabs = 0;  // 1: one K slab per TMA instruction everywhere (experiments)
 static int g_cfg_gated_warps = 0;  // gated form, 256-wide tiles: 0 heuristic, 8 or 16 epilogue warps
 static int g_cfg_mode = 0;  // 0 auto, 1 single-CTA tiles only, 2 CTA pairs with one accumulator, 3 CTA pairs with two
 
-template <int BN, int STAGES, int SPLIT, bool SWAP = false, bool GATED = false, int EW = kEpilogueWarps, int SL = 1, int AR = BM>
+template <int BN, int STAGES, int SPLIT, bool GATED = false, int EW = kEpilogueWarps, int SL = 1, int AR = BM>
 static int launch_gemm_form(const CUtensorMap& ta, const CUtensorMap& tw, const CUtensorMap& to,
                             const std::conditional_t<SPLIT == 4, LeanParams, GemmParams>& p, int grid, cudaStream_t s) {
   using L = SmemLayout<BN, STAGES, EW, SL, AR>;
@@ -1620,14 +1525,14 @@ static int launch_gemm_form(const CUtensorMap& ta, const CUtensorMap& tw, const 
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return IFLB200_ERR_DEVICE;
   if (!attr_set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_fp8_tc5_kernel<BN, STAGES, SPLIT, SWAP, GATED, EW, SL, AR>,
+    cudaError_t e = cudaFuncSetAttribute(gemm_fp8_tc5_kernel<BN, STAGES, SPLIT, GATED, EW, SL, AR>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, L::kDynamic);
     if (e != cudaSuccess) return (int)e;
     attr_set[dev] = true;
   }
-  const cudaError_t e = launch_dep(gemm_fp8_tc5_kernel<BN, STAGES, SPLIT, SWAP, GATED, EW, SL, AR>, dim3(grid),
+  const cudaError_t e = launch_dep(gemm_fp8_tc5_kernel<BN, STAGES, SPLIT, GATED, EW, SL, AR>, dim3(grid),
                                    dim3(96 + 32 * EW), L::kDynamic, s, p.split_k,
-                                   dependent_launch_for(SWAP ? p.N : p.M), ta, tw, to, p);
+                                   dependent_launch_for(p.M), ta, tw, to, p);
   note_captured_gemm(s);
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
@@ -1665,11 +1570,11 @@ static int launch_lean(const void* a, int64_t ld_a, const void* w, int64_t ld_w,
     memset(&p.w_tail, 0, sizeof(p.w_tail));
   }
   if (st != IFLB200_OK) return st;
-  return g.M <= 64 ? launch_gemm_form<64, 3, 4, false, false, kEpilogueWarps, 4, 64>(ta, tw, to, p, grid, s)
-                   : launch_gemm_form<64, 2, 4, false, false, kEpilogueWarps, 4>(ta, tw, to, p, grid, s);
+  return g.M <= 64 ? launch_gemm_form<64, 3, 4, false, kEpilogueWarps, 4, 64>(ta, tw, to, p, grid, s)
+                   : launch_gemm_form<64, 2, 4, false, kEpilogueWarps, 4>(ta, tw, to, p, grid, s);
 }
 
-template <int BN, int STAGES, int ACC, bool SWAP = false, bool PLANES = false, bool GATED = false, int EW = kEpilogueWarps>
+template <int BN, int STAGES, int ACC, bool PLANES = false, bool GATED = false, int EW = kEpilogueWarps>
 static int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tw, const CUtensorMap& to,
                             const GemmParams& p, int grid, cudaStream_t s) {
   using L = PairSmemLayout<BN, STAGES>;
@@ -1677,15 +1582,118 @@ static int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tw, const 
   int dev = 0;
   cudaGetDevice(&dev);
   if (!attr_set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_fp8_tc5_pair_kernel<BN, STAGES, ACC, SWAP, PLANES, GATED, EW>,
+    cudaError_t e = cudaFuncSetAttribute(gemm_fp8_tc5_pair_kernel<BN, STAGES, ACC, PLANES, GATED, EW>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, L::kDynamic);
     if (e != cudaSuccess) return (int)e;
     attr_set[dev] = true;
   }
-  const cudaError_t e = launch_dep(gemm_fp8_tc5_pair_kernel<BN, STAGES, ACC, SWAP, PLANES, GATED, EW>, dim3(grid), dim3(96 + 32 * EW),
-                                   L::kDynamic, s, 1, dependent_launch_for(SWAP ? p.N : p.M), ta, tw, to, p);
+  const cudaError_t e = launch_dep(gemm_fp8_tc5_pair_kernel<BN, STAGES, ACC, PLANES, GATED, EW>, dim3(grid), dim3(96 + 32 * EW),
+                                   L::kDynamic, s, 1, dependent_launch_for(p.M), ta, tw, to, p);
   note_captured_gemm(s);
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
+}
+
+// The [gate | up] weight [2F, K] seen as [F / 8][2][8][K]: box = 128 bytes x 8 x 2 x 8, so that one load brings 64
+// hidden units as sixteens of eight gate rows and their eight up rows.
+static int make_gated_pairs_map(CUtensorMap* tm, const void* ptr, int F, int K, int64_t ld) {
+  EncodeTiledFn enc = get_encode_fn();
+  if (!enc) return IFLB200_ERR_DRIVER;
+  const cuuint64_t dims[4] = {(cuuint64_t)K, 8, 2, (cuuint64_t)F / 8};
+  const cuuint64_t strides[3] = {(cuuint64_t)ld, (cuuint64_t)ld * (cuuint64_t)F, (cuuint64_t)ld * 8};
+  const cuuint32_t box[4] = {(cuuint32_t)BK, 8, 2, 8};
+  const cuuint32_t estr[4] = {1, 1, 1, 1};
+  const CUresult r = enc(tm, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, const_cast<void*>(ptr), dims, strides, box, estr,
+                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? IFLB200_OK : IFLB200_ERR_DRIVER;
+}
+
+// The tokens form over tiles of `bt` tokens; g is the problem as the other forms take it, g.partials the K ranges of the
+// planes form.
+template <int EPI>
+static int launch_tokens(const void* a, int64_t ld_a, const void* w, int64_t ld_w, const GemmParams& g, int bt,
+                         int sm_count, cudaStream_t s) {
+  using L = TokenLayout<EPI>;
+  static bool attr_set[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) return IFLB200_ERR_DEVICE;
+  if (!attr_set[dev]) {
+    const cudaError_t e =
+        cudaFuncSetAttribute(gemm_fp8_tc5_tokens_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kMaxBytes);
+    if (e != cudaSuccess) return (int)e;
+    attr_set[dev] = true;
+  }
+  const int rows = EPI == TOK_GATED ? BM : 2 * BM;  // output columns of a weight block
+  TokenParams p = {};
+  p.M = g.M; p.N = g.N; p.K = g.K;
+  p.bt = bt;
+  p.num_m = (g.M + bt - 1) / bt;
+  p.num_n = (g.N + rows - 1) / rows;
+  p.num_k = (g.K + BK - 1) / BK;
+  p.num_tiles = p.num_m * p.num_n;
+  // bands as in the pair kernel
+  p.group_m = g_cfg_group_m > 0 ? g_cfg_group_m : (p.num_m <= 24 ? p.num_m : 16);
+  p.parts = EPI == TOK_PLANES ? g.partials : 1;
+  p.slots = L::slots(bt);
+  p.pairs = L::pairs(bt);
+  p.idesc = make_idesc_e4m3_f32(2 * BM, bt);
+  p.exact = g.exact;
+  p.row = g.row; p.row_stride = g.row_stride;
+  p.col = g.col; p.col_stride = g.col_stride;
+  p.bias = g.bias; p.bias_dtype = g.bias_dtype;
+  p.out = reinterpret_cast<uint8_t*>(g.out);
+  p.out_dtype = g.out_dtype;
+  p.ld_out = g.ld_out * (g.out_dtype == IFLB200_F32 ? 4 : 2);
+  p.plane = p.ld_out * g.M;
+  p.act = g.act;
+  p.amax = g.amax;
+  CUtensorMap tt, tw;
+  int st = make_tensor_map(&tt, a, g.M, g.K, ld_a, bt / 2);
+  if (st == IFLB200_OK)
+    st = EPI == TOK_GATED ? make_gated_pairs_map(&tw, w, g.N, g.K, ld_w) : make_tensor_map(&tw, w, g.N, g.K, ld_w, BM);
+  if (st != IFLB200_OK) return st;
+  const int64_t units = (int64_t)p.num_tiles * p.parts, pairs = sm_count / 2;
+  g_last_launch[0] = 3 + 4 + (EPI == TOK_GATED ? 8 : (EPI == TOK_PLANES ? 16 : 0));
+  g_last_launch[1] = bt; g_last_launch[2] = p.parts; g_last_launch[3] = p.slots;
+  const cudaError_t e = launch_dep(gemm_fp8_tc5_tokens_kernel<EPI>, dim3(2 * (unsigned)(units < pairs ? units : pairs)),
+                                   dim3(L::kThreads), L::kFixed + p.slots * L::slab_bytes(bt), s, 1,
+                                   dependent_launch_for(g.M), tt, tw, p);
+  note_captured_gemm(s);
+  return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
+}
+
+// Estimated time of the tokens form, in the units of the costs it is compared with (each set of constants belongs to one
+// comparison): a slab takes at least `floor` clocks (commit and barriers) and `slab` + `slab_token` a token of the tile
+// (rows through the L2 port), times `ragged` where rows are off 64-byte boundaries; a tile's epilogue `tile` +
+// `tile_token` a token; a partly filled last wave counts 1 - `whole` of its share.
+struct TokenCost {
+  double floor, slab, slab_token, tile, tile_token, ends, whole, ragged;
+};
+constexpr int kTokensMinRows = 65;  // up to 64 rows the lean form's 64-row MMAs have less to do
+// M tokens, `cols` weight rows, `ranges` K ranges of `steps` slabs.
+static double tokens_cost(int M, int64_t cols, int steps, int ranges, bool aligned, const TokenCost& c, int sm_count, int bt) {
+  const int64_t pairs = sm_count / 2, units = (int64_t)((M + bt - 1) / bt) * ((cols + 2 * BM - 1) / (2 * BM)) * ranges;
+  const int64_t waves = (units + pairs - 1) / pairs;
+  const double row = c.slab + c.slab_token * bt;
+  const double wave = steps * (row > c.floor ? row : c.floor) * (aligned ? 1.0 : c.ragged) + c.tile + c.tile_token * bt;
+  return (waves == 1 ? wave : c.whole * waves * wave + (1.0 - c.whole) * units * wave / pairs) + c.ends;
+}
+// The width of least cost.  Narrower tiles than 48 tokens wait for barriers, and for more than 1500 tokens nothing
+// below 144 was ever the fastest.
+static int tokens_width(int M, int64_t cols, int steps, int ranges, bool aligned, const TokenCost& c, int sm_count, double& cost) {
+  int best = 0, tiles_before = 0;
+  for (int bt = M > 1500 ? 144 : 48; bt <= 256; bt += 16) {
+    const int tiles = (M + bt - 1) / bt;
+    if (tiles == tiles_before) continue;  // a narrower tile needs no more of them
+    tiles_before = tiles;
+    const double t = tokens_cost(M, cols, steps, ranges, aligned, c, sm_count, bt);
+    if (best == 0 || t < cost) {
+      cost = t;
+      best = bt;
+    }
+  }
+  return best;
 }
 
 static int run_gemm(const void* a, int64_t ld_a, const void* w, int64_t ld_w, GemmParams p, void* stream) {
@@ -1783,11 +1791,31 @@ static int run_gemm(const void* a, int64_t ld_a, const void* w, int64_t ld_w, Ge
       }
     }
     bn = best_bn;
-    if (g_cfg_mode == 0 && g_cfg_tile_n == 0 && g_cfg_split_k == 0 && g_cfg_swap != 2 && p.M > BM && p.N >= 256) {
+    const bool tokens_forced = g_cfg_tokens == 2;
+    if (g_cfg_mode == 0 && g_cfg_tile_n == 0 && g_cfg_split_k == 0 && g_cfg_tokens != 2 && p.M > BM && p.N >= 256) {
       const int64_t tiles = (int64_t)((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + 255) / 256);
       const int64_t pairs = dev->sm_count / 2;
       const int64_t step = aligned ? (tiles <= pairs ? 750 : 690) : (tiles <= pairs ? 585 : 650);
-      pair = waves_cost(tiles, pairs, steps * step + 4285) + 3595 + (arithmetic ? 5200 : 0) < best;
+      const int64_t cost = waves_cost(tiles, pairs, steps * step + 4285) + 3595 + (arithmetic ? 5200 : 0);
+      pair = cost < best;
+      if (pair) best = cost;
+    }
+    // Tokens on the MMA's N side, where the tile's width fits the tokens (see gemm_tokens.cuh).  The constants are the ones
+    // whose choice is closest to the fastest form over 700 sizes (65 to 16384 rows, 256 to 15360 columns, K 512 to
+    // 14336): 1.3 % slower than it on average, 10 % less time than without the form, 25 sizes more than 3 % slower.
+    // Where the choice above is the pair kernel, a tile of 256 tokens is the same tile: only a narrower one that saves
+    // 3 % of it is taken.  With scales in the epilogue only when asked for.
+    if (g_cfg_mode == 0 && g_cfg_stages == 0 && p.tma_store && g_cfg_tokens != 1 &&
+        (tokens_forced || (g_cfg_tile_n == 0 && g_cfg_split_k <= 1 && p.M >= kTokensMinRows && !arithmetic))) {
+      static constexpr TokenCost raw = {407, 68.5, 2.043, 771, 7.39, 3446, 0.8, 1.176};
+      double cost = 0.0;
+      int bt = tokens_width(p.M, p.N, (int)steps, 1, aligned, raw, dev->sm_count, cost);
+      if (g_cfg_tile_n) bt = g_cfg_tile_n;
+      bool take = tokens_forced || cost < (double)best;
+      if (take && pair && !tokens_forced) take = bt < 256 && cost < 0.97 * tokens_cost(p.M, p.N, (int)steps, 1, aligned, raw, dev->sm_count, 256);
+      if (take)
+        return p.epilogue == EPI_RAW ? launch_tokens<TOK_RAW>(a, ld_a, w, ld_w, p, bt, dev->sm_count, s)
+                                     : launch_tokens<TOK_DEQUANT>(a, ld_a, w, ld_w, p, bt, dev->sm_count, s);
     }
   }
   if ((g_cfg_mode >= 2 || pair) && p.N >= 256) {
@@ -1818,61 +1846,6 @@ static int run_gemm(const void* a, int64_t ld_a, const void* w, int64_t ld_w, Ge
   }
   if (bn == 0) return IFLB200_ERR_ARG;  // the forced configuration does not fit this problem
 
-  // Swapped form for a few hundred tokens: the tokens go on the MMA's N side in tiles of the width
-  // that fits them (816 tokens = 4 x 208 with 2 % padding, where 7 row blocks of 128 carry 9 %), the
-  // weight rows on its M side in blocks of 128 (256 on a CTA pair), and the epilogue stores the
-  // tile transposed.  Same K loop, same accumulator bits.  Two-byte raw or dequantised outputs.
-  // Measured on 816 x 32768 x 2048: 54.1 us on CTA pairs, 55.7 on single CTAs, against 53.9 for the
-  // ordinary form (the main loops alone 44.8 / 46.2 / 45.5 us).  That was with one producer warp for both
-  // operands, when a K step took 0.41 us whatever the tile; it has not been measured again since each operand has
-  // its own.  The heuristic does not take it; iflb200_gemm_set_mode(256) does.
-  if (g_cfg_swap != 1 && g_cfg_mode == 0 && g_cfg_tile_n == 0 && g_cfg_split_k == 0 && g_cfg_stages == 0 &&
-      p.M > 256 && p.M <= 1024 && oes == 2 && p.tma_store && (p.epilogue == EPI_RAW || p.epilogue == EPI_DEQUANT)) {
-    const int t_tiles = (p.M + 255) / 256;
-    const int fit = ((p.M + t_tiles - 1) / t_tiles + 15) / 16 * 16;
-    const int bt = fit <= 128 ? 128 : (fit <= 208 ? 208 : 256);  // the widths this form is built for
-    const int64_t steps = (p.K + BK - 1) / BK;
-    if (g_cfg_swap == 2) {
-      GemmParams q = p;
-      q.M = p.N;  // rows of the MMA's M side: output columns
-      q.N = p.M;  // tokens
-      q.num_m = (p.N + BM - 1) / BM;
-      q.num_n = (p.M + bt - 1) / bt;
-      q.num_k = (int)steps;
-      q.num_tiles = q.num_m * q.num_n;
-      q.group_m = g_cfg_group_m > 0 ? g_cfg_group_m : 8;
-      q.split_k = 1;
-      q.a_bytes = BM * BK;
-      const int grid = q.num_tiles < dev->sm_count ? q.num_tiles : dev->sm_count;
-      CUtensorMap tw_rows, ta_tokens, to_swapped;
-      st = make_tensor_map(&tw_rows, w, p.N, p.K, ld_w, BM);
-      if (st != IFLB200_OK) return st;
-      st = make_tensor_map(&ta_tokens, a, p.M, p.K, ld_a, bt);
-      if (st != IFLB200_OK) return st;
-      st = make_out_map_swapped(&to_swapped, p.out, p.M, p.N, p.ld_out);
-      if (st != IFLB200_OK) return st;
-      if (p.N >= 2 * BM && bt >= 208 && g_cfg_pair_swap) {
-        // weight rows in blocks of 256 on a CTA pair, each CTA loading half of the token tile
-        q.num_m = (p.N + 2 * BM - 1) / (2 * BM);
-        q.num_tiles = q.num_m * q.num_n;
-        q.group_m = g_cfg_group_m > 0 ? g_cfg_group_m : 4;
-        const int pairs = dev->sm_count / 2;
-        const int pgrid = 2 * (q.num_tiles < pairs ? q.num_tiles : pairs);
-        CUtensorMap ta_half;
-        st = make_tensor_map(&ta_half, a, p.M, p.K, ld_a, bt / 2);
-        if (st != IFLB200_OK) return st;
-        g_last_launch[0] = 3 + 4; g_last_launch[1] = bt; g_last_launch[2] = 1; g_last_launch[3] = 6;
-        return bt == 208 ? launch_gemm_pair<208, 6, 2, true>(tw_rows, ta_half, to_swapped, q, pgrid, s)
-                         : launch_gemm_pair<256, 6, 2, true>(tw_rows, ta_half, to_swapped, q, pgrid, s);
-      }
-      g_last_launch[0] = 1 + 4; g_last_launch[1] = bt; g_last_launch[2] = 1; g_last_launch[3] = bt == 128 ? 6 : 4;
-      switch (bt) {
-        case 128: return launch_gemm_form<128, 6, 0, true>(tw_rows, ta_tokens, to_swapped, q, grid, s);
-        case 208: return launch_gemm_form<208, 4, 0, true>(tw_rows, ta_tokens, to_swapped, q, grid, s);
-        default: return launch_gemm_form<256, 4, 0, true>(tw_rows, ta_tokens, to_swapped, q, grid, s);
-      }
-    }
-  }
   p.split_k = split;
   p.num_n = (p.N + bn - 1) / bn;
   p.num_k = (p.K + BK - 1) / BK;
@@ -1913,7 +1886,7 @@ static int run_gemm(const void* a, int64_t ld_a, const void* w, int64_t ld_w, Ge
     if (p.K % BK == 0 && make_slab_map(&sa_map, a, p.M, p.K, ld_a, a_rows, 4) == IFLB200_OK &&
         make_slab_map(&sw_map, w, p.N, p.K, ld_w, bn, 4) == IFLB200_OK) {
       g_last_launch[3] = 104;
-      return launch_gemm_form<64, 2, 2, false, false, kEpilogueWarps, 4>(sa_map, sw_map, to, p, grid, s);
+      return launch_gemm_form<64, 2, 2, false, kEpilogueWarps, 4>(sa_map, sw_map, to, p, grid, s);
     }
   }
   switch (bn) {
@@ -1968,15 +1941,30 @@ static int run_gemm_partials(const void* a, int64_t ld_a, const void* w, int64_t
   p.tma_store = 1;
   p.num_m = (M + BM - 1) / BM;
   // more than 128 rows: the width with the least waves x steps x clocks (as in run_gemm; an fp32 tile's epilogue
-  // and the prologue are 4000 a wave)
+  // and the prologue are 4000 a wave); more than 64: tokens on the MMA's N side where that takes less
+  // (constants over 1200 of 3462 sizes and numbers of ranges: 0.4 % slower than the fastest form on average, 28 % less time
+  // than without the form, nine more than 3 % slower; 816 x 2048 x 16384 in two ranges 29.4 -> 23.1 us)
   int bn = 64;
+  const int steps = ((num_k + 3) / 4 + splits - 1) / splits * 4;
+  auto cost = [&](int width, int clocks) {
+    const int64_t units = (int64_t)p.num_m * ((N + width - 1) / width) * splits;
+    return (units + dev->sm_count - 1) / dev->sm_count * ((int64_t)steps * clocks + 4000);
+  };
+  int64_t least = cost(64, 385);
   if (M > BM && N >= 256) {
-    auto cost = [&](int width, int clocks) {
-      const int64_t units = (int64_t)p.num_m * ((N + width - 1) / width) * splits;
-      const int steps = ((num_k + 3) / 4 + splits - 1) / splits * 4;
-      return (units + dev->sm_count - 1) / dev->sm_count * ((int64_t)steps * clocks + 4000);
-    };
-    if (cost(256, 720) <= cost(64, 385)) bn = 256;
+    const int64_t wide = cost(256, 720);
+    if (wide <= least) {
+      bn = 256;
+      least = wide;
+    }
+  }
+  if (g_cfg_mode == 0 && g_cfg_tokens != 1 && (M >= kTokensMinRows || g_cfg_tokens == 2)) {
+    static constexpr TokenCost planes = {314, 37.8, 1.986, 1706, 8, 2056, 0.848, 0.947};
+    double time = 0.0;
+    int bt = tokens_width(M, N, steps, splits, (ld_a | ld_w) % 64 == 0, planes, dev->sm_count, time);
+    if (g_cfg_tokens == 2 && g_cfg_tile_n) bt = g_cfg_tile_n;
+    if (time < 1.331 * least + 1370 || g_cfg_tokens == 2)
+      return launch_tokens<TOK_PLANES>(a, ld_a, w, ld_w, p, bt, dev->sm_count, reinterpret_cast<cudaStream_t>(stream));
   }
   p.num_n = (N + bn - 1) / bn;
   p.num_k = num_k;
@@ -2006,7 +1994,7 @@ static int run_gemm_partials(const void* a, int64_t ld_a, const void* w, int64_t
     p.num_m = pair_m;
     p.num_tiles = p.num_m * p.num_n;
     g_last_launch[0] = 3 + 16; g_last_launch[1] = bn; g_last_launch[2] = splits; g_last_launch[3] = 6;
-    return launch_gemm_pair<256, 6, 2, false, true>(ta, tw, to, p, 2 * (int)(pair_units < sm_pairs ? pair_units : sm_pairs), s);
+    return launch_gemm_pair<256, 6, 2, true>(ta, tw, to, p, 2 * (int)(pair_units < sm_pairs ? pair_units : sm_pairs), s);
   }
   st = make_tensor_map(&ta, a, M, K, ld_a, a_rows);
   if (st != IFLB200_OK) return st;
@@ -2111,20 +2099,33 @@ static int run_gemm_gated(const void* a, int64_t ld_a, const void* w, int64_t ld
   };
   int bn = g_cfg_tile_n == 256 || g_cfg_tile_n == 128 || g_cfg_tile_n == 64 ? g_cfg_tile_n : 0;
   bool pair = g_cfg_mode == 3 && F >= 128;
+  int64_t least = 0;
   if (bn == 0) {
-    int64_t best = 0;
     for (int i = 0; i < 3; ++i) {
       const int64_t c = cost((int64_t)p.num_m * ((F + widths[i] / 2 - 1) / (widths[i] / 2)), dev->sm_count, step_cycles[aligned][i], 2000);
-      if (bn == 0 || c < best) {
-        best = c;
+      if (bn == 0 || c < least) {
+        least = c;
         bn = widths[i];
       }
     }
     if (g_cfg_mode == 0 && M > BM && F >= 128) {
       const int64_t tiles = (int64_t)((M + 2 * BM - 1) / (2 * BM)) * ((F + 127) / 128), pairs = dev->sm_count / 2;
       const bool one_wave = tiles <= pairs;
-      pair = cost(tiles, pairs, aligned ? (one_wave ? 660 : 600) : (one_wave ? 870 : 830), 2500) + 1000 < best;
+      const int64_t c = cost(tiles, pairs, aligned ? (one_wave ? 660 : 600) : (one_wave ? 870 : 830), 2500) + 1000;
+      pair = c < least;
+      if (pair) least = c;
     }
+  }
+  if (g_cfg_mode == 0 && g_cfg_tokens != 1 && g_cfg_gated_warps == 0 &&
+      (g_cfg_tokens == 2 || (g_cfg_tile_n == 0 && M >= kTokensMinRows && F >= 2048))) {
+    // tokens on the MMA's N side (constants over 700 sizes: 0.6 % slower than the fastest form on average, 1.7 % less time
+    // than without it, eleven more than 3 % slower; hidden widths below 2048 were not among them)
+    static constexpr TokenCost gated = {265, 46, 2.225, 1375, 7.51, 1554, 0.911, 1.152};
+    double time = 0.0;
+    int bt = tokens_width(M, 2 * (int64_t)F, p.num_k, 1, aligned, gated, dev->sm_count, time);
+    if (g_cfg_tile_n) bt = g_cfg_tile_n;
+    if (time < (double)least || g_cfg_tokens == 2)
+      return launch_tokens<TOK_GATED>(a, ld_a, w, ld_w, p, bt, dev->sm_count, reinterpret_cast<cudaStream_t>(stream));
   }
   if (pair) {
     // as in the ordinary form: 256 tokens x 128 hidden units, each CTA 128 rows of A and of the gate or up weights
@@ -2141,7 +2142,7 @@ static int run_gemm_gated(const void* a, int64_t ld_a, const void* w, int64_t ld
     st = make_out_map(&to, h, M, F, ld_h, 4, 64);
     if (st != IFLB200_OK) return st;
     g_last_launch[0] = 3 + 8; g_last_launch[1] = 256; g_last_launch[2] = 1; g_last_launch[3] = 6;
-    return launch_gemm_pair<256, 6, 2, false, false, true, 16>(ta, tw, to, p, 2 * (p.num_tiles < pairs ? p.num_tiles : pairs),
+    return launch_gemm_pair<256, 6, 2, false, true, 16>(ta, tw, to, p, 2 * (p.num_tiles < pairs ? p.num_tiles : pairs),
                                                               reinterpret_cast<cudaStream_t>(stream));
   }
   p.num_n = (F + bn / 2 - 1) / (bn / 2);
@@ -2165,10 +2166,10 @@ static int run_gemm_gated(const void* a, int64_t ld_a, const void* w, int64_t ld
   switch (bn) {
     case 256:
       // sixteen epilogue warps (64 bytes of staging per row each), or eight
-      if (sixteen) return launch_gemm_form<256, 4, 0, false, true, 16>(ta, tw, to, p, grid, s);
-      return launch_gemm_form<256, 4, 0, false, true>(ta, tw, to, p, grid, s);
-    case 128: return launch_gemm_form<128, 6, 0, false, true>(ta, tw, to, p, grid, s);
-    default: return launch_gemm_form<64, 8, 0, false, true>(ta, tw, to, p, grid, s);
+      if (sixteen) return launch_gemm_form<256, 4, 0, true, 16>(ta, tw, to, p, grid, s);
+      return launch_gemm_form<256, 4, 0, true>(ta, tw, to, p, grid, s);
+    case 128: return launch_gemm_form<128, 6, 0, true>(ta, tw, to, p, grid, s);
+    default: return launch_gemm_form<64, 8, 0, true>(ta, tw, to, p, grid, s);
   }
 }
 
@@ -2206,8 +2207,7 @@ extern "C" int iflb200_gemm_set_mode(int mode) {
     return IFLB200_ERR_ARG;
   g_cfg_gated_warps = (mode & 1024) ? 16 : ((mode & 2048) ? 8 : 0);
   g_cfg_slabs = (mode & 4096) ? 1 : 0;
-  g_cfg_swap = (mode & 128) ? 1 : ((mode & 256) ? 2 : 0);  // 128: never the swapped form, 256: wherever it exists
-  g_cfg_pair_swap = (mode & 512) ? 0 : 1;                  // 512: the swapped form on single CTAs only
+  g_cfg_tokens = (mode & 128) ? 1 : ((mode & 256) ? 2 : 0);  // 128: never the tokens form, 256: wherever it exists (512, once its single-CTA variant, changes nothing)
   g_cfg_mode = family;
   g_cfg_direct_store = (mode & 16) ? 1 : 0;
   return IFLB200_OK;

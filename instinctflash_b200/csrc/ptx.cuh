@@ -282,6 +282,10 @@ __device__ __forceinline__ void cluster_arrive() {
 __device__ __forceinline__ void cluster_wait() {
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// Arrival that orders no memory accesses.
+__device__ __forceinline__ void cluster_arrive_relaxed() {
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+}
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -304,6 +308,15 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t smem_dst, const void* 
       "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes "
       "[%0], [%1, {%3, %4}], [%2];"
       ::"r"(smem_dst), "l"(tensor_map), "r"(leader_bar), "r"(x), "r"(y)
+      : "memory");
+}
+// The same for a 4-D tiled tensor.
+__device__ __forceinline__ void tma_load_4d_pair(uint32_t smem_dst, const void* tensor_map, uint32_t leader_bar, int32_t x,
+                                                 int32_t y, int32_t z, int32_t w) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes "
+      "[%0], [%1, {%3, %4, %5, %6}], [%2];"
+      ::"r"(smem_dst), "l"(tensor_map), "r"(leader_bar), "r"(x), "r"(y), "r"(z), "r"(w)
       : "memory");
 }
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t smem_dst, uint32_t cols) {
