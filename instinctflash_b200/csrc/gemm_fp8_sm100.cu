@@ -1801,19 +1801,25 @@ static int run_gemm(const void* a, int64_t ld_a, const void* w, int64_t ld_w, Ge
       if (pair) best = cost;
     }
     // Tokens on the MMA's N side, where the tile's width fits the tokens (see gemm_tokens.cuh).  The constants are the ones
-    // whose choice is closest to the fastest form over 700 sizes (65 to 16384 rows, 256 to 15360 columns, K 512 to
-    // 14336): 1.3 % slower than it on average, 10 % less time than without the form, 25 sizes more than 3 % slower.
+    // whose choice is closest to the fastest form over 700 raw sizes one after the other and 900 dequantised ones
+    // behind their quantiser (65 to 16384 rows, 256 to 15360 columns, K 512 to 14336): 1.3 and 0.6 % slower than it on
+    // average, the calls 10 and 14 % faster than without the form, 25 and 15 of them more than 3 % slower.
     // Where the choice above is the pair kernel, a tile of 256 tokens is the same tile: only a narrower one that saves
-    // 3 % of it is taken.  With scales in the epilogue only when asked for.
+    // 3 % of it is taken, or with scales, whose epilogue takes longer in the pair kernel, over fewer than 32 K steps any.
+    // Very deep reductions with few tiles stay split over a cluster, scales or not (228 x 1056 x 14320 with scales
+    // 23.1 us, 25.6 in this form), so that the fused linear's bits stay those of the raw output's.
     if (g_cfg_mode == 0 && g_cfg_stages == 0 && p.tma_store && g_cfg_tokens != 1 &&
-        (tokens_forced || (g_cfg_tile_n == 0 && g_cfg_split_k <= 1 && p.M >= kTokensMinRows && !arithmetic))) {
+        (tokens_forced || (g_cfg_tile_n == 0 && g_cfg_split_k <= 1 && p.M >= kTokensMinRows))) {
       static constexpr TokenCost raw = {407, 68.5, 2.043, 771, 7.39, 3446, 0.8, 1.176};
+      static constexpr TokenCost dequant = {356, 92.2, 2.004, 1226, 4.70, 3070, 0.744, 1.21};
+      const TokenCost& c = arithmetic ? dequant : raw;
       double cost = 0.0;
-      int bt = tokens_width(p.M, p.N, (int)steps, 1, aligned, raw, dev->sm_count, cost);
+      int bt = tokens_width(p.M, p.N, (int)steps, 1, aligned, c, dev->sm_count, cost);
       if (g_cfg_tile_n) bt = g_cfg_tile_n;
-      bool take = tokens_forced || cost < (double)best;
-      if (take && pair && !tokens_forced) take = bt < 256 && cost < 0.97 * tokens_cost(p.M, p.N, (int)steps, 1, aligned, raw, dev->sm_count, 256);
-      if (take)
+      bool take = cost < (double)best && (split == 1 || steps < 112);
+      if (take && pair && (!arithmetic || steps >= 32))
+        take = bt < 256 && cost < 0.97 * tokens_cost(p.M, p.N, (int)steps, 1, aligned, c, dev->sm_count, 256);
+      if (take || tokens_forced)
         return p.epilogue == EPI_RAW ? launch_tokens<TOK_RAW>(a, ld_a, w, ld_w, p, bt, dev->sm_count, s)
                                      : launch_tokens<TOK_DEQUANT>(a, ld_a, w, ld_w, p, bt, dev->sm_count, s);
     }

@@ -85,6 +85,26 @@ __device__ __forceinline__ uint4 ld_shared_v4(uint32_t addr) {
   return v;
 }
 
+// wait_bounded for a thread on its own.
+__device__ __forceinline__ bool wait_bounded_one(uint32_t bar, uint32_t parity, volatile uint32_t* abort, uint32_t code) {
+  if (mbar_try_wait(bar, parity)) return true;
+  uint64_t t0 = 0;
+  uint32_t spins = 0;
+  while (true) {
+    if (mbar_try_wait(bar, parity)) return true;
+    if (*abort) return false;
+    if (++spins > 2048) {
+      if (t0 == 0) t0 = globaltimer_ns();
+      __nanosleep(128);
+      if (globaltimer_ns() - t0 > g_gemm_wait_budget_ns) {
+        *abort = 1;
+        atomicCAS(&g_timeout_record[0], 0u, code);
+        return false;
+      }
+    }
+  }
+}
+
 template <int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TokenLayout<EPI>::kThreads, 1)
 gemm_fp8_tc5_tokens_kernel(const __grid_constant__ CUtensorMap tm_t, const __grid_constant__ CUtensorMap tm_w,
@@ -134,6 +154,8 @@ gemm_fp8_tc5_tokens_kernel(const __grid_constant__ CUtensorMap tm_t, const __gri
   };
 
   if (threadIdx.x == 0) {
+    prefetch_tensormap(&tm_w);
+    prefetch_tensormap(&tm_t);
     for (int i = 0; i < slots; ++i) mbar_init(full_bar(i), 2);  // the leader's producers of the slab arm it; bytes of both CTAs complete it
     for (int i = 0; i < slots >> pairs; ++i) mbar_init(bar0 + 8u * (slots + i), 1);  // one multicast commit from the leader
     for (int a = 0; a < 2; ++a) {
@@ -144,18 +166,17 @@ gemm_fp8_tc5_tokens_kernel(const __grid_constant__ CUtensorMap tm_t, const __gri
     fence_barrier_init();
     fence_proxy_async_smem();
   }
+  __syncwarp();
+  cluster_arrive_relaxed();  // (the initialisation has its own fence)
   if (warp == 1) {
     tmem_alloc_pair(smem_u32(tmem_slot), kTmemCols);
     tmem_relinquish_pair();
   }
-  if (warp == 0 && lane == 0) {
-    prefetch_tensormap(&tm_w);
-    prefetch_tensormap(&tm_t);
-  }
   tc_fence_before();
-  cluster_sync_all();  // barriers of both CTAs initialised before any remote signal
+  __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  cluster_wait();  // barriers of both CTAs initialised before any remote signal
 
   // producers: warp 0 and the warps behind the epilogue's, W and T in turn
   const int producer = warp == 0 ? 0 : (warp < 2 + EW ? -1 : warp - 1 - EW);
@@ -204,7 +225,8 @@ gemm_fp8_tc5_tokens_kernel(const __grid_constant__ CUtensorMap tm_t, const __gri
     if (t_producer) grid_launch_dependents();  // last loads issued: the next kernel may be scheduled
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (leader only)
-    if (leader) {
+    // One thread runs the whole loop: votes and elections per slab took the warp about 100 clocks more.
+    if (leader && elect_one()) {
       int slot = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -215,7 +237,7 @@ gemm_fp8_tc5_tokens_kernel(const __grid_constant__ CUtensorMap tm_t, const __gri
         steps_of(unit, kb0, kb1);
         const int slabs = kb1 - kb0;
         const uint32_t acc = it & 1u, acc_phase = (it >> 1) & 1u;
-        ok = wait_bounded(tempty_bar(acc), acc_phase ^ 1, abort_flag, (2u << 24) | (2u << 16) | (it & 0xFFFF));
+        ok = wait_bounded_one(tempty_bar(acc), acc_phase ^ 1, abort_flag, (2u << 24) | (2u << 16) | (it & 0xFFFF));
         if (!ok) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * kAccStride;
@@ -223,21 +245,18 @@ gemm_fp8_tc5_tokens_kernel(const __grid_constant__ CUtensorMap tm_t, const __gri
           for (int i = 0; i < slabs; i += 2) {
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-              ok = ok && wait_bounded(full_bar(slot + h), phase, abort_flag, (2u << 24) | (3u << 16) | (it & 0xFFFF));
+              ok = ok && wait_bounded_one(full_bar(slot + h), phase, abort_flag, (2u << 24) | (3u << 16) | (it & 0xFFFF));
               if (!ok) break;
               tc_fence_after();
-              if (elect_one()) {
-                const uint64_t at = (uint64_t)(((slot + h) * slab_bytes) >> 4);
-                if (i + h < slabs) {
+              const uint64_t at = (uint64_t)(((slot + h) * slab_bytes) >> 4);
+              if (i + h < slabs) {
 #pragma unroll
-                  for (int j = 0; j < BK / 32; ++j)
-                    mma_f8f6f4_pair(d_tmem, dw0 + at + 2 * j, dt0 + at + 2 * j, p.idesc, i > 0 || h > 0 || j > 0 ? 1u : 0u);
-                }
-                if (h == 1) mma_commit_pair(empty_bar(slot), 3);  // both free in both CTAs
+                for (int j = 0; j < BK / 32; ++j)
+                  mma_f8f6f4_pair(d_tmem, dw0 + at + 2 * j, dt0 + at + 2 * j, p.idesc, i > 0 || h > 0 || j > 0 ? 1u : 0u);
               }
-              __syncwarp();
             }
             if (!ok) break;
+            mma_commit_pair(empty_bar(slot), 3);  // both free in both CTAs
             slot += 2;
             if (slot == slots) {
               slot = 0;
@@ -246,17 +265,14 @@ gemm_fp8_tc5_tokens_kernel(const __grid_constant__ CUtensorMap tm_t, const __gri
           }
         } else {
           for (int i = 0; i < slabs; ++i) {
-            ok = wait_bounded(full_bar(slot), phase, abort_flag, (2u << 24) | (3u << 16) | (it & 0xFFFF));
+            ok = wait_bounded_one(full_bar(slot), phase, abort_flag, (2u << 24) | (3u << 16) | (it & 0xFFFF));
             if (!ok) break;
             tc_fence_after();
-            if (elect_one()) {
-              const uint64_t at = (uint64_t)((slot * slab_bytes) >> 4);
+            const uint64_t at = (uint64_t)((slot * slab_bytes) >> 4);
 #pragma unroll
-              for (int j = 0; j < BK / 32; ++j)
-                mma_f8f6f4_pair(d_tmem, dw0 + at + 2 * j, dt0 + at + 2 * j, p.idesc, i > 0 || j > 0 ? 1u : 0u);
-              mma_commit_pair(empty_bar(slot), 3);  // free in both CTAs
-            }
-            __syncwarp();
+            for (int j = 0; j < BK / 32; ++j)
+              mma_f8f6f4_pair(d_tmem, dw0 + at + 2 * j, dt0 + at + 2 * j, p.idesc, i > 0 || j > 0 ? 1u : 0u);
+            mma_commit_pair(empty_bar(slot), 3);  // free in both CTAs
             if (++slot == slots) {
               slot = 0;
               phase ^= 1;
@@ -264,10 +280,10 @@ gemm_fp8_tc5_tokens_kernel(const __grid_constant__ CUtensorMap tm_t, const __gri
           }
         }
         if (!ok) break;
-        if (elect_one()) mma_commit_pair(tfull_bar(acc), 3);  // accumulator complete in both CTAs
-        __syncwarp();
+        mma_commit_pair(tfull_bar(acc), 3);  // accumulator complete in both CTAs
       }
     }
+    __syncwarp();
   } else {
     // ------------------------------------------------------------------ epilogue warps (both CTAs)
     // A warp owns 32 weight rows (its lanes of tensor memory) and every PARTS-th block of 16 tokens.
