@@ -78,14 +78,6 @@ struct GemmParams {
   const CUtensorMap* out_maps;
 };
 
-// The lean form's arguments: K need not be a multiple of 128.  Stages of whole slabs come through the slab maps
-// (K / 128 slabs); the stage that holds the ragged slab comes slab by slab through these, which read
-// zeros past the end of a row.
-struct LeanParams : GemmParams {
-  CUtensorMap a_tail, w_tail;
-  int full_slabs;  // K / 128
-};
-
 // role << 24 | barrier kind << 16 | low 16 bits of the tile counter; 0 = no timeout.
 __device__ uint32_t g_timeout_record[4];
 // Time budget of every wait inside the GEMM kernels (read only on the slow path of a wait).
@@ -132,15 +124,14 @@ __device__ __forceinline__ float ld_dsmem_f32(uint32_t addr) {
 // SL: 128-byte K slabs per stage.  With SL > 1 one TMA instruction per operand brings SL slabs (the
 // operands are mapped as [K / 128][rows][128 bytes]): a skinny GEMM's main loop is bound by the
 // rate at which one SM can issue TMA instructions (about 0.2 us each, measured), not by bytes.
-// AR: activation rows of a stage (64: the lean form for at most 64 rows).
-template <int BN, int STAGES, int EW = kEpilogueWarps, int SL = 1, int AR = BM>
+template <int BN, int STAGES, int EW = kEpilogueWarps, int SL = 1>
 struct SmemLayout {
-  static constexpr int kABytes = AR * BK * SL;
+  static constexpr int kABytes = BM * BK * SL;
   static constexpr int kBBytes = BN * BK * SL;
   static constexpr int kStageBytes = kABytes + kBBytes;
   // epilogue staging: one 32-row buffer per epilogue warp (TMA-store source), 128 bytes per row
   // with eight epilogue warps, 64 with sixteen; a warp of the 64-row form has 16 rows
-  static constexpr int kWarpStaging = EW > 8 || AR == 64 ? 2048 : 4096;
+  static constexpr int kWarpStaging = EW > 8 ? 2048 : 4096;
   static constexpr int kStagingOffset = STAGES * kStageBytes;
   static constexpr int kBarOffset = kStagingOffset + EW * kWarpStaging;
   // full[STAGES], empty[STAGES], tmem_full[2], tmem_empty[2], then the TMEM base word and the
@@ -430,10 +421,9 @@ __device__ __forceinline__ void epilogue_values(const GemmParams& p, const uint3
 // Consumer arithmetic and output cast of 32 consecutive columns of this lane's row, written into
 // the lane's 128-byte staging row (128-byte swizzle: 16-byte chunk index ^ (lane & 7)).  `sub` is
 // the column offset inside the staged piece: 0 or 32 for two-byte outputs, 0 for four-byte ones.
-// `live`: the lane holds a row (a warp of the 64-row form has sixteen, and staging for no more).
 __device__ __forceinline__ void stage_columns(const GemmParams& p, const uint32_t (&r)[32], int n_abs, float rs,
                                               uint8_t* mine, int sub, int lane, bool pre = false, float csl = 0.0f,
-                                              float bsl = 0.0f, bool live = true) {
+                                              float bsl = 0.0f) {
   const int es = (p.out_dtype == IFLB200_F32) ? 4 : 2;
   if (es == 2) {
     // 32 values = 64 bytes = four 16-byte chunks; chunk index within the 128-byte row
@@ -448,7 +438,7 @@ __device__ __forceinline__ void stage_columns(const GemmParams& p, const uint32_
         u.y = pack_bf16x2(__uint_as_float(r[8 * j + 2]), __uint_as_float(r[8 * j + 3]));
         u.z = pack_bf16x2(__uint_as_float(r[8 * j + 4]), __uint_as_float(r[8 * j + 5]));
         u.w = pack_bf16x2(__uint_as_float(r[8 * j + 6]), __uint_as_float(r[8 * j + 7]));
-        if (live) *reinterpret_cast<uint4*>(mine + (((first + j) ^ sw) * 16)) = u;
+        *reinterpret_cast<uint4*>(mine + (((first + j) ^ sw) * 16)) = u;
       }
     } else {
       float y[32];
@@ -467,7 +457,7 @@ __device__ __forceinline__ void stage_columns(const GemmParams& p, const uint32_
           u.z = pack_f16x2(y[8 * j + 4], y[8 * j + 5]);
           u.w = pack_f16x2(y[8 * j + 6], y[8 * j + 7]);
         }
-        if (live) *reinterpret_cast<uint4*>(mine + (((first + j) ^ sw) * 16)) = u;
+        *reinterpret_cast<uint4*>(mine + (((first + j) ^ sw) * 16)) = u;
       }
     }
   } else {
@@ -475,8 +465,7 @@ __device__ __forceinline__ void stage_columns(const GemmParams& p, const uint32_
     epilogue_values(p, r, n_abs, rs, y, pre, csl, bsl);
 #pragma unroll
     for (int j = 0; j < 8; ++j)
-      if (live)
-        *reinterpret_cast<float4*>(mine + ((j ^ (lane & 7)) * 16)) =
+      *reinterpret_cast<float4*>(mine + ((j ^ (lane & 7)) * 16)) =
             make_float4(y[4 * j + 0], y[4 * j + 1], y[4 * j + 2], y[4 * j + 3]);
   }
 }
@@ -485,7 +474,7 @@ __device__ __forceinline__ void stage_columns(const GemmParams& p, const uint32_
 // memory.  128 bytes of each output row (64 two-byte or 32 four-byte columns) are staged with
 // the 128-byte swizzle and written by one TMA store, so global memory sees whole 128-byte lines
 // instead of 16-byte pieces of 32 different rows.
-template <int BN, int ROWS = 32>
+template <int BN>
 __device__ __forceinline__ void epilogue_tma_store(const GemmParams& p, const CUtensorMap* tm_out, uint32_t t_row,
                                                    uint32_t staging, uint8_t* staging_ptr, int row0, int n_base,
                                                    int col_begin, int col_end, float rs, int lane, int z = -1,
@@ -510,9 +499,9 @@ __device__ __forceinline__ void epilogue_tma_store(const GemmParams& p, const CU
         const int k = (c + sub - col_begin) >> 5;  // which of the warp's 32-column chunks (uniform)
         const float csl = k == 0 ? cv->cs[0] : (k == 1 ? cv->cs[1] : (k == 2 ? cv->cs[2] : cv->cs[3]));
         const float bsl = k == 0 ? cv->bs[0] : (k == 1 ? cv->bs[1] : (k == 2 ? cv->bs[2] : cv->bs[3]));
-        stage_columns(p, r, n0 + sub, rs, mine, sub, lane, true, csl, bsl, lane < ROWS);
+        stage_columns(p, r, n0 + sub, rs, mine, sub, lane, true, csl, bsl);
       } else {
-        stage_columns(p, r, n0 + sub, rs, mine, sub, lane, false, 0.0f, 0.0f, lane < ROWS);
+        stage_columns(p, r, n0 + sub, rs, mine, sub, lane, false, 0.0f, 0.0f);
       }
       GEMM_TRACE_IN_HELPER(11, threadIdx.x == 64 && c == col_begin && sub == 0);  // first chunk staged
     }
@@ -676,30 +665,25 @@ __device__ __forceinline__ void epilogue_gated(const GemmParams& p, const CUtens
 // SPLIT: 0 = never a cluster split-K, 1 = always (p.split_k > 1), 2 = decided by p.split_k.  The
 // wide-tile kernels of the large-M regime exist in forms 0 and 1: measured inside the M = 816 layer
 // stack, a kernel that carries both code paths ran the stack 5 % slower than the two specialised
-// ones.  The 64-wide kernel exists in form 2, for what the lean form (4) below leaves out: residual and direct-store
+// ones.  The 64-wide kernel exists in form 2, for what the lean kernel (gemm_lean.cuh) leaves out: residual and direct-store
 // epilogues, fewer than four K steps, a K split over a cluster that was asked for.
 // SPLIT 3: the planes form for more than 128 rows: (tile, K range) units on a persistent grid, each leaving
 // its fp32 partial sums in a plane; K is cut as in the skinny form, so the planes' bits are the same.
-// SPLIT 4: the lean form of the skinny regime: planes or one range, TMA stores, no cluster and no direct stores.
-// Every launch of a 4 us kernel fetches its instructions cold, so the code that a skinny layer stack never
-// reaches is left out; and up to 64 rows its MMAs read 64 activation rows instead of 128 (38 clocks each
-// for 48: a third of the main loop of a K = 1024 tile).
 // GATED: the gated form (see epilogue_gated): a tile pairs BN/2 gate columns with the BN/2 up
 // columns of the same hidden units; p.N counts hidden units.
 // EW: epilogue warps (8, or 16 for the gated form: EW / 4 per TMEM lane quadrant).
-template <int BN, int STAGES, int SPLIT, bool GATED = false, int EW = kEpilogueWarps, int SL = 1, int AR = BM>
+template <int BN, int STAGES, int SPLIT, bool GATED = false, int EW = kEpilogueWarps, int SL = 1>
 __global__ void __launch_bounds__(96 + 32 * EW, 1)
 gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w,
                     const __grid_constant__ CUtensorMap tm_out,
-                    const __grid_constant__ std::conditional_t<SPLIT == 4, LeanParams, GemmParams> p) {
-  using L = SmemLayout<BN, STAGES, EW, SL, AR>;
-  static_assert(AR == BM || SPLIT == 4, "64-row stages: lean form only");
+                    const __grid_constant__ GemmParams p) {
+  using L = SmemLayout<BN, STAGES, EW, SL>;
   static_assert(EW == kEpilogueWarps || GATED, "only the gated epilogue is written for more than eight warps");
   static_assert(SL == 1 || !GATED, "several slabs per load: ordinary form only");
   // two accumulators, each at a power-of-two column offset; BN in {64, 128, 192, 224, 256}
   constexpr uint32_t kAccStride = BN <= 64 ? 64 : (BN <= 128 ? 128 : 256);
   constexpr uint32_t kTmemCols = 2 * kAccStride;
-  constexpr uint32_t kIdesc = make_idesc_e4m3_f32(AR, BN);
+  constexpr uint32_t kIdesc = make_idesc_e4m3_f32(BM, BN);
 
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
@@ -732,13 +716,10 @@ gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
   // Split-K: the S CTAs of a cluster work on the same tile, CTA r on K steps [kb0, kb1); one
   // tile per CTA (the host launches tiles x S CTAs, at most one wave).
   // Partials: K split over independent CTAs (no cluster), each writing its fp32 partial sums.
-  constexpr bool PLANES = SPLIT == 3, LEAN = SPLIT == 4;
-  const bool partials = LEAN && p.partials > 1;
+  constexpr bool PLANES = SPLIT == 3;
   const bool split = SPLIT == 1 || (SPLIT == 2 && p.split_k > 1);
-  // At most 64 rows: MMAs of M = 64, whose row i lies in lane i % 16 of quadrant i / 16
-  constexpr int quad_rows = AR / 4;
-  const int k_parts = partials || PLANES ? p.partials : (split ? p.split_k : 1);
-  const int split_rank = partials ? (int)blockIdx.x % k_parts : (split ? (int)cluster_ctarank() : 0);
+  const int k_parts = PLANES ? p.partials : (split ? p.split_k : 1);
+  const int split_rank = split ? (int)cluster_ctarank() : 0;
   // a unit of work is a tile, or (tile, K range) in the planes form
   const int tile_first = !PLANES && k_parts > 1 ? (int)blockIdx.x / k_parts : (int)blockIdx.x;
   const int tile_stride = !PLANES && k_parts > 1 ? p.num_tiles : (int)gridDim.x;
@@ -809,23 +790,6 @@ gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
       for (int kb = kb0; kb < kb1; kb += SL) {
         ok = wait_bounded(empty_bar(ring.stage), ring.phase ^ 1, abort_flag, (1u << 24) | (1u << 16) | (it & 0xFFFF));
         if (!ok) break;
-        if constexpr (LEAN) {
-          const int have = min(SL, kb1 - kb);
-          if (kb + have > p.full_slabs) {  // the stage of the ragged slab
-            if (elect_one()) {
-              const uint32_t bar = full_bar(ring.stage), sa = base + ring.stage * L::kStageBytes, sw = sa + L::kABytes;
-              mbar_arrive_expect_tx(bar, (uint32_t)have * (bytes / SL));
-              for (int sl = 0; sl < have; ++sl) {
-                if (w_producer) tma_load_2d(sw + sl * BN * BK, &p.w_tail, bar, (kb + sl) * BK, n_blk * BN);
-                else tma_load_2d(sa + sl * p.a_bytes, &p.a_tail, bar, (kb + sl) * BK, a_row);
-              }
-            }
-            __syncwarp();
-            ring.arm();
-            ring.advance();
-            continue;
-          }
-        }
         if (elect_one()) {
           const uint32_t bar = full_bar(ring.stage), sa = base + ring.stage * L::kStageBytes, sw = sa + L::kABytes;
           mbar_arrive_expect_tx(bar, bytes);
@@ -846,9 +810,6 @@ gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
         if (weights && it == 0 && kb == kb0 + (STAGES - 1) * SL && elect_one()) {
           // the ring is full: until its first stage is free, pull the boxes behind it towards L2
           for (int kp = kb + SL; kp < kb1 && kp < kb0 + kPrefetchSteps; kp += SL) {
-            if constexpr (LEAN) {
-              if (kp >= p.full_slabs) break;
-            }
             if constexpr (GATED) tma_prefetch_l2_3d(&tm_w, kp * BK, n_blk * (BN / 2), 0);
             else if constexpr (SL > 1) tma_prefetch_l2_3d(&tm_w, 0, n_blk * BN, kp);
             else tma_prefetch_l2_2d(&tm_w, kp * BK, n_blk * BN);
@@ -935,9 +896,9 @@ gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
       // same thing before its first load), then this tile's per-column operands and row scale, so
       // that their latency runs under the main loop instead of after it.
       if (it == 0) grid_dependency_wait();
-      const int m = m_blk * BM + quad * quad_rows + lane;
-      const bool row_ok = m < p.M && (!LEAN || lane < quad_rows);
-      const bool prefetch = !GATED && !split && (LEAN || p.tma_store) && p.epilogue != EPI_RAW && col_end - col_begin <= 128;
+      const int m = m_blk * BM + quad * 32 + lane;
+      const bool row_ok = m < p.M;
+      const bool prefetch = !GATED && !split && p.tma_store && p.epilogue != EPI_RAW && col_end - col_begin <= 128;
       ColumnVectors cv;
       float rs_early = 1.0f;
       if (prefetch) {
@@ -967,14 +928,14 @@ gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
       if (split) {
         // one tile per CTA: the partial accumulator stays in tensor memory; the exchange with
         // the other CTAs of the cluster follows the role loops
-      } else if (LEAN || p.tma_store) {
+      } else if (p.tma_store) {
         // whole 128-byte pieces through shared memory and TMA; a 32-column remainder of a
         // 224-wide tile (two-byte outputs) straight from registers
         const int per_store = (p.out_dtype == IFLB200_F32 || p.half_rows) ? 32 : 64;
         const int col_tma_end = col_begin + (col_end - col_begin) / per_store * per_store;
-        epilogue_tma_store<BN, quad_rows>(p, tm_dst, t_row, staging, staging_ptr, m_blk * BM + quad * quad_rows, n_blk * BN,
+        epilogue_tma_store<BN>(p, tm_dst, t_row, staging, staging_ptr, m_blk * BM + quad * 32, n_blk * BN,
                                col_begin, col_tma_end, rs, lane,
-                               PLANES ? unit % k_parts : (LEAN && p.partials >= 1 ? split_rank : -1),  // a plane map takes a 3-D store
+                               PLANES ? unit % k_parts : -1,  // a plane map takes a 3-D store
                                prefetch ? &cv : nullptr);
         if (BN % 64 != 0 && col_tma_end < col_end) {
           const int n0 = n_blk * BN + col_tma_end;
@@ -1384,6 +1345,7 @@ gemm_fp8_tc5_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
 }  // namespace iflb200
 
 #include "gemm_tokens.cuh"
+#include "gemm_lean.cuh"
 
 namespace iflb200 {
 
@@ -1515,22 +1477,22 @@ static int g_cfg_slabs = 0;  // 1: one K slab per TMA instruction everywhere (ex
 static int g_cfg_gated_warps = 0;  // gated form, 256-wide tiles: 0 heuristic, 8 or 16 epilogue warps
 static int g_cfg_mode = 0;  // 0 auto, 1 single-CTA tiles only, 2 CTA pairs with one accumulator, 3 CTA pairs with two
 
-template <int BN, int STAGES, int SPLIT, bool GATED = false, int EW = kEpilogueWarps, int SL = 1, int AR = BM>
+template <int BN, int STAGES, int SPLIT, bool GATED = false, int EW = kEpilogueWarps, int SL = 1>
 static int launch_gemm_form(const CUtensorMap& ta, const CUtensorMap& tw, const CUtensorMap& to,
-                            const std::conditional_t<SPLIT == 4, LeanParams, GemmParams>& p, int grid, cudaStream_t s) {
-  using L = SmemLayout<BN, STAGES, EW, SL, AR>;
+                            const GemmParams& p, int grid, cudaStream_t s) {
+  using L = SmemLayout<BN, STAGES, EW, SL>;
   static_assert(L::kDynamic <= 227 * 1024, "stage ring + staging exceed the shared memory of an SM");
   static bool attr_set[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return IFLB200_ERR_DEVICE;
   if (!attr_set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_fp8_tc5_kernel<BN, STAGES, SPLIT, GATED, EW, SL, AR>,
+    cudaError_t e = cudaFuncSetAttribute(gemm_fp8_tc5_kernel<BN, STAGES, SPLIT, GATED, EW, SL>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, L::kDynamic);
     if (e != cudaSuccess) return (int)e;
     attr_set[dev] = true;
   }
-  const cudaError_t e = launch_dep(gemm_fp8_tc5_kernel<BN, STAGES, SPLIT, GATED, EW, SL, AR>, dim3(grid),
+  const cudaError_t e = launch_dep(gemm_fp8_tc5_kernel<BN, STAGES, SPLIT, GATED, EW, SL>, dim3(grid),
                                    dim3(96 + 32 * EW), L::kDynamic, s, p.split_k,
                                    dependent_launch_for(p.M), ta, tw, to, p);
   note_captured_gemm(s);
@@ -1553,8 +1515,26 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tw, const CUten
 static int make_tensor_map(CUtensorMap* tm, const void* ptr, int rows, int K, int64_t ld, int box_rows);
 static int make_slab_map(CUtensorMap* tm, const void* ptr, int rows, int K, int64_t ld, int box_rows, int slabs);
 
-static int launch_lean(const void* a, int64_t ld_a, const void* w, int64_t ld_w, const CUtensorMap& to, const GemmParams& g,
-                       int grid, cudaStream_t s) {
+template <int AR, int EPI>
+static int launch_lean_form(const CUtensorMap& ta, const CUtensorMap& tw, const LeanParams& p, int grid, cudaStream_t s) {
+  static bool attr_set[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) return IFLB200_ERR_DEVICE;
+  if (!attr_set[dev]) {
+    const cudaError_t e = cudaFuncSetAttribute(gemm_fp8_tc5_lean_kernel<AR, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               LeanLayout<AR>::kDynamic);
+    if (e != cudaSuccess) return (int)e;
+    attr_set[dev] = true;
+  }
+  const cudaError_t e = launch_dep(gemm_fp8_tc5_lean_kernel<AR, EPI>, dim3(grid), dim3(LeanLayout<AR>::kThreads),
+                                   LeanLayout<AR>::kDynamic, s, 1, dependent_launch_for(p.M), ta, tw, p);
+  note_captured_gemm(s);
+  return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
+}
+
+template <int EPI>
+static int launch_lean(const void* a, int64_t ld_a, const void* w, int64_t ld_w, const GemmParams& g, int grid, cudaStream_t s) {
   LeanParams p;
   static_cast<GemmParams&>(p) = g;
   p.full_slabs = g.K / BK;
@@ -1570,8 +1550,7 @@ static int launch_lean(const void* a, int64_t ld_a, const void* w, int64_t ld_w,
     memset(&p.w_tail, 0, sizeof(p.w_tail));
   }
   if (st != IFLB200_OK) return st;
-  return g.M <= 64 ? launch_gemm_form<64, 3, 4, false, kEpilogueWarps, 4, 64>(ta, tw, to, p, grid, s)
-                   : launch_gemm_form<64, 2, 4, false, kEpilogueWarps, 4>(ta, tw, to, p, grid, s);
+  return g.M <= 64 ? launch_lean_form<64, EPI>(ta, tw, p, grid, s) : launch_lean_form<128, EPI>(ta, tw, p, grid, s);
 }
 
 template <int BN, int STAGES, int ACC, bool PLANES = false, bool GATED = false, int EW = kEpilogueWarps>
@@ -1666,9 +1645,11 @@ static int launch_tokens(const void* a, int64_t ld_a, const void* w, int64_t ld_
 // Estimated time of the tokens form, in the units of the costs it is compared with (each set of constants belongs to one
 // comparison): a slab takes at least `floor` clocks (commit and barriers) and `slab` + `slab_token` a token of the tile
 // (rows through the L2 port), times `ragged` where rows are off 64-byte boundaries; a tile's epilogue `tile` +
-// `tile_token` a token; a partly filled last wave counts 1 - `whole` of its share.
+// `tile_token` a token; a partly filled last wave counts 1 - `whole` of its share; a single wave of more than 7 in 8 of
+// the pairs waits `full` for the last SMs of the kernel before it (333 x 2560 x 2048 behind its pack: 70 pairs 13.1 us, 60
+// pairs 11.6).
 struct TokenCost {
-  double floor, slab, slab_token, tile, tile_token, ends, whole, ragged;
+  double floor, slab, slab_token, tile, tile_token, ends, whole, ragged, full;
 };
 constexpr int kTokensMinRows = 65;  // up to 64 rows the lean form's 64-row MMAs have less to do
 // M tokens, `cols` weight rows, `ranges` K ranges of `steps` slabs.
@@ -1677,7 +1658,7 @@ static double tokens_cost(int M, int64_t cols, int steps, int ranges, bool align
   const int64_t waves = (units + pairs - 1) / pairs;
   const double row = c.slab + c.slab_token * bt;
   const double wave = steps * (row > c.floor ? row : c.floor) * (aligned ? 1.0 : c.ragged) + c.tile + c.tile_token * bt;
-  return (waves == 1 ? wave : c.whole * waves * wave + (1.0 - c.whole) * units * wave / pairs) + c.ends;
+  return (waves == 1 ? wave + (units * 8 > pairs * 7 ? c.full : 0.0) : c.whole * waves * wave + (1.0 - c.whole) * units * wave / pairs) + c.ends;
 }
 // The width of least cost.  Narrower tiles than 48 tokens wait for barriers, and for more than 1500 tokens nothing
 // below 144 was ever the fastest.
@@ -1810,8 +1791,8 @@ static int run_gemm(const void* a, int64_t ld_a, const void* w, int64_t ld_w, Ge
     // 23.1 us, 25.6 in this form), so that the fused linear's bits stay those of the raw output's.
     if (g_cfg_mode == 0 && g_cfg_stages == 0 && p.tma_store && g_cfg_tokens != 1 &&
         (tokens_forced || (g_cfg_tile_n == 0 && g_cfg_split_k <= 1 && p.M >= kTokensMinRows))) {
-      static constexpr TokenCost raw = {407, 68.5, 2.043, 771, 7.39, 3446, 0.8, 1.176};
-      static constexpr TokenCost dequant = {356, 92.2, 2.004, 1226, 4.70, 3070, 0.744, 1.21};
+      static constexpr TokenCost raw = {407, 68.5, 2.043, 771, 7.39, 3446, 0.8, 1.176, 0};
+      static constexpr TokenCost dequant = {297, 169, 1.897, 1336, 6.95, 3571, 0.588, 0.818, 460};
       const TokenCost& c = arithmetic ? dequant : raw;
       double cost = 0.0;
       int bt = tokens_width(p.M, p.N, (int)steps, 1, aligned, c, dev->sm_count, cost);
@@ -1881,12 +1862,9 @@ static int run_gemm(const void* a, int64_t ld_a, const void* w, int64_t ld_w, Ge
   // them; the K order is unchanged, so are the bits.
   if (bn == 64 && g_cfg_slabs != 1 && p.num_k / split >= 4 && stages == 0) {
     if (split == 1 && p.tma_store) {
-      if (p.M <= 64) {  // the lean form stores sixteen rows at a time then
-        st = make_out_map(&to, p.out, p.M, p.N, p.ld_out, oes, p.half_rows ? 64 : 128, 16);
-        if (st != IFLB200_OK) return st;
-      }
       g_last_launch[3] = 104;
-      return launch_lean(a, ld_a, w, ld_w, to, p, grid, s);
+      return p.epilogue == EPI_RAW ? launch_lean<LEAN_RAW>(a, ld_a, w, ld_w, p, grid, s)
+                                   : launch_lean<LEAN_DEQUANT>(a, ld_a, w, ld_w, p, grid, s);
     }
     CUtensorMap sa_map, sw_map;
     if (p.K % BK == 0 && make_slab_map(&sa_map, a, p.M, p.K, ld_a, a_rows, 4) == IFLB200_OK &&
@@ -1965,7 +1943,7 @@ static int run_gemm_partials(const void* a, int64_t ld_a, const void* w, int64_t
     }
   }
   if (g_cfg_mode == 0 && g_cfg_tokens != 1 && (M >= kTokensMinRows || g_cfg_tokens == 2)) {
-    static constexpr TokenCost planes = {314, 37.8, 1.986, 1706, 8, 2056, 0.848, 0.947};
+    static constexpr TokenCost planes = {314, 37.8, 1.986, 1706, 8, 2056, 0.848, 0.947, 0};
     double time = 0.0;
     int bt = tokens_width(M, N, steps, splits, (ld_a | ld_w) % 64 == 0, planes, dev->sm_count, time);
     if (g_cfg_tokens == 2 && g_cfg_tile_n) bt = g_cfg_tile_n;
@@ -1979,12 +1957,12 @@ static int run_gemm_partials(const void* a, int64_t ld_a, const void* w, int64_t
   const int a_rows = activation_box_rows(M);
   p.a_bytes = a_rows * BK;
   CUtensorMap ta, tw, to;
-  st = make_partials_map(&to, out, M, N, ld_out, splits, M <= 64 ? 16 : 32);
+  st = make_partials_map(&to, out, M, N, ld_out, splits, 32);
   if (st != IFLB200_OK) return st;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (M <= BM) {
     g_last_launch[0] = 1 + 16; g_last_launch[1] = 64; g_last_launch[2] = splits; g_last_launch[3] = 104;
-    return launch_lean(a, ld_a, w, ld_w, to, p, p.num_tiles * splits, s);
+    return launch_lean<LEAN_PLANES>(a, ld_a, w, ld_w, p, p.num_tiles * splits, s);
   }
   // CTA pairs where blocks of 256 rows pad little and their units need no more waves: two thirds of the traffic per K step, which is what these launches wait for.
   // 816 x 2048 x 16384 in two ranges 28.6 against 29.7 us, 640 rows in three 22.8 against 23.3.
@@ -2126,7 +2104,7 @@ static int run_gemm_gated(const void* a, int64_t ld_a, const void* w, int64_t ld
       (g_cfg_tokens == 2 || (g_cfg_tile_n == 0 && M >= kTokensMinRows && F >= 2048))) {
     // tokens on the MMA's N side (constants over 700 sizes: 0.6 % slower than the fastest form on average, 1.7 % less time
     // than without it, eleven more than 3 % slower; hidden widths below 2048 were not among them)
-    static constexpr TokenCost gated = {265, 46, 2.225, 1375, 7.51, 1554, 0.911, 1.152};
+    static constexpr TokenCost gated = {265, 46, 2.225, 1375, 7.51, 1554, 0.911, 1.152, 0};
     double time = 0.0;
     int bt = tokens_width(M, 2 * (int64_t)F, p.num_k, 1, aligned, gated, dev->sm_count, time);
     if (g_cfg_tile_n) bt = g_cfg_tile_n;
