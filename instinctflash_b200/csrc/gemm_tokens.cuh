@@ -40,6 +40,7 @@ struct TokenParams {
   int64_t ld_out, plane;  // bytes from one token to the next, from one plane to the next
   int out_dtype;
   int act;
+  int evict;  // gated form: weights leave L2 first
   uint32_t* amax;
 };
 
@@ -186,6 +187,7 @@ gemm_fp8_tc5_tokens_kernel(const __grid_constant__ CUtensorMap tm_t, const __gri
     // Two warps for each operand, which take the slabs in turn; the weights' ahead of the dependency wait, as in the
     // other forms.
     if (t_producer) grid_dependency_wait();
+    const uint64_t policy = l2_evict_first();
     int slot = producer >> 1, skip = producer >> 1;  // skip: slabs of the other warp until this one's next
     uint32_t phase = 0;
     bool ok = true;
@@ -207,7 +209,10 @@ gemm_fp8_tc5_tokens_kernel(const __grid_constant__ CUtensorMap tm_t, const __gri
           if (i < slabs) {
             if (leader) mbar_arrive_expect_tx(bar, 2u * (w_producer ? w_bytes : t_bytes));
             if (t_producer) tma_load_2d_pair(dst + w_bytes, &tm_t, bar & kPeerBitMask, x, t_row);
-            else if constexpr (EPI == TOK_GATED) tma_load_4d_pair(dst, &tm_w, bar & kPeerBitMask, x, 0, 0, w_row / 16);
+            else if constexpr (EPI == TOK_GATED) {
+              if (p.evict) tma_load_4d_pair_hint(dst, &tm_w, bar & kPeerBitMask, x, 0, 0, w_row / 16, policy);
+              else tma_load_4d_pair(dst, &tm_w, bar & kPeerBitMask, x, 0, 0, w_row / 16);
+            }
             else tma_load_2d_pair(dst, &tm_w, bar & kPeerBitMask, x, w_row);
           } else if (leader) {
             mbar_arrive(bar);  // an odd number of slabs: nothing to load, but the slot's phases stay in step

@@ -319,6 +319,21 @@ __device__ __forceinline__ void tma_load_4d_pair(uint32_t smem_dst, const void* 
       ::"r"(smem_dst), "l"(tensor_map), "r"(leader_bar), "r"(x), "r"(y), "r"(z), "r"(w)
       : "memory");
 }
+// A policy under which lines that a load brings to L2 are the first to go again.
+__device__ __forceinline__ uint64_t l2_evict_first() {
+  uint64_t policy;
+  asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
+  return policy;
+}
+// tma_load_4d_pair under an L2 policy.
+__device__ __forceinline__ void tma_load_4d_pair_hint(uint32_t smem_dst, const void* tensor_map, uint32_t leader_bar, int32_t x,
+                                                      int32_t y, int32_t z, int32_t w, uint64_t policy) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint "
+      "[%0], [%1, {%3, %4, %5, %6}], [%2], %7;"
+      ::"r"(smem_dst), "l"(tensor_map), "r"(leader_bar), "r"(x), "r"(y), "r"(z), "r"(w), "l"(policy)
+      : "memory");
+}
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t smem_dst, uint32_t cols) {
   asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst),
                "r"(cols)

@@ -262,15 +262,15 @@ bool gelu_width(const GeluStreamArgs& a, int sms, cudaStream_t s) {
 //     res += fma(delta * drow, dcol, bias) * gate;   y = norm(res) * scale + shift;   q, s = e4m3(y)
 // Bound by HBM and by the shared-memory port that delivers the vectors (20 bytes per element, 0.8 of the
 // port's cycles): 16384 x 5120 217 -> 111 us (5.3 TB/s; 3 bytes per element, no vectors: 112 -> 50),
-// 4680 x 3072 38 -> 28.5.
+// 4680 x 3072 38 -> 23.5.
 // The same structure: the residual and delta rows of the next turn are fetched into private slots, the
 // five vectors are in shared memory, the three meetings of a row (mean, variance, maximum) cost the
 // CTA's other groups nothing.
 // --------------------------------------------------------------------------------------------
-constexpr int kResNormThreads = 640;
+constexpr int kResNormThreads = 640, kResNormMore = 768;
 
-template <bool DELTA, bool GATE, bool AFFINE>
-__global__ void __launch_bounds__(kResNormThreads, 1) residual_norm_stream_kernel(const ResNormStreamArgs a, int tg) {
+template <bool DELTA, bool GATE, bool AFFINE, int THREADS>
+__global__ void __launch_bounds__(THREADS, 1) residual_norm_stream_kernel(const ResNormStreamArgs a, int tg) {
   constexpr int kVectors = (DELTA ? 2 : 0) + (GATE ? 1 : 0) + (AFFINE ? 2 : 0);
   extern __shared__ __align__(16) uint8_t smem[];
   __shared__ __align__(16) float red[3][kMaxGroups][kMaxWarps];
@@ -396,12 +396,26 @@ __global__ void __launch_bounds__(kResNormThreads, 1) residual_norm_stream_kerne
   }
 }
 
+template <bool DELTA, bool GATE, bool AFFINE, int THREADS>
+bool resnorm_launch(const ResNormStreamArgs& a, const StreamGeom& g, int sms, cudaStream_t s) {
+  return g.groups != 0 && launch_stream<residual_norm_stream_kernel<DELTA, GATE, AFFINE, THREADS>>(g, sms, s, a);
+}
 template <bool DELTA, bool GATE, bool AFFINE>
 bool resnorm_form(const ResNormStreamArgs& a, int sms, cudaStream_t s) {
-  const StreamGeom g = stream_geom(a.M, a.D, (DELTA ? 2 : 0) + (GATE ? 1 : 0) + (AFFINE ? 2 : 0), a.D * (DELTA ? 4 : 2),
-                                   kResNormThreads, sms);
-  if (g.groups == 0) return false;
-  return launch_stream<residual_norm_stream_kernel<DELTA, GATE, AFFINE>>(g, sms, s, a);
+  auto geom = [&](int threads) {
+    return stream_geom(a.M, a.D, (DELTA ? 2 : 0) + (GATE ? 1 : 0) + (AFFINE ? 2 : 0), a.D * (DELTA ? 4 : 2), threads, sms);
+  };
+  const StreamGeom g = geom(kResNormThreads);
+  if constexpr (DELTA) {
+    // More groups on fewer registers a thread where the rows then fill the turns better, by one row place in twenty at
+    // least: 4680 x 3072 takes four turns of eight rows an SM instead of six of six, 26.9 -> 23.5 us with a gate and 24.3
+    // -> 21.0 without, and of 59 other sizes none more than 2 % slower. With the same places the spills cost more (16384 x 5120 107 -> 115).
+    const StreamGeom more = geom(kResNormMore);
+    auto places = [&](const StreamGeom& x) { return (a.M + x.groups * sms - 1) / (x.groups * sms) * x.groups; };
+    if (g.groups != 0 && more.groups > g.groups && places(more) * 20 <= places(g) * 19)
+      return resnorm_launch<DELTA, GATE, AFFINE, kResNormMore>(a, more, sms, s);
+  }
+  return resnorm_launch<DELTA, GATE, AFFINE, kResNormThreads>(a, g, sms, s);
 }
 
 // --------------------------------------------------------------------------------------------
