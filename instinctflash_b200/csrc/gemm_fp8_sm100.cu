@@ -1708,7 +1708,7 @@ static int run_gemm(const void* a, int64_t ld_a, const void* w, int64_t ld_w, Ge
   // Tile shape by a measured cost model: waves x (K steps x clocks of a step + what a tile's epilogue holds up), and what
   // the first loads and the last stores take.  A partly filled last wave, which has the L2 and the store path to itself,
   // counts 0.7 and 0.3 of its share.  A 128-byte K step of a 64 / 128 / 256 wide tile is about 490 / 555 / 800 clocks:
-  // 24 / 32 / 48 KB are written to shared memory and read back by the tensor core through one port of 128 bytes a clock
+  // 24 / 32 / 48 KB come from L2 at about 64 bytes a clock and SM
   // (192 and 224 interpolate; the lean form's 64 rows 315).  A CTA pair's 256 x 256 tile is 32 KB per SM and 690, or 750
   // in a single wave, where latency shows.  Rows that do not start on 64-byte boundaries (K and strides in odd multiples
   // of 16 or 32) make every 128-byte piece two L2 requests: 570 / 630 / 815, lean 395, pairs 650 and 585.  The constants
@@ -1800,7 +1800,10 @@ static int run_gemm(const void* a, int64_t ld_a, const void* w, int64_t ld_w, Ge
       double cost = 0.0;
       int bt = tokens_width(p.M, p.N, (int)steps, 1, aligned, c, dev->sm_count, cost);
       if (g_cfg_tile_n) bt = g_cfg_tile_n;
-      bool take = cost < (double)best && (split == 1 || steps < 112);
+      // Nor is fp32 output of unrounded accumulators moved from a split K to an unsplit one: there, not behind a 16-bit
+      // rounding, the shorter sums are the more exact ones (K = 4096: 0.9e-7 in four ranges, 3.5e-7 in one).
+      const bool sums_show = arithmetic && p.exact && p.out_dtype == IFLB200_F32;
+      bool take = cost < (double)best && (split == 1 || (steps < 112 && !sums_show));
       if (take && pair && (!arithmetic || steps >= 32))
         take = bt < 256 && cost < 0.97 * tokens_cost(p.M, p.N, (int)steps, 1, aligned, c, dev->sm_count, 256);
       if (take || tokens_forced)
@@ -2105,9 +2108,9 @@ static int run_gemm_gated(const void* a, int64_t ld_a, const void* w, int64_t ld
   }
   if (g_cfg_mode == 0 && g_cfg_tokens != 1 && g_cfg_gated_warps == 0 &&
       (g_cfg_tokens == 2 || (g_cfg_tile_n == 0 && M >= kTokensMinRows && F >= 2048))) {
-    // tokens on the MMA's N side (constants over 700 sizes: 0.6 % slower than the fastest form on average, 1.7 % less time
-    // than without it, eleven more than 3 % slower; hidden widths below 2048 were not among them)
-    static constexpr TokenCost gated = {265, 46, 2.225, 1375, 7.51, 1554, 0.911, 1.152, 0};
+    // tokens on the MMA's N side (constants over 800 of 1051 sizes: 0.7 % slower than the fastest form on average, 3.7 %
+    // less time than without it, 44 more than 3 % slower; hidden widths below 2048 were not among them)
+    static constexpr TokenCost gated = {150, 47.9, 2.298, 731, 7.51, 1656, 0.737, 1.083, 0};
     double time = 0.0;
     int bt = tokens_width(M, 2 * (int64_t)F, p.num_k, 1, aligned, gated, dev->sm_count, time);
     if (g_cfg_tile_n) bt = g_cfg_tile_n;
