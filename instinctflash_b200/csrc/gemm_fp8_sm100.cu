@@ -2108,9 +2108,10 @@ static int run_gemm_gated(const void* a, int64_t ld_a, const void* w, int64_t ld
   }
   if (g_cfg_mode == 0 && g_cfg_tokens != 1 && g_cfg_gated_warps == 0 &&
       (g_cfg_tokens == 2 || (g_cfg_tile_n == 0 && M >= kTokensMinRows && F >= 2048))) {
-    // tokens on the MMA's N side (constants over 800 of 1051 sizes: 0.7 % slower than the fastest form on average, 3.7 %
-    // less time than without it, 44 more than 3 % slower; hidden widths below 2048 were not among them)
-    static constexpr TokenCost gated = {150, 47.9, 2.298, 731, 7.51, 1656, 0.737, 1.083, 0};
+    // tokens on the MMA's N side (constants over 700 sizes; over 1750 others 2.7 % less time than without the form, 21 more
+    // than 3 % slower; constants closer to the fastest form on average, 3.5 % less time, were slower at 106 of them, 13 % at
+    // 396 x 2 x 11008 x 2048; hidden widths below 2048 were not among them)
+    static constexpr TokenCost gated = {265, 46, 2.225, 1375, 7.51, 1554, 0.911, 1.152, 0};
     double time = 0.0;
     int bt = tokens_width(M, 2 * (int64_t)F, p.num_k, 1, aligned, gated, dev->sm_count, time);
     if (g_cfg_tile_n) bt = g_cfg_tile_n;
