@@ -191,33 +191,36 @@ def partial_splits(M: int, N: int, K: int, sm_count: int = 148) -> int:
     128-byte K slabs, at most eight planes.  1, the unsplit GEMM, for outputs wider than the residual kernel
     over planes takes.
 
-    Above 128 rows the number with the least estimated time, 1 where the unsplit GEMM is as good: the time of the
-    GEMM with tokens on the MMA's N side at the width it takes (the estimate that chooses that width, see
-    ``run_gemm_partials``), and for the planes 2.28 clocks per thousand elements written and read back (the unsplit
-    bf16 output 1.38).  The constants are the ones whose choice is closest to the fastest number for the GEMM and the
-    residual kernel after it over 600 of 1345 sizes (129 to 1600 rows, 768 to 2048 columns, K 2048 to 16384): 0.9 %
-    above it on average; the estimate of the row-block form that it replaces 4.9 %.  301 x 2048 x 16384 with its
-    residual 19.8 us in six ranges, 16.8 in four.  The sums differ from 64-bit ones by 2.2e-7 in six ranges and 3.4e-7
-    in four; the consumer rounds them to bf16 before anything else, 1.658737e-3 from the 64-bit ones either way."""
+    Above 128 rows the number with the least estimated time, 1 where the unsplit GEMM is as good.  The number fixes the
+    order and the length of the fp32 sums and with them the output's bits, so the estimate stays that of the
+    row-block form it was fitted to (63 sizes: 130 to 1024 rows, seven shapes) whatever form runs the ranges: fewer
+    ranges are longer sums (301 x 2048 x 16384: 2.2e-7 from the 64-bit ones in six ranges, 3.4e-7 in four).  In SM
+    clocks: a slab of a 128 x 64 / 256 tile 380 / 700 and a wave 7500 for prologue and fp32 epilogue, every plane
+    written and read back at 3200 bytes a clock; unsplit 440 / 480 / 850 for 64 / 128 / 256 columns and 1600 a
+    wave, over a cluster 11700 and 80 a column handed over."""
     if K % 128 or N > PLANES_MAX_WIDTH:
         return 1
     slabs = K // 128
     if M <= 128:
         return max(1, min(8, sm_count // max(1, (N + 63) // 64), slabs // 4))
-    blocks, pairs, elements = (N + 255) // 256, sm_count // 2, M * N / 1000.0
+    blocks, plane = (M + 127) // 128, 8 * M * N // 3200
 
-    def gemm(splits):
-        steps, times = 4 * -(-(-(-slabs // 4)) // splits), []
-        for width in range(144 if M > 1500 else 48, 257, 16):
-            units = -(-M // width) * blocks * splits
-            wave = steps * max(314.0, 37.8 + 1.986 * width) + 1706.0 + 8.0 * width
-            waves = -(-units // pairs)
-            times.append(wave if waves == 1 else wave * (0.848 * waves + 0.152 * units / pairs))
-        return min(times) + 2056.0
+    def cost(splits, width, clocks, wave):
+        units = blocks * ((N + width - 1) // width) * splits
+        steps = min(slabs, 4 * -(-(-(-slabs // 4)) // splits))
+        return -(-units // sm_count) * (steps * clocks + wave)
 
-    best, least = 1, 1.072 * gemm(1) + 1.381 * elements
+    plain = [(width, clocks) for width, clocks in ((64, 440), (128, 480), (256, 850)) if width == 64 or N >= width]
+    unsplit = min(cost(1, w, c, 1600) for w, c in plain)
+    # over a cluster: one wave, partial sums handed over through distributed shared memory (35 clusters of four
+    # do not fit the chip at once)
+    for ranges, room in ((2, sm_count), (4, sm_count - 16)):
+        for width, clocks in plain[1:]:
+            if blocks * ((N + width - 1) // width) * ranges <= room and slabs // ranges >= 8:
+                unsplit = min(unsplit, slabs // ranges * clocks + 11700 + 80 * width * (ranges - 1) // ranges)
+    best, least = 1, unsplit + plane // 2
     for splits in range(2, min(8, (slabs + 3) // 4) + 1):
-        time = gemm(splits) + 330.0 + 2.28 * splits * elements
+        time = min(cost(splits, w, c, 7500) for w, c in ((64, 380), (256, 700)) if w == 64 or N >= w) + splits * plane
         if time < least:
             best, least = splits, time
     return best

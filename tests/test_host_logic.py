@@ -163,3 +163,13 @@ def test_no_planes_for_rows_wider_than_their_consumer_takes(M, N, K):
 
 def test_planes_up_to_the_widest_row_of_their_consumer():
     assert fp8.PLANES_MAX_WIDTH == 8192 and fp8.partial_splits(129, 8192, 16384) > 1
+
+
+# The number of K ranges fixes which fp32 sums are formed, so it is part of the result: an estimate refitted to a
+# faster kernel must not change it.
+@pytest.mark.parametrize("M,N,K,splits", [
+    (50, 1024, 4096, 8), (50, 1024, 2048, 4), (128, 2048, 2048, 4), (129, 2048, 16384, 8), (147, 1024, 2816, 1), (200, 2048, 8192, 8),
+    (230, 768, 4096, 4), (301, 2048, 2048, 1), (301, 2048, 16384, 6), (384, 3072, 8192, 4), (400, 1024, 4096, 2), (640, 2048, 16384, 3),
+    (816, 2048, 2048, 1), (816, 2048, 8192, 1), (816, 2048, 16384, 2), (1040, 2048, 11008, 1), (1500, 2048, 16384, 3)])
+def test_number_of_planes_stays(M, N, K, splits):
+    assert fp8.partial_splits(M, N, K) == splits
