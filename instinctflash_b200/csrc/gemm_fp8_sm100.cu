@@ -1790,8 +1790,9 @@ static int run_gemm(const void* a, int64_t ld_a, const void* w, int64_t ld_w, Ge
     // average, the calls 10 and 14 % faster than without the form, 25 and 15 of them more than 3 % slower.
     // Where the choice above is the pair kernel, a tile of 256 tokens is the same tile: only a narrower one that saves
     // 3 % of it is taken, or with scales, whose epilogue takes longer in the pair kernel, over fewer than 32 K steps any.
-    // Very deep reductions with few tiles stay split over a cluster, scales or not (228 x 1056 x 14320 with scales
-    // 23.1 us, 25.6 in this form), so that the fused linear's bits stay those of the raw output's.
+    // A reduction that the choice above splits over a cluster stays split, whatever its time: the number of ranges is part
+    // of the result, and shorter fp32 sums are the more exact ones (K = 4096: 0.9e-7 from the 64-bit ones in four ranges,
+    // 3.5e-7 in one).  So this form never changes a bit of what the others write.
     if (g_cfg_mode == 0 && g_cfg_stages == 0 && p.tma_store && g_cfg_tokens != 1 &&
         (tokens_forced || (g_cfg_tile_n == 0 && g_cfg_split_k <= 1 && p.M >= kTokensMinRows))) {
       static constexpr TokenCost raw = {407, 68.5, 2.043, 771, 7.39, 3446, 0.8, 1.176, 0};
@@ -1800,10 +1801,7 @@ static int run_gemm(const void* a, int64_t ld_a, const void* w, int64_t ld_w, Ge
       double cost = 0.0;
       int bt = tokens_width(p.M, p.N, (int)steps, 1, aligned, c, dev->sm_count, cost);
       if (g_cfg_tile_n) bt = g_cfg_tile_n;
-      // Nor is fp32 output of unrounded accumulators moved from a split K to an unsplit one: there, not behind a 16-bit
-      // rounding, the shorter sums are the more exact ones (K = 4096: 0.9e-7 in four ranges, 3.5e-7 in one).
-      const bool sums_show = arithmetic && p.exact && p.out_dtype == IFLB200_F32;
-      bool take = cost < (double)best && (split == 1 || (steps < 112 && !sums_show));
+      bool take = cost < (double)best && (split == 1 || pair);
       if (take && pair && (!arithmetic || steps >= 32))
         take = bt < 256 && cost < 0.97 * tokens_cost(p.M, p.N, (int)steps, 1, aligned, c, dev->sm_count, 256);
       if (take || tokens_forced)

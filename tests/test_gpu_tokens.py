@@ -104,3 +104,32 @@ def test_gated(M, N, K, tile, act):
         assert torch.equal(amax[:M], h[:M, :F].abs().amax(1))
         return [h, amax]
     both(run, tile)
+
+
+# Reductions that are split over a cluster without the form, over sizes at which it is estimated faster unsplit; the last
+# rows on both sides of K = 14336
+@pytest.mark.parametrize("M,N,K", [(71, 304, 4864), (166, 1232, 5184), (411, 2112, 8896), (510, 320, 9296), (260, 3072, 13824),
+                                   (260, 3072, 14208), (260, 3072, 14336), (260, 3072, 16384)])
+def test_the_choice_keeps_the_k_split(M, N, K):
+    from instinctflash_b200 import _lib
+    from instinctflash_b200.kernels import fp8
+    lib = _lib.lib()
+    g, a, w = operands(M, N, K)
+    s = torch.rand(M, device=DEV, generator=g)
+    W = fp8.Fp8Weight(w, torch.rand(N, device=DEV, generator=g) * 1e-2, torch.randn(N, device=DEV, generator=g))
+    calls = [lambda o: fp8.gemm(a, W, o), lambda o: fp8.fp8_linear(a, s, W, o), lambda o: fp8.fp8_linear(a, s, W, o, exact=True)]
+    outs, splits = [], []
+    try:
+        for mode in (128, 0):
+            assert lib.iflb200_gemm_set_mode(mode) == 0
+            for call in calls:
+                outs.append(torch.full((M, N), float("nan"), device=DEV, dtype=torch.bfloat16))
+                call(outs[-1])
+                split = ctypes.c_int(0)
+                assert lib.iflb200_gemm_last_launch(None, None, ctypes.byref(split)) == 0
+                splits.append(split.value)
+    finally:
+        lib.iflb200_gemm_set_mode(0)
+    assert splits[:3] == splits[3:] and max(splits) > 1
+    for without, default in zip(outs[:3], outs[3:]):
+        assert torch.equal(bits(without), bits(default))
