@@ -1793,8 +1793,9 @@ static int run_gemm(const void* a, int64_t ld_a, const void* w, int64_t ld_w, Ge
     // A reduction that the choice above splits over a cluster stays split, whatever its time: the number of ranges is part
     // of the result, and shorter fp32 sums are the more exact ones (K = 4096: 0.9e-7 from the 64-bit ones in four ranges,
     // 3.5e-7 in one).  So this form never changes a bit of what the others write.
-    if (g_cfg_mode == 0 && g_cfg_stages == 0 && p.tma_store && g_cfg_tokens != 1 &&
-        (tokens_forced || (g_cfg_tile_n == 0 && g_cfg_split_k <= 1 && p.M >= kTokensMinRows))) {
+    // (a forced split over a cluster is not this form's: it runs or is refused below, in every mode)
+    if (g_cfg_mode == 0 && g_cfg_stages == 0 && p.tma_store && g_cfg_tokens != 1 && g_cfg_split_k <= 1 &&
+        (tokens_forced || (g_cfg_tile_n == 0 && p.M >= kTokensMinRows))) {
       static constexpr TokenCost raw = {407, 68.5, 2.043, 771, 7.39, 3446, 0.8, 1.176, 0};
       static constexpr TokenCost dequant = {297, 169, 1.897, 1336, 6.95, 3571, 0.588, 0.818, 460};
       const TokenCost& c = arithmetic ? dequant : raw;

@@ -1,4 +1,6 @@
 """Forced GEMM configurations that do not fit a problem are refused, whatever they are combined with."""
+import ctypes
+
 import pytest
 import torch
 
@@ -24,6 +26,29 @@ def test_a_split_that_does_not_fit_is_refused(mode, M, N, K, split):
         lib.iflb200_gemm_set_split_k(0)
     torch.cuda.synchronize()
     assert st == _lib.ERR_ARG and (out == 7.0).all()
+
+
+# the tokens form has no split over a cluster: asked for together, the split is taken where it fits and refused where not
+@pytest.mark.parametrize("M,N,K,split,fits", [(50, 64, 512, 4, False), (300, 128, 1024, 2, False), (300, 256, 4096, 4, True), (301, 2048, 2048, 2, True)])
+def test_a_forced_split_stands_above_the_tokens_form(M, N, K, split, fits):
+    from instinctflash_b200 import _lib
+    lib = _lib.lib()
+    g = torch.Generator(device=DEV).manual_seed(K)
+    a, w = (torch.randn(n, K, device=DEV, generator=g).to(E4M3) for n in (M, N))
+    stream, outs, ran = torch.cuda.current_stream().cuda_stream, [], ctypes.c_int(0)
+    try:
+        assert lib.iflb200_gemm_set_split_k(split) == 0
+        for mode in (128, 256):
+            assert lib.iflb200_gemm_set_mode(mode) == 0
+            outs.append(torch.full((M, N), 7.0, device=DEV, dtype=torch.bfloat16))
+            st = lib.iflb200_gemm_fp8_raw(a.data_ptr(), K, w.data_ptr(), K, M, N, K, outs[-1].data_ptr(), N, stream)
+            assert st == (0 if fits else _lib.ERR_ARG)
+            assert not fits or (lib.iflb200_gemm_last_launch(None, None, ctypes.byref(ran)) == 0 and ran.value == split)
+    finally:
+        lib.iflb200_gemm_set_mode(0)
+        lib.iflb200_gemm_set_split_k(0)
+    torch.cuda.synchronize()
+    assert torch.equal(*outs) and bool((outs[0] == 7.0).all()) == (not fits)
 
 
 # small calls of the fused linear: no K split over a cluster, whose epilogue costs more than the K steps it saves
