@@ -1802,7 +1802,11 @@ static int run_gemm(const void* a, int64_t ld_a, const void* w, int64_t ld_w, Ge
       double cost = 0.0;
       int bt = tokens_width(p.M, p.N, (int)steps, 1, aligned, c, dev->sm_count, cost);
       if (g_cfg_tile_n) bt = g_cfg_tile_n;
-      bool take = cost < (double)best && (split == 1 || pair);
+      // For more than 1500 rows the widths begin at 144 tokens, so that fewer than 512 columns are too few tiles for the
+      // pairs: where the 64-wide form is the alternative, 21 of 31 such sizes were slower in this one, all 1.06 times on
+      // average (6808 x 32 x 2224 8.7 and 10.7 us, 2588 x 288 x 3984 13.9 and 15.3).
+      const bool narrow = p.M > 1500 && p.N < 512 && bn == 64 && !pair;
+      bool take = cost < (double)best && (split == 1 || pair) && !narrow;
       if (take && pair && (!arithmetic || steps >= 32))
         take = bt < 256 && cost < 0.97 * tokens_cost(p.M, p.N, (int)steps, 1, aligned, c, dev->sm_count, 256);
       if (take || tokens_forced)

@@ -133,3 +133,18 @@ def test_the_choice_keeps_the_k_split(M, N, K):
     assert splits[:3] == splits[3:] and max(splits) > 1
     for without, default in zip(outs[:3], outs[3:]):
         assert torch.equal(bits(without), bits(default))
+
+
+# more than 1500 rows: few columns stay with the 64-wide form, up to 512 of them; the sizes around the line keep theirs
+@pytest.mark.parametrize("M,N,K,taken", [(6808, 32, 2224, False), (2588, 288, 3984, False), (4394, 16, 3456, False), (1500, 80, 6560, True),
+                                         (1650, 704, 1376, True), (7032, 416, 4416, True)])
+def test_few_columns_of_many_rows(M, N, K, taken):
+    from instinctflash_b200 import _lib
+    from instinctflash_b200.kernels import fp8
+    g, a, w = operands(M, N, K)
+    s, W = torch.rand(M, device=DEV, generator=g), fp8.Fp8Weight(w, torch.rand(N, device=DEV, generator=g), None)
+    family = ctypes.c_int(0)
+    for call in (lambda o: fp8.gemm(a, W, o), lambda o: fp8.fp8_linear(a, s, W, o)):
+        call(torch.empty(M, N, device=DEV, dtype=torch.bfloat16))
+        assert _lib.lib().iflb200_gemm_last_launch(ctypes.byref(family), None, None) == 0
+        assert bool(family.value & 4) == taken
