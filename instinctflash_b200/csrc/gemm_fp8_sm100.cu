@@ -1806,7 +1806,12 @@ static int run_gemm(const void* a, int64_t ld_a, const void* w, int64_t ld_w, Ge
       // pairs: where the 64-wide form is the alternative, 21 of 31 such sizes were slower in this one, all 1.06 times on
       // average (6808 x 32 x 2224 8.7 and 10.7 us, 2588 x 288 x 3984 13.9 and 15.3).
       const bool narrow = p.M > 1500 && p.N < 512 && bn == 64 && !pair;
-      bool take = cost < (double)best && (split == 1 || pair) && !narrow;
+      // Raw tiles of five K steps and fewer wait for their stores in every wave but the last: where the 256-wide form, which
+      // stores through TMA, is the alternative, 61 of 74 such sizes were slower in this one, all 1.09 times on average
+      // (5117 x 7424 x 448 30.0 and 25.8 us, 2967 x 14016 x 384 31.6 and 23.4).
+      const int64_t units = (int64_t)((p.M + bt - 1) / bt) * ((p.N + 2 * BM - 1) / (2 * BM));
+      const bool stores = !arithmetic && aligned && steps <= 5 && bn == 256 && !pair && units > dev->sm_count / 2;
+      bool take = cost < (double)best && (split == 1 || pair) && !narrow && !stores;
       if (take && pair && (!arithmetic || steps >= 32))
         take = bt < 256 && cost < 0.97 * tokens_cost(p.M, p.N, (int)steps, 1, aligned, c, dev->sm_count, 256);
       if (take || tokens_forced)

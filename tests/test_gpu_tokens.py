@@ -213,3 +213,15 @@ def test_few_columns_of_many_rows(M, N, K, taken):
         call(torch.empty(M, N, device=DEV, dtype=torch.bfloat16))
         assert _lib.lib().iflb200_gemm_last_launch(ctypes.byref(family), None, None) == 0
         assert bool(family.value & 4) == taken
+
+
+# raw outputs of five K steps and fewer in more than one wave stay with the 256-wide form, six steps and one wave do not
+@pytest.mark.parametrize("M,N,K,taken", [(2967, 14016, 384, False), (5117, 7424, 640, False), (3732, 10016, 768, True), (1222, 3552, 512, True)])
+def test_short_raw_reductions(M, N, K, taken):
+    from instinctflash_b200 import _lib
+    from instinctflash_b200.kernels import fp8
+    _, a, w = operands(M, N, K)
+    fp8.gemm(a, fp8.Fp8Weight(w, None, None), torch.empty(M, N, device=DEV, dtype=torch.bfloat16))
+    family = ctypes.c_int(0)
+    assert _lib.lib().iflb200_gemm_last_launch(ctypes.byref(family), None, None) == 0
+    assert bool(family.value & 4) == taken
