@@ -1938,32 +1938,26 @@ static int run_gemm_partials(const void* a, int64_t ld_a, const void* w, int64_t
   p.partials = splits;
   p.tma_store = 1;
   p.num_m = (M + BM - 1) / BM;
-  // more than 128 rows: the width with the least waves x steps x clocks (as in run_gemm; an fp32 tile's epilogue
-  // and the prologue are 4000 a wave); more than 64: tokens on the MMA's N side where that takes less
-  // (constants over 1200 of 3462 sizes and numbers of ranges: 0.4 % slower than the fastest form on average, 28 % less time
-  // than without the form, nine more than 3 % slower; 816 x 2048 x 16384 in two ranges 29.4 -> 23.1 us)
-  int bn = 64;
+  // More than 64 rows: tokens on the MMA's N side (410 sizes of 64 to 2560 columns 0.71 of the time before this form; 816 x 2048 x 16384
+  // in two ranges 29.4 -> 23.1 us), but not up to 64 columns for more than 1500 rows, which fill a quarter of its 256 weight
+  // rows at the most and are as many tiles of the row blocks: 1.15 times as long over 86 sizes, up to 1.7 (19882 x 32 x 2688 in
+  // five ranges 27.5 us, 16.2 in row blocks).  The constants of the width: fitted over 1200 sizes.
   const int steps = ((num_k + 3) / 4 + splits - 1) / splits * 4;
+  const bool tokens_forced = g_cfg_tokens == 2;
+  if (g_cfg_mode == 0 && g_cfg_tokens != 1 && (tokens_forced || (M >= kTokensMinRows && (N > 64 || M <= 1500)))) {
+    static constexpr TokenCost planes = {314, 37.8, 1.986, 1706, 8, 2056, 0.848, 0.947, 0};
+    double time = 0.0;
+    int bt = tokens_width(M, N, steps, splits, (ld_a | ld_w) % 64 == 0, planes, dev->sm_count, time);
+    if (tokens_forced && g_cfg_tile_n) bt = g_cfg_tile_n;
+    return launch_tokens<TOK_PLANES>(a, ld_a, w, ld_w, p, bt, dev->sm_count, reinterpret_cast<cudaStream_t>(stream));
+  }
+  // the row blocks' width: the one with the least waves x steps x clocks (as in run_gemm; an fp32 tile's epilogue and
+  // the prologue are 4000 a wave)
   auto cost = [&](int width, int clocks) {
     const int64_t units = (int64_t)p.num_m * ((N + width - 1) / width) * splits;
     return (units + dev->sm_count - 1) / dev->sm_count * ((int64_t)steps * clocks + 4000);
   };
-  int64_t least = cost(64, 385);
-  if (M > BM && N >= 256) {
-    const int64_t wide = cost(256, 720);
-    if (wide <= least) {
-      bn = 256;
-      least = wide;
-    }
-  }
-  if (g_cfg_mode == 0 && g_cfg_tokens != 1 && (M >= kTokensMinRows || g_cfg_tokens == 2)) {
-    static constexpr TokenCost planes = {314, 37.8, 1.986, 1706, 8, 2056, 0.848, 0.947, 0};
-    double time = 0.0;
-    int bt = tokens_width(M, N, steps, splits, (ld_a | ld_w) % 64 == 0, planes, dev->sm_count, time);
-    if (g_cfg_tokens == 2 && g_cfg_tile_n) bt = g_cfg_tile_n;
-    if (time < 1.331 * least + 1370 || g_cfg_tokens == 2)
-      return launch_tokens<TOK_PLANES>(a, ld_a, w, ld_w, p, bt, dev->sm_count, reinterpret_cast<cudaStream_t>(stream));
-  }
+  const int bn = M > BM && N >= 256 && cost(256, 720) <= cost(64, 385) ? 256 : 64;
   p.num_n = (N + bn - 1) / bn;
   p.num_k = num_k;
   p.num_tiles = p.num_m * p.num_n;

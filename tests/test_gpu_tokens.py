@@ -225,3 +225,22 @@ def test_short_raw_reductions(M, N, K, taken):
     family = ctypes.c_int(0)
     assert _lib.lib().iflb200_gemm_last_launch(ctypes.byref(family), None, None) == 0
     assert bool(family.value & 4) == taken
+
+
+@pytest.mark.parametrize("M,N,taken", [(19882, 32, False), (1501, 64, False), (1500, 64, True), (1501, 80, True), (65, 16, True)])
+def test_planes_of_few_columns(M, N, taken):
+    from instinctflash_b200 import _lib
+    from instinctflash_b200.kernels import fp8
+    _, a, w = operands(M, N, 2688)
+    out = torch.full((6, M, N), float("nan"), device=DEV)
+    fp8.gemm_partials(a, fp8.Fp8Weight(w, None, None), out[:5])
+    family = ctypes.c_int(0)
+    assert _lib.lib().iflb200_gemm_last_launch(ctypes.byref(family), None, None) == 0
+    assert bool(family.value & 4) == taken and family.value & 16
+    # row 5 * M of the planes is the guard's first; 21 slabs in five ranges of whole stages of four
+    assert torch.isnan(out[5]).all()
+    cuts = [512 * (6 * i // 5) for i in range(5)] + [2688]
+    for i in range(5):
+        want = a[:70, cuts[i]:cuts[i + 1]].double() @ w[:, cuts[i]:cuts[i + 1]].double().T
+        assert (out[i, :70].double() - want).norm() < 1e-5 * want.norm()
+    torch.cuda.synchronize()
