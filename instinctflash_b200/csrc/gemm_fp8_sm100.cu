@@ -667,8 +667,9 @@ __device__ __forceinline__ void epilogue_gated(const GemmParams& p, const CUtens
 // stack, a kernel that carries both code paths ran the stack 5 % slower than the two specialised
 // ones.  The 64-wide kernel exists in form 2, for what the lean kernel (gemm_lean.cuh) leaves out: residual and direct-store
 // epilogues, fewer than four K steps, a K split over a cluster that was asked for.
-// SPLIT 3: the planes form for more than 128 rows: (tile, K range) units on a persistent grid, each leaving
-// its fp32 partial sums in a plane; K is cut as in the skinny form, so the planes' bits are the same.
+// SPLIT 3: planes for more than 128 rows where the tokens form does not pay (up to 64 columns) or is forbidden: (tile, K
+// range) units on a persistent grid, each leaving its fp32 partial sums in a plane; K is cut as in the skinny form, so
+// the planes' bits are the same.
 // GATED: the gated form (see epilogue_gated): a tile pairs BN/2 gate columns with the BN/2 up
 // columns of the same hidden units; p.N counts hidden units.
 // EW: epilogue warps (8, or 16 for the gated form: EW / 4 per TMEM lane quadrant).
@@ -1117,11 +1118,10 @@ struct PairSmemLayout {
   static constexpr int kDynamic = kTotal + 1024;
 };
 
-// PLANES: (tile, K range) units as in the single-CTA kernel's planes form.
 // GATED: the gated form (see epilogue_gated).  The leader loads the gate rows of the tile's BN/2 hidden units,
 // its peer the up rows, so both accumulators hold BN/2 gate columns followed by their up columns; p.N counts
 // hidden units and EW is 16, as in the single-CTA kernel.
-template <int BN, int STAGES, int ACC, bool PLANES = false, bool GATED = false, int EW = kEpilogueWarps>
+template <int BN, int STAGES, int ACC, bool GATED = false, int EW = kEpilogueWarps>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(96 + 32 * EW, 1)
 gemm_fp8_tc5_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w,
                          const __grid_constant__ CUtensorMap tm_out, const GemmParams p) {
@@ -1150,16 +1150,6 @@ gemm_fp8_tc5_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
   const bool leader = rank == 0;
   const int pair_id = blockIdx.x >> 1;
   const int pair_stride = gridDim.x >> 1;
-  const int parts = PLANES ? p.partials : 1;
-  const int units = p.num_tiles * parts;
-  auto range_begin = [&](int part) { return PLANES ? (int)(((int64_t)((p.num_k + 3) / 4) * part) / parts) * 4 : 0; };
-  int kb0 = 0, kb1 = p.num_k;
-  auto enter_unit = [&](int unit) {
-    if constexpr (PLANES) {
-      kb0 = range_begin(unit % parts);
-      kb1 = min(p.num_k, range_begin(unit % parts + 1));
-    }
-  };
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -1196,13 +1186,12 @@ gemm_fp8_tc5_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
     Ring<STAGES> ring;
     bool ok = true;
     uint32_t it = 0;
-    for (int unit = pair_id; ok && unit < units; unit += pair_stride, ++it) {
+    for (int tile = pair_id; ok && tile < p.num_tiles; tile += pair_stride, ++it) {
       int m_blk, n_blk;
-      tile_coords(p, unit / parts, m_blk, n_blk);
-      enter_unit(unit);
+      tile_coords(p, tile, m_blk, n_blk);
       const int w_row = GATED ? n_blk * (BN / 2) + (int)rank * p.N : n_blk * BN + (int)rank * (BN / 2);
       const int row = w_producer ? w_row : m_blk * 2 * BM + (int)rank * BM;
-      for (int kb = kb0; kb < kb1; ++kb) {
+      for (int kb = 0; kb < p.num_k; ++kb) {
         ok = wait_bounded(empty_bar(ring.stage), ring.phase ^ 1, abort_flag, (1u << 24) | (1u << 16) | (it & 0xFFFF));
         if (!ok) break;
         if (elect_one()) {
@@ -1222,15 +1211,14 @@ gemm_fp8_tc5_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
       uint32_t phase = 0;
       bool ok = true;
       uint32_t it = 0;
-      for (int unit = pair_id; ok && unit < units; unit += pair_stride, ++it) {
-        enter_unit(unit);
+      for (int tile = pair_id; ok && tile < p.num_tiles; tile += pair_stride, ++it) {
         const uint32_t acc = (ACC == 2) ? (it & 1u) : 0u;
         const uint32_t acc_phase = (ACC == 2) ? ((it >> 1) & 1u) : (it & 1u);
         ok = wait_bounded(tempty_bar(acc), acc_phase ^ 1, abort_flag, (2u << 24) | (2u << 16) | (it & 0xFFFF));
         if (!ok) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * kAccStride;
-        for (int kb = kb0; kb < kb1; ++kb) {
+        for (int kb = 0; kb < p.num_k; ++kb) {
           ok = wait_bounded(full_bar(stage), phase, abort_flag, (2u << 24) | (3u << 16) | (it & 0xFFFF));
           if (!ok) break;
           tc_fence_after();
@@ -1240,7 +1228,7 @@ gemm_fp8_tc5_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
             const uint64_t db = make_kmajor_sw128_desc(sa + L::kABytes);
 #pragma unroll
             for (int j = 0; j < BK / 32; ++j)
-              mma_f8f6f4_pair(d_tmem, da + 2 * j, db + 2 * j, kIdesc, kb > kb0 || j > 0 ? 1u : 0u);
+              mma_f8f6f4_pair(d_tmem, da + 2 * j, db + 2 * j, kIdesc, kb > 0 || j > 0 ? 1u : 0u);
             mma_commit_pair(empty_bar(stage), 3);  // stage free in both CTAs
           }
           __syncwarp();
@@ -1270,10 +1258,9 @@ gemm_fp8_tc5_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
     bool ok = true;
     uint32_t it = 0;
     grid_dependency_wait();  // scales and residual operands may come from the kernel before this one
-    for (int unit = pair_id; ok && unit < units; unit += pair_stride, ++it) {
+    for (int tile = pair_id; ok && tile < p.num_tiles; tile += pair_stride, ++it) {
       int m_blk, n_blk;
-      tile_coords(p, unit / parts, m_blk, n_blk);
-      enter_unit(unit);
+      tile_coords(p, tile, m_blk, n_blk);
       const uint32_t acc = (ACC == 2) ? (it & 1u) : 0u;
       const uint32_t acc_phase = (ACC == 2) ? ((it >> 1) & 1u) : (it & 1u);
       const int m = m_blk * 2 * BM + (int)rank * BM + quad * 32 + lane;
@@ -1308,7 +1295,7 @@ gemm_fp8_tc5_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
       if (p.tma_store) {
         epilogue_tma_store<BN>(p, &tm_out, t_row, staging, staging_ptr,
                                m_blk * 2 * BM + (int)rank * BM + quad * 32, n_blk * BN, col_begin, col_end, rs, lane,
-                               PLANES ? unit % parts : -1, prefetch ? &cv : nullptr);
+                               -1, prefetch ? &cv : nullptr);
       } else {
 #pragma unroll 1
         for (int c = col_begin / 32; c < col_end / 32; ++c) {
@@ -1553,7 +1540,7 @@ static int launch_lean(const void* a, int64_t ld_a, const void* w, int64_t ld_w,
   return g.M <= 64 ? launch_lean_form<64, EPI>(ta, tw, p, grid, s) : launch_lean_form<128, EPI>(ta, tw, p, grid, s);
 }
 
-template <int BN, int STAGES, int ACC, bool PLANES = false, bool GATED = false, int EW = kEpilogueWarps>
+template <int BN, int STAGES, int ACC, bool GATED = false, int EW = kEpilogueWarps>
 static int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tw, const CUtensorMap& to,
                             const GemmParams& p, int grid, cudaStream_t s) {
   using L = PairSmemLayout<BN, STAGES>;
@@ -1561,12 +1548,12 @@ static int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tw, const 
   int dev = 0;
   cudaGetDevice(&dev);
   if (!attr_set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_fp8_tc5_pair_kernel<BN, STAGES, ACC, PLANES, GATED, EW>,
+    cudaError_t e = cudaFuncSetAttribute(gemm_fp8_tc5_pair_kernel<BN, STAGES, ACC, GATED, EW>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, L::kDynamic);
     if (e != cudaSuccess) return (int)e;
     attr_set[dev] = true;
   }
-  const cudaError_t e = launch_dep(gemm_fp8_tc5_pair_kernel<BN, STAGES, ACC, PLANES, GATED, EW>, dim3(grid), dim3(96 + 32 * EW),
+  const cudaError_t e = launch_dep(gemm_fp8_tc5_pair_kernel<BN, STAGES, ACC, GATED, EW>, dim3(grid), dim3(96 + 32 * EW),
                                    L::kDynamic, s, 1, dependent_launch_for(p.M), ta, tw, to, p);
   note_captured_gemm(s);
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
@@ -1951,13 +1938,7 @@ static int run_gemm_partials(const void* a, int64_t ld_a, const void* w, int64_t
     if (tokens_forced && g_cfg_tile_n) bt = g_cfg_tile_n;
     return launch_tokens<TOK_PLANES>(a, ld_a, w, ld_w, p, bt, dev->sm_count, reinterpret_cast<cudaStream_t>(stream));
   }
-  // the row blocks' width: the one with the least waves x steps x clocks (as in run_gemm; an fp32 tile's epilogue and
-  // the prologue are 4000 a wave)
-  auto cost = [&](int width, int clocks) {
-    const int64_t units = (int64_t)p.num_m * ((N + width - 1) / width) * splits;
-    return (units + dev->sm_count - 1) / dev->sm_count * ((int64_t)steps * clocks + 4000);
-  };
-  const int bn = M > BM && N >= 256 && cost(256, 720) <= cost(64, 385) ? 256 : 64;
+  constexpr int bn = 64;
   p.num_n = (N + bn - 1) / bn;
   p.num_k = num_k;
   p.num_tiles = p.num_m * p.num_n;
@@ -1972,29 +1953,14 @@ static int run_gemm_partials(const void* a, int64_t ld_a, const void* w, int64_t
     g_last_launch[0] = 1 + 16; g_last_launch[1] = 64; g_last_launch[2] = splits; g_last_launch[3] = 104;
     return launch_lean<LEAN_PLANES>(a, ld_a, w, ld_w, p, p.num_tiles * splits, s);
   }
-  // CTA pairs where blocks of 256 rows pad little and their units need no more waves: two thirds of the traffic per K step, which is what these launches wait for.
-  // 816 x 2048 x 16384 in two ranges 28.6 against 29.7 us, 640 rows in three 22.8 against 23.3.
-  const int pair_m = (M + 2 * BM - 1) / (2 * BM), sm_pairs = dev->sm_count / 2;
-  const int64_t pair_units = (int64_t)pair_m * p.num_n * splits, single_units = (int64_t)p.num_tiles * splits;
-  const int64_t pair_waves = (pair_units + sm_pairs - 1) / sm_pairs;
-  const int64_t single_waves = (single_units + dev->sm_count - 1) / dev->sm_count;
-  if (bn == 256 && g_cfg_mode != 1 && pair_m * 2 * BM * 4 <= M * 5 + 16 && pair_waves <= single_waves) {
-    st = make_tensor_map(&ta, a, M, K, ld_a, BM);
-    if (st != IFLB200_OK) return st;
-    st = make_tensor_map(&tw, w, N, K, ld_w, BM);
-    if (st != IFLB200_OK) return st;
-    p.num_m = pair_m;
-    p.num_tiles = p.num_m * p.num_n;
-    g_last_launch[0] = 3 + 16; g_last_launch[1] = bn; g_last_launch[2] = splits; g_last_launch[3] = 6;
-    return launch_gemm_pair<256, 6, 2, true>(ta, tw, to, p, 2 * (int)(pair_units < sm_pairs ? pair_units : sm_pairs), s);
-  }
   st = make_tensor_map(&ta, a, M, K, ld_a, a_rows);
   if (st != IFLB200_OK) return st;
   st = make_tensor_map(&tw, w, N, K, ld_w, bn);
   if (st != IFLB200_OK) return st;
-  const int grid = single_units < dev->sm_count ? (int)single_units : dev->sm_count;
+  const int64_t units = (int64_t)p.num_tiles * splits;
+  const int grid = units < dev->sm_count ? (int)units : dev->sm_count;
   g_last_launch[0] = 1 + 16; g_last_launch[1] = bn; g_last_launch[2] = splits; g_last_launch[3] = 0;
-  return bn == 64 ? launch_gemm_form<64, 8, 3>(ta, tw, to, p, grid, s) : launch_gemm_form<256, 4, 3>(ta, tw, to, p, grid, s);
+  return launch_gemm_form<64, 8, 3>(ta, tw, to, p, grid, s);
 }
 
 // Row blocks to several destinations: a holds `groups` blocks of `group_rows` rows; block g's
@@ -2135,7 +2101,7 @@ static int run_gemm_gated(const void* a, int64_t ld_a, const void* w, int64_t ld
     st = make_out_map(&to, h, M, F, ld_h, 4, 64);
     if (st != IFLB200_OK) return st;
     g_last_launch[0] = 3 + 8; g_last_launch[1] = 256; g_last_launch[2] = 1; g_last_launch[3] = 6;
-    return launch_gemm_pair<256, 6, 2, false, true, 16>(ta, tw, to, p, 2 * (p.num_tiles < pairs ? p.num_tiles : pairs),
+    return launch_gemm_pair<256, 6, 2, true, 16>(ta, tw, to, p, 2 * (p.num_tiles < pairs ? p.num_tiles : pairs),
                                                               reinterpret_cast<cudaStream_t>(stream));
   }
   p.num_n = (F + bn / 2 - 1) / (bn / 2);
