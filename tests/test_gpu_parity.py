@@ -350,9 +350,10 @@ def test_gemm_odd_tile_widths_all_epilogues(ops, unsplit, tile_n, out_dtype):
 
 @pytest.mark.parametrize("M,N,K", [(816, 1040, 512), (300, 640, 256), (1000, 2048, 384), (512, 256, 128), (257, 144, 2048),
                                    (816, 8192, 256), (600, 20480, 128)])
-def test_gemm_swapped_form_is_bit_identical(ops, unsplit, M, N, K):
+def test_gemm_tokens_form_is_bit_identical(ops, unsplit, M, N, K):
     """A few hundred tokens: tokens on the MMA's N side, tile stored transposed.  Same K loop, so
-    the raw accumulator and the dequantised outputs equal the ordinary form bit for bit."""
+    the raw accumulator and the dequantised outputs equal the ordinary form bit for bit.  Mode bit 512 is reserved:
+    accepted, and without effect."""
     fp8, lib = ops["fp8"], ops["lib"]
     g = torch.Generator().manual_seed(M + N + K)
     a = dev((torch.randn(M, K, generator=g) * 60).clamp(-448, 448).to(E4M3))
@@ -360,23 +361,26 @@ def test_gemm_swapped_form_is_bit_identical(ops, unsplit, M, N, K):
     s = dev(cases.vector(M, 911, lo=0.001, hi=0.02))
     W = fp8.Fp8Weight(w, dev(cases.vector(N, 912, lo=0.0001, hi=0.001)), dev(cases.vector(N, 913, sigma=0.05)))
 
-    def run():
+    def run(tokens):
+        def done(out):
+            assert bool(last_launch(ops)[0] & 4) == tokens
+            return out
         raw = torch.full((M, N), float("nan"), device=DEV, dtype=torch.bfloat16)
-        fp8.gemm(a, W, raw)
+        done(fp8.gemm(a, W, raw))
         y16 = torch.full((M, N), float("nan"), device=DEV, dtype=torch.float16)
-        fp8.fp8_linear(a, s, W, y16)
+        done(fp8.fp8_linear(a, s, W, y16))
         ybf = torch.full((M, N), float("nan"), device=DEV, dtype=torch.bfloat16)
-        fp8.fp8_linear(a, s, W, ybf, exact=True)
+        done(fp8.fp8_linear(a, s, W, ybf, exact=True))
         view = torch.full((M, N + 48), float("nan"), device=DEV, dtype=torch.bfloat16)
-        fp8.gemm(a, W, view[:, 16:16 + N])            # a strided output view
+        done(fp8.gemm(a, W, view[:, 16:16 + N]))      # a strided output view
         return raw, y16, ybf, view
     try:
-        assert lib.iflb200_gemm_set_mode(128) == 0     # never swapped
-        want = run()
+        assert lib.iflb200_gemm_set_mode(128) == 0     # never the tokens form
+        want = run(False)
         results = []
-        for mode in (256, 256 + 512):                  # swapped wherever the form exists: CTA pairs, single CTAs
+        for mode in (256, 256 + 512):                  # wherever the form exists
             assert lib.iflb200_gemm_set_mode(mode) == 0
-            results.append(run())
+            results.append(run(True))
     finally:
         lib.iflb200_gemm_set_mode(0)
     for got in results:
