@@ -87,6 +87,32 @@ def test_residual_norm_rows(M, D, delta, gate, affine):
     assert steps.max().item() <= 1 and (steps != 0).float().mean().item() < 2e-3
 
 
+# 1777 rows of 3072 take two turns of seven groups on 768 threads, the first 1480 of them two of five on 640: the same
+# threads own a row, so its bits are the same
+@pytest.mark.parametrize("gate", [False, True])
+def test_residual_norm_rows_on_more_groups(gate):
+    from instinctflash_b200.kernels import norm
+    M, few, D = 1777, 1480, 3072
+    g = torch.Generator(device=DEV).manual_seed(D)
+
+    def randn(*shape, scale=1.0):
+        return torch.randn(*shape, device=DEV, generator=g) * scale
+
+    res, delta, row = randn(M, D).to(torch.bfloat16), randn(M, D, scale=100.0).to(torch.bfloat16), torch.rand(M, device=DEV, generator=g) * 0.02
+    kw = {"delta_col": randn(D), "bias": randn(D), "mod_scale": randn(D, scale=0.2), "mod_shift": randn(D, scale=0.2)}
+    if gate:
+        kw["gate"] = randn(D)
+    outs = []
+    for rows in (M, few):
+        r, q, s = res[:rows].clone(), torch.full((rows, D + 8), 1.0, device=DEV).to(E4M3), torch.full((rows,), -1.0, device=DEV)
+        norm.residual_norm_quant(r, delta=delta[:rows], delta_row=row[:rows], layernorm=True, q=q[:, :D], q_scale=s, **kw)
+        outs.append((r, u8(q), i32(s)))
+    torch.cuda.synchronize()
+    for all_rows, first_rows in zip(*outs):
+        assert torch.equal(all_rows[:few], first_rows)
+    assert (outs[0][2][few:] > 0).all() and (outs[0][1][:, D:] == 0x38).all()
+
+
 # heads narrower than a thread's stride (its chunks lie at different pairs), one part only, no norm, pool slots
 @pytest.mark.parametrize("B,T,H,HD,parts,norm,dtype", [(2, 700, 24, 128, 3, True, torch.float16), (1, 1801, 9, 120, 3, False, torch.bfloat16),
                                                        (1, 1900, 12, 128, 1, True, torch.bfloat16), (1, 593, 40, 128, 3, True, torch.float16)])
