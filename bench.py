@@ -985,10 +985,11 @@ def main():
     reps = max(args.steps, 10)
     for lw in weights[:3]:
         dom_call(lw.w[name])
-    family = ctypes.c_int(0)
-    _lib.lib().iflb200_gemm_last_launch(ctypes.byref(family), None, None)
+    family, tile = ctypes.c_int(0), ctypes.c_int(0)
+    _lib.lib().iflb200_gemm_last_launch(ctypes.byref(family), ctypes.byref(tile), None)
+    # the skinny kernel runs every plain 64-wide tile over at least four K slabs
     kernel_name = ("gemm_fp8_tc5_tokens_kernel" if family.value & 4 else "gemm_fp8_tc5_pair_kernel" if family.value & 3 > 1
-                   else "gemm_fp8_tc5_lean_kernel" if spec.M <= 64 else "gemm_fp8_tc5_kernel") + \
+                   else "gemm_fp8_tc5_lean_kernel" if family.value == 1 and tile.value == 64 and k_dom > 384 else "gemm_fp8_tc5_kernel") + \
         f"{' (gated epilogue)' if gated_dom else ''} {spec.M}x{n_dom}x{k_dom} ({name})"
     torch.cuda.synchronize(dev)
     g0, g1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)

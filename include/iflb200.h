@@ -528,11 +528,12 @@ IFLB200_API int iflb200_set_dependent_launch(int enable);
  * (cta_group::2) with one / two tensor-memory accumulators; add 16 to store the epilogue
  * straight from registers instead of through shared memory and TMA; add 256 to take the
  * tokens form (tokens on the MMA's N side; raw, dequantised, partial-sum and gated outputs) wherever it
- * exists, in tiles of tile_n tokens if that is set, 128 to forbid it (512, once its single-CTA variant,
- * changes nothing); add 1024 / 2048 to run the gated form's 256-wide tiles with sixteen / eight
- * epilogue warps; add 4096 to keep the skinny-regime kernel on one K slab per TMA instruction.
- * Any other bit is refused.  Every mode writes the same output bits.  For
- * experiments and tests.  No reference counterpart. */
+ * exists, in tiles of tile_n tokens if that is set, 128 to forbid it (512 is reserved: accepted, without
+ * effect); a K split over a cluster that iflb200_gemm_set_split_k asks for stands above it; add 1024 / 2048
+ * to run the gated form's 256-wide tiles with sixteen / eight epilogue warps; add 4096 to keep the
+ * skinny-regime kernel on one K slab per TMA instruction.  Any other bit is refused.  Modes write the
+ * same output bits for the same K split: 0 and 128 always do, every one after
+ * iflb200_gemm_set_split_k(1).  For experiments and tests.  No reference counterpart. */
 IFLB200_API int iflb200_gemm_set_mode(int mode);
 
 #ifdef __cplusplus

@@ -130,7 +130,7 @@ struct SmemLayout {
   static constexpr int kBBytes = BN * BK * SL;
   static constexpr int kStageBytes = kABytes + kBBytes;
   // epilogue staging: one 32-row buffer per epilogue warp (TMA-store source), 128 bytes per row
-  // with eight epilogue warps, 64 with sixteen; a warp of the 64-row form has 16 rows
+  // with eight epilogue warps, 64 with sixteen
   static constexpr int kWarpStaging = EW > 8 ? 2048 : 4096;
   static constexpr int kStagingOffset = STAGES * kStageBytes;
   static constexpr int kBarOffset = kStagingOffset + EW * kWarpStaging;
@@ -466,7 +466,7 @@ __device__ __forceinline__ void stage_columns(const GemmParams& p, const uint32_
 #pragma unroll
     for (int j = 0; j < 8; ++j)
       *reinterpret_cast<float4*>(mine + ((j ^ (lane & 7)) * 16)) =
-            make_float4(y[4 * j + 0], y[4 * j + 1], y[4 * j + 2], y[4 * j + 3]);
+          make_float4(y[4 * j + 0], y[4 * j + 1], y[4 * j + 2], y[4 * j + 3]);
   }
 }
 
@@ -1614,7 +1614,8 @@ static int launch_tokens(const void* a, int64_t ld_a, const void* w, int64_t ld_
   p.plane = p.ld_out * g.M;
   p.act = g.act;
   // 32 MB of weights and more would push h, which the quantiser pass reads next, and one another's boxes out of L2:
-  // 816 x 2 x 16384 x 2048 50.7 -> 49.1 us, with the pass behind it 58.3 -> 55.9
+  // 816 x 2 x 16384 x 2048 50.7 -> 49.1 us, with the pass behind it 58.3 -> 55.9.  Over 70 sizes (66 to 2850 tokens, 4352 to
+  // 16128 hidden units, 32 to 144 MB) GEMM and pass took 0.94 to 1.01 of the time without the policy, 0.984 on average
   p.evict = EPI == TOK_GATED && (int64_t)g.N * g.K > (16ll << 20);
   p.amax = g.amax;
   CUtensorMap tt, tw;
@@ -1632,11 +1633,12 @@ static int launch_tokens(const void* a, int64_t ld_a, const void* w, int64_t ld_
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
 
-// Estimated time of the tokens form, in the units of the costs it is compared with (each set of constants belongs to one
-// comparison): a slab takes at least `floor` clocks (commit and barriers) and `slab` + `slab_token` a token of the tile
-// (rows through the L2 port), times `ragged` where rows are off 64-byte boundaries; a tile's epilogue `tile` +
-// `tile_token` a token; a partly filled last wave counts 1 - `whole` of its share; a single wave of more than 7 in 8 of
-// the pairs waits `full` for the last SMs of the kernel before it (333 x 2560 x 2048 behind its pack: 70 pairs 13.1 us, 60
+// Estimated time of the tokens form, in the units of the costs it is compared with: a slab takes at least `floor` clocks and
+// `slab` + `slab_token` a token of the tile, times `ragged` where rows are off 64-byte boundaries; a tile's epilogue `tile` +
+// `tile_token` a token; a partly filled last wave counts 1 - `whole` of its share.  The names say where a constant enters,
+// not what was measured of the kernel: each set was fitted by itself to the sizes where this form and the others cross, and
+// takes up what is off in the costs on the other side (a `ragged` below 1: they charge such rows too little).  A single
+// wave of more than 7 in 8 of the pairs waits `full` for the last SMs of the kernel before it (333 x 2560 x 2048 behind its pack: 70 pairs 13.1 us, 60
 // pairs 11.6).
 struct TokenCost {
   double floor, slab, slab_token, tile, tile_token, ends, whole, ragged, full;
@@ -1772,9 +1774,10 @@ static int run_gemm(const void* a, int64_t ld_a, const void* w, int64_t ld_w, Ge
       if (pair) best = cost;
     }
     // Tokens on the MMA's N side, where the tile's width fits the tokens (see gemm_tokens.cuh).  The constants are the ones
-    // whose choice is closest to the fastest form over 700 raw sizes one after the other and 900 dequantised ones
-    // behind their quantiser (65 to 16384 rows, 256 to 15360 columns, K 512 to 14336): 1.3 and 0.6 % slower than it on
-    // average, the calls 10 and 14 % faster than without the form, 25 and 15 of them more than 3 % slower.
+    // whose choice was closest to the fastest form over 700 raw sizes one after the other and 900 dequantised ones
+    // behind their quantiser (65 to 16384 rows, 256 to 15360 columns, K 512 to 14336).  With the rules below, over 796 raw
+    // and 804 dequantised other sizes of these ranges (to 8192 rows): 10 and 16 % less time than without the form, eight and one of
+    // them more than 3 % slower.
     // Where the choice above is the pair kernel, a tile of 256 tokens is the same tile: only a narrower one that saves
     // 3 % of it is taken, or with scales, whose epilogue takes longer in the pair kernel, over fewer than 32 K steps any.
     // A reduction that the choice above splits over a cluster stays split, whatever its time: the number of ranges is part
@@ -2166,7 +2169,7 @@ extern "C" int iflb200_gemm_set_mode(int mode) {
     return IFLB200_ERR_ARG;
   g_cfg_gated_warps = (mode & 1024) ? 16 : ((mode & 2048) ? 8 : 0);
   g_cfg_slabs = (mode & 4096) ? 1 : 0;
-  g_cfg_tokens = (mode & 128) ? 1 : ((mode & 256) ? 2 : 0);  // 128: never the tokens form, 256: wherever it exists (512, once its single-CTA variant, changes nothing)
+  g_cfg_tokens = (mode & 128) ? 1 : ((mode & 256) ? 2 : 0);  // 128: never the tokens form, 256: wherever it exists (512: reserved, without effect)
   g_cfg_mode = family;
   g_cfg_direct_store = (mode & 16) ? 1 : 0;
   return IFLB200_OK;

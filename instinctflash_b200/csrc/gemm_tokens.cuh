@@ -510,9 +510,10 @@ gemm_fp8_tc5_tokens_kernel(const __grid_constant__ CUtensorMap tm_t, const __gri
   }
 
   // Neither CTA leaves while its peer can still reach its shared or tensor memory: the leader's MMAs read and write the
-  // peer's until the last accumulator is complete, and every remote arrival has been waited for by then.  The barrier
-  // orders no data, so that it need not wait for the stores above.  After a timed-out wait the loads in flight get
-  // time to land.
+  // peer's until the last accumulator is complete, which both CTAs' epilogue warps have waited for.  Arrivals that free an
+  // accumulator have been waited for by then too; those of the last ring turn on the `empty` barriers, which nothing waits
+  // for, were committed ahead of that accumulator.  The barrier orders no data, so that it need not wait for the stores
+  // above.  After a timed-out wait the loads in flight get time to land.
   if (*abort_flag) {
     for (int i = 0; i < 64; ++i) __nanosleep(1000);
   }
