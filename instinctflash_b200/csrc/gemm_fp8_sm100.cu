@@ -1867,8 +1867,8 @@ static int run_gemm(const void* a, int64_t ld_a, const void* w, int64_t ld_w, Ge
   if (bn == 64 && g_cfg_slabs != 1 && p.num_k / split >= 4 && stages == 0) {
     if (split == 1 && p.tma_store) {
       g_last_launch[3] = 104;
-      return p.epilogue == EPI_RAW ? launch_lean<LEAN_RAW>(a, ld_a, w, ld_w, p, grid, s)
-                                   : launch_lean<LEAN_DEQUANT>(a, ld_a, w, ld_w, p, grid, s);
+      if (p.epilogue == EPI_RAW) return launch_lean<LEAN_RAW>(a, ld_a, w, ld_w, p, grid, s);
+      return oes == 4 ? launch_lean<LEAN_F32>(a, ld_a, w, ld_w, p, grid, s) : launch_lean<LEAN_DEQUANT>(a, ld_a, w, ld_w, p, grid, s);
     }
     CUtensorMap sa_map, sw_map;
     if (p.K % BK == 0 && make_slab_map(&sa_map, a, p.M, p.K, ld_a, a_rows, 4) == IFLB200_OK &&

@@ -4,7 +4,7 @@
 // A launch over 50 rows takes 3 to 5 us, most of it latencies in a row: the kernel before it, first operands, MMAs,
 // epilogue, completion.  It fetches its instructions cold, so the kernel holds nothing that such a launch does not run:
 // the output kind is a template argument, and a lane stores its row straight from registers (6 KB a tile are not worth
-// staging).  With one epilogue for all output kinds, through shared memory and TMA, the last store of a 64 x 4096 x 1024
+// staging; fp32 rows of many tiles are).  With one epilogue for all output kinds, through shared memory and TMA, the last store of a 64 x 4096 x 1024
 // launch was issued 2600 clocks after its last MMA; 18 expert layers over 50 rows (72 such launches) took 476 us, 417 now.
 // Four K slabs of 128 bytes a stage come with one TMA instruction per operand; up to 64 rows the MMAs are 64 rows high
 // (38 clocks each for 48), and row i of the accumulator lies in lane i % 16 of quadrant i / 16.
@@ -12,7 +12,7 @@
 
 namespace iflb200 {
 
-enum : int { LEAN_RAW = 0, LEAN_DEQUANT = 1, LEAN_PLANES = 2 };
+enum : int { LEAN_RAW = 0, LEAN_DEQUANT = 1, LEAN_PLANES = 2, LEAN_F32 = 3 };  // LEAN_F32: dequantised, fp32 output
 
 // The lean form's arguments: K need not be a multiple of 128.  Stages of whole slabs come through the slab maps
 // (K / 128 slabs); the stage that holds the ragged slab comes slab by slab through these, which read
@@ -26,7 +26,9 @@ template <int AR>
 struct LeanLayout {
   static constexpr int kSlabs = 4, kTile = 64, kStages = AR == 64 ? 3 : 2;
   static constexpr int kABytes = AR * BK * kSlabs, kWBytes = kTile * BK * kSlabs, kStageBytes = kABytes + kWBytes;
-  static constexpr int kBarOffset = kStages * kStageBytes;
+  // fp32 rows of the 128-row form on their way to memory, 32 x 128 bytes a warp
+  static constexpr int kStagingOffset = kStages * kStageBytes, kStaging = AR == 128 ? 4096 : 0;
+  static constexpr int kBarOffset = kStagingOffset + 8 * kStaging;
   static constexpr int kDynamic = kBarOffset + (2 * kStages + 4) * 8 + 16 + 1024;
   static constexpr int kThreads = 32 * 11;  // W producer, MMA, eight epilogue warps, A producer
 };
@@ -37,6 +39,7 @@ gemm_fp8_tc5_lean_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
                          const __grid_constant__ LeanParams p) {
   using L = LeanLayout<AR>;
   constexpr int SL = L::kSlabs, BN = L::kTile, STAGES = L::kStages, quad_rows = AR / 4;
+  constexpr bool kDequant = EPI == LEAN_DEQUANT || EPI == LEAN_F32, kWide = EPI == LEAN_PLANES || EPI == LEAN_F32;
   constexpr uint32_t kTmemCols = 2 * BN;
   constexpr uint32_t kIdesc = make_idesc_e4m3_f32(AR, BN);
   extern __shared__ uint8_t smem_raw[];
@@ -180,7 +183,7 @@ gemm_fp8_tc5_lean_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
       // this tile's scales and bias, fetched under the main loop: lane l holds column n0 + l; what is absent is a factor
       // of 1 or an addend of -0
       float rs = 1.0f, cs = 1.0f, bs = -0.0f;
-      if constexpr (EPI == LEAN_DEQUANT) {
+      if constexpr (kDequant) {
         if (row_ok && p.row) rs = __ldg(p.row + (int64_t)m * p.row_stride);
         if (n0 + lane < p.N) {
           if (p.col) cs = __ldg(p.col + (int64_t)(n0 + lane) * p.col_stride);
@@ -198,7 +201,7 @@ gemm_fp8_tc5_lean_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(tempty_bar(acc));
-      if constexpr (EPI == LEAN_DEQUANT) {
+      if constexpr (kDequant) {
 #pragma unroll
         for (int i = 0; i < 32; i += 2) {
           float a = __uint_as_float(r[i]), b = __uint_as_float(r[i + 1]);
@@ -221,8 +224,25 @@ gemm_fp8_tc5_lean_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
         }
       }
       const int valid = row_ok ? min(32, p.N - n0) : 0;  // a multiple of 16, or not positive
-      const bool wide = EPI == LEAN_PLANES || (EPI == LEAN_DEQUANT && p.out_dtype == IFLB200_F32);
-      if (wide) {
+      if constexpr (EPI == LEAN_F32 && AR == 128) {
+        // Many tiles of fp32 are bound by their stores, so whole 128-byte pieces of four rows leave at a time, through shared
+        // memory (16-byte pieces swizzled by the row): 0.93 of the time of 16 bytes of 32 rows over 261 sizes
+        // (1946 x 224 x 1744 8.7 -> 7.1 us); 16 columns, half of a piece, 1.05.
+        const uint32_t mine = base + L::kStagingOffset + (uint32_t)(warp - 2) * L::kStaging;
+        __syncwarp();  // the rows of the tile before this one have been read
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          st_shared_v4(mine + lane * 128 + ((j ^ (lane & 7)) << 4), make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]));
+        __syncwarp();
+        const int row0 = m_blk * BM + quad * 32, piece = lane & 7;
+        float* o = reinterpret_cast<float*>(p.out) + (int64_t)row0 * p.ld_out + n0 + 4 * piece;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int t = 4 * i + (lane >> 3);
+          const uint4 v = ld_shared_v4(mine + t * 128 + ((piece ^ (t & 7)) << 4));
+          if (row0 + t < p.M && n0 + 4 * piece < p.N) *reinterpret_cast<uint4*>(o + (int64_t)t * p.ld_out) = v;
+        }
+      } else if constexpr (kWide) {
         float* o = reinterpret_cast<float*>(p.out) + ((EPI == LEAN_PLANES ? (int64_t)part * p.M : 0) + m) * p.ld_out + n0;
 #pragma unroll
         for (int j = 0; j < 8; ++j)

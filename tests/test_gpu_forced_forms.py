@@ -74,3 +74,33 @@ def test_fused_linear_keeps_the_unsplit_bits(M, N, K):
             lib.iflb200_gemm_set_config(0, 0, 0)
             lib.iflb200_gemm_set_split_k(0)
     assert torch.equal(*outs)
+
+
+# fp32 outputs of the skinny kernel over one row block and several, against the kernel with one K slab a load: last rows in
+# each quadrant of a block, columns that end inside a warp's 32, several tiles for a CTA, no scales and all of them
+@pytest.mark.parametrize("M,N,K", [(65, 16, 512), (100, 208, 640), (129, 80, 640), (300, 48, 1040), (477, 144, 784), (2100, 720, 512)])
+@pytest.mark.parametrize("exact", [False, True])
+def test_skinny_fp32_rows(M, N, K, exact):
+    from instinctflash_b200 import _lib
+    from instinctflash_b200.kernels import fp8
+    lib = _lib.lib()
+    g = torch.Generator(device=DEV).manual_seed(M)
+    a, w = (torch.randn(n, K, device=DEV, generator=g).to(E4M3) for n in (M, N))
+    s, c, b = (torch.rand(n, device=DEV, generator=g) for n in (M, N, N))
+    outs, tile = [], ctypes.c_int(0)
+    try:
+        assert lib.iflb200_gemm_set_config(64, 0, 0) == 0 and lib.iflb200_gemm_set_split_k(1) == 0
+        for mode in (128, 128 + 4096):
+            assert lib.iflb200_gemm_set_mode(mode) == 0
+            for row, weight in ((s, fp8.Fp8Weight(w, c, b)), (None, fp8.Fp8Weight(w, None, None))):
+                outs.append(torch.full((M + 2, N + 48), float("nan"), device=DEV))
+                fp8.fp8_linear(a, row, weight, outs[-1][:M, 16:16 + N], exact=exact)
+                assert lib.iflb200_gemm_last_launch(None, ctypes.byref(tile), None) == 0 and tile.value == 64
+    finally:
+        lib.iflb200_gemm_set_mode(0)
+        lib.iflb200_gemm_set_config(0, 0, 0)
+        lib.iflb200_gemm_set_split_k(0)
+    torch.cuda.synchronize()
+    for skinny, general in zip(outs[:2], outs[2:]):
+        assert not torch.isnan(skinny[:M, 16:16 + N]).any()
+        assert torch.equal(skinny.view(torch.int32), general.view(torch.int32))   # guard rows and columns included
