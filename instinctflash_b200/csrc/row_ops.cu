@@ -134,6 +134,14 @@ __device__ __forceinline__ void unpack(const Raw8<float>& r, float (&o)[8]) {
 }
 // float32 vector operand (scales, bias, gates, norm weights) for one chunk.
 template <bool FAST>
+// Two elements of a 16-bit type as a packed pair.
+__device__ __forceinline__ uint64_t widen2(uint32_t w, __nv_bfloat16) {
+  return pack2(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u));
+}
+__device__ __forceinline__ uint64_t widen2(uint32_t w, __half) {
+  const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w));
+  return pack2(f.x, f.y);
+}
 __device__ __forceinline__ void load_f32(const float* p, int c0, int width, float (&o)[8]) {
   if (FAST) {
     unpack(raw_load<float>(p + c0), o);
@@ -474,6 +482,72 @@ gated_act_quant_kernel(const GatedArgs a) {
 
 // --------------------------------------------------------------------------------------------
 // dequant_rows: 2D in + out bytes per row; flat, one chunk per thread.
+// The same for few rows (a skinny decoder layer: 50 x 4096): no bytes to speak of, a launch is round trips to L2 and the
+// instructions of one row, fetched cold.  So a row has a thread for every four columns (eight, sixteen beyond 4096, 8192), every
+// load -- gate, up, their column scales, the row scale -- is issued before the first use, and the code is one
+// activation's: 50 x 4096 2.45 -> 1.92 us behind one another, 18 expert layers 418 -> 403; over 50 sizes and both
+// activations 0.79 of the time.  Two or four CTAs a row as a cluster took 0.4 us longer than one.
+constexpr int kGatedFewThreads = 1024;
+
+template <typename XT, int ACT, int Q>
+__global__ void __launch_bounds__(kGatedFewThreads) gated_act_quant_few_kernel(const GatedArgs a) {
+  __shared__ float red[kGatedFewThreads / 32];
+  row_begin(a.early);  // inputs may come from the kernel before this one in the stream
+  const int m = blockIdx.x, step = blockDim.x * 4, c0 = threadIdx.x * 4;
+  const XT* gr = reinterpret_cast<const XT*>(a.gu) + (int64_t)m * a.ld_gu + c0;
+  uint2 rg[Q], ru[Q];
+  float4 cg[Q], cu[Q];
+#pragma unroll
+  for (int i = 0; i < Q; ++i) {
+    cg[i] = cu[i] = make_float4(1.0f, 1.0f, 1.0f, 1.0f);  // an absent scale is a factor of 1
+    rg[i] = ru[i] = make_uint2(0u, 0u);
+    if (c0 + i * step < a.F) {
+      rg[i] = *reinterpret_cast<const uint2*>(gr + i * step);
+      ru[i] = *reinterpret_cast<const uint2*>(gr + a.F + i * step);
+      if (a.col) {
+        cg[i] = *reinterpret_cast<const float4*>(a.col + c0 + i * step);
+        cu[i] = *reinterpret_cast<const float4*>(a.col + a.F + c0 + i * step);
+      }
+    }
+  }
+  const float rs = a.row ? a.row[m] : 1.0f;
+  const uint64_t rs2 = pack2(rs, rs);
+  float h[Q][4], amax = 0.0f;
+#pragma unroll
+  for (int i = 0; i < Q; ++i) {
+    uint64_t g[2] = {widen2(rg[i].x, XT()), widen2(rg[i].y, XT())}, u[2] = {widen2(ru[i].x, XT()), widen2(ru[i].y, XT())};
+    g[0] = mul2(mul2(g[0], rs2), pack2(cg[i].x, cg[i].y));
+    g[1] = mul2(mul2(g[1], rs2), pack2(cg[i].z, cg[i].w));
+    u[0] = mul2(mul2(u[0], rs2), pack2(cu[i].x, cu[i].y));
+    u[1] = mul2(mul2(u[1], rs2), pack2(cu[i].z, cu[i].w));
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      if (ACT == IFLB200_ACT_GELU_TANH) {
+        g[j] = gelu_tanh_ref2(g[j]);
+      } else {
+        float x, y;
+        unpack2(g[j], x, y);
+        g[j] = pack2(silu_ref(x), silu_ref(y));
+      }
+      unpack2(mul2(u[j], g[j]), h[i][2 * j], h[i][2 * j + 1]);
+    }
+    if (c0 + i * step < a.F) amax = max_abs_f32(max_abs_f32(amax, h[i][0], h[i][1]), h[i][2], h[i][3]);
+  }
+  amax = warp_max_abs_f32(amax);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = amax;
+  __syncthreads();
+  amax = warp_max_abs_f32((threadIdx.x & 31) < blockDim.x / 32 ? red[threadIdx.x & 31] : 0.0f);
+  float scale, inv;
+  quant_scales(amax, scale, inv);
+  if (threadIdx.x == 0) a.qs[m] = scale;
+  uint8_t* q = a.q + (int64_t)m * a.ld_q + c0;
+#pragma unroll
+  for (int i = 0; i < Q; ++i)
+    if (c0 + i * step < a.F)
+      *reinterpret_cast<uint32_t*>(q + i * step) =
+          cvt_e4m3x4(__fmul_rn(h[i][0], inv), __fmul_rn(h[i][1], inv), __fmul_rn(h[i][2], inv), __fmul_rn(h[i][3], inv));
+}
+
 // --------------------------------------------------------------------------------------------
 struct DequantArgs {
   const void* x;
@@ -1275,6 +1349,26 @@ static void launch_resnorm(ResNormArgs a, bool fast, cudaStream_t s) {
   }
   a.iters = g.iters;
   dispatch_geom(g, [&](auto tpr, auto it) {
+  if constexpr (sizeof(XT) == 2) {
+    // A CTA for every row at once: while each has an SM of its own, and up to three an SM for rows that are one or two quads a
+    // thread.  us behind one another, this form against groups of 256 threads: 50 x 4096 1.92 / 2.45, 148 x 512 1.38 / 1.84, 148 x
+    // 8192 2.74 / 3.87, 148 x 16384 4.21 / 5.94, 444 x 4096 3.78 / 3.83, 444 x 5120 4.18 / 4.61; beyond, 200 x 8192 4.51 / 4.29, 600 x
+    // 4096 5.29 / 4.86.
+    const int sms = device_sm_count() > 0 ? device_sm_count() : 148, q = (a.F + 4 * kGatedFewThreads - 1) / (4 * kGatedFewThreads);
+    if (g_row_tpr_override == 0 && (a.M <= sms || (a.F <= 5120 && a.M <= 3 * sms))) {
+      auto few = [&](auto quads) {
+        constexpr int Q = decltype(quads)::value;
+        const int threads = ((a.F / 4 + Q - 1) / Q + 31) / 32 * 32;
+        const bool gelu = a.act == IFLB200_ACT_GELU_TANH;
+        launch_dep(gelu ? gated_act_quant_few_kernel<XT, IFLB200_ACT_GELU_TANH, Q> : gated_act_quant_few_kernel<XT, IFLB200_ACT_SILU, Q>,
+                   dim3(a.M), dim3(threads), 0, s, 1, dependent_launch_for(a.M), a);
+      };
+      if (q <= 1) few(IntTag<1>{});
+      else if (q <= 2) few(IntTag<2>{});
+      else few(IntTag<4>{});
+      return;
+    }
+  }
     constexpr int TPR = decltype(tpr)::value, IT = decltype(it)::value;
     const int grid = (a.M + kRowThreads / TPR - 1) / (kRowThreads / TPR);
     launch_dep(residual_norm_quant_kernel<RT, TPR, IT, true>, dim3(grid), dim3(kRowThreads), 0, s, 1, dependent_launch_for(a.M), a);
