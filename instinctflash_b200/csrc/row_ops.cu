@@ -4,6 +4,8 @@
 // stored 8 at a time.  All of them are HBM-bound: bytes per row are in the comments.
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "../../include/iflb200.h"
 #include "launch.cuh"
 #include "row_stream.cuh"
@@ -132,8 +134,6 @@ __device__ __forceinline__ void unpack(const Raw8<float>& r, float (&o)[8]) {
   o[0] = r.a.x; o[1] = r.a.y; o[2] = r.a.z; o[3] = r.a.w;
   o[4] = r.b.x; o[5] = r.b.y; o[6] = r.b.z; o[7] = r.b.w;
 }
-// float32 vector operand (scales, bias, gates, norm weights) for one chunk.
-template <bool FAST>
 // Two elements of a 16-bit type as a packed pair.
 __device__ __forceinline__ uint64_t widen2(uint32_t w, __nv_bfloat16) {
   return pack2(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u));
@@ -142,6 +142,8 @@ __device__ __forceinline__ uint64_t widen2(uint32_t w, __half) {
   const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w));
   return pack2(f.x, f.y);
 }
+// float32 vector operand (scales, bias, gates, norm weights) for one chunk.
+template <bool FAST>
 __device__ __forceinline__ void load_f32(const float* p, int c0, int width, float (&o)[8]) {
   if (FAST) {
     unpack(raw_load<float>(p + c0), o);
@@ -480,8 +482,6 @@ gated_act_quant_kernel(const GatedArgs a) {
   }
 }
 
-// --------------------------------------------------------------------------------------------
-// dequant_rows: 2D in + out bytes per row; flat, one chunk per thread.
 // The same for few rows (a skinny decoder layer: 50 x 4096): no bytes to speak of, a launch is round trips to L2 and the
 // instructions of one row, fetched cold.  So a row has a thread for every four columns (eight, sixteen beyond 4096, 8192), every
 // load -- gate, up, their column scales, the row scale -- is issued before the first use, and the code is one
@@ -548,6 +548,8 @@ __global__ void __launch_bounds__(kGatedFewThreads) gated_act_quant_few_kernel(c
           cvt_e4m3x4(__fmul_rn(h[i][0], inv), __fmul_rn(h[i][1], inv), __fmul_rn(h[i][2], inv), __fmul_rn(h[i][3], inv));
 }
 
+// --------------------------------------------------------------------------------------------
+// dequant_rows: 2D in + out bytes per row; flat, one chunk per thread.
 // --------------------------------------------------------------------------------------------
 struct DequantArgs {
   const void* x;
@@ -621,6 +623,11 @@ struct ResNormArgs {
   int mirrors;
 };
 
+// Whether a call is what the PLAIN instantiations below hold (the residual is float32 or bfloat16, any delta).
+static inline bool resnorm_plain(const ResNormArgs& a) {
+  return a.drow && a.dcol && a.write_res && a.q && !(a.bias || a.gate || a.layernorm || a.weight || a.beta || a.mod_scale || a.y || a.mirrors);
+}
+
 template <typename RT>
 __device__ __forceinline__ float round_through(float x);
 template <>
@@ -632,7 +639,10 @@ __device__ __forceinline__ float round_through<__nv_bfloat16>(float x) {
 
 // PART: the delta arrives as fp32 planes of a K-split GEMM (a.dpart) instead of a raw bf16 accumulator; an
 // instantiation of its own, so that the ordinary one keeps its registers.
-template <typename RT, int TPR, int IT, bool FAST, bool PART = false>
+// PLAIN: a scaled delta, RMS norm, codes -- what a decoder layer asks for (resnorm_plain).  A launch over a few hundred rows
+// fetches its instructions cold and holds the registers of its longest path, so this instantiation has no other
+// (816 x 2048 4.60 -> 4.39 us, 1100 x 2048 6.96 -> 4.43).
+template <typename RT, int TPR, int IT, bool FAST, bool PART = false, bool PLAIN = false>
 __global__ void __launch_bounds__(kRowThreads, PART ? 2 : resnorm_min_blocks<IT>())
 residual_norm_quant_kernel(const ResNormArgs a) {
   row_begin(a.early);  // inputs may come from the kernel before this one in the stream
@@ -641,11 +651,11 @@ residual_norm_quant_kernel(const ResNormArgs a) {
   const int m = blockIdx.x * (kRowThreads / TPR) + threadIdx.x / TPR;
   const bool live = m < a.M;
   RT* rr = reinterpret_cast<RT*>(a.res) + (live ? (int64_t)m * a.ld_res : 0);
-  const __nv_bfloat16* dr = a.delta ? a.delta + (live ? (int64_t)m * a.ld_delta : 0) : nullptr;
+  const __nv_bfloat16* dr = PLAIN || a.delta ? a.delta + (live ? (int64_t)m * a.ld_delta : 0) : nullptr;
   const float* dp = PART ? a.dpart + (live ? (int64_t)m * a.ld_delta : 0) : nullptr;
   const int64_t dp_plane = (int64_t)a.M * a.ld_delta;
-  const int64_t mofs = (live && a.mod_index) ? (int64_t)a.mod_index[m] * a.D : 0;
-  const float drs = (live && a.drow) ? a.drow[m] : 1.0f;
+  const int64_t mofs = (!PLAIN && live && a.mod_index) ? (int64_t)a.mod_index[m] * a.D : 0;
+  const float drs = (live && (PLAIN || a.drow)) ? a.drow[m] : 1.0f;
   const float fD = (float)a.D;
 
   Raw8<RT> rres[IT];
@@ -655,7 +665,7 @@ residual_norm_quant_kernel(const ResNormArgs a) {
     const int c0 = (it * TPR + t) * 8;
     const bool on = it < a.iters && live && c0 < a.D;
     rres[it] = fetch<FAST, RT>(rr, c0, a.D, on);
-    rdel[it] = fetch<FAST, __nv_bfloat16>(dr, c0, a.D, on && dr != nullptr && !PART);
+    rdel[it] = fetch<FAST, __nv_bfloat16>(dr, c0, a.D, on && (PLAIN || dr != nullptr) && !PART);
   }
   float x[IT][8];
   float sum = 0.0f, sumsq = 0.0f;
@@ -664,7 +674,7 @@ residual_norm_quant_kernel(const ResNormArgs a) {
     const int c0 = (it * TPR + t) * 8;
     unpack(rres[it], x[it]);
     if (it < a.iters && live && c0 < a.D) {
-      if (dr || PART) {
+      if (PLAIN || dr || PART) {
         float d[8], cs[8], bs[8], gs[8];
         if constexpr (PART) {
           // four planes in flight together, added in split order
@@ -690,34 +700,34 @@ residual_norm_quant_kernel(const ResNormArgs a) {
         } else {
           unpack(rdel[it], d);
         }
-        if (a.dcol) load_f32<FAST>(a.dcol, c0, a.D, cs);
-        if (a.bias) load_f32<FAST>(a.bias, c0, a.D, bs);
-        if (a.gate) load_f32<FAST>(a.gate + mofs, c0, a.D, gs);
+        if (PLAIN || a.dcol) load_f32<FAST>(a.dcol, c0, a.D, cs);
+        if (!PLAIN && a.bias) load_f32<FAST>(a.bias, c0, a.D, bs);
+        if (!PLAIN && a.gate) load_f32<FAST>(a.gate + mofs, c0, a.D, gs);
         Chain8 ch(d);
-        if (a.drow) ch.mul(drs);
-        if (a.dcol) ch.mul(cs);
-        if (a.bias) ch.add(bs);
-        if (a.gate) ch.mul(gs);
+        if (PLAIN || a.drow) ch.mul(drs);
+        if (PLAIN || a.dcol) ch.mul(cs);
+        if (!PLAIN && a.bias) ch.add(bs);
+        if (!PLAIN && a.gate) ch.mul(gs);
         ch.add(x[it]);  // x + d, contracted with d's last multiply when there is one
         ch.done(x[it]);
-        if (a.write_res) {
+        if (PLAIN || a.write_res) {
 #pragma unroll
           for (int i = 0; i < 8; ++i) x[it][i] = round_through<RT>(x[it][i]);
         }
         mask_tail<FAST>(x[it], c0, a.D);
-        if (a.write_res) store_out<FAST>(a.res, dtype_of<RT>(), (int64_t)m * a.ld_res, c0, a.D, x[it]);
+        if (PLAIN || a.write_res) store_out<FAST>(a.res, dtype_of<RT>(), (int64_t)m * a.ld_res, c0, a.D, x[it]);
       }
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        sum = __fadd_rn(sum, x[it][i]);
+        if (!PLAIN) sum = __fadd_rn(sum, x[it][i]);
         sumsq = __fmaf_rn(x[it][i], x[it][i], sumsq);
       }
     }
   }
-  if (a.q == nullptr && a.y == nullptr) return;  // residual update only (uniform across the CTA)
+  if (!PLAIN && a.q == nullptr && a.y == nullptr) return;  // residual update only (uniform across the CTA)
 
   float rstd;
-  if (a.layernorm) {
+  if (!PLAIN && a.layernorm) {
     const float mean = div_full(row_reduce<TPR, false>(sum, red[0]), fD);
     float sq = 0.0f;
 #pragma unroll
@@ -745,17 +755,17 @@ residual_norm_quant_kernel(const ResNormArgs a) {
     const int c0 = (it * TPR + t) * 8;
     if (it < a.iters && live && c0 < a.D) {
       float ws[8], bs[8], ms[8], mh[8];
-      if (a.weight) load_f32<FAST>(a.weight, c0, a.D, ws);
-      if (a.beta) load_f32<FAST>(a.beta, c0, a.D, bs);
-      if (a.mod_scale) {
+      if (!PLAIN && a.weight) load_f32<FAST>(a.weight, c0, a.D, ws);
+      if (!PLAIN && a.beta) load_f32<FAST>(a.beta, c0, a.D, bs);
+      if (!PLAIN && a.mod_scale) {
         load_f32<FAST>(a.mod_scale + mofs, c0, a.D, ms);
         load_f32<FAST>(a.mod_shift + mofs, c0, a.D, mh);
       }
       Chain8 ch(x[it]);
       ch.mul(rstd);
-      if (a.weight) ch.mul(ws);
-      if (a.beta) ch.add(bs);
-      if (a.mod_scale) {
+      if (!PLAIN && a.weight) ch.mul(ws);
+      if (!PLAIN && a.beta) ch.add(bs);
+      if (!PLAIN && a.mod_scale) {
 #pragma unroll
         for (int i = 0; i < 8; i += 2) unpack2(add2(pack2(ms[i], ms[i + 1]), pack2(1.0f, 1.0f)), ms[i], ms[i + 1]);
         ch.mul(ms);
@@ -765,10 +775,10 @@ residual_norm_quant_kernel(const ResNormArgs a) {
       mask_tail<FAST>(x[it], c0, a.D);
 #pragma unroll
       for (int i = 0; i < 8; ++i) amax = max_f32(amax, fabsf(x[it][i]));
-      if (a.y) store_out<FAST>(a.y, a.y_dtype, (int64_t)m * a.ld_y, c0, a.D, x[it]);
+      if (!PLAIN && a.y) store_out<FAST>(a.y, a.y_dtype, (int64_t)m * a.ld_y, c0, a.D, x[it]);
     }
   }
-  if (a.q == nullptr) return;
+  if (!PLAIN && a.q == nullptr) return;
   amax = row_reduce<TPR, true>(amax, red[2]);
   float scale, inv;
   quant_scales(amax, scale, inv);
@@ -807,6 +817,9 @@ residual_norm_quant_kernel(const ResNormArgs a) {
 // so that a few hundred rows are resident together.  Eight columns a thread, chunk after chunk and plane
 // group after plane group before: 50 x 1024 with eight planes 2.9 -> 2.3 us, 816 x 2048 with two 7.6 -> 5.6.
 // PL: planes loaded together (further ones follow in groups of PL).
+// PLAIN: the decoder layer's operands alone (resnorm_plain), in a quarter of the code and with one meeting of the row's
+// warps for the sum and the maximum: 50 x 1024 with eight planes 2.42 -> 1.77 us, 816 x 2048 with two 5.59 -> 3.89, 18 expert
+// layers 403 -> 381; over 250 sizes of 1 to 2000 rows 0.80 of the time, one more than 3 % slower (2000 x 2048, eight planes 27.0, 28.3).
 // --------------------------------------------------------------------------------------------
 template <typename T>
 struct Quad;
@@ -866,7 +879,7 @@ __host__ __device__ constexpr int row_cta_min_blocks() {
   return IT * (PL + 4) <= 12 ? 4 : (IT * (PL + 4) <= 18 ? 3 : 2);
 }
 
-template <typename RT, int IT, int PL>
+template <typename RT, int IT, int PL, bool PLAIN>
 __global__ void __launch_bounds__(kRowThreads, row_cta_min_blocks<IT, PL>())
 residual_norm_planes_kernel(const ResNormArgs a) {
   static_assert(kRowThreads == 256, "eight warps per row");
@@ -875,8 +888,8 @@ residual_norm_planes_kernel(const ResNormArgs a) {
   const int m = blockIdx.x, c = threadIdx.x * 4;
   row_begin(a.early);  // inputs may come from the kernel before this one in the stream
   RT* rr = reinterpret_cast<RT*>(a.res) + (int64_t)m * a.ld_res + c;
-  const int64_t mofs = a.mod_index ? (int64_t)a.mod_index[m] * a.D + c : c;
-  const float drs = a.drow ? a.drow[m] : 1.0f;
+  const int64_t mofs = !PLAIN && a.mod_index ? (int64_t)a.mod_index[m] * a.D + c : c;
+  const float drs = PLAIN || a.drow ? a.drow[m] : 1.0f;
 
   Quad<RT> rres[IT];
   Quad<float> plane[PL][IT], dcol[IT];
@@ -886,7 +899,7 @@ residual_norm_planes_kernel(const ResNormArgs a) {
   for (int it = 0; it < IT; ++it) {
     if (it * kStep + c < a.D) {
       rres[it].load(rr + it * kStep);
-      if (a.dcol) dcol[it].load(a.dcol + c + it * kStep);
+      if (PLAIN || a.dcol) dcol[it].load(a.dcol + c + it * kStep);
     }
 #pragma unroll
     for (int s = 0; s < PL; ++s)
@@ -931,35 +944,42 @@ residual_norm_planes_kernel(const ResNormArgs a) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) d[i] = __bfloat162float(__float2bfloat16_rn(d[i]));
       ChainV<4> ch(d);
-      if (a.drow) ch.mul(drs);
-      if (a.dcol) {
+      if (PLAIN || a.drow) ch.mul(drs);
+      if (PLAIN || a.dcol) {
         dcol[it].widen(op);
         ch.mul(op);
       }
-      if (a.bias) {
+      if (!PLAIN && a.bias) {
         load_quad(a.bias + c + o, op);
         ch.add(op);
       }
-      if (a.gate) {
+      if (!PLAIN && a.gate) {
         load_quad(a.gate + mofs + o, op);
         ch.mul(op);
       }
       ch.add(x[it]);  // x + d, contracted with d's last multiply when there is one
       ch.done(x[it]);
-      if (a.write_res) {
+      if (PLAIN || a.write_res) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) x[it][i] = round_through<RT>(x[it][i]);
         store_quad(a.res, dtype_of<RT>(), (int64_t)m * a.ld_res + c + o, x[it]);
       }
 #pragma unroll
-      for (int i = 0; i < 4; ++i) sum = a.layernorm ? __fadd_rn(sum, x[it][i]) : __fmaf_rn(x[it][i], x[it][i], sum);
+      for (int i = 0; i < 4; ++i) sum = !PLAIN && a.layernorm ? __fadd_rn(sum, x[it][i]) : __fmaf_rn(x[it][i], x[it][i], sum);
     }
   }
-  if (a.q == nullptr && a.y == nullptr) return;  // residual update only (uniform across the CTA)
+  if (!PLAIN && a.q == nullptr && a.y == nullptr) return;  // residual update only (uniform across the CTA)
 
   const float fD = (float)a.D;
+  float amax = 0.0f;
+  if (PLAIN) {  // rounding keeps the order of the |x| rstd, so that the largest |x| gives the largest of them: one meeting for both
+#pragma unroll
+    for (int it = 0; it < IT; ++it) amax = max_abs_f32(max_abs_f32(amax, x[it][0], x[it][1]), x[it][2], x[it][3]);
+    amax = warp_max_abs_f32(amax);
+    if ((threadIdx.x & 31) == 0) red[2][threadIdx.x >> 5] = amax;
+  }
   sum = row_cta_reduce<false>(sum, red[0]);
-  if (a.layernorm) {
+  if (!PLAIN && a.layernorm) {
     const float mean = div_full(sum, fD);
     sum = 0.0f;
 #pragma unroll
@@ -975,7 +995,6 @@ residual_norm_planes_kernel(const ResNormArgs a) {
     sum = row_cta_reduce<false>(sum, red[1]);
   }
   const float rstd = rsqrt_approx_ftz(__fadd_rn(div_full(sum, fD), a.eps));
-  float amax = 0.0f;
 #pragma unroll
   for (int it = 0; it < IT; ++it) {
     const int o = it * kStep;
@@ -983,15 +1002,15 @@ residual_norm_planes_kernel(const ResNormArgs a) {
       float op[4];
       ChainV<4> ch(x[it]);
       ch.mul(rstd);
-      if (a.weight) {
+      if (!PLAIN && a.weight) {
         load_quad(a.weight + c + o, op);
         ch.mul(op);
       }
-      if (a.beta) {
+      if (!PLAIN && a.beta) {
         load_quad(a.beta + c + o, op);
         ch.add(op);
       }
-      if (a.mod_scale) {
+      if (!PLAIN && a.mod_scale) {
         load_quad(a.mod_scale + mofs + o, op);
 #pragma unroll
         for (int i = 0; i < 4; ++i) op[i] = __fadd_rn(op[i], 1.0f);
@@ -1000,12 +1019,17 @@ residual_norm_planes_kernel(const ResNormArgs a) {
         ch.add(op);
       }
       ch.done(x[it]);
-      amax = max_abs_f32(max_abs_f32(amax, x[it][0], x[it][1]), x[it][2], x[it][3]);
-      if (a.y) store_quad(a.y, a.y_dtype, (int64_t)m * a.ld_y + c + o, x[it]);
+      if (!PLAIN) amax = max_abs_f32(max_abs_f32(amax, x[it][0], x[it][1]), x[it][2], x[it][3]);
+      if (!PLAIN && a.y) store_quad(a.y, a.y_dtype, (int64_t)m * a.ld_y + c + o, x[it]);
     }
   }
-  if (a.q == nullptr) return;
-  amax = row_cta_reduce<true>(amax, red[2]);
+  if (!PLAIN && a.q == nullptr) return;
+  if (PLAIN) {
+    const float4 lo = reinterpret_cast<const float4*>(red[2])[0], hi = reinterpret_cast<const float4*>(red[2])[1];
+    amax = __fmul_rn(max_f32(max_f32(max_f32(lo.x, lo.y), max_f32(lo.z, lo.w)), max_f32(max_f32(hi.x, hi.y), max_f32(hi.z, hi.w))), rstd);
+  } else {
+    amax = row_cta_reduce<true>(amax, red[2]);
+  }
   float scale, inv;
   quant_scales(amax, scale, inv);
   if (threadIdx.x == 0) a.qs[m] = scale;
@@ -1019,13 +1043,13 @@ residual_norm_planes_kernel(const ResNormArgs a) {
       *reinterpret_cast<uint32_t*>(q + it * kStep) = code;
 #pragma unroll
       for (int k = 0; k < kMaxMirrors; ++k)
-        if (k < a.mirrors) *reinterpret_cast<uint32_t*>(a.q_mirror[k] + (int64_t)m * a.ld_q + c + it * kStep) = code;
+        if (!PLAIN && k < a.mirrors) *reinterpret_cast<uint32_t*>(a.q_mirror[k] + (int64_t)m * a.ld_q + c + it * kStep) = code;
     }
   }
   if (threadIdx.x == 0) {
 #pragma unroll
     for (int k = 0; k < kMaxMirrors; ++k)
-      if (k < a.mirrors) a.qs_mirror[k][m] = scale;
+      if (!PLAIN && k < a.mirrors) a.qs_mirror[k][m] = scale;
   }
 }
 
@@ -1040,7 +1064,13 @@ residual_norm_planes_kernel(const ResNormArgs a) {
 //   not elsewhere (4096, 816 rows, 8 planes 28.9 / 26.3; 8192, 500 rows, 2 / 8 planes 16.6 / 13.5 and 70.8 / 30.8).
 template <typename RT, int IT, int PL>
 static void launch_resnorm_planes_form(const ResNormArgs& a, cudaStream_t s) {
-  launch_dep(residual_norm_planes_kernel<RT, IT, PL>, dim3(a.M), dim3(kRowThreads), 0, s, 1, dependent_launch_for(a.M), a);
+  if constexpr (IT <= 2) {
+    if (resnorm_plain(a)) {
+      launch_dep(residual_norm_planes_kernel<RT, IT, PL, true>, dim3(a.M), dim3(kRowThreads), 0, s, 1, dependent_launch_for(a.M), a);
+      return;
+    }
+  }
+  launch_dep(residual_norm_planes_kernel<RT, IT, PL, false>, dim3(a.M), dim3(kRowThreads), 0, s, 1, dependent_launch_for(a.M), a);
 }
 template <typename RT, int TPR, int IT>
 static void launch_resnorm_part_form(ResNormArgs a, cudaStream_t s) {
@@ -1319,6 +1349,26 @@ static void launch_gated(GatedArgs a, bool fast, cudaStream_t s) {
     launch_dep(gated_act_quant_kernel<XT, kRowThreads, 8, false>, dim3(a.M), dim3(kRowThreads), 0, s, 1, dependent_launch_for(a.M), a);
     return;
   }
+  if constexpr (sizeof(XT) == 2) {
+    // A CTA for every row at once: while each has an SM of its own, and up to three an SM for rows that are one or two quads a
+    // thread.  us behind one another, this form against groups of 256 threads: 50 x 4096 1.92 / 2.45, 148 x 512 1.38 / 1.84, 148 x
+    // 8192 2.74 / 3.87, 148 x 16384 4.21 / 5.94, 444 x 4096 3.78 / 3.83, 444 x 5120 4.18 / 4.61; beyond, 200 x 8192 4.51 / 4.29, 600 x
+    // 4096 5.29 / 4.86.
+    const int sms = device_sm_count() > 0 ? device_sm_count() : 148, q = (a.F + 4 * kGatedFewThreads - 1) / (4 * kGatedFewThreads);
+    if (g_row_tpr_override == 0 && (a.M <= sms || (a.F <= 5120 && a.M <= 3 * sms))) {
+      auto few = [&](auto quads) {
+        constexpr int Q = decltype(quads)::value;
+        const int threads = ((a.F / 4 + Q - 1) / Q + 31) / 32 * 32;
+        const bool gelu = a.act == IFLB200_ACT_GELU_TANH;
+        launch_dep(gelu ? gated_act_quant_few_kernel<XT, IFLB200_ACT_GELU_TANH, Q> : gated_act_quant_few_kernel<XT, IFLB200_ACT_SILU, Q>,
+                   dim3(a.M), dim3(threads), 0, s, 1, dependent_launch_for(a.M), a);
+      };
+      if (q <= 1) few(IntTag<1>{});
+      else if (q <= 2) few(IntTag<2>{});
+      else few(IntTag<4>{});
+      return;
+    }
+  }
   const RowGeom g = pick_geom(a.F);
   a.iters = g.iters;
   dispatch_geom(g, [&](auto tpr, auto it) {
@@ -1349,28 +1399,14 @@ static void launch_resnorm(ResNormArgs a, bool fast, cudaStream_t s) {
   }
   a.iters = g.iters;
   dispatch_geom(g, [&](auto tpr, auto it) {
-  if constexpr (sizeof(XT) == 2) {
-    // A CTA for every row at once: while each has an SM of its own, and up to three an SM for rows that are one or two quads a
-    // thread.  us behind one another, this form against groups of 256 threads: 50 x 4096 1.92 / 2.45, 148 x 512 1.38 / 1.84, 148 x
-    // 8192 2.74 / 3.87, 148 x 16384 4.21 / 5.94, 444 x 4096 3.78 / 3.83, 444 x 5120 4.18 / 4.61; beyond, 200 x 8192 4.51 / 4.29, 600 x
-    // 4096 5.29 / 4.86.
-    const int sms = device_sm_count() > 0 ? device_sm_count() : 148, q = (a.F + 4 * kGatedFewThreads - 1) / (4 * kGatedFewThreads);
-    if (g_row_tpr_override == 0 && (a.M <= sms || (a.F <= 5120 && a.M <= 3 * sms))) {
-      auto few = [&](auto quads) {
-        constexpr int Q = decltype(quads)::value;
-        const int threads = ((a.F / 4 + Q - 1) / Q + 31) / 32 * 32;
-        const bool gelu = a.act == IFLB200_ACT_GELU_TANH;
-        launch_dep(gelu ? gated_act_quant_few_kernel<XT, IFLB200_ACT_GELU_TANH, Q> : gated_act_quant_few_kernel<XT, IFLB200_ACT_SILU, Q>,
-                   dim3(a.M), dim3(threads), 0, s, 1, dependent_launch_for(a.M), a);
-      };
-      if (q <= 1) few(IntTag<1>{});
-      else if (q <= 2) few(IntTag<2>{});
-      else few(IntTag<4>{});
-      return;
-    }
-  }
     constexpr int TPR = decltype(tpr)::value, IT = decltype(it)::value;
     const int grid = (a.M + kRowThreads / TPR - 1) / (kRowThreads / TPR);
+    if constexpr (std::is_same<RT, float>::value && IT <= 3) {
+      if (a.delta && resnorm_plain(a)) {
+        launch_dep(residual_norm_quant_kernel<RT, TPR, IT, true, false, true>, dim3(grid), dim3(kRowThreads), 0, s, 1, dependent_launch_for(a.M), a);
+        return;
+      }
+    }
     launch_dep(residual_norm_quant_kernel<RT, TPR, IT, true>, dim3(grid), dim3(kRowThreads), 0, s, 1, dependent_launch_for(a.M), a);
   });
 }

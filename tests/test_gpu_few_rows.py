@@ -38,3 +38,31 @@ def test_gated_quantiser_bits(M, F):
             torch.cuda.synchronize()
             assert torch.equal(u8(outs[0][0]), u8(outs[1][0])) and torch.equal(i32(outs[0][1]), i32(outs[1][1]))
 
+
+# A weight of ones takes the general form and multiplies by one.  Widths: quads and chunks with ragged ends, the widest of
+# the planes form (2048) and of the bf16 delta's (3072 and beyond); planes: 0 is a bf16 delta, then either side of the groups.
+@pytest.mark.parametrize("D", [8, 1016, 1024, 1032, 2048, 2056, 3072, 6152])
+@pytest.mark.parametrize("planes", [0, 1, 2, 3, 4, 5, 8])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_plain_residual_bits(D, planes, dtype):
+    from instinctflash_b200.kernels import norm
+    M = 9
+    g = torch.Generator(device=DEV).manual_seed(D + planes)
+    res0 = (torch.randn(M, D, device=DEV, generator=g) * 2).to(dtype)
+    delta = torch.randn(*((planes, M, D) if planes else (M, D)), device=DEV, generator=g)
+    if not planes:
+        delta = delta.to(torch.bfloat16)
+    res0[1], delta[..., 1, :] = 0.0, 0.0                      # nothing: eps alone
+    res0[2], delta[..., 2, :] = 1e-25, 0.0                    # squares below the smallest number
+    res0[3], delta[..., 3, :] = 1e30, 0.0                     # and above the largest
+    res0[4, D // 2], res0[5, D - 1], res0[6, 0] = float("nan"), float("inf"), float("-inf")
+    row, col = torch.rand(M, device=DEV, generator=g), torch.rand(D, device=DEV, generator=g)
+    for eps in (1e-6, 0.0):
+        outs = []
+        for weight in (None, torch.ones(D, device=DEV)):
+            res, q, s = res0.clone(), torch.full((M, D + 8), 1.0, device=DEV).to(E4M3), torch.empty(M, device=DEV)
+            norm.residual_norm_quant(res, delta=delta, delta_row=row, delta_col=col, weight=weight, q=q[:, :D], q_scale=s, eps=eps)
+            outs.append((res, q, s))
+        torch.cuda.synchronize()
+        (r0, q0, s0), (r1, q1, s1) = outs
+        assert torch.equal(u8(r0), u8(r1)) and torch.equal(u8(q0), u8(q1)) and torch.equal(i32(s0), i32(s1))
