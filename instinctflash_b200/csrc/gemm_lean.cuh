@@ -3,9 +3,9 @@
 //
 // A launch over 50 rows takes 3 to 5 us, most of it latencies in a row: the kernel before it, first operands, MMAs,
 // epilogue, completion.  It fetches its instructions cold, so the kernel holds nothing that such a launch does not run:
-// the output kind is a template argument, and a lane stores its row straight from registers (6 KB a tile are not worth
-// staging; fp32 rows of many tiles are).  With one epilogue for all output kinds, through shared memory and TMA, the last store of a 64 x 4096 x 1024
-// launch was issued 2600 clocks after its last MMA; 18 expert layers over 50 rows (72 such launches) took 476 us, 417 now.
+// the output kind is a template argument, and the accumulator goes to memory straight from registers.  With one epilogue for all
+// output kinds, through shared memory and TMA, the last store of a 64 x 4096 x 1024 launch was issued 2600 clocks after its
+// last MMA.
 // Four K slabs of 128 bytes a stage come with one TMA instruction per operand; up to 64 rows the MMAs are 64 rows high
 // (38 clocks each for 48), and row i of the accumulator lies in lane i % 16 of quadrant i / 16.
 #pragma once
@@ -26,9 +26,7 @@ template <int AR>
 struct LeanLayout {
   static constexpr int kSlabs = 4, kTile = 64, kStages = AR == 64 ? 3 : 2;
   static constexpr int kABytes = AR * BK * kSlabs, kWBytes = kTile * BK * kSlabs, kStageBytes = kABytes + kWBytes;
-  // fp32 rows of the 128-row form on their way to memory, 32 x 128 bytes a warp
-  static constexpr int kStagingOffset = kStages * kStageBytes, kStaging = AR == 128 ? 4096 : 0;
-  static constexpr int kBarOffset = kStagingOffset + 8 * kStaging;
+  static constexpr int kBarOffset = kStages * kStageBytes;
   static constexpr int kDynamic = kBarOffset + (2 * kStages + 4) * 8 + 16 + 1024;
   static constexpr int kThreads = 32 * 11;  // W producer, MMA, eight epilogue warps, A producer
 };
@@ -170,7 +168,14 @@ gemm_fp8_tc5_lean_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
     __syncwarp();
   } else {
     // ------------------------------------------------------------------ epilogue warps: 32 columns of a quadrant's rows
+    // Tensor memory is read in the 16 x 256-bit shape: a thread holds two neighbouring columns of rows r4 and r4 + 8 of
+    // every eight, so that four lanes write a whole 32-byte sector of a row (fp32, straight from the registers), or after
+    // a 4 x 4 transpose among them 64 bytes (two-byte outputs).  A lane per row wrote half a sector at a time, and up to 64
+    // rows half of the lanes held nothing: 64 x 4096 x 1024 with scales 3.68 -> 3.18 us behind one another, 50 x 1024 x 4096 in
+    // eight planes 3.44 -> 3.26, 18 expert layers 381 -> 368; over 147 sizes dequantised 0.96 of the time, planes 0.95, raw 1.00.
+    constexpr int kBlocks = AR / 64;  // sixteens of rows of a quadrant
     const int quad = warp & 3, c0 = ((warp - 2) >> 2) * 32;
+    const int r4 = lane >> 2, c4 = lane & 3;
     bool ok = true;
     uint32_t it = 0;
     grid_dependency_wait();
@@ -178,87 +183,82 @@ gemm_fp8_tc5_lean_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
       int m_blk, n_blk;
       tile_coords(p, tile, m_blk, n_blk);
       const uint32_t acc = it & 1u, acc_phase = (it >> 1) & 1u;
-      const int m = m_blk * BM + quad * quad_rows + lane, n0 = n_blk * BN + c0;
-      const bool row_ok = lane < quad_rows && m < p.M;
-      // this tile's scales and bias, fetched under the main loop: lane l holds column n0 + l; what is absent is a factor
-      // of 1 or an addend of -0
-      float rs = 1.0f, cs = 1.0f, bs = -0.0f;
+      const int m0 = m_blk * BM + quad * quad_rows + r4, n0 = n_blk * BN + c0;
+      // where this thread's first row goes, and the rows and columns that there are from it on
+      constexpr int kEs = kWide ? 4 : 2;
+      uint8_t* out = reinterpret_cast<uint8_t*>(p.out) + ((EPI == LEAN_PLANES ? (int64_t)part * p.M : 0) + m0) * p.ld_out * kEs +
+                     (int64_t)(n0 + (kWide ? 2 : 8) * c4) * kEs;
+      const int64_t eight_rows = 8 * p.ld_out * kEs;
+      const int rows = p.M - m0, columns = p.N - n0;
+      // this tile's scales and bias, fetched under the main loop; what is absent is a factor of 1 or an addend of -0
+      float rs[2 * kBlocks], cs[8], bs[8];
       if constexpr (kDequant) {
-        if (row_ok && p.row) rs = __ldg(p.row + (int64_t)m * p.row_stride);
-        if (n0 + lane < p.N) {
-          if (p.col) cs = __ldg(p.col + (int64_t)(n0 + lane) * p.col_stride);
-          if (p.bias)
-            bs = p.bias_dtype == IFLB200_F32 ? __ldg(reinterpret_cast<const float*>(p.bias) + n0 + lane)
-                                             : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.bias)[n0 + lane]);
+#pragma unroll
+        for (int i = 0; i < 2 * kBlocks; ++i) {
+          const int m = m0 + 8 * i;
+          rs[i] = p.row && m < p.M ? __ldg(p.row + (int64_t)m * p.row_stride) : 1.0f;
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int n = n0 + 8 * (i >> 1) + 2 * c4 + (i & 1);
+          cs[i] = p.col && n < p.N ? __ldg(p.col + (int64_t)n * p.col_stride) : 1.0f;
+          bs[i] = !p.bias || n >= p.N ? -0.0f
+                  : p.bias_dtype == IFLB200_F32 ? __ldg(reinterpret_cast<const float*>(p.bias) + n)
+                                                : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.bias)[n]);
         }
       }
       ok = wait_bounded(tfull_bar(acc), acc_phase, abort_flag, (3u << 24) | (4u << 16) | (it & 0xFFFF));
       if (!ok) break;
       tc_fence_after();
-      uint32_t r[32];
-      tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(quad * 32) << 16) + acc * BN + c0, r);
+      uint32_t r[kBlocks][16];  // r[b][4j + 2h + e]: row 16 b + 8 h + r4, column 8 j + 2 c4 + e
+      const uint32_t t_acc = tmem_base + ((uint32_t)(quad * 32) << 16) + acc * BN + c0;
+#pragma unroll
+      for (int b = 0; b < kBlocks; ++b) tmem_ld_16x256b_x4(t_acc + ((uint32_t)(16 * b) << 16), r[b]);
       tmem_ld_wait();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(tempty_bar(acc));
-      if constexpr (kDequant) {
 #pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          float a = __uint_as_float(r[i]), b = __uint_as_float(r[i + 1]);
-          const float ca = __shfl_sync(0xFFFFFFFFu, cs, i), cb = __shfl_sync(0xFFFFFFFFu, cs, i + 1);
-          const float ba = __shfl_sync(0xFFFFFFFFu, bs, i), bb = __shfl_sync(0xFFFFFFFFu, bs, i + 1);
-          if (p.exact == 2) {  // (acc * (row * col)) + bias, each operation rounded (scalar: see gemm_tokens.cuh)
-            a = __fadd_rn(__fmul_rn(a, __fmul_rn(rs, ca)), ba);
-            b = __fadd_rn(__fmul_rn(b, __fmul_rn(rs, cb)), bb);
-          } else {  // ((acc * row) * col) + bias, the addition contracted with the last factor there is
-            if (!p.exact) {
-              const uint32_t w = pack_bf16x2(a, b);
-              a = __uint_as_float(w << 16);
-              b = __uint_as_float(w & 0xFFFF0000u);
-            }
-            const uint64_t x = pack2(a, b), r2 = pack2(rs, rs), b2 = pack2(ba, bb);
-            unpack2(p.col ? fma2(mul2(x, r2), pack2(ca, cb), b2) : fma2(x, r2, b2), a, b);
-          }
-          r[i] = __float_as_uint(a);
-          r[i + 1] = __float_as_uint(b);
-        }
-      }
-      const int valid = row_ok ? min(32, p.N - n0) : 0;  // a multiple of 16, or not positive
-      if constexpr (EPI == LEAN_F32 && AR == 128) {
-        // Many tiles of fp32 are bound by their stores, so whole 128-byte pieces of four rows leave at a time, through shared
-        // memory (16-byte pieces swizzled by the row): 0.93 of the time of 16 bytes of 32 rows over 261 sizes
-        // (1946 x 224 x 1744 8.7 -> 7.1 us); 16 columns, half of a piece, 1.05.
-        const uint32_t mine = base + L::kStagingOffset + (uint32_t)(warp - 2) * L::kStaging;
-        __syncwarp();  // the rows of the tile before this one have been read
+      for (int b = 0; b < kBlocks; ++b) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
-          st_shared_v4(mine + lane * 128 + ((j ^ (lane & 7)) << 4), make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]));
-        __syncwarp();
-        const int row0 = m_blk * BM + quad * 32, piece = lane & 7;
-        float* o = reinterpret_cast<float*>(p.out) + (int64_t)row0 * p.ld_out + n0 + 4 * piece;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int t = 4 * i + (lane >> 3);
-          const uint4 v = ld_shared_v4(mine + t * 128 + ((piece ^ (t & 7)) << 4));
-          if (row0 + t < p.M && n0 + 4 * piece < p.N) *reinterpret_cast<uint4*>(o + (int64_t)t * p.ld_out) = v;
-        }
-      } else if constexpr (kWide) {
-        float* o = reinterpret_cast<float*>(p.out) + ((EPI == LEAN_PLANES ? (int64_t)part * p.M : 0) + m) * p.ld_out + n0;
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-          if (4 * j < valid) *reinterpret_cast<uint4*>(o + 4 * j) = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
-      } else {
-        uint16_t* o = reinterpret_cast<uint16_t*>(p.out) + (int64_t)m * p.ld_out + n0;
-        const bool f16 = EPI == LEAN_DEQUANT && p.out_dtype == IFLB200_F16;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int h = 0; h < 2; ++h) {
+          if (16 * b + 8 * h >= rows + r4) continue;  // none of the warp's
+          const bool in = 16 * b + 8 * h < rows;
+          uint8_t* o = out + (2 * b + h) * eight_rows;
           uint32_t v[4];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const float a = __uint_as_float(r[8 * j + 2 * i]), b = __uint_as_float(r[8 * j + 2 * i + 1]);
-            v[i] = f16 ? pack_f16x2(a, b) : pack_bf16x2(a, b);
+          for (int j = 0; j < 4; ++j) {
+            float x = __uint_as_float(r[b][4 * j + 2 * h]), y = __uint_as_float(r[b][4 * j + 2 * h + 1]);
+            if constexpr (kDequant) {
+              const float rsc = rs[2 * b + h];
+              if (p.exact == 2) {  // (acc * (row * col)) + bias, each operation rounded (scalar: see gemm_tokens.cuh)
+                x = __fadd_rn(__fmul_rn(x, __fmul_rn(rsc, cs[2 * j])), bs[2 * j]);
+                y = __fadd_rn(__fmul_rn(y, __fmul_rn(rsc, cs[2 * j + 1])), bs[2 * j + 1]);
+              } else {  // ((acc * row) * col) + bias, the addition contracted with the last factor there is
+                if (!p.exact) {
+                  const uint32_t w = pack_bf16x2(x, y);
+                  x = __uint_as_float(w << 16);
+                  y = __uint_as_float(w & 0xFFFF0000u);
+                }
+                const uint64_t x2 = pack2(x, y), r2 = pack2(rsc, rsc), b2 = pack2(bs[2 * j], bs[2 * j + 1]);
+                unpack2(p.col ? fma2(mul2(x2, r2), pack2(cs[2 * j], cs[2 * j + 1]), b2) : fma2(x2, r2, b2), x, y);
+              }
+            }
+            if constexpr (kWide) {
+              if (in && 8 * j < columns) *reinterpret_cast<float2*>(o + 32 * j) = make_float2(x, y);
+            } else {
+              v[j] = EPI == LEAN_DEQUANT && p.out_dtype == IFLB200_F16 ? pack_f16x2(x, y) : pack_bf16x2(x, y);
+            }
           }
-          if (8 * j < valid) *reinterpret_cast<uint4*>(o + 8 * j) = make_uint4(v[0], v[1], v[2], v[3]);
+          if constexpr (!kWide) {
+            // lane c4 of four hands over its columns of the other lanes' eights and ends up with eight columns of its own
+            const bool odd = c4 & 1, high = c4 & 2;
+            const uint32_t s0 = __shfl_xor_sync(0xFFFFFFFFu, odd ? v[0] : v[1], 1), s1 = __shfl_xor_sync(0xFFFFFFFFu, odd ? v[2] : v[3], 1);
+            const uint32_t w0 = odd ? s0 : v[0], w1 = odd ? v[1] : s0, w2 = odd ? s1 : v[2], w3 = odd ? v[3] : s1;
+            const uint32_t u0 = __shfl_xor_sync(0xFFFFFFFFu, high ? w0 : w2, 2), u1 = __shfl_xor_sync(0xFFFFFFFFu, high ? w1 : w3, 2);
+            if (in && 8 * c4 < columns)
+              *reinterpret_cast<uint4*>(o) = high ? make_uint4(u0, u1, w2, w3) : make_uint4(w0, w1, u0, u1);
+          }
         }
       }
     }
