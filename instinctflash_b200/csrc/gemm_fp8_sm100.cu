@@ -1686,14 +1686,15 @@ static int run_gemm(const void* a, int64_t ld_a, const void* w, int64_t ld_w, Ge
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   // Raw and dequant epilogues go through shared memory and TMA stores; the residual epilogue
   // updates its operand in place with plain loads and stores.
+  // (The tokens and the skinny form store from registers or by ordinary stores, and the skinny one loads through maps of its own:
+  // a map is encoded where a form takes it.  Four of the six of a 64 x 4096 x 1024 call went unused.)
   CUtensorMap to;
   p.tma_store = (p.epilogue != EPI_RESIDUAL && g_cfg_direct_store == 0) ? 1 : 0;
-  if (p.tma_store) {
-    st = make_out_map(&to, p.out, p.M, p.N, p.ld_out, oes);
-    if (st != IFLB200_OK) return st;
-  } else {
+  const auto make_out = [&](int row_bytes) {
+    if (p.tma_store) return make_out_map(&to, p.out, p.M, p.N, p.ld_out, oes, row_bytes);
     memset(&to, 0, sizeof(to));
-  }
+    return (int)IFLB200_OK;
+  };
   // Tile shape by a measured cost model: waves x (K steps x clocks of a step + what a tile's epilogue holds up), and what
   // the first loads and the last stores take.  A partly filled last wave, which has the L2 and the store path to itself,
   // counts 0.7 and 0.3 of its share.  A 128-byte K step of a 64 / 128 / 256 wide tile is about 490 / 555 / 800 clocks:
@@ -1827,9 +1828,9 @@ static int run_gemm(const void* a, int64_t ld_a, const void* w, int64_t ld_w, Ge
     const int pairs = dev->sm_count / 2;
     const int grid = 2 * (p.num_tiles < pairs ? p.num_tiles : pairs);
     CUtensorMap ta, tw;
-    st = make_tensor_map(&ta, a, p.M, p.K, ld_a, BM);
-    if (st != IFLB200_OK) return st;
-    st = make_tensor_map(&tw, w, p.N, p.K, ld_w, PBN / 2);
+    st = make_out(128);
+    if (st == IFLB200_OK) st = make_tensor_map(&ta, a, p.M, p.K, ld_a, BM);
+    if (st == IFLB200_OK) st = make_tensor_map(&tw, w, p.N, p.K, ld_w, PBN / 2);
     if (st != IFLB200_OK) return st;
     g_last_launch[0] = g_cfg_mode == 2 ? 2 : 3; g_last_launch[1] = PBN; g_last_launch[2] = 1; g_last_launch[3] = 6;
     return g_cfg_mode == 2 ? launch_gemm_pair<PBN, 6, 1>(ta, tw, to, p, grid, s)
@@ -1844,32 +1845,26 @@ static int run_gemm(const void* a, int64_t ld_a, const void* w, int64_t ld_w, Ge
   p.group_m = g_cfg_group_m > 0 ? g_cfg_group_m : 8;
   const int grid = split > 1 ? p.num_tiles * split : (p.num_tiles < dev->sm_count ? p.num_tiles : dev->sm_count);
 
-  // 64-wide tiles of two-byte outputs with consumer arithmetic: a 64-byte piece per warp instead of
-  // one 128-byte piece that the first warp of each quadrant stages alone (the epilogue of a skinny
-  // launch overlaps nothing: 64 x 4096 x 1024 with scales and bias 5.7 -> 5.1 us; raw outputs, whose
-  // staging is a handful of instructions, gain nothing from the second store and keep one piece).
-  if (bn == 64 && split == 1 && p.tma_store && oes == 2 && p.epilogue != EPI_RAW) {
-    st = make_out_map(&to, p.out, p.M, p.N, p.ld_out, oes, 64);
-    if (st != IFLB200_OK) return st;
-    p.half_rows = 1;
-  }
-  CUtensorMap ta, tw;
   const int a_rows = activation_box_rows(p.M);
   p.a_bytes = a_rows * BK;
-  st = make_tensor_map(&ta, a, p.M, p.K, ld_a, a_rows);
-  if (st != IFLB200_OK) return st;
-  st = make_tensor_map(&tw, w, p.N, p.K, ld_w, bn);
-  if (st != IFLB200_OK) return st;
   const int stages = g_cfg_stages;
   g_last_launch[0] = 1; g_last_launch[1] = bn; g_last_launch[2] = split; g_last_launch[3] = stages;
   // Skinny regime (64-wide tiles): four K slabs per TMA instruction where a CTA has at least one full stage of
   // them; the K order is unchanged, so are the bits.
-  if (bn == 64 && g_cfg_slabs != 1 && p.num_k / split >= 4 && stages == 0) {
-    if (split == 1 && p.tma_store) {
-      g_last_launch[3] = 104;
-      if (p.epilogue == EPI_RAW) return launch_lean<LEAN_RAW>(a, ld_a, w, ld_w, p, grid, s);
-      return oes == 4 ? launch_lean<LEAN_F32>(a, ld_a, w, ld_w, p, grid, s) : launch_lean<LEAN_DEQUANT>(a, ld_a, w, ld_w, p, grid, s);
-    }
+  const bool skinny = bn == 64 && g_cfg_slabs != 1 && p.num_k / split >= 4 && stages == 0;
+  if (skinny && split == 1 && p.tma_store) {
+    g_last_launch[3] = 104;
+    if (p.epilogue == EPI_RAW) return launch_lean<LEAN_RAW>(a, ld_a, w, ld_w, p, grid, s);
+    return oes == 4 ? launch_lean<LEAN_F32>(a, ld_a, w, ld_w, p, grid, s) : launch_lean<LEAN_DEQUANT>(a, ld_a, w, ld_w, p, grid, s);
+  }
+  // 64-wide tiles of two-byte outputs with consumer arithmetic: a 64-byte piece per warp instead of
+  // one 128-byte piece that the first warp of each quadrant stages alone (the epilogue of a skinny
+  // launch overlaps nothing: 64 x 4096 x 1024 with scales and bias 5.7 -> 5.1 us; raw outputs, whose
+  // staging is a handful of instructions, gain nothing from the second store and keep one piece).
+  p.half_rows = bn == 64 && split == 1 && p.tma_store && oes == 2 && p.epilogue != EPI_RAW;
+  st = make_out(p.half_rows ? 64 : 128);
+  if (st != IFLB200_OK) return st;
+  if (skinny) {
     CUtensorMap sa_map, sw_map;
     if (p.K % BK == 0 && make_slab_map(&sa_map, a, p.M, p.K, ld_a, a_rows, 4) == IFLB200_OK &&
         make_slab_map(&sw_map, w, p.N, p.K, ld_w, bn, 4) == IFLB200_OK) {
@@ -1877,6 +1872,10 @@ static int run_gemm(const void* a, int64_t ld_a, const void* w, int64_t ld_w, Ge
       return launch_gemm_form<64, 2, 2, false, kEpilogueWarps, 4>(sa_map, sw_map, to, p, grid, s);
     }
   }
+  CUtensorMap ta, tw;
+  st = make_tensor_map(&ta, a, p.M, p.K, ld_a, a_rows);
+  if (st == IFLB200_OK) st = make_tensor_map(&tw, w, p.N, p.K, ld_w, bn);
+  if (st != IFLB200_OK) return st;
   switch (bn) {
     case 256: return (stages == 3) ? launch_gemm<256, 3>(ta, tw, to, p, grid, s) : launch_gemm<256, 4>(ta, tw, to, p, grid, s);
     case 224: return launch_gemm<224, 4>(ta, tw, to, p, grid, s);
@@ -1948,17 +1947,15 @@ static int run_gemm_partials(const void* a, int64_t ld_a, const void* w, int64_t
   p.group_m = g_cfg_group_m > 0 ? g_cfg_group_m : 8;
   const int a_rows = activation_box_rows(M);
   p.a_bytes = a_rows * BK;
-  CUtensorMap ta, tw, to;
-  st = make_partials_map(&to, out, M, N, ld_out, splits, 32);
-  if (st != IFLB200_OK) return st;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (M <= BM) {
     g_last_launch[0] = 1 + 16; g_last_launch[1] = 64; g_last_launch[2] = splits; g_last_launch[3] = 104;
     return launch_lean<LEAN_PLANES>(a, ld_a, w, ld_w, p, p.num_tiles * splits, s);
   }
-  st = make_tensor_map(&ta, a, M, K, ld_a, a_rows);
-  if (st != IFLB200_OK) return st;
-  st = make_tensor_map(&tw, w, N, K, ld_w, bn);
+  CUtensorMap ta, tw, to;
+  st = make_partials_map(&to, out, M, N, ld_out, splits, 32);
+  if (st == IFLB200_OK) st = make_tensor_map(&ta, a, M, K, ld_a, a_rows);
+  if (st == IFLB200_OK) st = make_tensor_map(&tw, w, N, K, ld_w, bn);
   if (st != IFLB200_OK) return st;
   const int64_t units = (int64_t)p.num_tiles * splits;
   const int grid = units < dev->sm_count ? (int)units : dev->sm_count;
