@@ -11,10 +11,12 @@ namespace iflb200 {
 
 // 0: plain stream order; 1 (default): dependent launch for kernels over at most
 // kDependentLaunchMaxRows activation rows; 2: always.  Measured on B200: with a few hundred rows
-// (kernels of 3-50 us) early scheduling of the next kernel shortens a layer stack by 5-15 %;
-// with thousands of rows (kernels of 40-300 us) the same stack got 3-6 % slower.
+// (kernels of 3-50 us) early scheduling of the next kernel shortens a layer stack by 5-15 %, with thousands (kernels of
+// 20-150 us) by 1-7 %: diffusion blocks of 3072 columns 0.93 of the time at 2100 rows, 0.97 at 4680, 0.98 at 8192, 0.99
+// at 16384, of 1536 columns 0.93 at 3000 and 0.98 at 16384, of 5120 columns 0.96 at 2200 and 0.99 to 1.00 from 8192 on;
+// pack and GEMM of 4680 x 3072 x 3072 0.90.  More rows than that were not measured and have nothing to gain.
 extern int g_dependent_launch;
-constexpr long long kDependentLaunchMaxRows = 2048;
+constexpr long long kDependentLaunchMaxRows = 16384;
 inline bool dependent_launch_for(long long rows) {
   return g_dependent_launch == 2 || (g_dependent_launch == 1 && rows <= kDependentLaunchMaxRows);
 }
