@@ -1140,8 +1140,7 @@ amax_partial_kernel(const uint16_t* __restrict__ x, int64_t n, uint32_t* __restr
     for (int64_t i = (int64_t)blockIdx.x * kPackThreads + threadIdx.x; i < n; i += stride)
       best = max(best, (uint32_t)x[i] & 0x7FFFu);
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) best = max(best, __shfl_xor_sync(0xFFFFFFFFu, best, o));
+  best = __reduce_max_sync(0xFFFFFFFFu, best);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = best;
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -1152,54 +1151,66 @@ amax_partial_kernel(const uint16_t* __restrict__ x, int64_t n, uint32_t* __restr
 
 // n_partial > 0: dynamic scale from the partial maxima (every CTA recomputes it; CTA 0 writes
 // it out).  n_partial == 0: fixed scale read from scale_in.
+// ONE: dynamic, and the grid holds every element at four chunks a thread (n <= kPackOnePass).  The elements are then on their way before the
+// maxima are awaited: amax_partial_kernel, which is the kernel before, lets this one start only when everything before it has
+// completed, x included.  Both kernels for 2^19 elements 4.14 -> 3.48 us, 682 thousand 4.21 -> 3.57, 2^22 7.69 -> 6.80, 2^23 10.3 ->
+// 8.7; with more than one pass the loads ahead were slower (2^24 15.8 -> 16.2, 2^26 71 -> 76).
+constexpr int64_t kPackOnePass = (int64_t)kPackMaxCtas * kPackThreads * 8 * 4;
+template <bool ONE>
 __global__ void __launch_bounds__(kPackThreads)
 pack_kernel(const uint16_t* __restrict__ x, int64_t n, const uint32_t* __restrict__ partial,
             int n_partial, const float* __restrict__ scale_in, float* __restrict__ scale_out,
             uint8_t* __restrict__ q) {
-  row_dependency_wait();  // inputs may come from the kernel before this one in the stream
-  row_trigger();
   __shared__ uint32_t red[kPackThreads / 32];
-  __shared__ float s_scale;
-  if (n_partial > 0) {
-    uint32_t best = 0;
-    for (int i = threadIdx.x; i < n_partial; i += kPackThreads) best = max(best, partial[i]);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) best = max(best, __shfl_xor_sync(0xFFFFFFFFu, best, o));
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = best;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      for (int i = 1; i < kPackThreads / 32; ++i) best = max(best, red[i]);
-      const float sc = scale_of_bits(best);
-      s_scale = sc;
-      if (blockIdx.x == 0) *scale_out = sc;
-    }
-    __syncthreads();
-  } else {
-    if (threadIdx.x == 0) s_scale = *scale_in;
-    __syncthreads();
-  }
-  const float scale = s_scale;
   const bool vec = ((reinterpret_cast<uintptr_t>(x) & 15) == 0) && ((reinterpret_cast<uintptr_t>(q) & 7) == 0);
-  const int64_t stride = (int64_t)gridDim.x * kPackThreads;
+  const int64_t stride = (int64_t)gridDim.x * kPackThreads, first = (int64_t)blockIdx.x * kPackThreads + threadIdx.x;
   const int64_t nvec = vec ? n / 8 : 0;
   const uint4* xv = reinterpret_cast<const uint4*>(x);
-  // with a caller's own scale the row may hold NaN or a quotient out of range: by division
-  const float r = n_partial > 0 ? reciprocal_for_pack(scale) : __uint_as_float(0x7FC00000u);
-  for (int64_t i0 = (int64_t)blockIdx.x * kPackThreads + threadIdx.x; i0 < nvec; i0 += 4 * stride) {
-    uint4 u[4];
+  uint4 u[4];
+  auto load = [&](int64_t i0) {
 #pragma unroll
     for (int k = 0; k < 4; ++k) u[k] = i0 + k * stride < nvec ? xv[i0 + k * stride] : make_uint4(0u, 0u, 0u, 0u);
+  };
+  if (ONE) load(first);
+  row_dependency_wait();  // inputs may come from the kernel before this one in the stream
+  row_trigger();
+  float scale;
+  if (ONE || n_partial > 0) {
+    uint32_t best = 0;
+    for (int i = threadIdx.x; i < n_partial; i += kPackThreads) best = max(best, partial[i]);
+    best = __reduce_max_sync(0xFFFFFFFFu, best);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = best;
+    __syncthreads();
+    best = red[0];
+#pragma unroll
+    for (int i = 1; i < kPackThreads / 32; ++i) best = max(best, red[i]);
+    scale = scale_of_bits(best);
+    if (blockIdx.x == 0 && threadIdx.x == 0) *scale_out = scale;
+  } else {
+    scale = *scale_in;
+  }
+  // with a caller's own scale the row may hold NaN or a quotient out of range: by division
+  const float r = ONE || n_partial > 0 ? reciprocal_for_pack(scale) : __uint_as_float(0x7FC00000u);
+  auto store = [&](int64_t i0) {
 #pragma unroll
     for (int k = 0; k < 4; ++k)
       if (i0 + k * stride < nvec) reinterpret_cast<uint2*>(q)[i0 + k * stride] = pack_eight(u[k], scale, r);
+  };
+  if (ONE) {
+    store(first);
+  } else {
+    for (int64_t i0 = first; i0 < nvec; i0 += 4 * stride) {
+      load(i0);
+      store(i0);
+    }
   }
-  for (int64_t i = nvec * 8 + (int64_t)blockIdx.x * kPackThreads + threadIdx.x; i < n; i += stride)
+  for (int64_t i = nvec * 8 + first; i < n; i += stride)
     q[i] = (uint8_t)(cvt_e4m3x2(pack_one(__uint_as_float((uint32_t)x[i] << 16), scale), 0.0f) & 0xFF);
 }
 
 // Small tensors: the whole dynamic pack in one launch.  A cluster of eight CTAs (sixteen above 2^18
 // elements) keeps the tensor in registers between the maximum and the cast; the maxima of the CTAs meet in
-// distributed shared memory.  The two kernels above are two launches and two passes: 4.1 us whatever the size,
+// distributed shared memory.  The two kernels above are two launches and two passes: 3.6 us up to 700 thousand elements,
 // against 2.0 here at 2^16 elements, 3.2 at 2^18, 3.4 at 2^19; a cluster takes 4.3 for 680 thousand, so above
 // 2^19 they stay.
 constexpr int kPackClusterThreads = 1024;
@@ -1798,8 +1809,8 @@ extern "C" int iflb200_dynamic_pack_bf16_e4m3(const void* x, int64_t n, void* q,
   launch_dep(amax_partial_kernel, dim3(grid), dim3(kPackThreads), 0, s, 1, dependent_launch_for(n >> 12), reinterpret_cast<const uint16_t*>(x), n, partial);
   // The pass over the maxima is the kernel before at any size, and it is short beside a GEMM: its
   // successor starts early however large the tensor is (4680 x 3072 15.2 -> 14.9 us).
-  launch_dep(pack_kernel, dim3(grid), dim3(kPackThreads), 0, s, 1, dependent_launch_for(0), reinterpret_cast<const uint16_t*>(x), n, partial, grid, nullptr,
-                                            scale, reinterpret_cast<uint8_t*>(q));
+  launch_dep(n <= kPackOnePass ? pack_kernel<true> : pack_kernel<false>, dim3(grid), dim3(kPackThreads), 0, s, 1, dependent_launch_for(0),
+             reinterpret_cast<const uint16_t*>(x), n, partial, grid, nullptr, scale, reinterpret_cast<uint8_t*>(q));
   return (int)cudaGetLastError();
 }
 
@@ -1809,7 +1820,7 @@ extern "C" int iflb200_pack_bf16_e4m3(const void* x, int64_t n, const float* sca
   if (n == 0) return IFLB200_OK;
   if (!x || !q) return IFLB200_ERR_ARG;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  launch_dep(pack_kernel, dim3(pack_grid(n)), dim3(kPackThreads), 0, s, 1, dependent_launch_for(n >> 12), reinterpret_cast<const uint16_t*>(x), n, nullptr,
+  launch_dep(pack_kernel<false>, dim3(pack_grid(n)), dim3(kPackThreads), 0, s, 1, dependent_launch_for(n >> 12), reinterpret_cast<const uint16_t*>(x), n, nullptr,
                                                     0, scale, nullptr, reinterpret_cast<uint8_t*>(q));
   return (int)cudaGetLastError();
 }
@@ -1862,8 +1873,8 @@ extern "C" int iflb200_dynamic_pack_bf16_e4m3_noalloc(const void* x, int64_t n, 
   const int grid = pack_grid(n);  // <= kPackMaxCtas words of scratch, all written before they are read
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   launch_dep(amax_partial_kernel, dim3(grid), dim3(kPackThreads), 0, s, 1, dependent_launch_for(n >> 12), reinterpret_cast<const uint16_t*>(x), n, partial);
-  launch_dep(pack_kernel, dim3(grid), dim3(kPackThreads), 0, s, 1, dependent_launch_for(0), reinterpret_cast<const uint16_t*>(x), n, partial, grid, nullptr,
-                                            scale, reinterpret_cast<uint8_t*>(q));
+  launch_dep(n <= kPackOnePass ? pack_kernel<true> : pack_kernel<false>, dim3(grid), dim3(kPackThreads), 0, s, 1, dependent_launch_for(0),
+             reinterpret_cast<const uint16_t*>(x), n, partial, grid, nullptr, scale, reinterpret_cast<uint8_t*>(q));
   return (int)cudaGetLastError();
 }
 #endif
