@@ -9,8 +9,8 @@ buffer is allocated once (the engines' arena pattern, instinctflash/engines/comm
 The same driver runs any set of operators with the reference's signatures (``ops`` argument),
 so the reference's own kernels can be timed through it.
 
-With this package's operators the driver uses the fused forms by default (``fused="auto"``: for
-more than 64 rows): the gated activation is evaluated in the gate_up GEMM's epilogue (``fp8_linear_gated`` +
+With this package's operators the driver uses the fused forms by default for all but few and short rows
+(``fused="auto"``): the gated activation is evaluated in the gate_up GEMM's epilogue (``fp8_linear_gated`` +
 ``row_quant_from_amax`` instead of ``gemm`` + ``gated_act_quant``), bit-identical to the unfused
 sequence; ``fused=False`` keeps the reference's three-launch structure per linear.
 """
@@ -104,12 +104,13 @@ class LinearStack:
         split_rows = spec.M if split_rows is None else split_rows
         self.spec, self.weights, self.dev = spec, weights, torch.device(device)
         self.ops = ops or native_ops()
-        # fused forms exist only in this package's operator set; "auto" takes the gated epilogue where its
-        # extra short launch costs no more than the row kernel it replaces (a layer of 1024 x 4096: 26.6
-        # against 27.1 us at 50 rows, equal at 64, 30.9 against 30.4 at 96; 2048 x 16384 at 80 rows 58.1
-        # against 54.0)
+        # fused forms exist only in this package's operator set; "auto" takes the gated epilogue where its extra short
+        # launch costs no more than the row kernel it replaces, which serves few and short rows in one round of loads.  A layer
+        # unfused / fused: 1024 x 4096 17.5 / 18.2 us at 80 rows, 0.95 to 0.98 of the time up to 330, 1.00 to 1.03 at 360 to 500;
+        # 768 x 2560 0.92 to 0.98 up to 560; 1280 x 5120 0.95 to 0.99 up to 280; 2048 x 8192 0.96 to 0.99 up to 148, 1.02 to 1.04 at
+        # 150 to 240; 2048 x 11008 0.99 at 80, 1.01 to 1.10 from 96 on; 2048 x 16384 0.97 at 80, 1.01 to 1.12 from 112 on
         if fused == "auto":
-            fused = spec.M > 64
+            fused = spec.M > 64 and (spec.ffn > 8192 or spec.M * spec.ffn > 1_200_000)
         self.fused = bool(fused) and hasattr(self.ops, "fp8_linear_gated")
         self.fuse_residual = fuse_residual and hasattr(self.ops, "fp8_linear_residual")
         # deep, narrow projections (down, o) whose tiles do not fill the GPU run split-K over independent CTAs, the
