@@ -775,10 +775,7 @@ gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
   if (w_producer || a_producer) {
     // ------------------------------------------------------------------ TMA producers
     const bool weights = w_producer;
-    if (!weights) {
-      grid_dependency_wait();
-      if (lane == 0) GEMM_TRACE(3);  // the kernel before this one has completed
-    }
+    bool waited = weights;
     const uint32_t bytes = w_producer ? (uint32_t)L::kBBytes : (uint32_t)(SL * p.a_bytes);
     Ring<STAGES> ring;
     bool ok = true;
@@ -794,6 +791,11 @@ gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
         if (elect_one()) {
           const uint32_t bar = full_bar(ring.stage), sa = base + ring.stage * L::kStageBytes, sw = sa + L::kABytes;
           mbar_arrive_expect_tx(bar, bytes);
+          if (!waited) {  // directly before the first load (see gemm_lean.cuh)
+            grid_dependency_wait();
+            GEMM_TRACE(3);  // the kernel before this one has completed
+            waited = true;
+          }
           if (w_producer) {
             // SL slabs per instruction (slabs past the end of K read as zeros); the gated form's weight is mapped
             // as [2][F][K]: gate rows, then the up rows of the same hidden units, in one load
@@ -821,7 +823,10 @@ gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
     // This CTA's last loads are in flight: the next kernel in the stream may be scheduled now
     // (it becomes resident as CTAs of this grid leave and waits for the grid to complete).
     // Not earlier: CTAs parked at their dependency wait for the length of a long GEMM slow it.
-    if (!weights) grid_launch_dependents();
+    if (!weights) {
+      grid_dependency_wait();  // (a lane that has issued no load has not waited yet)
+      grid_launch_dependents();
+    }
     ring.drain(full_bar(0));
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
@@ -1182,7 +1187,7 @@ gemm_fp8_tc5_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
     // ------------------------------------------------------------------ TMA producers (both CTAs)
     // A warp per operand, the weights' one ahead of the dependency wait, as in the single-CTA kernel.
     const bool weights = w_producer;
-    if (!weights) grid_dependency_wait();
+    bool waited = weights;
     Ring<STAGES> ring;
     bool ok = true;
     uint32_t it = 0;
@@ -1197,13 +1202,18 @@ gemm_fp8_tc5_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
         if (elect_one()) {
           if (leader) mbar_arrive_expect_tx(full_bar(ring.stage), 2u * (w_producer ? L::kBBytes : L::kABytes));
           const uint32_t dst = base + ring.stage * L::kStageBytes + (w_producer ? L::kABytes : 0);
+          if (!waited) grid_dependency_wait();  // directly before the first load (see gemm_lean.cuh)
+          waited = true;
           tma_load_2d_pair(dst, w_producer ? &tm_w : &tm_a, full_bar(ring.stage) & kPeerBitMask, kb * BK, row);
         }
         __syncwarp();
         ring.advance();
       }
     }
-    if (!weights) grid_launch_dependents();  // last loads issued: the next kernel may be scheduled
+    if (!weights) {  // last loads issued: the next kernel may be scheduled
+      grid_dependency_wait();  // (a lane that has issued no load has not waited yet)
+      grid_launch_dependents();
+    }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (leader only)
     if (leader) {

@@ -198,7 +198,7 @@ gemm_fp8_tc5_tokens_kernel(const __grid_constant__ CUtensorMap tm_t, const __gri
     // ------------------------------------------------------------------ TMA producers (both CTAs)
     // Two warps for each operand, which take the slabs in turn; the weights' ahead of the dependency wait, as in the
     // other forms.
-    if (t_producer) grid_dependency_wait();
+    bool waited = w_producer;
     const uint64_t policy = l2_evict_first();
     int slot = producer >> 1, skip = producer >> 1;  // skip: slabs of the other warp until this one's next
     uint32_t phase = 0;
@@ -220,6 +220,8 @@ gemm_fp8_tc5_tokens_kernel(const __grid_constant__ CUtensorMap tm_t, const __gri
           const int x = (kb0 + i) * BK;
           if (i < slabs) {
             if (leader) mbar_arrive_expect_tx(bar, 2u * (w_producer ? w_bytes : t_bytes));
+            if (!waited) grid_dependency_wait();  // directly before the first load (see gemm_lean.cuh)
+            waited = true;
             if (t_producer) tma_load_2d_pair(dst + w_bytes, &tm_t, bar & kPeerBitMask, x, t_row);
             else if constexpr (EPI == TOK_GATED) {
               if (p.evict) tma_load_4d_pair_hint(dst, &tm_w, bar & kPeerBitMask, x, 0, 0, w_row / 16, policy);
@@ -239,7 +241,10 @@ gemm_fp8_tc5_tokens_kernel(const __grid_constant__ CUtensorMap tm_t, const __gri
       }
       skip = i - taken;
     }
-    if (t_producer) grid_launch_dependents();  // last loads issued: the next kernel may be scheduled
+    if (t_producer) {  // last loads issued: the next kernel may be scheduled
+      grid_dependency_wait();  // (a lane that has issued no load has not waited yet)
+      grid_launch_dependents();
+    }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (leader only)
     // One thread runs the whole loop: votes and elections per slab took the warp about 100 clocks more.
