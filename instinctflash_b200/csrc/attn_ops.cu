@@ -54,8 +54,6 @@ template <int IT, bool CL, int kGroup>
 __global__ void __launch_bounds__(kCombineThreads, kGroup == 4 ? 2 : 1) attn_combine_quant_kernel(const CombineArgs a) {
   const int threads = blockDim.x;
   if (CL) cluster_arrive();  // this CTA runs: its shared memory may be written from now on
-  grid_dependency_wait();  // the partials come from the kernel before this one in the stream
-  grid_launch_dependents();
   __shared__ float red[kCombineThreads / 32];
   __shared__ float maxima[kCombineMaxCluster];
   const int t = CL ? blockIdx.x / a.cluster : blockIdx.x, b = blockIdx.y;
@@ -67,6 +65,20 @@ __global__ void __launch_bounds__(kCombineThreads, kGroup == 4 ? 2 : 1) attn_com
   const int total = min(all, first + share);  // this CTA's chunks: [first, total)
   const int n_rows = a.tokens * a.group;
   const int64_t plane = (int64_t)a.batch * a.heads_kv * n_rows;  // rows of one split
+  // where the first chunk's partials are, worked out ahead of the wait, which its divisions used to follow (708 tokens x 8 x 64, 14
+  // splits 6.54 -> 5.91 us behind one another; 0.96 of the time over 41 sizes)
+  const auto place = [&](int c, int& head, int& d, int64_t& row) {
+    head = c / chunks_per_head;
+    d = (c - head * chunks_per_head) * 4;
+    const int kvh = head / a.group, h = head - kvh * a.group;
+    row = ((int64_t)b * a.heads_kv + kvh) * n_rows + (int64_t)t * a.group + h;
+  };
+  int head0, d0;
+  int64_t row0;
+  place(first + threadIdx.x, head0, d0, row0);
+  asm volatile("" : "+r"(head0), "+r"(d0), "+l"(row0));
+  grid_dependency_wait();  // the partials come from the kernel before this one in the stream
+  grid_launch_dependents();
   float out[IT][4];
   float amax = 0.0f;
 #pragma unroll
@@ -75,9 +87,9 @@ __global__ void __launch_bounds__(kCombineThreads, kGroup == 4 ? 2 : 1) attn_com
 #pragma unroll
     for (int i = 0; i < 4; ++i) out[it][i] = 0.0f;
     if (c < total) {
-      const int head = c / chunks_per_head, d = (c - head * chunks_per_head) * 4;
-      const int kvh = head / a.group, h = head - kvh * a.group;
-      const int64_t row = ((int64_t)b * a.heads_kv + kvh) * n_rows + (int64_t)t * a.group + h;
+      int head = head0, d = d0;
+      int64_t row = row0;
+      if (it > 0) place(c, head, d, row);
       const float *pm = a.pm + row, *pl = a.pl + row, *po = a.po + row * a.block_d + d;
       float gm[kGroup], gl[kGroup];
       float4 gv[kGroup];
@@ -168,7 +180,7 @@ __global__ void __launch_bounds__(kCombineThreads, kGroup == 4 ? 2 : 1) attn_com
   for (int it = 0; it < IT; ++it) {
     const int c = first + it * threads + threadIdx.x;
     if (c < total) {
-      const int head = c / chunks_per_head, d = (c - head * chunks_per_head) * 4;
+      const int head = it == 0 ? head0 : c / chunks_per_head, d = it == 0 ? d0 : (c - head * chunks_per_head) * 4;
       *reinterpret_cast<uint32_t*>(qr + (int64_t)head * a.head_dim + d) =
           cvt_e4m3x4(__fmul_rn(out[it][0], inv), __fmul_rn(out[it][1], inv), __fmul_rn(out[it][2], inv),
                      __fmul_rn(out[it][3], inv));

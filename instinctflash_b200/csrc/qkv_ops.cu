@@ -191,19 +191,23 @@ __device__ __forceinline__ void load_vec_f32(const float* p, float (&o)[VEC]) {
 template <typename OT, int VEC>
 __global__ void __launch_bounds__(256) qkv_split_vec_kernel(const QkvSplitArgs a) {
   using P = typename Pack<VEC>::type;
-  if (threadIdx.x == 0) grid_dependency_wait();
-  __syncthreads();
-  grid_launch_dependents();
+  // Which token and head, and where they are, is worked out ahead of the wait, which the two 64-bit divisions used to follow:
+  // 69 x 24 heads x 128 2.15 -> 1.95 us behind one another, 0.96 of the time over 40 sizes (with the token kernel's, unchanged).
   const int lane = threadIdx.x & 31;
   const int heads = a.HQ + 2 * a.HKV;
   const int64_t unit = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (unit >= (int64_t)a.T * heads) return;
-  const int t = (int)(unit / heads);
-  const int h = (int)(unit % heads);
+  const bool one_word = (int64_t)a.T * heads < (1ll << 31);
+  int t = one_word ? (int)((uint32_t)unit / (uint32_t)heads) : (int)(unit / heads);
+  int h = (int)(unit - (int64_t)t * heads);
   constexpr int half = 32 * VEC;
   const int i0 = lane * VEC;
   const __nv_bfloat16* src =
       reinterpret_cast<const __nv_bfloat16*>(a.qkv) + (int64_t)t * a.ld_qkv + (int64_t)h * (2 * half) + i0;
+  asm volatile("" : "+r"(t), "+r"(h), "+l"(src));
+  if (threadIdx.x == 0) grid_dependency_wait();
+  __syncthreads();
+  grid_launch_dependents();
+  if (t >= a.T) return;
   const P pl = *reinterpret_cast<const P*>(src);
   const P ph = *reinterpret_cast<const P*>(src + half);
   const bool has_row = a.row != nullptr;

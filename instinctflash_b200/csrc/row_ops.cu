@@ -1541,17 +1541,19 @@ template <int Q>
 __global__ void __launch_bounds__(kRowThreads)
 quant_from_amax_kernel(const float* __restrict__ h, int64_t ld_h, int M, int F, const float* __restrict__ amax,
                        float* __restrict__ amax_zero, uint8_t* __restrict__ q, int64_t ld_q, float* __restrict__ qs, int early) {
-  row_begin(early);  // h and amax come from the kernel before this one in the stream
+  row_open(early);
   const int m = blockIdx.y;
   const int c0 = blockIdx.x * (kRowThreads * 4 * Q) + threadIdx.x * 4;
-  const float* src = h + (int64_t)m * ld_h + c0;
+  const float *src = h + (int64_t)m * ld_h + c0, *top = amax + m;
   uint8_t* dst = q + (int64_t)m * ld_q + c0;
+  keep(F); keep(src); keep(top); keep(dst);
+  row_enter(early);  // h and amax come from the kernel before this one in the stream
   float4 v[Q];
 #pragma unroll
   for (int i = 0; i < Q; ++i)
     if (c0 + i * kRowThreads * 4 < F) v[i] = *reinterpret_cast<const float4*>(src + i * kRowThreads * 4);
   float scale, inv;
-  quant_scales(amax[m], scale, inv);
+  quant_scales(*top, scale, inv);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     qs[m] = scale;
     if (amax_zero) amax_zero[m] = 0.0f;
