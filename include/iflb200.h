@@ -247,10 +247,11 @@ IFLB200_API int iflb200_residual_norm_quant_peers(void* res, int res_dtype, int6
  * accumulation on the tcgen05 tensor cores, unit scales.  K, N multiples of 16.
  * Ordering on the stream (this and every other GEMM entry point): with dependent launch enabled
  * (iflb200_set_dependent_launch, the default) the kernel becomes resident while the kernel enqueued
- * immediately before it is still running and loads its first weight boxes before it waits for that
- * kernel; `a`, the scales and everything else are read
- * after the wait.  So `w` must not be an OUTPUT of the kernel enqueued immediately before on the
- * same stream (weights are packed at load time; activations may of course come from that kernel).
+ * immediately before it is still running and, with M <= 2048, loads its first weight boxes before it waits
+ * for that kernel; `a`, the scales and everything else are read
+ * after the wait.  So with M <= 2048 `w` must not be an OUTPUT of the kernel enqueued immediately before on the
+ * same stream (weights are packed at load time; activations may of course come from that kernel).  With more
+ * rows `w` is read after the wait too, in every mode, and may be such an output.
  * Replaces: instinctflash/kernels/fp8.py:50-53 (gemm -> torch._scaled_mm).
  */
 IFLB200_API int iflb200_gemm_fp8_raw(const void* a, int64_t ld_a, const void* w, int64_t ld_w,
@@ -519,9 +520,10 @@ IFLB200_API int iflb200_gemm_set_split_k(int split_k);
 IFLB200_API int iflb200_row_set_group(int threads_per_row);
 /* Programmatic dependent launch: a kernel launched this way may be scheduled while its
  * predecessor in the stream drains; it waits for the predecessor's results before its first
- * access to memory a kernel can write, and the GEMM warms L2 with its first weight boxes
+ * access to memory a kernel can write, except that a GEMM of at most 2048 rows loads its first weight boxes
  * meanwhile.  1 (default) = for calls over at most 16384 activation rows (it shortens a layer
- * stack by up to a tenth; longer kernels have nothing to gain), 0 = never, 2 = always.  Results are identical in every mode.  No reference counterpart. */
+ * stack by up to a tenth; longer kernels have nothing to gain), 0 = never, 2 = always.  Results are identical in every
+ * mode for calls that keep the rule on weights of iflb200_gemm_fp8_raw.  No reference counterpart. */
 IFLB200_API int iflb200_set_dependent_launch(int enable);
 /* Kernel family: 0 = heuristic, 1 = single-CTA tiles only, 2 / 3 = 256x256 tiles on CTA pairs
  * (cta_group::2) with one / two tensor-memory accumulators; add 16 to store the epilogue

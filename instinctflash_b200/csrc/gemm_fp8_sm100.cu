@@ -770,12 +770,12 @@ gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
   // written waits for that kernel first: the producer of the activations and the epilogue warps.  The
   // weights are not an output of the kernel before this one (contract: see iflb200_gemm_fp8_raw), so their
   // producer starts at once, and their DRAM round trip -- the longest single latency of a 4 us
-  // skinny kernel -- runs while that kernel drains.
+  // skinny kernel -- runs while that kernel drains.  With more rows than kEarlyWeightsMaxRows it waits too.
   const bool w_producer = warp == 0, a_producer = warp == 2 + EW;
   if (w_producer || a_producer) {
     // ------------------------------------------------------------------ TMA producers
     const bool weights = w_producer;
-    bool waited = weights;
+    bool waited = weights && p.M <= kEarlyWeightsMaxRows;
     const uint32_t bytes = w_producer ? (uint32_t)L::kBBytes : (uint32_t)(SL * p.a_bytes);
     Ring<STAGES> ring;
     bool ok = true;
@@ -1185,9 +1185,9 @@ gemm_fp8_tc5_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
   const bool w_producer = warp == 0, a_producer = warp == 2 + EW;
   if (w_producer || a_producer) {
     // ------------------------------------------------------------------ TMA producers (both CTAs)
-    // A warp per operand, the weights' one ahead of the dependency wait, as in the single-CTA kernel.
+    // A warp per operand, the weights' one ahead of the dependency wait for few rows, as in the single-CTA kernel.
     const bool weights = w_producer;
-    bool waited = weights;
+    bool waited = weights && p.M <= kEarlyWeightsMaxRows;
     Ring<STAGES> ring;
     bool ok = true;
     uint32_t it = 0;

@@ -87,11 +87,11 @@ gemm_fp8_tc5_lean_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  // As in the other forms: only the activations and the epilogue wait for the kernel before this one.
+  // As in the other forms: up to kEarlyWeightsMaxRows only the activations and the epilogue wait for the kernel before this one.
   const bool w_producer = warp == 0, a_producer = warp == 10;
   if (w_producer || a_producer) {
     // ------------------------------------------------------------------ TMA producers
-    bool waited = w_producer;
+    bool waited = w_producer && p.M <= kEarlyWeightsMaxRows;
     const uint32_t slab_bytes = w_producer ? (uint32_t)(BN * BK) : (uint32_t)p.a_bytes;
     Ring<STAGES> ring;
     bool ok = true;

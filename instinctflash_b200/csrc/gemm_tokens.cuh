@@ -196,9 +196,9 @@ gemm_fp8_tc5_tokens_kernel(const __grid_constant__ CUtensorMap tm_t, const __gri
   const bool w_producer = (producer & 1) == 0, t_producer = !w_producer;
   if (producer >= 0) {
     // ------------------------------------------------------------------ TMA producers (both CTAs)
-    // Two warps for each operand, which take the slabs in turn; the weights' ahead of the dependency wait, as in the
-    // other forms.
-    bool waited = w_producer;
+    // Two warps for each operand, which take the slabs in turn; the weights' ahead of the dependency wait for few rows, as
+    // in the other forms.
+    bool waited = w_producer && p.M <= kEarlyWeightsMaxRows;
     const uint64_t policy = l2_evict_first();
     int slot = producer >> 1, skip = producer >> 1;  // skip: slabs of the other warp until this one's next
     uint32_t phase = 0;

@@ -68,7 +68,10 @@ def _operands(a: torch.Tensor, w: Fp8Weight):
 
 
 def gemm(a: torch.Tensor, w: Fp8Weight, out: torch.Tensor) -> torch.Tensor:
-    """out[M, N] (bf16) = a[M, K] (e4m3) @ w.w[N, K]^T, unscaled raw accumulator."""
+    """out[M, N] (bf16) = a[M, K] (e4m3) @ w.w[N, K]^T, unscaled raw accumulator.
+
+    With at most 2048 rows, here and in every function below, the kernel reads its first weights while the kernel
+    enqueued directly before it still runs: ``w.w`` must not be that kernel's output (include/iflb200.h)."""
     if native.gemm(a, w.w, out):
         return out
     M, N, K = _operands(a, w)
