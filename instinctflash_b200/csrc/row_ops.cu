@@ -908,37 +908,44 @@ __host__ __device__ constexpr int row_cta_min_blocks() {
 template <typename RT, int IT, int PL, bool PLAIN>
 __global__ void __launch_bounds__(kRowThreads, row_cta_min_blocks<IT, PL>())
 residual_norm_planes_kernel(const ResNormArgs a) {
-  row_open(a.early);
   static_assert(kRowThreads == 256, "eight warps per row");
   __shared__ __align__(16) float red[3][kRowThreads / 32];
   constexpr int kStep = kRowThreads * 4;
   const int m = blockIdx.x, c = threadIdx.x * 4;
-  int D = a.D, splits = a.dsplits;
-  RT* rr = reinterpret_cast<RT*>(a.res) + (int64_t)m * a.ld_res + c;
-  const float* dp = a.dpart + (int64_t)m * a.ld_delta + c;
-  int64_t dp_plane = (int64_t)a.M * a.ld_delta;
-  const float *col = a.dcol + c, *row = a.drow + m;
-  uint8_t* q = a.q + (int64_t)m * a.ld_q + c;
-  float *qs = a.qs + m, eps = a.eps;
+  // What PLAIN computes from its arguments ahead of the wait.  The general form has no registers for it: with these
+  // held it took up to 1.2 times as long (1677 x 1456 in eight planes 20.6 -> 23.7 us).
+  int D_kept = a.D, splits_kept = a.dsplits;
+  RT* rr_kept = reinterpret_cast<RT*>(a.res) + (int64_t)m * a.ld_res + c;
+  const float *dp_kept = a.dpart + (int64_t)m * a.ld_delta + c, *col_kept = a.dcol + c, *row_kept = a.drow + m;
+  int64_t plane_kept = (int64_t)a.M * a.ld_delta;
+  uint8_t* q_kept = a.q + (int64_t)m * a.ld_q + c;
+  float *qs_kept = a.qs + m, eps_kept = a.eps;
   if (PLAIN) {
-    keep(D); keep(splits); keep(rr); keep(dp); keep(col); keep(row); keep(q); keep(qs);
-    asm volatile("" : "+l"(dp_plane), "+f"(eps));
+    row_open(a.early);
+    keep(D_kept); keep(splits_kept); keep(rr_kept); keep(dp_kept); keep(col_kept); keep(row_kept); keep(q_kept); keep(qs_kept);
+    asm volatile("" : "+l"(plane_kept), "+f"(eps_kept));
+    row_enter(a.early);  // inputs may come from the kernel before this one in the stream
+  } else {
+    row_begin(a.early);
   }
-  row_enter(a.early);  // inputs may come from the kernel before this one in the stream
+#define KEPT(kept, value) (PLAIN ? (kept) : (value))
+  RT* rr = KEPT(rr_kept, reinterpret_cast<RT*>(a.res) + (int64_t)m * a.ld_res + c);
   const int64_t mofs = !PLAIN && a.mod_index ? (int64_t)a.mod_index[m] * a.D + c : c;
-  const float drs = PLAIN || a.drow ? *row : 1.0f;
+  const float drs = PLAIN ? *row_kept : a.drow ? a.drow[m] : 1.0f;
 
   Quad<RT> rres[IT];
   Quad<float> plane[PL][IT], dcol[IT];
+  const float* dp = KEPT(dp_kept, a.dpart + (int64_t)m * a.ld_delta + c);
+  const int64_t dp_plane = KEPT(plane_kept, (int64_t)a.M * a.ld_delta);
 #pragma unroll
   for (int it = 0; it < IT; ++it) {
-    if (it * kStep + c < D) {
+    if (it * kStep + c < KEPT(D_kept, a.D)) {
       rres[it].load(rr + it * kStep);
-      if (PLAIN || a.dcol) dcol[it].load(col + it * kStep);
+      if (PLAIN || a.dcol) dcol[it].load(KEPT(col_kept, a.dcol + c) + it * kStep);
     }
 #pragma unroll
     for (int s = 0; s < PL; ++s)
-      if (s < splits && it * kStep + c < D) plane[s][it].load(dp + s * dp_plane + it * kStep);
+      if (s < KEPT(splits_kept, a.dsplits) && it * kStep + c < KEPT(D_kept, a.D)) plane[s][it].load(dp + s * dp_plane + it * kStep);
   }
   float x[IT][4];
   float sum = 0.0f;
@@ -947,13 +954,13 @@ residual_norm_planes_kernel(const ResNormArgs a) {
     const int o = it * kStep;
 #pragma unroll
     for (int i = 0; i < 4; ++i) x[it][i] = 0.0f;
-    if (o + c < D) {
+    if (o + c < KEPT(D_kept, a.D)) {
       rres[it].widen(x[it]);
       float d[4], op[4];
       plane[0][it].widen(d);  // the planes in split order, then the raw accumulator's rounding point
 #pragma unroll
       for (int s = 1; s < PL; ++s) {
-        if (s < splits) {
+        if (s < KEPT(splits_kept, a.dsplits)) {
           float e[4];
           plane[s][it].widen(e);
 #pragma unroll
@@ -962,14 +969,14 @@ residual_norm_planes_kernel(const ResNormArgs a) {
       }
       if (PL < 8) {
 #pragma unroll 1
-        for (int s0 = PL; s0 < splits; s0 += PL) {
+        for (int s0 = PL; s0 < KEPT(splits_kept, a.dsplits); s0 += PL) {
           float e[PL][4];
 #pragma unroll
           for (int s = 0; s < PL; ++s)
-            if (s0 + s < splits) load_quad(dp + (s0 + s) * dp_plane + o, e[s]);
+            if (s0 + s < KEPT(splits_kept, a.dsplits)) load_quad(dp + (s0 + s) * dp_plane + o, e[s]);
 #pragma unroll
           for (int s = 0; s < PL; ++s) {
-            if (s0 + s < splits) {
+            if (s0 + s < KEPT(splits_kept, a.dsplits)) {
 #pragma unroll
               for (int i = 0; i < 4; ++i) d[i] = __fadd_rn(d[i], e[s][i]);
             }
@@ -997,7 +1004,7 @@ residual_norm_planes_kernel(const ResNormArgs a) {
       if (PLAIN || a.write_res) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) x[it][i] = round_through<RT>(x[it][i]);
-        store_quad(rr, dtype_of<RT>(), o, x[it]);
+        store_quad(KEPT((void*)rr, a.res), dtype_of<RT>(), KEPT(0, (int64_t)m * a.ld_res + c) + o, x[it]);
       }
 #pragma unroll
       for (int i = 0; i < 4; ++i) sum = !PLAIN && a.layernorm ? __fadd_rn(sum, x[it][i]) : __fmaf_rn(x[it][i], x[it][i], sum);
@@ -1005,7 +1012,7 @@ residual_norm_planes_kernel(const ResNormArgs a) {
   }
   if (!PLAIN && a.q == nullptr && a.y == nullptr) return;  // residual update only (uniform across the CTA)
 
-  const float fD = (float)D;
+  const float fD = (float)KEPT(D_kept, a.D);
   float amax = 0.0f;
   if (PLAIN) {  // rounding keeps the order of the |x| rstd, so that the largest |x| gives the largest of them: one meeting for both
 #pragma unroll
@@ -1019,7 +1026,7 @@ residual_norm_planes_kernel(const ResNormArgs a) {
     sum = 0.0f;
 #pragma unroll
     for (int it = 0; it < IT; ++it) {
-      if (it * kStep + c < D) {
+      if (it * kStep + c < KEPT(D_kept, a.D)) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           x[it][i] = __fadd_rn(x[it][i], -mean);
@@ -1029,11 +1036,11 @@ residual_norm_planes_kernel(const ResNormArgs a) {
     }
     sum = row_cta_reduce<false>(sum, red[1]);
   }
-  const float rstd = rsqrt_approx_ftz(__fadd_rn(div_full(sum, fD), eps));
+  const float rstd = rsqrt_approx_ftz(__fadd_rn(div_full(sum, fD), KEPT(eps_kept, a.eps)));
 #pragma unroll
   for (int it = 0; it < IT; ++it) {
     const int o = it * kStep;
-    if (o + c < D) {
+    if (o + c < KEPT(D_kept, a.D)) {
       float op[4];
       ChainV<4> ch(x[it]);
       ch.mul(rstd);
@@ -1067,10 +1074,11 @@ residual_norm_planes_kernel(const ResNormArgs a) {
   }
   float scale, inv;
   quant_scales(amax, scale, inv);
-  if (threadIdx.x == 0) *qs = scale;
+  if (threadIdx.x == 0) *KEPT(qs_kept, a.qs + m) = scale;
+  uint8_t* q = KEPT(q_kept, a.q + (int64_t)m * a.ld_q + c);
 #pragma unroll
   for (int it = 0; it < IT; ++it) {
-    if (it * kStep + c < D) {
+    if (it * kStep + c < KEPT(D_kept, a.D)) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) x[it][i] = __fmul_rn(x[it][i], inv);
       const uint32_t code = cvt_e4m3x4(x[it][0], x[it][1], x[it][2], x[it][3]);
@@ -1086,6 +1094,7 @@ residual_norm_planes_kernel(const ResNormArgs a) {
       if (!PLAIN && k < a.mirrors) a.qs_mirror[k][m] = scale;
   }
 }
+#undef KEPT
 
 // Rows of at most 8192 columns on the aligned path.  The quads form takes its further plane groups quad by quad, each
 // a round trip, and that many registers let few rows be resident: it serves the widths and numbers of planes
