@@ -845,7 +845,7 @@ residual_norm_quant_kernel(const ResNormArgs a) {
 // PL: planes loaded together (further ones follow in groups of PL).
 // PLAIN: the decoder layer's operands alone (resnorm_plain), in a quarter of the code and with one meeting of the row's
 // warps for the sum and the maximum: 50 x 1024 with eight planes 2.42 -> 1.77 us, 816 x 2048 with two 5.59 -> 3.89, 18 expert
-// layers 403 -> 381; over 250 sizes of 1 to 2000 rows 0.80 of the time, one more than 3 % slower (2000 x 2048, eight planes 27.0, 28.3).
+// layers 403 -> 381; over 250 sizes of 1 to 2000 rows 0.80 of the time, but for many bytes of planes (launch_resnorm_planes_form).
 // --------------------------------------------------------------------------------------------
 template <typename T>
 struct Quad;
@@ -1108,7 +1108,11 @@ residual_norm_planes_kernel(const ResNormArgs a) {
 template <typename RT, int IT, int PL>
 static void launch_resnorm_planes_form(const ResNormArgs& a, cudaStream_t s) {
   if constexpr (IT <= 2) {
-    if (resnorm_plain(a)) {
+    // More than 32 MB of planes, five to eight of them and a wide row: the general form streams them
+    // faster (measured; why was not looked into).  PLAIN against general: 500 x 2048 in eight 1.00, 600 1.05, 1000 1.09,
+    // 600 x 1792 in seven 0.98, 700 1.08; under 10240 columns x planes PLAIN stays ahead (3000 x 1536 in six 0.98).
+    const bool many_bytes = IT == 2 && PL == 8 && a.D * a.dsplits >= 10240 && (int64_t)a.M * a.D * a.dsplits > (1 << 23);
+    if (!many_bytes && resnorm_plain(a)) {
       launch_dep(residual_norm_planes_kernel<RT, IT, PL, true>, dim3(a.M), dim3(kRowThreads), 0, s, 1, dependent_launch_for(a.M), a);
       return;
     }

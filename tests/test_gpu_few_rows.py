@@ -66,3 +66,19 @@ def test_plain_residual_bits(D, planes, dtype):
         torch.cuda.synchronize()
         (r0, q0, s0), (r1, q1, s1) = outs
         assert torch.equal(u8(r0), u8(r1)) and torch.equal(u8(q0), u8(q1)) and torch.equal(i32(s0), i32(s1))
+
+
+# either side of the 32 MB of planes from which a plain call takes the general form
+@pytest.mark.parametrize("M,D,planes", [(512, 2048, 8), (513, 2048, 8), (819, 1280, 8), (820, 1280, 8), (820, 2048, 5)])
+def test_plain_residual_bits_of_many_planes(M, D, planes):
+    from instinctflash_b200.kernels import norm
+    g = torch.Generator(device=DEV).manual_seed(M)
+    res0, delta = torch.randn(M, D, device=DEV, generator=g), torch.randn(planes, M, D, device=DEV, generator=g)
+    row, col = torch.rand(M, device=DEV, generator=g), torch.rand(D, device=DEV, generator=g)
+    outs = []
+    for weight in (None, torch.ones(D, device=DEV)):
+        res, q, s = res0.clone(), torch.empty(M, D, device=DEV, dtype=E4M3), torch.empty(M, device=DEV)
+        norm.residual_norm_quant(res, delta=delta, delta_row=row, delta_col=col, weight=weight, q=q, q_scale=s)
+        outs.append((res, q, s))
+    torch.cuda.synchronize()
+    assert all(torch.equal(u8(a), u8(b)) for a, b in zip(*outs))
