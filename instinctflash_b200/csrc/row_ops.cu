@@ -320,7 +320,7 @@ row_quant_kernel(const RowQuantArgs a) {
   int K = a.K;
   uint8_t* qr = a.q + (live ? (int64_t)m * a.ld_q : 0);
   float* qs = a.qs + (live ? m : 0);
-  keep(K); keep(xr); keep(qr); keep(qs);
+  if (PLAIN || sizeof(XT) == 2) { keep(K); keep(xr); keep(qr); keep(qs); }
   row_enter(a.early);  // inputs may come from the kernel before this one in the stream
   const float rs = (live && a.row) ? a.row[m] : 1.0f;
 
