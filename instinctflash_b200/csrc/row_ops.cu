@@ -912,26 +912,26 @@ residual_norm_planes_kernel(const ResNormArgs a) {
   __shared__ __align__(16) float red[3][kRowThreads / 32];
   constexpr int kStep = kRowThreads * 4;
   const int m = blockIdx.x, c = threadIdx.x * 4;
-  // What PLAIN computes from its arguments ahead of the wait.  The general form has no registers for it: with these
-  // held it took up to 1.2 times as long (1677 x 1456 in eight planes 20.6 -> 23.7 us).
+  // What is computed from the arguments ahead of the wait, for PLAIN certain to be in registers then.  The general form over up to
+  // eight planes has none to spare: with these ahead it took up to 1.2 times as long (1677 x 1456 in eight 20.6 -> 23.7 us);
+  // over up to four planes a group it gains by them (3770 x 392 18.9 -> 16.5, 334 x 136 in two 2.73 -> 2.39).
+  constexpr bool kAhead = PLAIN || PL < 8;
   int D_kept = a.D, splits_kept = a.dsplits;
   RT* rr_kept = reinterpret_cast<RT*>(a.res) + (int64_t)m * a.ld_res + c;
   const float *dp_kept = a.dpart + (int64_t)m * a.ld_delta + c, *col_kept = a.dcol + c, *row_kept = a.drow + m;
   int64_t plane_kept = (int64_t)a.M * a.ld_delta;
   uint8_t* q_kept = a.q + (int64_t)m * a.ld_q + c;
   float *qs_kept = a.qs + m, eps_kept = a.eps;
+  row_open(a.early);
   if (PLAIN) {
-    row_open(a.early);
     keep(D_kept); keep(splits_kept); keep(rr_kept); keep(dp_kept); keep(col_kept); keep(row_kept); keep(q_kept); keep(qs_kept);
     asm volatile("" : "+l"(plane_kept), "+f"(eps_kept));
-    row_enter(a.early);  // inputs may come from the kernel before this one in the stream
-  } else {
-    row_begin(a.early);
   }
-#define KEPT(kept, value) (PLAIN ? (kept) : (value))
+  row_enter(a.early);  // inputs may come from the kernel before this one in the stream
+#define KEPT(kept, value) (kAhead ? (kept) : (value))
   RT* rr = KEPT(rr_kept, reinterpret_cast<RT*>(a.res) + (int64_t)m * a.ld_res + c);
   const int64_t mofs = !PLAIN && a.mod_index ? (int64_t)a.mod_index[m] * a.D + c : c;
-  const float drs = PLAIN ? *row_kept : a.drow ? a.drow[m] : 1.0f;
+  const float drs = PLAIN || a.drow ? *KEPT(row_kept, a.drow + m) : 1.0f;
 
   Quad<RT> rres[IT];
   Quad<float> plane[PL][IT], dcol[IT];
