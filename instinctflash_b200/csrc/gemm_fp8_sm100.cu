@@ -1491,7 +1491,7 @@ static int launch_gemm_form(const CUtensorMap& ta, const CUtensorMap& tw, const 
   }
   const cudaError_t e = launch_dep(gemm_fp8_tc5_kernel<BN, STAGES, SPLIT, GATED, EW, SL>, dim3(grid),
                                    dim3(96 + 32 * EW), L::kDynamic, s, p.split_k,
-                                   dependent_launch_for(p.M), ta, tw, to, p);
+                                   dependent_launch_for(p.M, true), ta, tw, to, p);
   note_captured_gemm(s);
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
@@ -1525,7 +1525,7 @@ static int launch_lean_form(const CUtensorMap& ta, const CUtensorMap& tw, const 
     attr_set[dev] = true;
   }
   const cudaError_t e = launch_dep(gemm_fp8_tc5_lean_kernel<AR, EPI>, dim3(grid), dim3(LeanLayout<AR>::kThreads),
-                                   LeanLayout<AR>::kDynamic, s, 1, dependent_launch_for(p.M), ta, tw, p);
+                                   LeanLayout<AR>::kDynamic, s, 1, dependent_launch_for(p.M, true), ta, tw, p);
   note_captured_gemm(s);
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
@@ -1564,7 +1564,7 @@ static int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tw, const 
     attr_set[dev] = true;
   }
   const cudaError_t e = launch_dep(gemm_fp8_tc5_pair_kernel<BN, STAGES, ACC, GATED, EW>, dim3(grid), dim3(96 + 32 * EW),
-                                   L::kDynamic, s, 1, dependent_launch_for(p.M), ta, tw, to, p);
+                                   L::kDynamic, s, 1, dependent_launch_for(p.M, true), ta, tw, to, p);
   note_captured_gemm(s);
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
@@ -1638,7 +1638,7 @@ static int launch_tokens(const void* a, int64_t ld_a, const void* w, int64_t ld_
   g_last_launch[1] = bt; g_last_launch[2] = p.parts; g_last_launch[3] = p.slots;
   const cudaError_t e = launch_dep(gemm_fp8_tc5_tokens_kernel<EPI>, dim3(2 * (unsigned)(units < pairs ? units : pairs)),
                                    dim3(L::kThreads), L::kFixed + p.slots * L::slab_bytes(bt), s, 1,
-                                   dependent_launch_for(g.M), tt, tw, p);
+                                   dependent_launch_for(g.M, true), tt, tw, p);
   note_captured_gemm(s);
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }

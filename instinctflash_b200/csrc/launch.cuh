@@ -9,16 +9,26 @@
 
 namespace iflb200 {
 
-// 0: plain stream order; 1 (default): dependent launch for kernels over at most
-// kDependentLaunchMaxRows activation rows; 2: always.  Measured on B200: with a few hundred rows
-// (kernels of 3-50 us) early scheduling of the next kernel shortens a layer stack by 5-15 %, with thousands (kernels of
-// 20-150 us) by 1-7 %: diffusion blocks of 3072 columns 0.93 of the time at 2100 rows, 0.97 at 4680, 0.98 at 8192, 0.99
-// at 16384, of 1536 columns 0.93 at 3000 and 0.98 at 16384, of 5120 columns 0.96 at 2200 and 0.99 to 1.00 from 8192 on;
-// pack and GEMM of 4680 x 3072 x 3072 0.90.  More rows than that were not measured and have nothing to gain.
+// 0: plain stream order; 1 (default): dependent launch for kernels over at most kDependentRows activation rows, and up to
+// kDependentRowsLong where the kernel says so (`many`); 2: always.  Measured on B200: with a few hundred rows
+// (kernels of 3-50 us) early scheduling of the next kernel shortens a layer stack by 5-15 %.  Over more than 2048 rows a
+// launch's share of the time is small, and what is scheduled early can be in the way of what still runs.  Time with
+// dependent launch over time without it, 2049 to 16384 rows, each operator directly behind a GEMM, by elements:
+//   GEMM forms                   0.94 to 1.00 (0.97 in the mean; 16384 x 5120 x 5120 0.97)
+//   row quantiser                0.94 below 2^21, 0.98 at 2^23 to 2^24, 1.02 above 2^25 (up to 1.11 with few GEMM tiles)
+//   GELU quantiser               0.96 below 2^22, 0.99 at 2^23 to 2^24, 1.00 above
+//   dequantisation               0.98 below 2^22, 0.99 up to 2^24, 1.03 above 2^24.5
+//   quantiser from row maxima    0.96 below 2^21, 0.99 at 2^23, 1.00 at 2^24, 1.09 above
+//   gated quantiser              0.96 below 2^21, 0.98 up to 2^22, 1.01 at 2^23, 1.03 to 1.1 above
+//   streaming layer-norm rows    0.98 at 1536 columns, 0.99 to 1.00 from 2048 on; other residual rows 1.01 to 1.07 (1024 columns)
+//   residual over planes         1.11 in the mean, up to 1.27
+//   streaming wan_qkv            1.00; behind itself 0.95 to 0.98
+//   QKV split                    1.01, up to 1.06; behind itself up to 1.3 (64-wide heads, 3000 tokens)
+//   first kernel of the pack     1.01 below 2^25, 1.06 above
 extern int g_dependent_launch;
-constexpr long long kDependentLaunchMaxRows = 16384;
-inline bool dependent_launch_for(long long rows) {
-  return g_dependent_launch == 2 || (g_dependent_launch == 1 && rows <= kDependentLaunchMaxRows);
+constexpr long long kDependentRows = 2048, kDependentRowsLong = 16384;
+inline bool dependent_launch_for(long long rows, bool many = false) {
+  return g_dependent_launch == 2 || (g_dependent_launch == 1 && rows <= (many ? kDependentRowsLong : kDependentRows));
 }
 
 // A GEMM of up to so many rows fetches its first weights ahead of its dependency wait, a larger one behind it: there the early

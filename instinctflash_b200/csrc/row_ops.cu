@@ -1393,11 +1393,12 @@ static void launch_row_quant(RowQuantArgs a, bool fast, cudaStream_t s) {
   }
   const RowGeom g = pick_geom(a.K);
   a.iters = g.iters;
+  const bool dep = dependent_launch_for(a.M, a.phase == 0 && (int64_t)a.M * a.K <= 1 << 24);  // see launch.cuh
   dispatch_geom(g, [&](auto tpr, auto it) {
     constexpr int TPR = decltype(tpr)::value, IT = decltype(it)::value;
     const int grid = (a.M + kRowThreads / TPR - 1) / (kRowThreads / TPR);
-    if (plain) launch_dep(row_quant_kernel<XT, TPR, IT, true, true>, dim3(grid), dim3(kRowThreads), 0, s, 1, dependent_launch_for(a.M), a);
-    else launch_dep(row_quant_kernel<XT, TPR, IT, false, true>, dim3(grid), dim3(kRowThreads), 0, s, 1, dependent_launch_for(a.M), a);
+    if (plain) launch_dep(row_quant_kernel<XT, TPR, IT, true, true>, dim3(grid), dim3(kRowThreads), 0, s, 1, dep, a);
+    else launch_dep(row_quant_kernel<XT, TPR, IT, false, true>, dim3(grid), dim3(kRowThreads), 0, s, 1, dep, a);
   });
 }
 template <typename XT>
@@ -1432,7 +1433,8 @@ static void launch_gated(GatedArgs a, bool fast, cudaStream_t s) {
   dispatch_geom(g, [&](auto tpr, auto it) {
     constexpr int TPR = decltype(tpr)::value, IT = decltype(it)::value;
     const int grid = (a.M + kRowThreads / TPR - 1) / (kRowThreads / TPR);
-    launch_dep(gated_act_quant_kernel<XT, TPR, IT, true>, dim3(grid), dim3(kRowThreads), 0, s, 1, dependent_launch_for(a.M), a);
+    launch_dep(gated_act_quant_kernel<XT, TPR, IT, true>, dim3(grid), dim3(kRowThreads), 0, s, 1,
+               dependent_launch_for(a.M, (int64_t)a.M * a.F <= 1 << 22), a);  // see launch.cuh
   });
 }
 template <typename RT>
@@ -1609,7 +1611,7 @@ extern "C" int iflb200_quant_from_amax(const float* h, int64_t ld_h, int M, int 
   uint8_t* codes = reinterpret_cast<uint8_t*>(q);
   auto launch = [&](auto kernel, int columns) {
     launch_dep(kernel, dim3((unsigned)((F + columns - 1) / columns), (unsigned)M), dim3(kRowThreads), 0, s, 1,
-               dependent_launch_for(M), h, ld_h, M, F, amax, amax_zero, codes, ld_q, qs, early_trigger_for(s));
+               dependent_launch_for(M, fast && (int64_t)M * F <= 1 << 23), h, ld_h, M, F, amax, amax_zero, codes, ld_q, qs, early_trigger_for(s));
   };
   // Pieces of 4096 columns where there is work for every SM, of 1024 while six of them a SM hold all, of 2048 between
   // (a piece of 1024 columns is one load a thread): us for pieces of 1024 / 2048 / 4096 columns -- 50 x 4096 1.30 / 1.30 /
@@ -1678,9 +1680,10 @@ extern "C" int iflb200_dequant_rows(const void* x, int x_dtype, int64_t ld_x, in
     b.row = row ? row + m0 : nullptr;
     const dim3 grid(chunks, rows);
     if (fast) {
-      if (x_dtype == IFLB200_BF16) launch_dep(dequant_rows_kernel<__nv_bfloat16, true>, dim3(grid), dim3(256), 0, s, 1, dependent_launch_for(b.M), b);
-      else if (x_dtype == IFLB200_F16) launch_dep(dequant_rows_kernel<__half, true>, dim3(grid), dim3(256), 0, s, 1, dependent_launch_for(b.M), b);
-      else launch_dep(dequant_rows_kernel<float, true>, dim3(grid), dim3(256), 0, s, 1, dependent_launch_for(b.M), b);
+      const bool dep = dependent_launch_for(b.M, (int64_t)M * D <= 1 << 24);  // see launch.cuh
+      if (x_dtype == IFLB200_BF16) launch_dep(dequant_rows_kernel<__nv_bfloat16, true>, dim3(grid), dim3(256), 0, s, 1, dep, b);
+      else if (x_dtype == IFLB200_F16) launch_dep(dequant_rows_kernel<__half, true>, dim3(grid), dim3(256), 0, s, 1, dep, b);
+      else launch_dep(dequant_rows_kernel<float, true>, dim3(grid), dim3(256), 0, s, 1, dep, b);
     } else {
       if (x_dtype == IFLB200_BF16) launch_dep(dequant_rows_kernel<__nv_bfloat16, false>, dim3(grid), dim3(256), 0, s, 1, dependent_launch_for(b.M), b);
       else if (x_dtype == IFLB200_F16) launch_dep(dequant_rows_kernel<__half, false>, dim3(grid), dim3(256), 0, s, 1, dependent_launch_for(b.M), b);

@@ -162,7 +162,7 @@ bool launch_stream(const StreamGeom& g, int sms, cudaStream_t s, const KArgs& a)
     if (cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimit) != cudaSuccess) return false;
     granted[dev] = true;
   }
-  launch_dep(kKernel, dim3(sms), dim3(g.tg * g.groups), g.smem, s, 1, dependent_launch_for(a.rows_of_call()), a, g.tg);
+  launch_dep(kKernel, dim3(sms), dim3(g.tg * g.groups), g.smem, s, 1, dependent_launch_for(a.rows_of_call(), a.many()), a, g.tg);
   return true;
 }
 

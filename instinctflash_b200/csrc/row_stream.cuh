@@ -14,6 +14,7 @@ struct GeluStreamArgs {
   int64_t ld_x;
   int M, K;
   int rows_of_call() const { return M; }
+  bool many() const { return (int64_t)M * K <= 1 << 24; }  // dependent launch beyond kDependentRows
   const float* row;
   const float* col;
   const float* bias;
@@ -30,6 +31,7 @@ struct ResNormStreamArgs {
   int64_t ld_res;
   int M, D;
   int rows_of_call() const { return M; }
+  bool many() const { return true; }
   const __nv_bfloat16* delta;  // or null
   int64_t ld_delta;
   const float *drow, *dcol, *bias, *gate;
@@ -51,6 +53,7 @@ struct WanStreamArgs {
   int64_t ld_raw;
   int rows, tokens, parts, D, HD;
   int rows_of_call() const { return rows; }
+  bool many() const { return true; }
   const float *row, *col, *bias, *q_norm, *k_norm;
   float eps;
   const float *inv_freq, *pos;
