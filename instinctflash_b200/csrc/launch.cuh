@@ -16,7 +16,7 @@ namespace iflb200 {
 // dependent launch over time without it, 2049 to 16384 rows, each operator directly behind a GEMM, by elements:
 //   GEMM forms                   0.94 to 1.00 (0.97 in the mean; 16384 x 5120 x 5120 0.97)
 //   row quantiser                0.94 below 2^21, 0.98 at 2^23 to 2^24, 1.02 above 2^25 (up to 1.11 with few GEMM tiles)
-//   GELU quantiser               0.96 below 2^22, 0.99 at 2^23 to 2^24, 1.00 above
+//   GELU quantiser               0.96 below 2^22, 0.99 at 2^23 to 2^25, 1.00 above
 //   dequantisation               0.98 below 2^22, 0.99 up to 2^24, 1.03 above 2^24.5
 //   quantiser from row maxima    0.96 below 2^21, 0.99 at 2^23, 1.00 at 2^24, 1.09 above
 //   gated quantiser              0.96 below 2^21, 0.98 up to 2^22, 1.01 at 2^23, 1.03 to 1.1 above

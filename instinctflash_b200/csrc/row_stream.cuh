@@ -14,7 +14,7 @@ struct GeluStreamArgs {
   int64_t ld_x;
   int M, K;
   int rows_of_call() const { return M; }
-  bool many() const { return (int64_t)M * K <= 1 << 24; }  // dependent launch beyond kDependentRows
+  bool many() const { return (int64_t)M * K <= 1 << 25; }  // dependent launch beyond kDependentRows
   const float* row;
   const float* col;
   const float* bias;
