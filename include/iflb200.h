@@ -521,7 +521,7 @@ IFLB200_API int iflb200_row_set_group(int threads_per_row);
 /* Programmatic dependent launch: a kernel launched this way may be scheduled while its
  * predecessor in the stream drains; it waits for the predecessor's results before its first
  * access to memory a kernel can write, except that a GEMM of at most 2048 rows loads its first weight boxes
- * meanwhile.  1 (default) = for calls over at most 2048 activation rows, and over at most 16384 for the GEMMs and for
+ * meanwhile, and the second kernel of a dynamic pack its elements, which the first has waited for.  1 (default) = for calls over at most 2048 activation rows, and over at most 16384 for the GEMMs and for
  * row kernels of few enough elements (where it was measured to shorten a chain of calls), 0 = never, 2 = always.  Results are identical in every
  * mode for calls that keep the rule on weights of iflb200_gemm_fp8_raw.  No reference counterpart. */
 IFLB200_API int iflb200_set_dependent_launch(int enable);

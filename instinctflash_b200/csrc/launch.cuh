@@ -1,7 +1,8 @@
 // Host-side kernel launch with the attributes this library uses: an optional cluster width and
 // programmatic dependent launch (the kernel may be scheduled while its predecessor in the
 // stream drains; every kernel launched through here calls grid_dependency_wait() before its
-// first access to memory another kernel may write).
+// first access to memory another kernel may write, but for two reads: the first weights of a GEMM of few rows
+// (kEarlyWeightsMaxRows), and the elements in the one-pass pack, whose own first kernel stands before it (pack_kernel)).
 #pragma once
 #include <cuda_runtime.h>
 

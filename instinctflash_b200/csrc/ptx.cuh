@@ -200,7 +200,7 @@ __device__ __forceinline__ void named_bar_arrive(uint32_t id, uint32_t threads) 
 // Programmatic dependent launch.  A kernel launched with the programmatic-stream-serialization
 // attribute may start while its predecessor in the stream still runs; grid_dependency_wait()
 // returns once the predecessor has completed and its writes are visible.  Every global access
-// that can alias anything another kernel writes must come after it.  Both are no-ops in a
+// that can alias anything another kernel writes must come after it (the two exceptions: launch.cuh).  Both are no-ops in a
 // kernel launched without the attribute.
 // ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

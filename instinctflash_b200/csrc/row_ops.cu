@@ -1165,7 +1165,7 @@ __device__ __forceinline__ uint32_t max_bf16_bits(const uint4& u, uint32_t best)
 __global__ void __launch_bounds__(kPackThreads)
 amax_partial_kernel(const uint16_t* __restrict__ x, int64_t n, uint32_t* __restrict__ partial) {
   row_dependency_wait();  // inputs may come from the kernel before this one in the stream
-  row_trigger();
+  row_trigger();  // never ahead of the wait: pack_kernel<true> reads x without one of its own
   __shared__ uint32_t red[kPackThreads / 32];
   uint32_t best = 0;
   const int64_t nvec = n / 8;
@@ -1199,9 +1199,16 @@ amax_partial_kernel(const uint16_t* __restrict__ x, int64_t n, uint32_t* __restr
 // n_partial > 0: dynamic scale from the partial maxima (every CTA recomputes it; CTA 0 writes
 // it out).  n_partial == 0: fixed scale read from scale_in.
 // ONE: dynamic, and the grid holds every element at four chunks a thread (n <= kPackOnePass).  The elements are then on their way before the
-// maxima are awaited: amax_partial_kernel, which is the kernel before, lets this one start only when everything before it has
-// completed, x included.  Both kernels for 2^19 elements 4.14 -> 3.48 us, 682 thousand 4.21 -> 3.57, 2^22 7.69 -> 6.80, 2^23 10.3 ->
+// maxima are awaited, the one read of this library's row kernels ahead of their wait: amax_partial_kernel, which is the kernel
+// before, lets this one start only behind its own wait, when whatever wrote x has completed and its writes have reached
+// L2.  So these loads are strong ones at GPU scope, which L2 serves: a line that L1 or the read-only path kept from an earlier
+// launch cannot be the answer.  Both kernels for 2^19 elements 4.14 -> 3.48 us, 682 thousand 4.21 -> 3.57, 2^22 7.69 -> 6.80, 2^23 10.3 ->
 // 8.7; with more than one pass the loads ahead were slower (2^24 15.8 -> 16.2, 2^26 71 -> 76).
+__device__ __forceinline__ uint4 ld_relaxed_gpu_v4(const uint4* p) {
+  uint4 v;
+  asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+  return v;
+}
 constexpr int64_t kPackOnePass = (int64_t)kPackMaxCtas * kPackThreads * 8 * 4;
 template <bool ONE>
 __global__ void __launch_bounds__(kPackThreads)
@@ -1216,7 +1223,10 @@ pack_kernel(const uint16_t* __restrict__ x, int64_t n, const uint32_t* __restric
   uint4 u[4];
   auto load = [&](int64_t i0) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) u[k] = i0 + k * stride < nvec ? xv[i0 + k * stride] : make_uint4(0u, 0u, 0u, 0u);
+    for (int k = 0; k < 4; ++k) {
+      u[k] = make_uint4(0u, 0u, 0u, 0u);
+      if (i0 + k * stride < nvec) u[k] = ONE ? ld_relaxed_gpu_v4(xv + i0 + k * stride) : xv[i0 + k * stride];
+    }
   };
   if (ONE) load(first);
   row_dependency_wait();  // inputs may come from the kernel before this one in the stream
