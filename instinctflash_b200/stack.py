@@ -94,6 +94,17 @@ def make_inputs(spec: StackSpec, device, *, cpu_seeded: bool = True):
     return x.to(torch.bfloat16).to(device), attn.to(device)
 
 
+def gated_epilogue_pays(rows: int, ffn: int) -> bool:
+    """Whether a decoder layer of ``rows`` tokens runs its gated activation in the gate_up GEMM's epilogue plus a short quantiser
+    launch, rather than as a GEMM and one row kernel, which serves few and short rows in one round of loads.
+
+    A layer unfused / fused, geometric mean over 1100 sizes (512 to 4096 hidden columns, which do not move the lines, 65 to 6000
+    rows) by hidden units and millions of rows x units: up to 2048 units 0.93 at 1, 0.94 at 3, 0.99 at 5, 1.00 at 7 to 10; to 5120
+    0.97 at 1, 0.99 at 2, 0.97 at 3, 0.99 at 4, 1.02 at 5, 1.03 beyond; above 0.97 at 0.9, 0.99 at 1.2, 1.01 at 1.4, 1.03 at 1.7 to 2,
+    1.00 to 1.02 at 2.5 to 3, 1.03 to 1.1 beyond.  Left of a line some sizes lose up to 4 %, right of it too."""
+    return rows > 64 and rows * ffn > (6_000_000 if ffn <= 2048 else 3_500_000 if ffn <= 5120 else 1_200_000)
+
+
 class LinearStack:
     """Static buffers + the per-layer call sequence.  ``ops`` supplies the operators."""
 
@@ -104,13 +115,9 @@ class LinearStack:
         split_rows = spec.M if split_rows is None else split_rows
         self.spec, self.weights, self.dev = spec, weights, torch.device(device)
         self.ops = ops or native_ops()
-        # fused forms exist only in this package's operator set; "auto" takes the gated epilogue where its extra short
-        # launch costs no more than the row kernel it replaces, which serves few and short rows in one round of loads.  A layer
-        # unfused / fused: 1024 x 4096 17.5 / 18.2 us at 80 rows, 0.95 to 0.98 of the time up to 330, 1.00 to 1.03 at 360 to 500;
-        # 768 x 2560 0.92 to 0.98 up to 560; 1280 x 5120 0.95 to 0.99 up to 280; 2048 x 8192 0.96 to 0.99 up to 148, 1.02 to 1.04 at
-        # 150 to 240; 2048 x 11008 0.99 at 80, 1.01 to 1.10 from 96 on; 2048 x 16384 0.97 at 80, 1.01 to 1.12 from 112 on
+        # fused forms exist only in this package's operator set
         if fused == "auto":
-            fused = spec.M > 64 and (spec.ffn > 8192 or spec.M * spec.ffn > 1_200_000)
+            fused = gated_epilogue_pays(spec.M, spec.ffn)
         self.fused = bool(fused) and hasattr(self.ops, "fp8_linear_gated")
         self.fuse_residual = fuse_residual and hasattr(self.ops, "fp8_linear_residual")
         # deep, narrow projections (down, o) whose tiles do not fill the GPU run split-K over independent CTAs, the

@@ -81,3 +81,11 @@ def test_tensor_parallel_driver_two_gloo_ranks_match_single_process():
     assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-2000:]
     line = [l for l in r.stdout.splitlines() if l.startswith("TP_RESULT")][-1]
     assert "'exact_ok': True" in line, line
+
+
+@pytest.mark.parametrize("rows,ffn,pays", [(64, 16384, False), (65, 16384, False), (73, 16384, False), (74, 16384, True), (234, 5120, False),
+                                           (683, 5120, False), (684, 5120, True), (233, 5128, False), (235, 5128, True),
+                                           (2929, 2048, False), (2930, 2048, True), (816, 16384, True), (50, 4096, False)])
+def test_lines_of_the_gated_epilogue(rows, ffn, pays):
+    from instinctflash_b200.stack import gated_epilogue_pays
+    assert gated_epilogue_pays(rows, ffn) == pays
