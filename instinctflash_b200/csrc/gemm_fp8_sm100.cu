@@ -84,7 +84,7 @@ __device__ uint32_t g_timeout_record[4];
 __device__ uint64_t g_gemm_wait_budget_ns = kWaitBudgetNs;
 #ifdef IFLB200_TRACE
 // Experiment builds only (-DIFLB200_TRACE; never in the product library): block 0 of each launch of
-// the single-CTA kernel stamps the SM clock at a few points; slot 0 holds globaltimer at entry.
+// the single-CTA and of the skinny kernel stamps the SM clock at a few points; slot 0 holds globaltimer at entry.
 __device__ unsigned long long g_gemm_trace[64][16];
 __device__ unsigned int g_gemm_trace_launch;
 __device__ unsigned int g_gemm_trace_cur;  // id of the launch whose block 0 is tracing (helpers without the id)
@@ -96,7 +96,22 @@ __device__ unsigned int g_gemm_trace_cur;  // id of the launch whose block 0 is 
   do {                                                                                \
     if (blockIdx.x == 0) g_gemm_trace[trace_id & 63][slot] = (unsigned long long)clock64(); \
   } while (0)
+#define GEMM_TRACE_BEGIN()                                                         \
+  __shared__ unsigned int trace_id_s;                                              \
+  if (threadIdx.x == 0) {                                                          \
+    trace_id_s = blockIdx.x == 0 ? atomicAdd(&g_gemm_trace_launch, 1u) : 0u;       \
+    if (blockIdx.x == 0) {                                                         \
+      g_gemm_trace_cur = trace_id_s;                                               \
+      g_gemm_trace[trace_id_s & 63][0] = globaltimer_ns();                         \
+      g_gemm_trace[trace_id_s & 63][1] = (unsigned long long)clock64();            \
+    }                                                                              \
+  }                                                                                \
+  __syncthreads();                                                                 \
+  const unsigned int trace_id = trace_id_s
 #else
+#define GEMM_TRACE_BEGIN() \
+  do {                     \
+  } while (0)
 #define GEMM_TRACE(slot) \
   do {                   \
   } while (0)
@@ -701,19 +716,7 @@ gemm_fp8_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-#ifdef IFLB200_TRACE
-  __shared__ unsigned int trace_id_s;
-  if (threadIdx.x == 0) {
-    trace_id_s = blockIdx.x == 0 ? atomicAdd(&g_gemm_trace_launch, 1u) : 0u;
-    if (blockIdx.x == 0) {
-      g_gemm_trace_cur = trace_id_s;
-      g_gemm_trace[trace_id_s & 63][0] = globaltimer_ns();
-      g_gemm_trace[trace_id_s & 63][1] = (unsigned long long)clock64();
-    }
-  }
-  __syncthreads();
-  const unsigned int trace_id = trace_id_s;
-#endif
+  GEMM_TRACE_BEGIN();
   // Split-K: the S CTAs of a cluster work on the same tile, CTA r on K steps [kb0, kb1); one
   // tile per CTA (the host launches tiles x S CTAs, at most one wave).
   // Partials: K split over independent CTAs (no cluster), each writing its fp32 partial sums.

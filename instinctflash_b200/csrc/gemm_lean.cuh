@@ -54,6 +54,7 @@ gemm_fp8_tc5_lean_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
+  GEMM_TRACE_BEGIN();
   // K split over independent CTAs: each writes its fp32 partial sums to a plane of its own
   const int parts = EPI == LEAN_PLANES ? p.partials : 1;
   const int part = EPI == LEAN_PLANES ? (int)blockIdx.x % parts : 0;
@@ -86,6 +87,7 @@ gemm_fp8_tc5_lean_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if (threadIdx.x == 0) GEMM_TRACE(2);  // barriers initialised, tensor memory allocated
 
   // As in the other forms: up to kEarlyWeightsMaxRows only the activations and the epilogue wait for the kernel before this one.
   const bool w_producer = warp == 0, a_producer = warp == 10;
@@ -111,7 +113,10 @@ gemm_fp8_tc5_lean_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
           // The activations' dependency wait stands directly before their first load: everything ahead of it has been
           // fetched and computed when the kernel before this one ends.  At the top of the loop it left 930 clocks from the end
           // of the wait to the load, most of it cold instructions; now 170 (18 expert layers 372 -> 351 us).
-          if (!waited) grid_dependency_wait();
+          if (!waited) {
+            grid_dependency_wait();
+            if (a_producer) GEMM_TRACE(3);  // the kernel before this one has completed
+          }
           waited = true;
           if (whole) {
             tma_load_3d(dst, w_producer ? &tm_w : &tm_a, bar, 0, row, kb);
@@ -119,6 +124,7 @@ gemm_fp8_tc5_lean_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
             for (int sl = 0; sl < have; ++sl)
               tma_load_2d(dst + sl * slab_bytes, w_producer ? &p.w_tail : &p.a_tail, bar, (kb + sl) * BK, row);
           }
+          if (a_producer && it == 0 && kb == kb0) GEMM_TRACE(14);  // first activations asked for
         }
         __syncwarp();
         ring.arm();
@@ -151,6 +157,7 @@ gemm_fp8_tc5_lean_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
         for (int kb = kb0; kb < kb1; kb += SL) {
           ok = wait_bounded_one(full_bar(stage), phase, abort_flag, (2u << 24) | (3u << 16) | (it & 0xFFFF));
           if (!ok) break;
+          if (it == 0 && kb == kb0) GEMM_TRACE(4);  // first operands have landed
           tc_fence_after();
           const uint32_t sa = base + stage * L::kStageBytes;
 #pragma unroll
@@ -171,6 +178,7 @@ gemm_fp8_tc5_lean_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
         }
         if (!ok) break;
         mma_commit(tfull_bar(acc));
+        if (it == 0) GEMM_TRACE(5);  // last MMA of the first tile issued
       }
     }
     __syncwarp();
@@ -217,6 +225,7 @@ gemm_fp8_tc5_lean_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
       }
       ok = wait_bounded(tfull_bar(acc), acc_phase, abort_flag, (3u << 24) | (4u << 16) | (it & 0xFFFF));
       if (!ok) break;
+      if (warp == 2 && lane == 0 && it == 0) GEMM_TRACE(6);  // first accumulator complete
       tc_fence_after();
       uint32_t r[kBlocks][16];  // r[b][4j + 2h + e]: row 16 b + 8 h + r4, column 8 j + 2 c4 + e
       const uint32_t t_acc = tmem_base + ((uint32_t)(quad * 32) << 16) + acc * BN + c0;
@@ -270,12 +279,14 @@ gemm_fp8_tc5_lean_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_
         }
       }
     }
+    if (warp == 2 && lane == 0) GEMM_TRACE(7);  // last store issued
   }
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, kTmemCols);
+    if (lane == 0) GEMM_TRACE(9);  // all roles done
   }
 }
 
