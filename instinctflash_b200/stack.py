@@ -100,13 +100,13 @@ def gated_epilogue_pays(rows: int, ffn: int) -> bool:
 
     A layer unfused / fused, passes back to back until the clock has settled, geometric mean over 420 sizes (512 to 3072 hidden
     columns, which do not move the lines, 65 to 4000 rows) by hidden units and millions of rows x units: up to 2048 units 0.95 at
-    1, 0.97 at 2, 0.99 at 5, 0.99 at 6; to 5120 0.97 at 1, 0.99 at 1.6, 1.01 at 2 to 3, 1.02 beyond; above, where the row kernel of few
-    rows ends at a row an SM, 0.98 at 0.9, 1.00 at 1.2, 1.03 to 1.05 at 1.5 to 2, 1.02 to 1.1 beyond.  Either side of a line some
-    sizes lose 2 to 5 %; all together run 0.3 % longer than with the better form of each."""
+    1, 0.97 at 2, 0.99 at 5, 0.99 at 6; to 5120 0.97 at 1, 0.98 at 1.4, 1.00 at 1.6 (338 x 4608 1.03), 1.01 at 2 to 3, 1.02 beyond; above,
+    where the row kernel of few rows ends at a row an SM, 0.98 at 0.9, 1.00 at 1.2, 1.03 to 1.05 at 1.5 to 2, 1.02 to 1.1 beyond.
+    Either side of a line some sizes lose 2 to 5 %; all together run 0.3 % longer than with the better form of each."""
     if rows <= 64:
         return False
     if ffn <= 5120:
-        return rows * ffn > (6_000_000 if ffn <= 2048 else 1_600_000)
+        return rows * ffn > (6_000_000 if ffn <= 2048 else 1_400_000)
     return rows > 148 or rows * ffn > 1_200_000
 
 
