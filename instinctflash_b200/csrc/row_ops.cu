@@ -46,7 +46,9 @@ __device__ __forceinline__ void row_enter(int early) {
 
 // Holds a value in a register from here on: what a launch of a few microseconds computes from its arguments (whose first
 // reads miss the constant cache) is done when the kernel before it ends, and not between the wait and the first load
-// (18 expert layers 352 -> 344 us; 50 x 4096 gated 1.90 -> 1.74 behind one another, 350 sizes 0.97 of the time).
+// (18 expert layers 352 -> 344 us; 50 x 4096 gated on one buffer 1.90 -> 1.74 behind one another, 350 sizes 0.97 of the time).
+// Not in instantiations that have no registers to spare: float32 rows with scales (row_quant_kernel: 16 x 5120 2.68 -> 2.87 us with
+// them), eight planes with every operand (residual_norm_planes_kernel).
 template <typename T>
 __device__ __forceinline__ void keep(T*& p) {
   asm volatile("" : "+l"(p));
@@ -505,7 +507,7 @@ gated_act_quant_kernel(const GatedArgs a) {
 // The same for few rows (a skinny decoder layer: 50 x 4096): no bytes to speak of, a launch is round trips to L2 and the
 // instructions of one row, fetched cold.  So a row has a thread for every four columns (eight, sixteen beyond 4096, 8192), every
 // load -- gate, up, their column scales, the row scale -- is issued before the first use, and the code is one
-// activation's: 50 x 4096 2.45 -> 1.92 us behind one another, 18 expert layers 418 -> 403; over 50 sizes and both
+// activation's: 50 x 4096 2.48 -> 1.91 us behind one another, 18 expert layers 418 -> 403; over 50 sizes and both
 // activations 0.79 of the time.  Two or four CTAs a row as a cluster took 0.4 us longer than one.
 constexpr int kGatedFewThreads = 1024;
 
@@ -1420,9 +1422,9 @@ static void launch_gated(GatedArgs a, bool fast, cudaStream_t s) {
   }
   if constexpr (sizeof(XT) == 2) {
     // A CTA for every row at once: while each has an SM of its own, and up to three an SM for rows that are one or two quads a
-    // thread.  us behind one another, this form against groups of 256 threads: 50 x 4096 1.92 / 2.45, 148 x 512 1.38 / 1.84, 148 x
-    // 8192 2.74 / 3.87, 148 x 16384 4.21 / 5.94, 444 x 4096 3.78 / 3.83, 444 x 5120 4.18 / 4.61; beyond, 200 x 8192 4.51 / 4.29, 600 x
-    // 4096 5.29 / 4.86.
+    // thread.  us behind one another, this form against groups of 256 threads: 50 x 4096 1.91 / 2.48, 148 x 512 1.32 / 1.80, 148 x
+    // 8192 2.71 / 3.85, 148 x 16384 4.03 / 5.88, 444 x 4096 3.70 / 3.85, 444 x 5120 4.17 / 4.63; beyond, 200 x 8192 4.65 / 4.28, 149 x
+    // 6144 3.59 / 3.35, 445 x 4096 4.24 / 3.86, 600 x 4096 5.47 / 4.87 (up to 2048 columns it stays ahead: 600 x 512 1.54 / 2.19).
     const int sms = device_sm_count() > 0 ? device_sm_count() : 148, q = (a.F + 4 * kGatedFewThreads - 1) / (4 * kGatedFewThreads);
     if (g_row_tpr_override == 0 && (a.M <= sms || (a.F <= 5120 && a.M <= 3 * sms))) {
       auto few = [&](auto quads) {
@@ -1869,6 +1871,7 @@ extern "C" int iflb200_dynamic_pack_bf16_e4m3(const void* x, int64_t n, void* q,
   if (launch_pack_cluster(x, n, q, scale, s)) return (int)cudaGetLastError();
   uint32_t* partial = reinterpret_cast<uint32_t*>(workspace);
   launch_dep(amax_partial_kernel, dim3(grid), dim3(kPackThreads), 0, s, 1, dependent_launch_for(n >> 12), reinterpret_cast<const uint16_t*>(x), n, partial);
+  // (n >> 12: dependent up to 2^23 elements; above, the first kernel directly behind a GEMM took 1.01 to 1.08 times as long.)
   // The pass over the maxima is the kernel before at any size, and it is short beside a GEMM: its
   // successor starts early however large the tensor is (4680 x 3072 15.2 -> 14.9 us).
   launch_dep(n <= kPackOnePass ? pack_kernel<true> : pack_kernel<false>, dim3(grid), dim3(kPackThreads), 0, s, 1, dependent_launch_for(0),
